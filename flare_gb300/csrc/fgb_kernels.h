@@ -35,13 +35,14 @@ int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
                     double *d_dB2, double *d_force_dots, cudaStream_t st);
 
 // FP64 row energies E = K alpha and the local-variance finish
-// var = k_self - sum(part) (predict.cu).
+// var = k_self - scale sum(part) (predict.cu).
 int launch_row_energy(int Mr, int Ms, const double *Kmat, const double *alpha,
                       const int *perm, double *e_rows, double *e_atom,
                       cudaStream_t st);
 int launch_variance_final(int Mr, int ntiles, const double *part,
                           const int *perm, const double *norms, double sig2,
-                          double xi, double *var, cudaStream_t st);
+                          double xi, double *var, cudaStream_t st,
+                          double scale = 1.0);
 
 // FP64 triangular variance GEMM (Z = K L^T, row sums of Z^2 per 64-column
 // tile), ntiles = ceil(R / 64).

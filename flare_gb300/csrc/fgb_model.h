@@ -31,7 +31,9 @@ struct fgb_workspace {
   fgb::DevBuf kmat, wmat, erows, part;
   fgb::DevBuf b2f, yf;           // mixed path: FP32 normalised rows, D^ B
   fgb::DevBuf dB2, fdots, fdot, dots, kern;  // plain (stored-gradient) form
-  fgb::oz::Sliced ozA, ozK;      // tensor-core path: sliced rows per call
+  // tensor-core paths: sliced rows, kernel matrix and (FP64 path) adjoint
+  // weights of one row chunk
+  fgb::oz::Sliced ozA, ozK, ozW;
   fgb::DevBuf ozerr;
 };
 
@@ -78,6 +80,18 @@ struct fgb_model_s {
       ozL[fgb::oz::kF64Variants];
   bool ozS_ready[fgb::oz::kF64Variants] = {};
   bool ozL_ready[fgb::oz::kF64Variants] = {};
+  // FP64 path: 1/|s| of the sparse rows as an unevaluated sum of two FP64
+  // numbers (built with oz64S): a rounded norm would be the same error in
+  // every atom's kernel with that row, and those add up
+  fgb::DevBuf sinv;
+  // FP64 path: the raw sparse rows, the transposed unit rows (n_d x M_s) and the L_inv
+  // panels at kS64 slices, one set per B tile height (kTN64v), sliced the
+  // first time each runs; largest |alpha| per species (the adjoint weights'
+  // fixed scale); whether descriptors, alpha and L_inv are all finite
+  std::vector<std::unique_ptr<fgb::oz::Sliced>> oz64S[2], oz64ST[2], oz64L[2];
+  bool oz64S_ready[2] = {}, oz64ST_ready[2] = {}, oz64L_ready[2] = {};
+  std::vector<double> alpha_max;
+  bool finite = true;
   // slices of the kernel GEMM (9, 8 or 7) and of the variance GEMM (9, 8,
   // 7 or 6) with the largest energy (eV/atom) and local-variance
   // differences to 9 slices measured on the sparse set when they were
@@ -143,6 +157,15 @@ namespace fgb {
 int kernel_stage_fp64(fgb_model_s *m, int N, const std::vector<int> &counts,
                       bool want_grad, bool want_var, double *d_e_atom,
                       double *d_gB2, double *d_var, cudaStream_t st);
+// The FP64 stage of a power-1 or power-2 model with finite weights on the
+// tensor cores (ozaki.cu), else the FP64 SIMT kernels (predict.cu).
+// have_rowmax: ws.rowmax holds each row's largest |B2|; ws.ozerr is cleared
+// before and read after by the caller.
+bool fp64_stage_sliced(const fgb_model_s *m);
+int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
+                         bool want_grad, bool want_var, double *d_e_atom,
+                         double *d_gB2, double *d_var, cudaStream_t st,
+                         bool fixed, bool have_rowmax);
 // Bounded tensor-core waits report into ws.ozerr, which the caller clears
 // before and reads after; `fixed`: prepare nothing (operands must be ready).
 // `after_chunk(s, Mr, perm)` runs after each row chunk's kernel and

@@ -18,6 +18,14 @@ constexpr int kEpiWarps = 3; // epilogue warps per TMEM lane quarter (16 columns
 // accumulation in TMEM); the biggest group (a + b = 10) sums to at most
 // 11264 * K.  Longer K runs in segments summed in 64-bit integers.
 constexpr int kMaxK = 1472;
+// FP64 path: 10 slices (60 bits of each row's largest entry), so that what
+// is dropped lies below the FP64 rounding of the results even where errors
+// of the sparse rows add up over all atoms with large |alpha| (256 FCC
+// atoms, sum |alpha| 1e6: energy error 1.1e-7 eV at 9 slices).  The biggest
+// group then sums to at most 12288 * K.
+constexpr int kS64 = 10;
+constexpr int kMaxK64 = 1360;
+constexpr int kTN64v[2] = {48, 32};   // B tile heights of its products
 // FP32-level configuration (force GEMM of the mixed path): 4 slices, B tiles
 // of 128 rows; the biggest group (a + b = 5) sums to at most 6144 * K.
 constexpr int kSF32 = 4;
@@ -75,11 +83,11 @@ struct Sliced {
 int pad_to(int x, int m);
 // Size `out` for rows x K in S slices (no conversion).
 int prepare(int rows, int K, int TR, int S, Sliced &out);
-// Slice rows into S = kS (FP64-level), 8, 7 or 6 (the mixed path's kernel
+// Slice rows into S = kS64 (FP64 path), kS (FP64-level), 8, 7 or 6 (the mixed path's kernel
 // and variance GEMMs) or kSF32 (FP32-level) digits.
 int slice(const SliceSpec &sp, Sliced &out, cudaStream_t st, int S = kS);
 
-// Product of S-slice operands (S = 9, 8, 7 or 6; B.S == S, A.S >= S); the
+// Product of S-slice operands (S = 10, 9, 8, 7 or 6; B.S == S, A.S >= S); the
 // tile shape follows B.TR (one of kTNF64v).
 template <int S, class Epi>
 int gemm_s(const Sliced &A, const Sliced &B, bool tri, const Epi &epi,

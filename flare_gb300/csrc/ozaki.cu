@@ -94,7 +94,8 @@ constexpr int ring_depth(int S, int TN) {
 template <int S, int TN>
 using CfgS = typename std::conditional<
     S == kS, typename std::conditional<TN == 48, CfgF64, CfgF64n>::type,
-    Cfg<S, TN, ring_depth(S, TN), kMaxK, TN / 16>>::type;
+    Cfg<S, TN, ring_depth(S, TN), S == kS64 ? kMaxK64 : kMaxK,
+        TN / 16>>::type;
 static_assert(CfgS<8, 48>::EW == 3 && CfgS<8, 32>::EW == 2 &&
                   CfgS<8, 64>::EW == 4 && CfgS<7, 48>::WCOLS == 16 &&
                   CfgS<7, 32>::WCOLS == 16 && CfgS<7, 64>::WCOLS == 16,
@@ -883,6 +884,7 @@ static int slice_s(const SliceSpec &sp, Sliced &out, cudaStream_t st) {
 
 int slice(const SliceSpec &sp, Sliced &out, cudaStream_t st, int S) {
   if (S == kS) return slice_s<kS>(sp, out, st);
+  if (S == kS64) return slice_s<kS64>(sp, out, st);
   if (S == 8) return slice_s<8>(sp, out, st);
   if (S == 7) return slice_s<7>(sp, out, st);
   if (S == 6) return slice_s<6>(sp, out, st);
@@ -1155,6 +1157,146 @@ struct EpiKernel {
   }
 };
 
+// 1/|s| of each row as hi + lo (about 100 bits): the squared norm by exact
+// products and TwoSums, a warp per row, and one Newton step on 1/sqrt.
+__device__ __forceinline__ void dd_add(double &hi, double &lo, double b,
+                                       double b_lo) {
+  const double s = __dadd_rn(hi, b), bb = __dadd_rn(s, -hi);
+  const double e = __dadd_rn(__dadd_rn(hi, -__dadd_rn(s, -bb)),
+                             __dadd_rn(b, -bb));
+  const double l = __dadd_rn(e, __dadd_rn(lo, b_lo));
+  hi = __dadd_rn(s, l);
+  lo = __dadd_rn(l, -__dadd_rn(hi, -s));
+}
+__global__ void k_oz_row_inv(int M, int nd, const double *__restrict__ S,
+                             double2 *__restrict__ out) {
+  const int m = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (m >= M) return;
+  double hi = 0.0, lo = 0.0;
+  for (int k = lane; k < nd; k += 32) {
+    const double x = S[(long long)m * nd + k];
+    const double p = __dmul_rn(x, x);
+    dd_add(hi, lo, p, __fma_rn(x, x, -p));
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1)
+    dd_add(hi, lo, __shfl_xor_sync(0xffffffffu, hi, off),
+           __shfl_xor_sync(0xffffffffu, lo, off));
+  if (lane) return;
+  double y = 0.0, y_lo = 0.0;
+  if (hi > 0.0) {
+    y = 1.0 / sqrt(hi);
+    // r = 1 - (hi + lo) y^2, y y = q + qe exactly
+    const double q = __dmul_rn(y, y), qe = __fma_rn(y, y, -q);
+    double r = __fma_rn(-hi, q, 1.0);
+    r = __dadd_rn(r, -__fma_rn(hi, qe, __dmul_rn(lo, q)));
+    y_lo = 0.5 * y * r;
+  }
+  out[m] = make_double2(y, y_lo);
+}
+
+// Kernel GEMM epilogue of the FP64 path (power 1 or 2, finite weights): v =
+// d . s of the raw rows, c = v / (|d| |s|) with 1/|s| as hi + lo; the
+// partial sums of alpha c^xi, and c^xi and the adjoint weights alpha c
+// (power 1: alpha) each written straight as kS64 slices (A operands of the
+// variance and adjoint products) under fixed scales: |c| <= 1, so 2^1
+// and 2^eW > max|alpha| bound them.  The factors sigma^2 and xi sigma^2
+// are row constants that the final sums apply: an FP64 instruction of a
+// warp holds its SM quarter's pipe for 64 cycles, and these epilogues are
+// bound by that count (6 a value here).
+struct EpiKernel64 {
+  using Value = double;
+  static constexpr bool kFloat = false;
+  static constexpr int eK = 1;
+  __nv_bfloat16 *Ksl, *Wsl;   // either may be null
+  double *Kscale, *Wscale;    // row scales (all 2^eK, 2^eW)
+  int KPv, eW;
+  double *epart;              // M x nslots energy partials
+  int nslots;
+  const double *alpha;
+  const double2 *sinv;
+  const unsigned char *valid;
+  const int *perm;
+  const double *norms;
+  bool quad;                  // power 2 (else 1)
+  int N;
+  __device__ double chunk(int m, bool row_ok, int n0, const double (&v)[16],
+                          double acc) const {
+    const double nd = row_ok ? norms[perm[m]] : 0.0;
+    const bool dok = nd >= kEmptyThresh;
+    const double inv = dok ? 1.0 / nd : 0.0;
+    double k[16], w[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const int n = n0 + j;
+      k[j] = w[j] = 0.0;
+      if (dok && n < N && valid[n]) {
+        const double a = alpha[n];
+        const double2 si = sinv[n];
+        const double t = v[j] * inv, c = fma(t, si.y, t * si.x);
+        k[j] = quad ? c * c : c;
+        w[j] = quad ? c * a : a;
+        acc = fma(a, k[j], acc);
+      }
+    }
+    if (n0 < KPv) {
+      if (Ksl) store_k_slices<kS64>(k, eK, Ksl, m, n0, KPv);
+      if (Wsl) store_k_slices<kS64>(w, eW, Wsl, m, n0, KPv);
+    }
+    return acc;
+  }
+  __device__ void finish(int m, bool row_ok, int slot, double acc) const {
+    if (row_ok) epart[(long long)m * nslots + slot] = acc;
+    if (slot == 0) {
+      if (Ksl) Kscale[m] = ldexp(1.0, eK);
+      if (Wsl) Wscale[m] = ldexp(1.0, eW);
+    }
+  }
+};
+
+// Adjoint product of the FP64 path, G = scale (W S^) with scale = xi
+// sigma^2: dE/dB2 = (G - xi E d^) / |d| in atom order (E from e_atom,
+// complete before this launch).
+struct EpiGrad64 {
+  using Value = double;
+  static constexpr bool kFloat = false;
+  const int *perm;
+  const double *norms, *B2, *e_atom;
+  double xi, scale;
+  double *gB2;
+  int N;   // n_d
+  __device__ double chunk(int m, bool row_ok, int n0, const double (&v)[16],
+                          double acc) const {
+    if (!row_ok) return acc;
+    const int atom = perm[m];
+    const double nd = norms[atom];
+    const bool dok = nd >= kEmptyThresh;
+    const double inv = dok ? 1.0 / nd : 0.0;
+    const double sv = scale * inv, sb = -(xi * e_atom[atom] * inv) * inv;
+    const long long at = (long long)atom * N + n0;
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      if (n0 + j < N) gB2[at + j] = dok ? fma(v[j], sv, sb * B2[at + j]) : 0.0;
+    return acc;
+  }
+  __device__ void finish(int, bool, int, double) const {}
+};
+
+// out (cols x rows) = in^T, 32 x 32 tiles.
+__global__ void k_oz_transpose(int rows, int cols, const double *__restrict__ in,
+                               double *__restrict__ out) {
+  __shared__ double t[32][33];
+  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  for (int k = threadIdx.y; k < 32; k += blockDim.y)
+    if (r0 + k < rows && c0 + (int)threadIdx.x < cols)
+      t[k][threadIdx.x] = in[(long long)(r0 + k) * cols + c0 + threadIdx.x];
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += blockDim.y)
+    if (c0 + k < cols && r0 + (int)threadIdx.x < rows)
+      out[(long long)(c0 + k) * rows + r0 + threadIdx.x] = t[threadIdx.x][k];
+}
+
 // Variance GEMM epilogue: per-row sum of z^2 over this tile's columns.
 struct EpiZsq {
   using Value = double;
@@ -1174,15 +1316,16 @@ struct EpiZsq {
   }
 };
 
-// E_atom = sum of the row's energy partials (fixed order, row_slots_sum).
+// E_atom = scale x sum of the row's energy partials (fixed order,
+// row_slots_sum).
 __global__ void k_energy_final(int M, int ntiles, const double *__restrict__ part,
-                               const int *__restrict__ perm,
+                               const int *__restrict__ perm, double scale,
                                double *__restrict__ e_atom) {
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int m = (int)(gt / kRowLanes), q = (int)(gt % kRowLanes);
   if (m >= M) return;   // whole lane groups
   const double s = row_slots_sum(part, m, ntiles, q);
-  if (q == 0) e_atom[perm[m]] = s;
+  if (q == 0) e_atom[perm[m]] = s * scale;
 }
 
 }  // namespace
@@ -1228,6 +1371,65 @@ static int build_oz_L(fgb_model_s *m, int v, cudaStream_t st) {
       return rc;
   }
   m->ozL_ready[v] = true;
+  return FGB_OK;
+}
+
+// Operands of the FP64 path at kS64 slices for B tiles of kTN64v[v] rows,
+// per species: the sparse rows, their transpose or the L_inv panels.
+static int build_oz64(fgb_model_s *m, int v,
+                      std::vector<std::unique_ptr<oz::Sliced>> &out,
+                      const std::function<oz::SliceSpec(int, int &)> &spec,
+                      cudaStream_t st) {
+  out.clear();
+  int rc;
+  for (int s = 0; s < m->b2.n_species; s++) {
+    out.emplace_back(new oz::Sliced());
+    if (m->h_counts[s] == 0) continue;
+    rc = FGB_OK;
+    oz::SliceSpec sp = spec(s, rc);
+    sp.TR = oz::kTN64v[v];
+    if (rc || (rc = oz::slice(sp, *out[s], st, oz::kS64))) return rc;
+  }
+  return FGB_OK;
+}
+
+static int build_oz64_S(fgb_model_s *m, int v, cudaStream_t st) {
+  const int nd = m->b2.n_d;
+  int rc;
+  if ((rc = m->sinv.ensure(sizeof(double2) * (m->M + 1)))) return rc;
+  oz::k_oz_row_inv<<<ceil_div((long long)m->M * 32, 256), 256, 0, st>>>(
+      m->M, nd, m->Sraw.as<double>(), m->sinv.as<double2>());
+  FGB_LAUNCH_CHECK("k_oz_row_inv");
+  return build_oz64(m, v, m->oz64S[v], [&](int s, int &) {
+    return oz::SliceSpec{m->h_counts[s], nd, 0,
+                         m->Sraw.as<double>() + (size_t)m->h_offsets[s] * nd, nd,
+                         nullptr, nullptr};
+  }, st);
+}
+
+static int build_oz64_L(fgb_model_s *m, int v, cudaStream_t st) {
+  return build_oz64(m, v, m->oz64L[v], [&](int s, int &) {
+    return oz::SliceSpec{m->h_panel_rows[s], m->h_counts[s], 0,
+                         m->Lp.as<double>() + m->h_panel_off[s],
+                         m->h_counts[s], nullptr, nullptr};
+  }, st);
+}
+
+static int build_oz64_ST(fgb_model_s *m, int v, cudaStream_t st) {
+  const int nd = m->b2.n_d;
+  std::vector<DevBuf> T(m->b2.n_species);
+  const int rc = build_oz64(m, v, m->oz64ST[v], [&](int s, int &r) {
+    const int Ms = m->h_counts[s];
+    if (!(r = T[s].ensure(sizeof(double) * (size_t)Ms * nd)))
+      oz::k_oz_transpose<<<dim3(ceil_div(nd, 32), ceil_div(Ms, 32)),
+                           dim3(32, 8), 0, st>>>(
+          Ms, nd, m->S.as<double>() + (size_t)m->h_offsets[s] * nd,
+          T[s].as<double>());
+    return oz::SliceSpec{nd, Ms, 0, T[s].as<double>(), Ms, nullptr, nullptr};
+  }, st);
+  if (rc) return rc;
+  FGB_LAUNCH_CHECK("k_oz_transpose");
+  FGB_CUDA(cudaStreamSynchronize(st));   // T goes
   return FGB_OK;
 }
 
@@ -1298,7 +1500,7 @@ static int probe_sparse(fgb_model_s *m, int Sk, int Sv, std::vector<double> &E,
     if (rc) return rc;
     oz::k_energy_final<<<
         ceil_div((long long)Ms * kRowLanes, 128), 128, 0, st>>>(
-        Ms, slots, erows.as<double>(), ident.as<int>(),
+        Ms, slots, erows.as<double>(), ident.as<int>(), 1.0,
         eout.as<double>() + off);
     FGB_LAUNCH_CHECK("k_energy_final");
     if (Sv > 0) {
@@ -1516,7 +1718,7 @@ int kernel_stage_oz(fgb_model_s *m, int N, const std::vector<int> &counts,
         StageTimer _pt(kStRowEnergy, st);
         oz::k_energy_final<<<
             ceil_div((long long)Mr * kRowLanes, 128), 128, 0, st>>>(
-            Mr, m->ozS[vk][s]->RP / 16, m->ws.erows.as<double>(), perm,
+            Mr, m->ozS[vk][s]->RP / 16, m->ws.erows.as<double>(), perm, 1.0,
             d_e_atom);
         FGB_LAUNCH_CHECK("k_energy_final");
       }
@@ -1549,6 +1751,146 @@ int kernel_stage_oz(fgb_model_s *m, int N, const std::vector<int> &counts,
           return rc;
       }
       if (after_chunk && (rc = (*after_chunk)(s, Mr, perm))) return rc;
+    }
+  }
+  return FGB_OK;
+}
+
+// Power 1 or 2 and finite weights: k and the adjoint weights then stay below
+// fixed scales, and no infinity or NaN has to come through.  Other powers
+// (pow of a small or negative c) and non-finite weights keep the SIMT form.
+bool fp64_stage_sliced(const fgb_model_s *m) {
+  return (m->power == 2.0 || m->power == 1.0) && m->finite;
+}
+
+// Kernel, adjoint and variance products of the FP64 path as exact 10-slice
+// products (60 bits of each row's largest entry, integer sums, one
+// rounding): on this GPU an FP64 multiply-add pipe of 2 a clock an SM makes
+// one 64 x 64 x 144 SIMT tile 150 us, while the slice products run on the
+// tensor cores.
+int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
+                         bool want_grad, bool want_var, double *d_e_atom,
+                         double *d_gB2, double *d_var, cudaStream_t st,
+                         bool fixed, bool have_rowmax) {
+  int rc, dev = 0, sms = 0;
+  FGB_CUDA(cudaGetDevice(&dev));
+  FGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const B2Params &p = m->b2;
+  const int nd = p.n_d;
+  const double sig2 = m->sigma * m->sigma, xi = m->power;
+  constexpr int kRows = 32768;
+  // B tile height of a product of `rows` x `cols` (variant 0: 48 rows, 1:
+  // 32 rows): the fewer rounds of tiles over the SMs weighted by a tile's
+  // time.  A 48-row tile takes 1.25 times a 32-row tile (2 x 1,000 sparse,
+  // n_d 680, three products of both species: 500 atoms 417 against 335 us,
+  // 1,000 atoms 420 and 374, 1,500 atoms 426 and 480, 8,000 atoms 1,319 and
+  // 1,403).
+  const auto pick = [sms](int rows, int cols) {
+    const int mt = ceil_div(rows, oz::kTM);
+    return 4 * ceil_div((long long)mt * ceil_div(cols, oz::kTN64v[1]), sms) <
+                   5 * ceil_div((long long)mt * ceil_div(cols, oz::kTN64v[0]),
+                                sms)
+               ? 1 : 0;
+  };
+  const auto ready = [&](bool *flags, int v,
+                         int (*build)(fgb_model_s *, int, cudaStream_t)) -> int {
+    if (flags[v]) return FGB_OK;
+    if (fixed) {
+      set_error("FP64 kernel stage: operands not sliced before a fixed call");
+      return FGB_EINVAL;
+    }
+    const int r = build(m, v, st);
+    if (r == FGB_OK) flags[v] = true;
+    return r;
+  };
+  int base = 0;
+  for (int s = 0; s < p.n_species; s++) {
+    const int Ns = counts[s], Ms = m->h_counts[s];
+    const int *perm_s = m->ws.perm.as<int>() + base;
+    base += Ns;
+    if (Ns > 0 && Ms == 0 && want_var) {
+      // no sparse environments of this species: k = 0, var = k_self
+      if ((rc = launch_variance_final(Ns, 0, nullptr, perm_s,
+                                      m->ws.norms.as<double>(), sig2, xi,
+                                      d_var, st)))
+        return rc;
+    }
+    if (Ms == 0) continue;
+    const int R = m->h_panel_rows[s], off = m->h_offsets[s];
+    const double wmax = m->alpha_max[s];
+    const int eW = wmax > 0.0 ? std::ilogb(wmax) + 1 : 0;
+    for (int r0 = 0; r0 < Ns; r0 += kRows) {
+      const int Mr = std::min(kRows, Ns - r0);
+      const int *perm = perm_s + r0;
+      const int vk = pick(Mr, Ms), vv = pick(Mr, R), vg = pick(Mr, nd);
+      if ((rc = ready(m->oz64S_ready, vk, build_oz64_S)) ||
+          (want_var && (rc = ready(m->oz64L_ready, vv, build_oz64_L))) ||
+          (want_grad && (rc = ready(m->oz64ST_ready, vg, build_oz64_ST))))
+        return rc;
+      const oz::Sliced &Sk = *m->oz64S[vk][s];
+      const int kslots = Sk.RP / 16;
+      if ((rc = m->ws.erows.ensure(sizeof(double) * (size_t)Mr * kslots)) ||
+          (want_var &&
+           (rc = oz::prepare(Mr, Ms, oz::kTM, oz::kS64, m->ws.ozK))) ||
+          (want_grad &&
+           (rc = oz::prepare(Mr, Ms, oz::kTM, oz::kS64, m->ws.ozW))))
+        return rc;
+      {
+        StageTimer _pt(kStRowSlice, st, 2);
+        if ((rc = oz::slice({Mr, nd, oz::kTM, m->ws.B2.as<double>(), nd, perm,
+                             nullptr,
+                             have_rowmax ? m->ws.rowmax.as<double>() : nullptr},
+                            m->ws.ozA, st, oz::kS64)))
+          return rc;
+      }
+      {
+        StageTimer _pt(kStKernelGemm, st);
+        const oz::EpiKernel64 epi{
+            want_var ? m->ws.ozK.q.as<__nv_bfloat16>() : nullptr,
+            want_grad ? m->ws.ozW.q.as<__nv_bfloat16>() : nullptr,
+            want_var ? m->ws.ozK.scale.as<double>() : nullptr,
+            want_grad ? m->ws.ozW.scale.as<double>() : nullptr,
+            oz::pad_to(Ms, oz::kKC), eW, m->ws.erows.as<double>(), kslots,
+            m->alpha.as<double>() + off, m->sinv.as<double2>() + off,
+            m->svalid.as<unsigned char>() + off, perm,
+            m->ws.norms.as<double>(), xi == 2.0, Ms};
+        if ((rc = oz::gemm_s<oz::kS64>(m->ws.ozA, Sk, false, epi, m->ws.ozerr.as<int>(),
+                           st)))
+          return rc;
+      }
+      {
+        StageTimer _pt(kStRowEnergy, st);
+        oz::k_energy_final<<<
+            ceil_div((long long)Mr * kRowLanes, 128), 128, 0, st>>>(
+            Mr, kslots, m->ws.erows.as<double>(), perm, sig2, d_e_atom);
+        FGB_LAUNCH_CHECK("k_energy_final");
+      }
+      if (want_grad) {
+        StageTimer _pt(kStAdjointGemm, st);
+        const oz::EpiGrad64 epi{perm, m->ws.norms.as<double>(),
+                                m->ws.B2.as<double>(), d_e_atom, xi,
+                                xi * sig2, d_gB2, nd};
+        if ((rc = oz::gemm_s<oz::kS64>(m->ws.ozW, *m->oz64ST[vg][s], false, epi,
+                           m->ws.ozerr.as<int>(), st)))
+          return rc;
+      }
+      if (want_var) {
+        const oz::Sliced &L = *m->oz64L[vv][s];
+        const int vslots = L.RP / 16;
+        if ((rc = m->ws.part.ensure(sizeof(double) * (size_t)Mr * vslots)))
+          return rc;
+        {
+          StageTimer _pt(kStVarianceGemm, st);
+          const oz::EpiZsq epi{m->ws.part.as<double>(), vslots, R};
+          if ((rc = oz::gemm_s<oz::kS64>(m->ws.ozK, L, true, epi, m->ws.ozerr.as<int>(),
+                             st)))
+            return rc;
+        }
+        if ((rc = launch_variance_final(Mr, vslots, m->ws.part.as<double>(),
+                                        perm, m->ws.norms.as<double>(), sig2,
+                                        xi, d_var, st, sig2 * sig2)))
+          return rc;
+      }
     }
   }
   return FGB_OK;

@@ -150,7 +150,8 @@ k_variance_gemm(int M, int R, int Ms, const double *__restrict__ Kmat,
 __global__ void k_variance_final(int M, int ntiles, const double *__restrict__ part,
                                  const int *__restrict__ perm,
                                  const double *__restrict__ norms, double sig2,
-                                 double xi, double *__restrict__ var) {
+                                 double xi, double scale,
+                                 double *__restrict__ var) {
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int m = (int)(gt / kRowLanes), q = (int)(gt % kRowLanes);
   if (m >= M) return;   // whole lane groups
@@ -161,7 +162,7 @@ __global__ void k_variance_final(int M, int ntiles, const double *__restrict__ p
   // K_self = sig^2 (d.d/(|d||d|))^xi, zero for an empty environment.
   double kself = nd >= kEmptyThresh ? sig2 * powx((nd * nd) / (nd * nd), xi)
                                     : 0.0;
-  var[atom] = kself - s;
+  var[atom] = kself - s * scale;
 }
 
 __global__ void k_transpose_rm(int R, int C, const double *__restrict__ in,
@@ -302,11 +303,12 @@ int launch_row_energy(int Mr, int Ms, const double *Kmat, const double *alpha,
 
 int launch_variance_final(int Mr, int ntiles, const double *part,
                           const int *perm, const double *norms, double sig2,
-                          double xi, double *var, cudaStream_t st) {
+                          double xi, double *var, cudaStream_t st,
+                          double scale) {
   StageTimer _pt(kStVarianceFinal, st);
   k_variance_final<<<
       ceil_div((long long)Mr * kRowLanes, 128), 128, 0, st>>>(
-      Mr, ntiles, part, perm, norms, sig2, xi, var);
+      Mr, ntiles, part, perm, norms, sig2, xi, scale, var);
   FGB_LAUNCH_CHECK("k_variance_final");
   return FGB_OK;
 }
@@ -440,7 +442,7 @@ int kernel_stage_fp64(fgb_model_s *m, int N, const std::vector<int> &counts,
       k_variance_final<<<
           ceil_div((long long)Ns * kRowLanes, 128), 128, 0, st>>>(
           Ns, 0, nullptr, perm_s, m->ws.norms.as<double>(), sig2, m->power,
-          d_var);
+          1.0, d_var);
       FGB_LAUNCH_CHECK("k_variance_final");
     }
     for (int r0 = 0; r0 < Ns && Ms > 0; r0 += kRowChunk) {
@@ -501,7 +503,7 @@ int kernel_stage_fp64(fgb_model_s *m, int N, const std::vector<int> &counts,
           k_variance_final<<<
               ceil_div((long long)Mr * kRowLanes, 128), 128, 0, st>>>(
               Mr, ntiles, m->ws.part.as<double>(), perm,
-              m->ws.norms.as<double>(), sig2, m->power, d_var);
+              m->ws.norms.as<double>(), sig2, m->power, 1.0, d_var);
           FGB_LAUNCH_CHECK("k_variance_final");
         }
       }
@@ -593,12 +595,22 @@ extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
   for (bool &r : m->ozS_ready) r = false;
   for (bool &r : m->ozL_ready) r = false;
   for (bool &r : m->ozB_ready) r = false;
+  for (int v = 0; v < 2; v++)
+    m->oz64S_ready[v] = m->oz64ST_ready[v] = m->oz64L_ready[v] = false;
+  m->finite = true;
+  for (int t = 0; t < M; t++) m->finite &= std::isfinite(snorm[t]);
   if (!h_alpha || !h_L_inv) return FGB_OK;
   if ((rc = m->alpha.ensure(sizeof(double) * (M + 1)))) return rc;
   if (M > 0)
     FGB_CUDA(cudaMemcpy(m->alpha.p, h_alpha, sizeof(double) * M,
                         cudaMemcpyHostToDevice));
   m->h_alpha.assign(h_alpha, h_alpha + M);
+  m->alpha_max.assign(S, 0.0);
+  for (int s = 0; s < S; s++)
+    for (int t = m->h_offsets[s]; t < m->h_offsets[s + 1]; t++) {
+      m->finite &= std::isfinite(h_alpha[t]);
+      m->alpha_max[s] = std::max(m->alpha_max[s], std::fabs(h_alpha[t]));
+    }
   m->h_L_inv.assign(h_L_inv, h_L_inv + (size_t)M * M);
   // L_inv panels: species s uses rows [c_s, c_s + R_s) and columns
   // [c_s, c_s + M_s); R_s = M_s when everything below the diagonal block is
@@ -619,6 +631,7 @@ extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
       for (int c = 0; c < Ms; c++)
         panels.push_back(h_L_inv[(size_t)(cs + r) * M + cs + c]);
   }
+  for (double x : panels) m->finite &= std::isfinite(x);
   if ((rc = m->Lp.ensure(sizeof(double) * (panels.size() + 1)))) return rc;
   if (!panels.empty())
     FGB_CUDA(cudaMemcpy(m->Lp.p, panels.data(), sizeof(double) * panels.size(),
@@ -690,7 +703,8 @@ int predict_impl(fgb_model_s *m, int n_struc, const int *h_atom_offsets,
   // the bounded tensor-core waits report into ws.ozerr, read at the end (a
   // fixed call's caller clears and reads it)
   if ((rc = m->ws.ozerr.ensure(sizeof(int)))) return rc;
-  if (!fixed && mixed)
+  const bool sliced = mixed || fp64_stage_sliced(m);
+  if (!fixed && sliced)
     FGB_CUDA(cudaMemsetAsync(m->ws.ozerr.p, 0, sizeof(int), st));
   const bool want_e = want & FGB_WANT_ENERGY, want_f = want & FGB_WANT_FORCES,
              want_s = want & FGB_WANT_STRESS, want_v = want & FGB_WANT_LOCAL_VAR;
@@ -760,7 +774,7 @@ int predict_impl(fgb_model_s *m, int n_struc, const int *h_atom_offsets,
                                 adj32 ? nullptr : m->ws.A.as<double>(),
                                 m->ws.B2.as<double>(), m->ws.norms.as<double>(),
                                 st, mixed && !m->force_f64,
-                                mixed ? m->ws.rowmax.as<double>() : nullptr,
+                                sliced ? m->ws.rowmax.as<double>() : nullptr,
                                 adj32 ? m->ws.A.as<float>() : nullptr)))
       return rc;
   }
@@ -784,6 +798,13 @@ int predict_impl(fgb_model_s *m, int n_struc, const int *h_atom_offsets,
                                  m->ws.gB2.as<double>(),
                                  v_direct ? d_local_var : m->ws.var.as<double>(),
                                  st, fixed != nullptr)))
+      return rc;
+  } else if (sliced) {
+    if ((rc = kernel_stage_fp64_oz(m, counts, want_grad, want_v,
+                                   m->ws.e_atom.as<double>(),
+                                   m->ws.gB2.as<double>(),
+                                   v_direct ? d_local_var : m->ws.var.as<double>(),
+                                   st, fixed != nullptr, true)))
       return rc;
   } else {
     if ((rc = kernel_stage_fp64(m, N, counts, want_grad, want_v,
@@ -838,7 +859,7 @@ int predict_impl(fgb_model_s *m, int n_struc, const int *h_atom_offsets,
   int h[5] = {0, 0, 0, 0, 0};
   FGB_CUDA(cudaMemcpyAsync(h, m->nl.flag.p, sizeof(int) * 4,
                            cudaMemcpyDeviceToHost, st));
-  if (mixed)
+  if (sliced)
     FGB_CUDA(cudaMemcpyAsync(h + 4, m->ws.ozerr.p, sizeof(int),
                              cudaMemcpyDeviceToHost, st));
   FGB_CUDA(cudaStreamSynchronize(st));
