@@ -29,10 +29,12 @@ int launch_struct_reduce(int n_struc, const int *d_atom_off,
                          const double *d_virial, double *d_energy,
                          double *d_stress, cudaStream_t st);
 
-// Stored forward-mode gradients (the reference's algorithm).
+// Stored forward-mode gradients (the reference's algorithm); scratch: each
+// pair's centre atom (left for the caller) and the pairs' basis values.
 int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
                     const int *d_species, const double *d_A, const double *d_B2,
-                    double *d_dB2, double *d_force_dots, cudaStream_t st);
+                    double *d_dB2, double *d_force_dots, DevBuf &center,
+                    DevBuf &basis, cudaStream_t st);
 
 // FP64 row energies E = K alpha and the local-variance finish
 // var = k_self - scale sum(part) (predict.cu).

@@ -30,7 +30,7 @@ struct fgb_workspace {
   fgb::DevBuf gB2, pair_grad, forces, virial;
   fgb::DevBuf kmat, wmat, erows, part;
   fgb::DevBuf b2f, yf;           // mixed path: FP32 normalised rows, D^ B
-  fgb::DevBuf dB2, fdots, fdot, dots, kern;  // plain (stored-gradient) form
+  fgb::DevBuf basis, dB2, fdots, fdot, dots, kern;  // plain (stored-gradient) form
   // tensor-core paths: sliced rows, kernel matrix and (FP64 path) adjoint
   // weights of one row chunk
   fgb::oz::Sliced ozA, ozK, ozW;

@@ -3,6 +3,8 @@
 // and the FP64 QR solve.
 #include <cusolverDn.h>
 
+#include <type_traits>
+
 #include "fgb_dense.h"
 #include "fgb_internal.h"
 #include "fgb_kernels.h"
@@ -42,93 +44,154 @@ k_envs_envs(int M, int N, int K, const double *__restrict__ D1,
 
 
 // Stored forward-mode gradients (b2.cpp:181-242 with single-bond gradients
-// from :367-395): one CTA per atom, pairs in order.  For pair p (i -> j,
-// species s_j) the single-bond gradient is nonzero only in block s_j:
+// from :367-395).  For pair p (i -> j, species s_j) the single-bond gradient
+// is nonzero only in block s_j:
 // dA_p[c][n][lm] = dg_n (x_c/r) Y_lm + g_n dY_lm/dx_c, and
 // dB2_p[c][(n1,n2,l)] = sum_m A[n1][lm] dA_p[c][n2][lm] + dA_p[c][n1][lm] A[n2][lm].
-// Shared: A[nA] | B2[nd] | g,dg[nm] | Y[nh] | Yd[3nh] | dA[3 nm nh] | red[3*64]
-constexpr int kDT = 64;
+// Two kernels over the flat pair list, both bound by FP64 instructions (64
+// cycles each per warp on an SM quarter), so the pairs are spread over all
+// SMs.  One block per atom that walked its pairs in series, one thread
+// evaluating each pair's basis, took 913 us for 108 FCC atoms (3,456 pairs,
+// n_d 144) where these take 84 us (k_pair_basis 14, k_b2_dervs 70).
+constexpr int kBT = 32;   // pairs (threads) per block of k_pair_basis
 
-__global__ void __launch_bounds__(kDT)
-k_b2_dervs(B2Params p, int n_atoms, const long long *__restrict__ offsets,
-           const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
-           const int *__restrict__ species, const double *__restrict__ A_in,
-           const double *__restrict__ B2_in, double *__restrict__ dB2,
-           double *__restrict__ fdots) {
-  extern __shared__ double smem[];
-  const int i = blockIdx.x;
-  if (i >= n_atoms) return;
-  const int nA = p.n_A, nh = p.n_harm, nm = p.n_max, nr = p.n_rad,
-            L1 = p.l_max + 1, nd = p.n_d;
-  double *A = smem;
-  double *Bv = A + nA;
-  double *g = Bv + nd;
-  double *dg = g + nm;
-  double *Y = dg + nm;
-  double *Yd = Y + nh;
-  double *dA = Yd + 3 * nh;
-  double *red = dA + 3 * nm * nh;
-  const int t = threadIdx.x;
-  for (int e = t; e < nA; e += blockDim.x) A[e] = A_in[(long long)i * nA + e];
-  for (int q = t; q < nd; q += blockDim.x) Bv[q] = B2_in[(long long)i * nd + q];
-  const int si = species[i];
-  __syncthreads();
-  for (long long pp = offsets[i]; pp < offsets[i + 1]; pp++) {
-    const int j = nbr_j[pp];
-    const double4_16a r = rel[pp];
-    const int sj = species[j];
-    const double rc = p.cutoffs[si * kMaxSpecies + sj];
-    const bool keep = r.x <= rc;
-    if (t == 0 && keep) {
-      radial_eval<double>(p, r.x, rc, g, dg);
-      ylm_eval<double>(p.l_max, r.y, r.z, r.w, Y, Yd);
-    }
-    __syncthreads();
-    if (keep) {
-      const double ir = 1.0 / r.x;
-      const double e3[3] = {r.y * ir, r.z * ir, r.w * ir};
-      for (int e = t; e < 3 * nm * nh; e += blockDim.x) {
-        int c = e / (nm * nh), n = (e / nh) % nm, lm = e % nh;
-        dA[e] = dg[n] * e3[c] * Y[lm] + g[n] * Yd[3 * lm + c];
-      }
-    }
-    __syncthreads();
-    double fd[3] = {0.0, 0.0, 0.0};
-    for (int q = t; q < nd; q += blockDim.x) {
-      double v[3] = {0.0, 0.0, 0.0};
-      if (keep) {
-        int l = q % L1, pidx = q / L1, n1 = 0;
-        while (pidx >= nr - n1) { pidx -= nr - n1; n1++; }
-        int n2 = n1 + pidx;
-        int b1 = n1 / nm, b2 = n2 / nm;
-        const double *a1 = A + n1 * nh + l * l, *a2 = A + n2 * nh + l * l;
-        for (int c = 0; c < 3; c++) {
-          double acc = 0.0;
-          const double *d1 = dA + c * nm * nh + (n1 - b1 * nm) * nh + l * l;
-          const double *d2 = dA + c * nm * nh + (n2 - b2 * nm) * nh + l * l;
-          for (int m = 0; m < 2 * l + 1; m++) {
-            if (b2 == sj) acc += a1[m] * d2[m];
-            if (b1 == sj) acc += d1[m] * a2[m];
-          }
-          v[c] = acc;
-        }
-      }
-      for (int c = 0; c < 3; c++) {
-        dB2[(3 * pp + c) * nd + q] = v[c];
-        fd[c] += v[c] * Bv[q];
-      }
-    }
-    for (int c = 0; c < 3; c++) red[c * kDT + t] = fd[c];
-    __syncthreads();
-    for (int h = kDT / 2; h > 0; h >>= 1) {
-      if (t < h)
-        for (int c = 0; c < 3; c++) red[c * kDT + t] += red[c * kDT + t + h];
-      __syncthreads();
-    }
-    if (t == 0)
-      for (int c = 0; c < 3; c++) fdots[3 * pp + c] = red[c * kDT];
-    __syncthreads();
+// Basis values of every pair, value-major so that neighbouring pairs are
+// neighbouring addresses: rows g[nm] | dg[nm] | Y[nh] | dY/dx[nh] | dY/dy[nh]
+// | dY/dz[nh], each P long; zero for pairs beyond the species pair's cutoff.
+// LC > 0 fixes l_max (the recurrence stays in registers).
+template <int LC>
+__global__ void __launch_bounds__(kBT)
+k_pair_basis(B2Params p, long long P, const int *__restrict__ center,
+             const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
+             const int *__restrict__ species, double *__restrict__ basis) {
+  const long long pp = (long long)blockIdx.x * kBT + threadIdx.x;
+  if (pp >= P) return;
+  const double4_16a r = rel[pp];
+  const double rc =
+      p.cutoffs[species[center[pp]] * kMaxSpecies + species[nbr_j[pp]]];
+  const int nm = p.n_max, nh = p.n_harm;
+  double *o = basis + pp;
+  if (!(r.x <= rc)) {
+    for (int v = 0; v < 2 * nm + 4 * nh; v++) o[v * P] = 0.0;
+    return;
   }
+  double g[kMaxNmax], dg[kMaxNmax];
+  radial_eval<double>(p, r.x, rc, g, dg);
+  for (int n = 0; n < nm; n++) {
+    o[n * P] = g[n];
+    o[(nm + n) * P] = dg[n];
+  }
+  double *y = o + 2 * nm * P;
+  ylm_visit<double, LC, true>(
+      p.l_max, r.y, r.z, r.w,
+      [&](int idx, double v, double gx, double gy, double gz) {
+        y[idx * P] = v;
+        y[(nh + idx) * P] = gx;
+        y[(2 * nh + idx) * P] = gy;
+        y[(3 * nh + idx) * P] = gz;
+      });
+}
+
+// dB2 rows of PP consecutive pairs: dA in shared memory, then a thread per
+// descriptor q for all PP x 3 rows, and the rows' dots with B2 by a
+// fixed-order block sum.
+constexpr int kDT = 128;
+template <int PP>
+__global__ void __launch_bounds__(kDT)
+k_b2_dervs(B2Params p, long long P, const int *__restrict__ center,
+           const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
+           const int *__restrict__ species, const double *__restrict__ basis,
+           const double *__restrict__ A_in, const double *__restrict__ B2_in,
+           double *__restrict__ dB2, double *__restrict__ fdots) {
+  extern __shared__ double dA[];            // PP x 3 x nm x nh
+  __shared__ double red[3 * PP][kDT + 1];
+  const int nA = p.n_A, nh = p.n_harm, nm = p.n_max, nr = p.n_rad,
+            L1 = p.l_max + 1, nd = p.n_d, nmh = nm * nh;
+  const long long p0 = (long long)blockIdx.x * PP;
+  const int t = threadIdx.x;
+  int cen[PP], sj[PP];
+#pragma unroll
+  for (int k = 0; k < PP; k++) {
+    cen[k] = p0 + k < P ? center[p0 + k] : center[p0];
+    sj[k] = p0 + k < P ? species[nbr_j[p0 + k]] : -1;
+  }
+  for (int e = t; e < nmh; e += kDT) {
+    const int n = e / nh, lm = e - n * nh;
+    const double *bn = basis + n * P + p0;
+    const double *by = basis + (2 * nm + lm) * P + p0;
+#pragma unroll
+    for (int k = 0; k < PP; k++) {
+      if (p0 + k >= P) break;
+      const double4_16a r = rel[p0 + k];
+      const double ir = 1.0 / r.x;
+      const double g = bn[k], dgy = bn[nm * P + k] * ir * by[k];
+      double *d = dA + k * 3 * nmh + e;
+      d[0] = fma(dgy, r.y, g * by[nh * P + k]);
+      d[nmh] = fma(dgy, r.z, g * by[2 * nh * P + k]);
+      d[2 * nmh] = fma(dgy, r.w, g * by[3 * nh * P + k]);
+    }
+  }
+  __syncthreads();
+  double fd[3 * PP];
+#pragma unroll
+  for (int k = 0; k < 3 * PP; k++) fd[k] = 0.0;
+  for (int q = t; q < nd; q += kDT) {
+    const int l = q % L1;
+    int pidx = q / L1, n1 = 0;
+    while (pidx >= nr - n1) { pidx -= nr - n1; n1++; }
+    const int n2 = n1 + pidx, b1 = n1 / nm, b2 = n2 / nm;
+    const int o1 = n1 * nh + l * l, o2 = n2 * nh + l * l;
+    const int e1 = o1 - b1 * nmh, e2 = o2 - b2 * nmh;
+#pragma unroll
+    for (int k = 0; k < PP; k++) {
+      if (p0 + k >= P) break;
+      double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+      const double *A = A_in + (long long)cen[k] * nA;
+      const double *d = dA + k * 3 * nmh;
+      if (b2 == sj[k])
+        for (int m = 0; m < 2 * l + 1; m++) {
+          const double a = A[o1 + m];
+          v0 = fma(a, d[e2 + m], v0);
+          v1 = fma(a, d[nmh + e2 + m], v1);
+          v2 = fma(a, d[2 * nmh + e2 + m], v2);
+        }
+      if (b1 == sj[k])
+        for (int m = 0; m < 2 * l + 1; m++) {
+          const double a = A[o2 + m];
+          v0 = fma(a, d[e1 + m], v0);
+          v1 = fma(a, d[nmh + e1 + m], v1);
+          v2 = fma(a, d[2 * nmh + e1 + m], v2);
+        }
+      const double b = B2_in[(long long)cen[k] * nd + q];
+      double *out = dB2 + 3 * (p0 + k) * nd + q;
+      out[0] = v0;
+      out[nd] = v1;
+      out[2 * (long long)nd] = v2;
+      fd[3 * k] = fma(v0, b, fd[3 * k]);
+      fd[3 * k + 1] = fma(v1, b, fd[3 * k + 1]);
+      fd[3 * k + 2] = fma(v2, b, fd[3 * k + 2]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3 * PP; k++) red[k][t] = fd[k];
+  __syncthreads();
+  for (int k = t >> 5; k < 3 * PP; k += kDT / 32) {
+    double x = 0.0;
+    for (int q = t & 31; q < kDT; q += 32) x += red[k][q];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+      x += __shfl_down_sync(0xffffffffu, x, off);
+    if ((t & 31) == 0 && p0 + k / 3 < P) fdots[3 * p0 + k] = x;
+  }
+}
+
+// center[q] = a for the pairs q of atom a: a warp per atom.
+__global__ void k_pair_center(int N, const long long *__restrict__ off,
+                              int *__restrict__ center) {
+  const int a = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (a >= N) return;
+  for (long long q = off[a] + (threadIdx.x & 31); q < off[a + 1]; q += 32)
+    center[q] = a;
 }
 
 // Dots_s = B2[perm] S_s^T (raw descriptors), Ns x Ms.
@@ -187,7 +250,9 @@ k_force_kernel(int R, int Ms, int K, const double *__restrict__ dB2,
         double nij = ni * nj, nij3 = nij * nj * nj;
         double dv = dots[(long long)jl * Ms + n];
         double nd_ = dv / nij;
-        double dval = power * pow(nd_, power - 1.0);
+        double dval = power * (power == 2.0 ? nd_
+                                            : power == 1.0 ? 1.0
+                                                           : pow(nd_, power - 1.0));
         double f1 = acc[i][jj] / nij;
         double f2 = dv * fdots[gr] / nij3;
         v = sig2 * dval * (f1 - f2);
@@ -197,28 +262,97 @@ k_force_kernel(int R, int Ms, int K, const double *__restrict__ dB2,
   }
 }
 
-// Energy column: K[c_s + i][0] = sum_j sig2 (dot_ij / |s_i||d_j|)^power.
-__global__ void k_energy_col(int Ns, int Ms, const double *__restrict__ dots,
-                             const int *__restrict__ perm,
-                             const double *__restrict__ dnorm,
-                             const double *__restrict__ snorm, double sig2,
-                             double power, int c_s, long long ncol,
-                             double *__restrict__ kern) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= Ms) return;
-  double ni = snorm[i];
+// The energy and stress columns are sums over all atoms or pairs for every
+// sparse row: block (32 sparse rows x 8 groups) x chunk of atoms or pairs,
+// then k_col_final adds the chunks in order.  A thread per sparse row that
+// walked every pair alone took 1,751 us (108 FCC atoms, 3,456 pairs, 200
+// sparse rows) and every atom 406 us; the three kernels here take 12, 7 and
+// 9 us, the stress part at 1.4 TB/s of FK (16.6 MB, partly in L2).
+constexpr int kColRows = 32, kColGroups = 8;
+
+// part[ch][i] = sum over the chunk's atoms j of sig2 (dot_ij / |s_i||d_j|)^power
+__global__ void __launch_bounds__(kColRows * kColGroups)
+k_energy_part(int Ns, int Ms, int per, const double *__restrict__ dots,
+              const int *__restrict__ perm, const double *__restrict__ dnorm,
+              const double *__restrict__ snorm, double sig2, double power,
+              double *__restrict__ part, int ldp) {
+  __shared__ double red[kColGroups][kColRows + 1];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int i = blockIdx.x * kColRows + x, ch = blockIdx.y;
   double acc = 0.0;
-  if (ni >= kEmptyThresh)
-    for (int j = 0; j < Ns; j++) {
-      double nj = dnorm[perm[j]];
-      if (nj < kEmptyThresh) continue;
-      acc += sig2 * pow(dots[(long long)j * Ms + i] / (ni * nj), power);
+  if (i < Ms) {
+    const double ni = snorm[i];
+    const int j1 = min(Ns, (ch + 1) * per);
+    if (ni >= kEmptyThresh)
+      for (int j = ch * per + g; j < j1; j += kColGroups) {
+        const double nj = dnorm[perm[j]];
+        if (nj < kEmptyThresh) continue;
+        acc += sig2 * powx(dots[(long long)j * Ms + i] / (ni * nj), power);
+      }
+  }
+  red[g][x] = acc;
+  __syncthreads();
+  if (g == 0 && i < Ms) {
+    for (int q = 1; q < kColGroups; q++) acc += red[q][x];
+    part[(long long)ch * ldp + i] = acc;
+  }
+}
+
+// part[ch][k][i] = sum over the chunk's pairs of fk_a r_b (b >= a, flare order)
+__global__ void __launch_bounds__(kColRows * kColGroups)
+k_stress_part(int M, long long P, long long per,
+              const double4_16a *__restrict__ rel,
+              const double *__restrict__ FK, double *__restrict__ part) {
+  __shared__ double red[6][kColGroups][kColRows + 1];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int i = blockIdx.x * kColRows + x;
+  const long long ch = blockIdx.y;
+  double s[6] = {0, 0, 0, 0, 0, 0};
+  if (i < M) {
+    const long long p1 = min(P, (ch + 1) * per);
+    for (long long p = ch * per + g; p < p1; p += kColGroups) {
+      const double4_16a r = rel[p];
+      const double *f = FK + 3 * p * M + i;
+      const double f0 = f[0], f1 = f[M], f2 = f[2LL * M];
+      s[0] = fma(f0, r.y, s[0]);
+      s[1] = fma(f0, r.z, s[1]);
+      s[2] = fma(f0, r.w, s[2]);
+      s[3] = fma(f1, r.z, s[3]);
+      s[4] = fma(f1, r.w, s[4]);
+      s[5] = fma(f2, r.w, s[5]);
     }
-  kern[(long long)(c_s + i) * ncol] = acc;
+  }
+#pragma unroll
+  for (int k = 0; k < 6; k++) red[k][g][x] = s[k];
+  __syncthreads();
+  if (g < 6 && i < M) {
+    double t = 0.0;
+    for (int q = 0; q < kColGroups; q++) t += red[g][q][x];
+    part[(ch * 6 + g) * M + i] = t;
+  }
+}
+
+// Energy column (k = 0) and stress columns (k = 1..6, times -1/V) from the
+// chunks' partial sums: kern[i][col].
+__global__ void k_col_final(int M, int nce, int ncs,
+                            const double *__restrict__ epart,
+                            const double *__restrict__ spart, double vol_inv,
+                            int n_atoms, long long ncol,
+                            double *__restrict__ kern) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+  if (i >= M) return;
+  double s = 0.0;
+  if (k == 0) {
+    for (int c = 0; c < nce; c++) s += epart[(long long)c * M + i];
+    kern[(long long)i * ncol] = s;
+  } else {
+    for (int c = 0; c < ncs; c++) s += spart[((long long)c * 6 + k - 1) * M + i];
+    kern[(long long)i * ncol + 1 + 3LL * n_atoms + k - 1] = -s * vol_inv;
+  }
 }
 
 // Force columns by owner-computes: K[i][1+3a+c] = sum_{p in out(a)}
-// FK[3p+c][i] - FK[3 twin(p)+c][i].  Thread per (sparse i, atom a).
+[3p+c][i] - FK[3 twin(p)+c][i].  Thread per (sparse i, atom a).
 __global__ void k_force_cols(int M, int N, const long long *__restrict__ off,
                              const long long *__restrict__ twin,
                              const double *__restrict__ FK, long long ncol,
@@ -238,27 +372,6 @@ __global__ void k_force_cols(int M, int N, const long long *__restrict__ off,
   for (int c = 0; c < 3; c++) kern[(long long)i * ncol + 1 + 3 * a + c] = f[c];
 }
 
-// Stress columns: -(1/V) sum_p fk_a r_b for b >= a (flare order).
-__global__ void k_stress_cols(int M, long long P, const double4_16a *__restrict__ rel,
-                              const double *__restrict__ FK, double vol_inv,
-                              int n_atoms, long long ncol,
-                              double *__restrict__ kern) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M) return;
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (long long p = 0; p < P; p++) {
-    double4_16a r = rel[p];
-    double c3[3] = {r.y, r.z, r.w};
-    int k = 0;
-    for (int a = 0; a < 3; a++) {
-      double fk = FK[(3 * p + a) * M + i];
-      for (int b = a; b < 3; b++) s[k++] -= fk * c3[b] * vol_inv;
-    }
-  }
-  for (int k = 0; k < 6; k++)
-    kern[(long long)i * ncol + 1 + 3LL * n_atoms + k] = s[k];
-}
-
 // mean_efs[o] = sum_i kern[i][o] alpha[i]
 __global__ void k_kern_t_alpha(int M, long long ncol, const double *__restrict__ kern,
                                const double *__restrict__ alpha,
@@ -268,13 +381,6 @@ __global__ void k_kern_t_alpha(int M, long long ncol, const double *__restrict__
   double acc = 0.0;
   for (int i = 0; i < M; i++) acc += kern[(long long)i * ncol + o] * alpha[i];
   out[o] = acc;
-}
-
-__global__ void k_pair_center(int N, const long long *__restrict__ off,
-                              int *__restrict__ center) {
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= N) return;
-  for (long long p = off[a]; p < off[a + 1]; p++) center[p] = a;
 }
 
 __global__ void k_rownorms(int M, int nd, const double *__restrict__ S,
@@ -290,22 +396,60 @@ __global__ void k_rownorms(int M, int nd, const double *__restrict__ S,
 
 int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
                     const int *d_species, const double *d_A, const double *d_B2,
-                    double *d_dB2, double *d_force_dots, cudaStream_t st) {
+                    double *d_dB2, double *d_force_dots, DevBuf &center,
+                    DevBuf &basis, cudaStream_t st) {
   const int N = nl->n_atoms;
-  if (N == 0 || nl->n_pairs == 0) return FGB_OK;
-  size_t sm = sizeof(double) * ((size_t)p.n_A + p.n_d + 2 * p.n_max +
-                                4 * p.n_harm + 3 * (size_t)p.n_max * p.n_harm +
-                                3 * kDT);
+  const long long P = nl->n_pairs;
+  if (N == 0 || P == 0) return FGB_OK;
+  // dA of a pair: PP = 8 pairs a block while they leave room for two blocks
+  // on an SM, else 2
+  const size_t per = sizeof(double) * 3 * (size_t)p.n_max * p.n_harm;
+  const int PP = 8 * per <= 96 * 1024 ? 8 : 2;
+  // descriptors whose A, B2 row and pair basis together exceed 200 KB are
+  // refused by every stored-gradient entry point
+  const size_t sm = sizeof(double) * ((size_t)p.n_A + p.n_d + 2 * p.n_max +
+                                      4 * p.n_harm + 192) + per;
   if (sm > 200 * 1024) {
     set_error("stored-gradient form needs %zu bytes of shared memory", sm);
     return FGB_EINVAL;
   }
-  FGB_CUDA(cudaFuncSetAttribute(k_b2_dervs,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sm));
-  k_b2_dervs<<<N, kDT, sm, st>>>(p, N, nl->offsets.as<long long>(),
-                                 nl->nbr_j.as<int>(), nl->nbr_rel.as<double4_16a>(),
-                                 d_species, d_A, d_B2, d_dB2, d_force_dots);
+  int rc;
+  if ((rc = center.ensure(sizeof(int) * P)) ||
+      (rc = basis.ensure(sizeof(double) * (2 * p.n_max + 4 * p.n_harm) *
+                         (size_t)P)))
+    return rc;
+  k_pair_center<<<ceil_div((long long)N * 32, 128), 128, 0, st>>>(
+      N, nl->offsets.as<long long>(), center.as<int>());
+  FGB_LAUNCH_CHECK("k_pair_center");
+  const auto eval = [&](auto lc) {
+    k_pair_basis<decltype(lc)::value><<<ceil_div(P, kBT), kBT, 0, st>>>(
+        p, P, center.as<int>(), nl->nbr_j.as<int>(),
+        nl->nbr_rel.as<double4_16a>(), d_species, basis.as<double>());
+  };
+  switch (p.l_max) {
+    case 1: eval(std::integral_constant<int, 1>()); break;
+    case 2: eval(std::integral_constant<int, 2>()); break;
+    case 3: eval(std::integral_constant<int, 3>()); break;
+    case 4: eval(std::integral_constant<int, 4>()); break;
+    case 5: eval(std::integral_constant<int, 5>()); break;
+    case 6: eval(std::integral_constant<int, 6>()); break;
+    default: eval(std::integral_constant<int, 0>()); break;
+  }
+  FGB_LAUNCH_CHECK("k_pair_basis");
+  const auto dervs = [&](auto pp) -> int {
+    constexpr int K = decltype(pp)::value;
+    FGB_CUDA(cudaFuncSetAttribute(k_b2_dervs<K>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(K * per)));
+    k_b2_dervs<K><<<ceil_div(P, K), kDT, K * per, st>>>(
+        p, P, center.as<int>(), nl->nbr_j.as<int>(),
+        nl->nbr_rel.as<double4_16a>(), d_species, basis.as<double>(), d_A,
+        d_B2, d_dB2, d_force_dots);
+    return FGB_OK;
+  };
+  if ((rc = PP == 8 ? dervs(std::integral_constant<int, 8>())
+                    : dervs(std::integral_constant<int, 2>())))
+    return rc;
   FGB_LAUNCH_CHECK("k_b2_dervs");
   return FGB_OK;
 }
@@ -342,7 +486,7 @@ extern "C" int fgb_b2_forward_dervs(fgb_b2_t b2, fgb_nlist_t nl,
     return FGB_EINVAL;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  DevBuf A, flag;
+  DevBuf A, flag, center, basis;
   int rc;
   if ((rc = check_species(d_species, nl->n_atoms, b2->p.n_species, flag, st)))
     return rc;
@@ -352,7 +496,7 @@ extern "C" int fgb_b2_forward_dervs(fgb_b2_t b2, fgb_nlist_t nl,
                               d_norms, st)))
     return rc;
   rc = launch_b2_dervs(b2->p, nl, d_species, A.as<double>(), d_B2, d_dB2,
-                       d_force_dots, st);
+                       d_force_dots, center, basis, st);
   if (!rc) FGB_CUDA(cudaStreamSynchronize(st));
   return rc;
 }
@@ -397,7 +541,7 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
     return rc;
   if ((rc = launch_b2_dervs(p, nl, d_species, ws.A.as<double>(),
                             ws.B2.as<double>(), ws.dB2.as<double>(),
-                            ws.fdots.as<double>(), st)))
+                            ws.fdots.as<double>(), ws.pos, ws.basis, st)))
     return rc;
   // host-side species permutation and pair rows (plain path: sync is fine)
   std::vector<int> hs(N);
@@ -420,9 +564,6 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
                            cudaMemcpyHostToDevice, st));
   FGB_CUDA(cudaMemcpyAsync(ws.flags.p, inv.data(), sizeof(int) * N,
                            cudaMemcpyHostToDevice, st));
-  k_pair_center<<<ceil_div(N, 128), 128, 0, st>>>(
-      N, nl->offsets.as<long long>(), ws.pos.as<int>());
-  FGB_LAUNCH_CHECK("k_pair_center");
   DevBuf snorm, dots, rowsd;
   if ((rc = snorm.ensure(sizeof(double) * (M + 1)))) return rc;
   k_rownorms<<<ceil_div(M, 128), 128, 0, st>>>(M, nd, d_sparse,
@@ -430,6 +571,15 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
   FGB_LAUNCH_CHECK("k_rownorms");
   FGB_CUDA(cudaMemsetAsync(ws.kern.p, 0, sizeof(double) * 3 * P * M, st));
   const double sig2 = sigma * sigma;
+  // chunks of the energy (atoms) and stress (pairs) sums: at least 32 atoms
+  // or pairs each and at most 128 chunks
+  const int eper = std::max(32, ceil_div(N, 128)), nce = ceil_div(N, eper);
+  const long long sper = std::max(32LL, (P + 127) / 128);
+  const int ncs = ceil_div(P, sper);
+  if ((rc = ws.part.ensure(sizeof(double) * (size_t)M * (nce + 6 * ncs))))
+    return rc;
+  double *spart = ws.part.as<double>() + (size_t)M * nce;
+  FGB_CUDA(cudaMemsetAsync(ws.part.p, 0, sizeof(double) * (size_t)M * nce, st));
   for (int s = 0; s < S; s++) {
     const int Ns = sbase[s + 1] - sbase[s], Ms = h_counts[s];
     if (Ns == 0 || Ms == 0) continue;
@@ -440,10 +590,12 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
     k_dots<<<g1, GT, 0, st>>>(Ns, Ms, nd, ws.B2.as<double>(), perm_s, Ss,
                               dots.as<double>());
     FGB_LAUNCH_CHECK("k_dots");
-    k_energy_col<<<ceil_div(Ms, 128), 128, 0, st>>>(
-        Ns, Ms, dots.as<double>(), perm_s, ws.norms.as<double>(),
-        snorm.as<double>() + off[s], sig2, power, off[s], ncol, d_kern);
-    FGB_LAUNCH_CHECK("k_energy_col");
+    k_energy_part<<<dim3(ceil_div(Ms, kColRows), ceil_div(Ns, eper)),
+                    kColRows * kColGroups, 0, st>>>(
+        Ns, Ms, eper, dots.as<double>(), perm_s, ws.norms.as<double>(),
+        snorm.as<double>() + off[s], sig2, power,
+        ws.part.as<double>() + off[s], M);
+    FGB_LAUNCH_CHECK("k_energy_part");
     rows.clear();
     for (int k = sbase[s]; k < sbase[s + 1]; k++) {
       int a = perm[k];
@@ -468,10 +620,16 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
       M, N, nl->offsets.as<long long>(), nl->nbr_twin.as<long long>(),
       ws.kern.as<double>(), ncol, d_kern);
   FGB_LAUNCH_CHECK("k_force_cols");
-  k_stress_cols<<<ceil_div(M, 64), 64, 0, st>>>(
-      M, P, nl->nbr_rel.as<double4_16a>(), ws.kern.as<double>(),
-      1.0 / nl->h_volume[0], N, ncol, d_kern);
-  FGB_LAUNCH_CHECK("k_stress_cols");
+  if (P > 0) {
+    k_stress_part<<<dim3(ceil_div(M, kColRows), ncs), kColRows * kColGroups, 0,
+                    st>>>(M, P, sper, nl->nbr_rel.as<double4_16a>(),
+                          ws.kern.as<double>(), spart);
+    FGB_LAUNCH_CHECK("k_stress_part");
+  }
+  k_col_final<<<dim3(ceil_div(M, 128), 7), 128, 0, st>>>(
+      M, nce, ncs, ws.part.as<double>(), spart, 1.0 / nl->h_volume[0], N, ncol,
+      d_kern);
+  FGB_LAUNCH_CHECK("k_col_final");
   return FGB_OK;
 }
 }  // namespace fgb

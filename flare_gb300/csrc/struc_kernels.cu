@@ -505,7 +505,7 @@ int self_kernel_impl(const B2Params &p, double sigma, double power,
                                 ws.B2.as<double>(), ws.norms.as<double>(), st)) ||
         (rc = launch_b2_dervs(p, nl, d_species, ws.A.as<double>(),
                               ws.B2.as<double>(), ws.dB2.as<double>(),
-                              ws.fdots.as<double>(), st)))
+                              ws.fdots.as<double>(), ws.pos, ws.basis, st)))
       return rc;
   }
   // species-sorted rows (host: this is a synchronous FP64 path)
@@ -661,7 +661,7 @@ int ss_prepare(const B2Params &p, fgb_nlist_s *nl, const int *d_species,
                                ws.B2.as<double>(), ws.norms.as<double>(), st)) ||
        (rc = launch_b2_dervs(p, nl, d_species, ws.A.as<double>(),
                              ws.B2.as<double>(), ws.dB2.as<double>(),
-                             ws.fdots.as<double>(), st))))
+                             ws.fdots.as<double>(), ws.pos, ws.basis, st))))
     return rc;
   std::vector<int> hs(N), perm, inv(N), srow, item_row;
   std::vector<double> hn(N);
