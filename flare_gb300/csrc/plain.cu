@@ -352,7 +352,7 @@ __global__ void k_col_final(int M, int nce, int ncs,
 }
 
 // Force columns by owner-computes: K[i][1+3a+c] = sum_{p in out(a)}
-[3p+c][i] - FK[3 twin(p)+c][i].  Thread per (sparse i, atom a).
+// FK[3p+c][i] - FK[3 twin(p)+c][i].  Thread per (sparse i, atom a).
 __global__ void k_force_cols(int M, int N, const long long *__restrict__ off,
                              const long long *__restrict__ twin,
                              const double *__restrict__ FK, long long ncol,
