@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstring>
+#include <mutex>
 
 #include "fgb_internal.h"
 
@@ -31,12 +32,48 @@ static std::atomic<unsigned long long> g_allocations{0};
 
 unsigned long long devbuf_allocations() { return g_allocations.load(); }
 
+// The current device's scratch pool (nullptr: none can be had), made at
+// first use and kept until the process ends.
+static cudaMemPool_t scratch_pool() {
+  constexpr int kMaxDev = 64;
+  static std::mutex mu;
+  static cudaMemPool_t pools[kMaxDev] = {};
+  static bool tried[kMaxDev] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  std::lock_guard<std::mutex> g(mu);
+  if (!tried[dev]) {
+    tried[dev] = true;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    unsigned long long keep = kScratchKeep;
+    if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold,
+                                &keep) != cudaSuccess) {
+      cudaGetLastError();
+      pools[dev] = nullptr;
+    }
+  }
+  return pools[dev];
+}
+
 int DevBuf::ensure(size_t n) {
   if (n == 0) n = 16;
   if (n <= bytes) return FGB_OK;
-  g_allocations.fetch_add(1);
+  if (!scratch) g_allocations.fetch_add(1);
   release();
-  cudaError_t e = cudaMalloc(&p, n);
+  cudaError_t e = cudaErrorUnknown;
+  if (cudaMemPool_t pool = scratch ? scratch_pool() : nullptr) {
+    e = cudaMallocFromPoolAsync(&p, n, pool, st);
+    pooled = e == cudaSuccess;
+    if (!pooled) cudaGetLastError();
+  }
+  if (!pooled) e = cudaMalloc(&p, n);
   if (e != cudaSuccess) {
     p = nullptr;
     cudaGetLastError();
@@ -49,9 +86,13 @@ int DevBuf::ensure(size_t n) {
 }
 
 void DevBuf::release() {
-  if (p) cudaFree(p);
+  if (p) {
+    if (pooled) cudaFreeAsync(p, st);
+    else cudaFree(p);
+  }
   p = nullptr;
   bytes = 0;
+  pooled = false;
 }
 
 // Canonical 3x3 algebra (same formulas and order as the oracle's):

@@ -439,8 +439,7 @@ int cholqr_solve(int M, long long n, double *At, const double *b,
       return rc;
     if (pass < 2) {
       // Q becomes the next pass's input (A0's storage is free after pass 0)
-      std::swap(Q.p, A0.p);
-      std::swap(Q.bytes, A0.bytes);
+      Q.swap(A0);
       Qprev = A0.as<double>();
       if ((rc = Qt.ensure(sizeof(double) * nM))) return rc;
       if ((rc = transpose(ni, M, Qprev, M, Qt.as<double>(), n, st))) return rc;

@@ -2,18 +2,41 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>
+#include <utility>
 #include <vector>
 
 #include "fgb_common.cuh"
 
 namespace fgb {
 
-// Grow-only device buffer.
+// Grow-only device buffer.  on(st) makes it one call's scratch, allocated and
+// freed in the order of stream st from a pool that keeps at most
+// kScratchKeep bytes per device between calls (a cudaMalloc and cudaFree
+// pair takes about 115 us and waits for the device; a solve made 151).
+constexpr size_t kScratchKeep = 256u << 20;
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
+  bool scratch = false, pooled = false;
+  cudaStream_t st = nullptr;
+  DevBuf &on(cudaStream_t stream) {
+    scratch = true;
+    st = stream;
+    return *this;
+  }
   int ensure(size_t n);            // FGB_OK or FGB_ENOMEM
   void release();
+  DevBuf() = default;
+  explicit DevBuf(cudaStream_t stream) { on(stream); }
+  DevBuf(const DevBuf &) = delete;
+  DevBuf &operator=(const DevBuf &) = delete;
+  void swap(DevBuf &o) {
+    std::swap(p, o.p);
+    std::swap(bytes, o.bytes);
+    std::swap(scratch, o.scratch);
+    std::swap(pooled, o.pooled);
+    std::swap(st, o.st);
+  }
   ~DevBuf() { release(); }
   template <typename T> T *as() const { return static_cast<T *>(p); }
 };

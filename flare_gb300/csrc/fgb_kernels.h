@@ -36,21 +36,15 @@ int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
                     double *d_dB2, double *d_force_dots, DevBuf &center,
                     DevBuf &basis, cudaStream_t st);
 
-// FP64 row energies E = K alpha and the local-variance finish
-// var = k_self - scale sum(part) (predict.cu).
-int launch_row_energy(int Mr, int Ms, const double *Kmat, const double *alpha,
-                      const int *perm, double *e_rows, double *e_atom,
-                      cudaStream_t st);
+// The local-variance finish var = k_self - scale sum(part) (predict.cu).
 int launch_variance_final(int Mr, int ntiles, const double *part,
                           const int *perm, const double *norms, double sig2,
                           double xi, double *var, cudaStream_t st,
                           double scale = 1.0);
 
-// FP64 triangular variance GEMM (Z = K L^T, row sums of Z^2 per 64-column
-// tile), ntiles = ceil(R / 64).
-int launch_variance_fp64(int Mr, int R, int Ms, const double *Kmat,
-                         const double *Lp, double *part, int ntiles,
-                         cudaStream_t st);
+// mean_efs = K^T alpha from K^T (ncol x M).
+int launch_kt_alpha(int M, long long ncol, const double *KT,
+                    const double *alpha, double *out, cudaStream_t st);
 
 // Validate coded species in [0, n_species); returns FGB_EINVAL otherwise.
 int check_species(const int *d_species, int n, int n_species, DevBuf &flag,

@@ -7,17 +7,22 @@
 #include "fgb_internal.h"
 #include "fgb_ozaki.h"
 
-// Page-locked species counts (and range flag) of the species permutation
-// and the event recorded after their copy, so that the host can wait for
-// them after queueing more work.
+// Host copy of the species counts (and range flag; the stored-gradient form
+// also keeps its pair counts per species here): page-locked with the event
+// recorded after the copy, so that the host can wait for it after queueing
+// more work, or (pageable) plain host memory for a workspace of one call,
+// into which a copy returns complete.
 struct fgb_pinned_counts {
+  static constexpr int kInts = 2 * (fgb::kMaxSpecies + 1);
   int *h = nullptr;
   cudaEvent_t ev = nullptr;
+  bool pageable = false;
+  int host[kInts] = {};
   fgb_pinned_counts() = default;
   fgb_pinned_counts(const fgb_pinned_counts &) = delete;
   fgb_pinned_counts &operator=(const fgb_pinned_counts &) = delete;
   ~fgb_pinned_counts() {
-    if (h) cudaFreeHost(h);
+    if (h && !pageable) cudaFreeHost(h);
     if (ev) cudaEventDestroy(ev);
   }
 };
@@ -30,11 +35,25 @@ struct fgb_workspace {
   fgb::DevBuf gB2, pair_grad, forces, virial;
   fgb::DevBuf kmat, wmat, erows, part;
   fgb::DevBuf b2f, yf;           // mixed path: FP32 normalised rows, D^ B
-  fgb::DevBuf basis, dB2, fdots, fdot, dots, kern;  // plain (stored-gradient) form
+  // stored-gradient form: pairs grouped by species, basis values, gradients,
+  // cosines, force kernel, sparse norms and slices
+  fgb::DevBuf start, rows, basis, dB2, fdots, dots, kern, snorm;
+  fgb::oz::Sliced ozSp[2];
   // tensor-core paths: sliced rows, kernel matrix and (FP64 path) adjoint
   // weights of one row chunk
   fgb::oz::Sliced ozA, ozK, ozW;
   fgb::DevBuf ozerr;
+  // one call's scratch on stream st (DevBuf::on) for the buffers of the
+  // stored-gradient form
+  void scratch_on(cudaStream_t st) {
+    counts.pageable = true;
+    for (fgb::DevBuf *b :
+         {&perm, &flags, &pos, &scal, &flag, &A, &B2, &norms, &rowmax, &part,
+          &start, &rows, &basis, &dB2, &fdots, &dots, &kern, &snorm, &ozerr,
+          &ozA.q, &ozA.scale, &ozK.q, &ozK.scale, &ozSp[0].q, &ozSp[0].scale,
+          &ozSp[1].q, &ozSp[1].scale})
+      b->on(st);
+  }
 };
 
 struct fgb_io {
@@ -61,6 +80,9 @@ struct fgb_model_s {
   bool has_rinv = false;
   fgb::DevBuf Lfull;    // L_inv (M x M, lower triangular) for DTC, on demand
   bool lfull_ready = false;
+  // R_inv^T and L_inv as kS64-slice B operands (SOR and DTC variances)
+  fgb::oz::Sliced oz64R[2], oz64Lfull[2];
+  bool oz64R_ready[2] = {}, oz64Lfull_ready[2] = {};
   fgb::DevBuf Bmap;     // mixed path: per species n_d x n_d FP32 folded matrix
   fgb::DevBuf Bfold;    // the folded matrices in FP64 (power 2), per species
   // the folded matrices in FP32-level slices (tensor-core force GEMM), one
@@ -208,8 +230,9 @@ int species_permutation_finish(int S, fgb_workspace &ws,
                                std::vector<int> &counts);
 int envs_struc_impl(const B2Params &p, double sigma, double power,
                     const int *h_counts, const double *d_sparse,
-                    fgb_nlist_s *nl, const int *d_species, double *d_kern,
+                    fgb_nlist_s *nl, const int *d_species, double *d_kt,
                     fgb_workspace &ws, cudaStream_t st);
+int sliced_finish(fgb_workspace &ws, cudaStream_t st, const char *what);
 // self_kernel_struc of one structure into d_out[1 + 3N + 6] (struc_kernels.cu); with
 // have_dervs the workspace already holds B2, norms and dB2 of this list.
 int self_kernel_impl(const B2Params &p, double sigma, double power,

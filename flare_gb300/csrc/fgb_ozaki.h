@@ -77,7 +77,9 @@ struct SliceSpec {
 struct Sliced {
   int rows = 0, K = 0, TR = 0, RP = 0, KP = 0, S = 0;
   DevBuf q;       // bf16 slices, tiled canonical layout
-  DevBuf scale;   // per-row 2^e
+  DevBuf scale;   // per-row 2^e (kS64 slices: +inf for a non-finite row)
+  Sliced() = default;
+  explicit Sliced(cudaStream_t st) : q(st), scale(st) {}   // one call's scratch
 };
 
 int pad_to(int x, int m);
@@ -105,6 +107,40 @@ int gemm_store(const Sliced &A, const Sliced &B, double *C, long long ldc,
 // written), the same exact integer sums and one rounding of the product.
 int gemm_axpby(const Sliced &A, const Sliced &B, double *C, long long ldc,
                double a, double b, int *err, cudaStream_t st);
+// B tile height (index into kTN64v) of a kS64-slice product.
+int tile64(int rows, int cols);
+// Products of kS64-slice operands (B tiles of kTN64v rows) for the
+// stored-gradient form and the solved variances:
+//   C[m][n] = (A B^T) inv_a[m] / |s_n|, 1/|s| as hi + lo, zero where either
+//     row is empty (norm below 1e-8); a_norm gathered through perm
+int gemm_cosine(const Sliced &A, const Sliced &B, const int *perm,
+                const double *a_norm, const double2 *s_inv,
+                const double *s_norm, double *C, int *err, cudaStream_t st);
+//   FK[gr][c_s + n] = sig2 power c^(power-1) (f / (|s_n||d|) - c fdots / |d|^2)
+//     for gr = rows[m], f = (A B^T)[m][n], d the centre of pair gr / 3 and c
+//     its row (crow[centre] - crow0) of the cosines: normalized_dot_product.cpp:185-198
+struct ForceKernelArgs {
+  const int *rows, *center, *crow;
+  const double *cosine, *d_norm, *fdots, *s_norm;
+  const double2 *s_inv;
+  double sig2, power;
+  double *FK;
+  int c_s, M, crow0;
+};
+int gemm_force_kernel(const Sliced &A, const Sliced &B,
+                      const ForceKernelArgs &fk, int *err, cudaStream_t st);
+//   K[m][n] = sig2 ((A B^T) / (na_m nb_n))^power (normalized_dot_product.cpp:
+//     28-89), zero for empty rows
+int gemm_envs(const Sliced &A, const Sliced &B, const double *na,
+              const double *nb, double sig2, double power, double *K, int *err,
+              cudaStream_t st);
+//   part[m][slot]: sums of (A B^T)^2 over 16 columns each (B.RP / 16 slots);
+//     tri: B lower triangular
+int gemm_rowsq(const Sliced &A, const Sliced &B, bool tri, double *part,
+               int *err, cudaStream_t st);
+// |row| and 1/|row| as hi + lo of M rows of n_d values (norms may be null).
+int row_inverse(int M, int nd, const double *rows, double *norms, double2 *inv,
+                cudaStream_t st);
 // Y (A.rows x B.rows, leading dimension ldy) = A B^T rounded to FP32, from
 // kSF32-slice operands (A tiles of kTM rows, B tiles of 128 or 64 rows;
 // `ew` epilogue warps per lane quarter, 2 or 4 for 128-row tiles).  A may

@@ -340,7 +340,11 @@ k_oz_rowscale(int R, int K, int RP, const double *__restrict__ src,
     mb = max(mb, (unsigned long long)__shfl_xor_sync(0xffffffffu, (long long)mb, off));
   const double mx = __longlong_as_double((long long)mb) * inv;
   const int e = mx > 0.0 ? ilogb(mx) + 1 : 0;
-  if (lane == 0) scale[m] = ldexp(1.0, e);
+  // an infinity or NaN in the row: scale +inf, which makes every product of
+  // the row NaN at kS64 slices
+  const bool bad = mb >= 0x7FF0000000000000ULL;
+  if (lane == 0)
+    scale[m] = bad ? __longlong_as_double(0x7FF0000000000000LL) : ldexp(1.0, e);
 }
 
 // The same scales from each source row's largest |value| given up front
@@ -376,20 +380,22 @@ __global__ void k_oz_scale_from_max(int R, int RP, const int *__restrict__ perm,
 // columns, 32 consecutive k at a time, lane = row + 8 x (k group of 8), so
 // that the 16-byte row pieces a store instruction writes for one slice are
 // two contiguous 256-byte blocks (one 16-k chunk each) rather than 32
-// scattered pieces; the parts let a few thousand rows fill the GPU.
+// scattered pieces; the parts let a few thousand rows fill the GPU.  A warp
+// spends about 3 us in each 32-column step (1,500 instructions a lane), so
+// few rows take parts of one step (slice_s).
 constexpr int kSlicePart = 128;
 static_assert(kSlicePart % 32 == 0, "a part is whole 32-column steps");
 template <int S>
 __global__ void __launch_bounds__(256)
-k_oz_slice8(int R, int K, int RP, int KP, int TR, int nparts,
+k_oz_slice8(int R, int K, int RP, int KP, int TR, int npart, int ncols,
             const double *__restrict__ src, long long ld, int vec,
             const int *__restrict__ perm, const double *__restrict__ rownorm,
             double thresh, __nv_bfloat16 *__restrict__ out,
             const double *__restrict__ scale) {
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  const int part = (int)(gw % nparts);
-  const int m0 = (int)(gw / nparts) * 8;
+  const int part = (int)(gw % npart);
+  const int m0 = (int)(gw / npart) * 8;
   if (m0 >= RP) return;
   const int r = lane & 7, g = lane >> 3;
   const int m = m0 + r;
@@ -407,8 +413,8 @@ k_oz_slice8(int R, int K, int RP, int KP, int TR, int nparts,
   const double *sr = src + row * ld;
   const int e = pow2_exp(scale[m]);
   const size_t stride = (size_t)TR * kKC;
-  const int kend = min(KP, (part + 1) * kSlicePart);
-  for (int k0 = part * kSlicePart + g * 8; k0 < kend; k0 += 32) {
+  const int kend = min(KP, (part + 1) * ncols);
+  for (int k0 = part * ncols + g * 8; k0 < kend; k0 += 32) {
     // the lane's 8 values: four 16-byte loads when the source rows allow
     // (vec: 16-byte aligned rows) and all 8 lie inside the row
     double v[8];
@@ -732,7 +738,8 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
       for (int ch = 0; ch < NCH; ch++) {
 #pragma unroll
         for (int j = 0; j < 16; j++) {
-          const int e = er + pow2_exp(Bscale[n0 + c_lo + ch * 16 + j]);
+          const int eb = pow2_exp(Bscale[n0 + c_lo + ch * 16 + j]);
+          const int e = er + eb;
           if constexpr (Epi::kFloat) {
             static_assert(!C::HAS_LO, "FP32 results take at most 5 slices");
             v[ch][j] = scaled_float(hi[ch][j], e - 6 * C::TSPLIT);
@@ -740,6 +747,8 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
             double x = exact_scaled(hi[ch][j], e - 6 * C::TSPLIT);
             if constexpr (C::HAS_LO)
               x += exact_scaled(lo[ch][j], e - 6 * (S + 1));
+            if constexpr (S == kS64)   // a row scale of +inf
+              if (max(er, eb) > 1023) x = __longlong_as_double(0x7FF8000000000000LL);
             v[ch][j] = x;
           }
         }
@@ -869,13 +878,19 @@ static int slice_s(const SliceSpec &sp, Sliced &out, cudaStream_t st) {
         kEmptyThresh, out.scale.as<double>());
     FGB_LAUNCH_CHECK("k_oz_rowscale");
   }
-  const int nparts = ceil_div(out.KP, kSlicePart);
+  // parts of one step while the 128-column parts would leave SMs with fewer
+  // than 8 warps (256 rows x 144: 10.8 against 5.1 us; 16,000 x 680
+  // the same 54 us in either form)
+  const int ncols =
+      (long long)(out.RP / 8) * ceil_div(out.KP, kSlicePart) < 8 * 152
+          ? 32 : kSlicePart;
+  const int nparts = ceil_div(out.KP, ncols);
   const long long threads = (long long)(out.RP / 8) * nparts * 32;  // RP % 8 == 0
   // 16-byte loads need every row start 16-byte aligned
   const int vec = (sp.ld % 2 == 0 &&
                    reinterpret_cast<uintptr_t>(sp.src) % 16 == 0) ? 1 : 0;
   k_oz_slice8<S><<<ceil_div(threads, 256), 256, 0, st>>>(
-      sp.rows, sp.K, out.RP, out.KP, sp.TR, nparts, sp.src, sp.ld, vec,
+      sp.rows, sp.K, out.RP, out.KP, sp.TR, nparts, ncols, sp.src, sp.ld, vec,
       sp.perm, sp.rownorm, kEmptyThresh, out.q.as<__nv_bfloat16>(),
       out.scale.as<double>());
   FGB_LAUNCH_CHECK("k_oz_slice8");
@@ -1169,6 +1184,7 @@ __device__ __forceinline__ void dd_add(double &hi, double &lo, double b,
   lo = __dadd_rn(l, -__dadd_rn(hi, -s));
 }
 __global__ void k_oz_row_inv(int M, int nd, const double *__restrict__ S,
+                             double *__restrict__ norms,
                              double2 *__restrict__ out) {
   const int m = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -1194,6 +1210,7 @@ __global__ void k_oz_row_inv(int M, int nd, const double *__restrict__ S,
     y_lo = 0.5 * y * r;
   }
   out[m] = make_double2(y, y_lo);
+  if (norms) norms[m] = sqrt(hi);
 }
 
 // Kernel GEMM epilogue of the FP64 path (power 1 or 2, finite weights): v =
@@ -1316,6 +1333,100 @@ struct EpiZsq {
   }
 };
 
+// C = cosines of the rows (gemm_cosine).
+struct EpiCosine {
+  using Value = double;
+  static constexpr bool kFloat = false;
+  const int *perm;
+  const double *a_norm, *s_norm;
+  const double2 *s_inv;
+  double *C;
+  int N;
+  __device__ double chunk(int m, bool row_ok, int n0, const double (&v)[16],
+                          double acc) const {
+    if (!row_ok) return acc;
+    const double nd = a_norm[perm[m]];
+    const double inv = nd >= kEmptyThresh ? 1.0 / nd : 0.0;
+    double *c = C + (long long)m * N + n0;
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      if (n0 + j < N) {
+        const double t = v[j] * inv;
+        const double2 si = s_inv[n0 + j];
+        c[j] = inv != 0.0 && s_norm[n0 + j] >= kEmptyThresh
+                   ? fma(t, si.y, t * si.x) : 0.0;
+      }
+    return acc;
+  }
+  __device__ void finish(int, bool, int, double) const {}
+};
+
+// Force kernel values of gradient rows (gemm_force_kernel).
+struct EpiForceKernel {
+  using Value = double;
+  static constexpr bool kFloat = false;
+  ForceKernelArgs a;
+  int N;
+  __device__ double chunk(int m, bool row_ok, int n0, const double (&v)[16],
+                          double acc) const {
+    if (!row_ok) return acc;
+    const int gr = a.rows[m];
+    const int atom = a.center[gr / 3];
+    const double nd = a.d_norm[atom];
+    const bool dok = nd >= kEmptyThresh;
+    // row constants with the factor sig2 power in them: 6 FP64
+    // instructions a value, which bound this epilogue
+    const double inv = dok ? 1.0 / nd : 0.0;
+    const double kinv = a.sig2 * a.power * inv;
+    const double fdn = kinv * (a.fdots[gr] * inv);
+    const double *cs = a.cosine + (long long)(a.crow[atom] - a.crow0) * N + n0;
+    double *out = a.FK + (long long)gr * a.M + a.c_s + n0;
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      if (n0 + j < N) {
+        double x = 0.0;
+        if (dok && a.s_norm[n0 + j] >= kEmptyThresh) {
+          const double c = cs[j];
+          // both words of 1/|s|: the two terms nearly cancel, and an error
+          // common to a sparse row adds up over the pairs (stress rows)
+          const double t = v[j] * kinv;
+          const double2 si = a.s_inv[n0 + j];
+          x = fma(t, si.x, fma(t, si.y, -(c * fdn)));
+          if (a.power == 2.0) x *= c;
+          else if (a.power != 1.0) x *= pow(c, a.power - 1.0);
+        }
+        out[j] = x;
+      }
+    return acc;
+  }
+  __device__ void finish(int, bool, int, double) const {}
+};
+
+// Kernel matrix of two environment sets (gemm_envs).
+struct EpiEnvs {
+  using Value = double;
+  static constexpr bool kFloat = false;
+  const double *na, *nb;
+  double sig2, power;
+  double *K;
+  int N;
+  __device__ double chunk(int m, bool row_ok, int n0, const double (&v)[16],
+                          double acc) const {
+    if (!row_ok) return acc;
+    const double a = na[m];
+    double *k = K + (long long)m * N + n0;
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      if (n0 + j < N) {
+        const double b = nb[n0 + j];
+        k[j] = a >= kEmptyThresh && b >= kEmptyThresh
+                   ? sig2 * gemm64::powx(v[j] / (a * b), power) : 0.0;
+      }
+    return acc;
+  }
+  __device__ void finish(int, bool, int, double) const {}
+};
+
 // E_atom = scale x sum of the row's energy partials (fixed order,
 // row_slots_sum).
 __global__ void k_energy_final(int M, int ntiles, const double *__restrict__ part,
@@ -1331,6 +1442,58 @@ __global__ void k_energy_final(int M, int ntiles, const double *__restrict__ par
 }  // namespace
 }  // namespace oz
 
+
+namespace oz {
+
+int row_inverse(int M, int nd, const double *rows, double *norms, double2 *inv,
+                cudaStream_t st) {
+  if (M == 0) return FGB_OK;
+  k_oz_row_inv<<<ceil_div((long long)M * 32, 256), 256, 0, st>>>(M, nd, rows,
+                                                               norms, inv);
+  FGB_LAUNCH_CHECK("k_oz_row_inv");
+  return FGB_OK;
+}
+
+// The fewer rounds of tiles over the SMs weighted by a tile's time: a 48-row
+// tile takes 1.25 times a 32-row tile (2 x 1,000 sparse, n_d 680, the three
+// products of the FP64 path over both species: 500 atoms 417 us at 48 rows
+// against 335 at 32, 1,000 atoms 420 and 374, 1,500 atoms 426 and 480, 8,000
+// atoms 1,319 and 1,403).
+int tile64(int rows, int cols) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
+          cudaSuccess)
+    return 0;
+  const long long mt = ceil_div(rows, kTM);
+  return 4 * ceil_div(mt * ceil_div(cols, kTN64v[1]), sms) <
+                 5 * ceil_div(mt * ceil_div(cols, kTN64v[0]), sms)
+             ? 1 : 0;
+}
+
+int gemm_cosine(const Sliced &A, const Sliced &B, const int *perm,
+                const double *a_norm, const double2 *s_inv,
+                const double *s_norm, double *C, int *err, cudaStream_t st) {
+  return gemm_s<kS64>(A, B, false,
+                      EpiCosine{perm, a_norm, s_norm, s_inv, C, B.rows}, err,
+                      st);
+}
+int gemm_force_kernel(const Sliced &A, const Sliced &B,
+                      const ForceKernelArgs &fk, int *err, cudaStream_t st) {
+  return gemm_s<kS64>(A, B, false, EpiForceKernel{fk, B.rows}, err, st);
+}
+int gemm_envs(const Sliced &A, const Sliced &B, const double *na,
+              const double *nb, double sig2, double power, double *K, int *err,
+              cudaStream_t st) {
+  return gemm_s<kS64>(A, B, false, EpiEnvs{na, nb, sig2, power, K, B.rows},
+                      err, st);
+}
+int gemm_rowsq(const Sliced &A, const Sliced &B, bool tri, double *part,
+               int *err, cudaStream_t st) {
+  return gemm_s<kS64>(A, B, tri, EpiZsq{part, B.RP / 16, B.rows}, err, st);
+}
+
+}  // namespace oz
 
 // Slice the model operands for variant v (slice count and B tile height),
 // per species: the normalised sparse rows (B of the kernel GEMM) or the
@@ -1397,9 +1560,9 @@ static int build_oz64_S(fgb_model_s *m, int v, cudaStream_t st) {
   const int nd = m->b2.n_d;
   int rc;
   if ((rc = m->sinv.ensure(sizeof(double2) * (m->M + 1)))) return rc;
-  oz::k_oz_row_inv<<<ceil_div((long long)m->M * 32, 256), 256, 0, st>>>(
-      m->M, nd, m->Sraw.as<double>(), m->sinv.as<double2>());
-  FGB_LAUNCH_CHECK("k_oz_row_inv");
+  if ((rc = oz::row_inverse(m->M, nd, m->Sraw.as<double>(), nullptr,
+                            m->sinv.as<double2>(), st)))
+    return rc;
   return build_oz64(m, v, m->oz64S[v], [&](int s, int &) {
     return oz::SliceSpec{m->h_counts[s], nd, 0,
                          m->Sraw.as<double>() + (size_t)m->h_offsets[s] * nd, nd,
@@ -1772,26 +1935,11 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
                          bool want_grad, bool want_var, double *d_e_atom,
                          double *d_gB2, double *d_var, cudaStream_t st,
                          bool fixed, bool have_rowmax) {
-  int rc, dev = 0, sms = 0;
-  FGB_CUDA(cudaGetDevice(&dev));
-  FGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int rc;
   const B2Params &p = m->b2;
   const int nd = p.n_d;
   const double sig2 = m->sigma * m->sigma, xi = m->power;
   constexpr int kRows = 32768;
-  // B tile height of a product of `rows` x `cols` (variant 0: 48 rows, 1:
-  // 32 rows): the fewer rounds of tiles over the SMs weighted by a tile's
-  // time.  A 48-row tile takes 1.25 times a 32-row tile (2 x 1,000 sparse,
-  // n_d 680, three products of both species: 500 atoms 417 against 335 us,
-  // 1,000 atoms 420 and 374, 1,500 atoms 426 and 480, 8,000 atoms 1,319 and
-  // 1,403).
-  const auto pick = [sms](int rows, int cols) {
-    const int mt = ceil_div(rows, oz::kTM);
-    return 4 * ceil_div((long long)mt * ceil_div(cols, oz::kTN64v[1]), sms) <
-                   5 * ceil_div((long long)mt * ceil_div(cols, oz::kTN64v[0]),
-                                sms)
-               ? 1 : 0;
-  };
   const auto ready = [&](bool *flags, int v,
                          int (*build)(fgb_model_s *, int, cudaStream_t)) -> int {
     if (flags[v]) return FGB_OK;
@@ -1822,7 +1970,8 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
     for (int r0 = 0; r0 < Ns; r0 += kRows) {
       const int Mr = std::min(kRows, Ns - r0);
       const int *perm = perm_s + r0;
-      const int vk = pick(Mr, Ms), vv = pick(Mr, R), vg = pick(Mr, nd);
+      const int vk = oz::tile64(Mr, Ms), vv = oz::tile64(Mr, R),
+                vg = oz::tile64(Mr, nd);
       if ((rc = ready(m->oz64S_ready, vk, build_oz64_S)) ||
           (want_var && (rc = ready(m->oz64L_ready, vv, build_oz64_L))) ||
           (want_grad && (rc = ready(m->oz64ST_ready, vg, build_oz64_ST))))

@@ -52,7 +52,7 @@ k_envs_envs(int M, int N, int K, const double *__restrict__ D1,
 // cycles each per warp on an SM quarter), so the pairs are spread over all
 // SMs.  One block per atom that walked its pairs in series, one thread
 // evaluating each pair's basis, took 913 us for 108 FCC atoms (3,456 pairs,
-// n_d 144) where these take 84 us (k_pair_basis 14, k_b2_dervs 70).
+// n_d 144) where these take 78 us (k_pair_basis 15, k_b2_dervs 63).
 constexpr int kBT = 32;   // pairs (threads) per block of k_pair_basis
 
 // Basis values of every pair, value-major so that neighbouring pairs are
@@ -95,27 +95,27 @@ k_pair_basis(B2Params p, long long P, const int *__restrict__ center,
 // dB2 rows of PP consecutive pairs: dA in shared memory, then a thread per
 // descriptor q for all PP x 3 rows, and the rows' dots with B2 by a
 // fixed-order block sum.
-constexpr int kDT = 128;
+constexpr int kDTmax = 256;
 template <int PP>
-__global__ void __launch_bounds__(kDT)
+__global__ void __launch_bounds__(kDTmax)
 k_b2_dervs(B2Params p, long long P, const int *__restrict__ center,
            const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
            const int *__restrict__ species, const double *__restrict__ basis,
            const double *__restrict__ A_in, const double *__restrict__ B2_in,
            double *__restrict__ dB2, double *__restrict__ fdots) {
-  extern __shared__ double dA[];            // PP x 3 x nm x nh
-  __shared__ double red[3 * PP][kDT + 1];
+  extern __shared__ double dA[];   // PP x 3 x nm x nh | 3 PP x (threads + 1)
   const int nA = p.n_A, nh = p.n_harm, nm = p.n_max, nr = p.n_rad,
             L1 = p.l_max + 1, nd = p.n_d, nmh = nm * nh;
   const long long p0 = (long long)blockIdx.x * PP;
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, nt = blockDim.x;
+  double *red = dA + PP * 3 * nmh;
   int cen[PP], sj[PP];
 #pragma unroll
   for (int k = 0; k < PP; k++) {
     cen[k] = p0 + k < P ? center[p0 + k] : center[p0];
     sj[k] = p0 + k < P ? species[nbr_j[p0 + k]] : -1;
   }
-  for (int e = t; e < nmh; e += kDT) {
+  for (int e = t; e < nmh; e += nt) {
     const int n = e / nh, lm = e - n * nh;
     const double *bn = basis + n * P + p0;
     const double *by = basis + (2 * nm + lm) * P + p0;
@@ -135,7 +135,7 @@ k_b2_dervs(B2Params p, long long P, const int *__restrict__ center,
   double fd[3 * PP];
 #pragma unroll
   for (int k = 0; k < 3 * PP; k++) fd[k] = 0.0;
-  for (int q = t; q < nd; q += kDT) {
+  for (int q = t; q < nd; q += nt) {
     const int l = q % L1;
     int pidx = q / L1, n1 = 0;
     while (pidx >= nr - n1) { pidx -= nr - n1; n1++; }
@@ -173,11 +173,11 @@ k_b2_dervs(B2Params p, long long P, const int *__restrict__ center,
     }
   }
 #pragma unroll
-  for (int k = 0; k < 3 * PP; k++) red[k][t] = fd[k];
+  for (int k = 0; k < 3 * PP; k++) red[k * (nt + 1) + t] = fd[k];
   __syncthreads();
-  for (int k = t >> 5; k < 3 * PP; k += kDT / 32) {
+  for (int k = t >> 5; k < 3 * PP; k += nt / 32) {
     double x = 0.0;
-    for (int q = t & 31; q < kDT; q += 32) x += red[k][q];
+    for (int q = t & 31; q < nt; q += 32) x += red[k * (nt + 1) + q];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
       x += __shfl_down_sync(0xffffffffu, x, off);
@@ -194,85 +194,18 @@ __global__ void k_pair_center(int N, const long long *__restrict__ off,
     center[q] = a;
 }
 
-// Dots_s = B2[perm] S_s^T (raw descriptors), Ns x Ms.
-__global__ void __launch_bounds__(GT)
-k_dots(int M, int N, int K, const double *__restrict__ B2,
-       const int *__restrict__ perm, const double *__restrict__ S,
-       double *__restrict__ out) {
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  double acc[4][4];
-  gemm_mainloop<true>(acc, m0, n0, M, N, K, B2, K, perm, S, K);
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    int m = m0 + ty + 16 * i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      int n = n0 + tx + 16 * j;
-      if (n < N) out[(long long)m * N + n] = acc[i][j];
-    }
-  }
-}
-
-// Force-kernel values for the pairs of species-s centres
-// (normalized_dot_product.cpp:185-198): rows are dB2 rows 3p+c (gathered),
-// columns the species' sparse environments.  Written into FK[3P x M].
-__global__ void __launch_bounds__(GT)
-k_force_kernel(int R, int Ms, int K, const double *__restrict__ dB2,
-               const int *__restrict__ rows, const double *__restrict__ S,
-               const int *__restrict__ pair_center,
-               const int *__restrict__ inv_perm,
-               const double *__restrict__ dots, const double *__restrict__ dnorm,
-               const double *__restrict__ snorm,
-               const double *__restrict__ fdots, double sig2, double power,
-               int c_s, int M, double *__restrict__ FK) {
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  double acc[4][4];
-  gemm_mainloop<true>(acc, m0, n0, R, Ms, K, dB2, K, rows, S, K);
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    int m = m0 + ty + 16 * i;
-    if (m >= R) continue;
-    long long gr = rows[m];
-    int pair = (int)(gr / 3);
-    int atom = pair_center[pair];
-    int jl = inv_perm[atom];
-    double nj = dnorm[atom];
-#pragma unroll
-    for (int jj = 0; jj < 4; jj++) {
-      int n = n0 + tx + 16 * jj;
-      if (n >= Ms) continue;
-      double ni = snorm[n];
-      double v = 0.0;
-      if (ni >= kEmptyThresh && nj >= kEmptyThresh) {
-        double nij = ni * nj, nij3 = nij * nj * nj;
-        double dv = dots[(long long)jl * Ms + n];
-        double nd_ = dv / nij;
-        double dval = power * (power == 2.0 ? nd_
-                                            : power == 1.0 ? 1.0
-                                                           : pow(nd_, power - 1.0));
-        double f1 = acc[i][jj] / nij;
-        double f2 = dv * fdots[gr] / nij3;
-        v = sig2 * dval * (f1 - f2);
-      }
-      FK[gr * M + c_s + n] = v;
-    }
-  }
-}
-
 // The energy and stress columns are sums over all atoms or pairs for every
 // sparse row: block (32 sparse rows x 8 groups) x chunk of atoms or pairs,
 // then k_col_final adds the chunks in order.  A thread per sparse row that
 // walked every pair alone took 1,751 us (108 FCC atoms, 3,456 pairs, 200
-// sparse rows) and every atom 406 us; the three kernels here take 12, 7 and
-// 9 us, the stress part at 1.4 TB/s of FK (16.6 MB, partly in L2).
+// sparse rows) and every atom 406 us; the three kernels here take 15, 3 and
+// 3 us, the stress part at 1.1 TB/s of FK (16.6 MB, partly in L2).
 constexpr int kColRows = 32, kColGroups = 8;
 
-// part[ch][i] = sum over the chunk's atoms j of sig2 (dot_ij / |s_i||d_j|)^power
+// part[ch][i] = sum over the chunk's atoms j of sig2 c_ij^power (c zero for
+// empty rows, which add nothing)
 __global__ void __launch_bounds__(kColRows * kColGroups)
-k_energy_part(int Ns, int Ms, int per, const double *__restrict__ dots,
+k_energy_part(int Ns, int Ms, int per, const double *__restrict__ cosine,
               const int *__restrict__ perm, const double *__restrict__ dnorm,
               const double *__restrict__ snorm, double sig2, double power,
               double *__restrict__ part, int ldp) {
@@ -280,15 +213,11 @@ k_energy_part(int Ns, int Ms, int per, const double *__restrict__ dots,
   const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int i = blockIdx.x * kColRows + x, ch = blockIdx.y;
   double acc = 0.0;
-  if (i < Ms) {
-    const double ni = snorm[i];
+  if (i < Ms && snorm[i] >= kEmptyThresh) {
     const int j1 = min(Ns, (ch + 1) * per);
-    if (ni >= kEmptyThresh)
-      for (int j = ch * per + g; j < j1; j += kColGroups) {
-        const double nj = dnorm[perm[j]];
-        if (nj < kEmptyThresh) continue;
-        acc += sig2 * powx(dots[(long long)j * Ms + i] / (ni * nj), power);
-      }
+    for (int j = ch * per + g; j < j1; j += kColGroups)
+      if (dnorm[perm[j]] >= kEmptyThresh)
+        acc += sig2 * powx(cosine[(long long)j * Ms + i], power);
   }
   red[g][x] = acc;
   __syncthreads();
@@ -298,10 +227,24 @@ k_energy_part(int Ns, int Ms, int per, const double *__restrict__ dots,
   }
 }
 
+// First sparse row of each species: FK[gr][i] is written only where row i
+// and the centre of pair gr / 3 have one species; elsewhere it is zero by
+// definition and not read.
+struct SparseOffsets {
+  int o[kMaxSpecies + 1];
+  int n;
+  __device__ int species(int i) const {
+    int s = 0;
+    while (s + 1 < n && i >= o[s + 1]) s++;
+    return s;
+  }
+};
+
 // part[ch][k][i] = sum over the chunk's pairs of fk_a r_b (b >= a, flare order)
 __global__ void __launch_bounds__(kColRows * kColGroups)
-k_stress_part(int M, long long P, long long per,
+k_stress_part(int M, long long P, long long per, SparseOffsets so,
               const double4_16a *__restrict__ rel,
+              const int *__restrict__ center, const int *__restrict__ species,
               const double *__restrict__ FK, double *__restrict__ part) {
   __shared__ double red[6][kColGroups][kColRows + 1];
   const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -309,8 +252,10 @@ k_stress_part(int M, long long P, long long per,
   const long long ch = blockIdx.y;
   double s[6] = {0, 0, 0, 0, 0, 0};
   if (i < M) {
+    const int si = so.species(i);
     const long long p1 = min(P, (ch + 1) * per);
     for (long long p = ch * per + g; p < p1; p += kColGroups) {
+      if (species[center[p]] != si) continue;
       const double4_16a r = rel[p];
       const double *f = FK + 3 * p * M + i;
       const double f0 = f[0], f1 = f[M], f2 = f[2LL * M];
@@ -332,64 +277,137 @@ k_stress_part(int M, long long P, long long per,
   }
 }
 
-// Energy column (k = 0) and stress columns (k = 1..6, times -1/V) from the
-// chunks' partial sums: kern[i][col].
-__global__ void k_col_final(int M, int nce, int ncs,
-                            const double *__restrict__ epart,
-                            const double *__restrict__ spart, double vol_inv,
-                            int n_atoms, long long ncol,
-                            double *__restrict__ kern) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
-  if (i >= M) return;
+// Energy row (k = 0) and stress rows (k = 1..6, times -1/V) of K^T from the
+// chunks' partial sums: block of 32 sparse rows, 8 groups of chunks.
+__global__ void __launch_bounds__(kColRows * kColGroups)
+k_col_final(int M, int nce, int ncs, const double *__restrict__ epart,
+            const double *__restrict__ spart, double vol_inv, int n_atoms,
+            double *__restrict__ kt) {
+  __shared__ double red[kColGroups][kColRows + 1];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int i = blockIdx.x * kColRows + x, k = blockIdx.y;
+  const int nc = k ? ncs : nce;
+  const double *src = k ? spart + (long long)(k - 1) * M : epart;
+  const long long step = k ? 6LL * M : M;
   double s = 0.0;
-  if (k == 0) {
-    for (int c = 0; c < nce; c++) s += epart[(long long)c * M + i];
-    kern[(long long)i * ncol] = s;
-  } else {
-    for (int c = 0; c < ncs; c++) s += spart[((long long)c * 6 + k - 1) * M + i];
-    kern[(long long)i * ncol + 1 + 3LL * n_atoms + k - 1] = -s * vol_inv;
-  }
+  if (i < M)
+    for (int c = g; c < nc; c += kColGroups) s += src[c * step + i];
+  red[g][x] = s;
+  __syncthreads();
+  if (g || i >= M) return;
+  for (int q = 1; q < kColGroups; q++) s += red[q][x];
+  if (k == 0) kt[i] = s;
+  else kt[(3LL * n_atoms + k) * M + i] = -s * vol_inv;
 }
 
-// Force columns by owner-computes: K[i][1+3a+c] = sum_{p in out(a)}
-// FK[3p+c][i] - FK[3 twin(p)+c][i].  Thread per (sparse i, atom a).
-__global__ void k_force_cols(int M, int N, const long long *__restrict__ off,
-                             const long long *__restrict__ twin,
-                             const double *__restrict__ FK, long long ncol,
-                             double *__restrict__ kern) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)M * N) return;
-  int i = (int)(idx % M), a = (int)(idx / M);
+// Force rows of K^T by owner-computes: K^T[1+3a+c][i] = sum_{p in out(a)}
+// FK[3p+c][i] - FK[3 twin(p)+c][i].  Block: an atom x 32 sparse rows x 8
+// groups of its pairs (one group that walked all of them waited on each
+// twin: 37 us against 13, 108 FCC atoms, 200 sparse rows).
+__global__ void __launch_bounds__(kColRows * kColGroups)
+k_force_cols(int M, int N, SparseOffsets so, const long long *__restrict__ off,
+             const int *__restrict__ nbr_j, const long long *__restrict__ twin,
+             const int *__restrict__ species, const double *__restrict__ FK,
+             double *__restrict__ kt) {
+  __shared__ double red[3][kColGroups][kColRows + 1];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int i = blockIdx.y * kColRows + x, a = blockIdx.x;
   double f[3] = {0.0, 0.0, 0.0};
-  for (long long q = off[a]; q < off[a + 1]; q++) {
-    long long tw = twin[q];
-    for (int c = 0; c < 3; c++) {
-      double v = FK[(3 * q + c) * M + i];
-      if (tw >= 0) v -= FK[(3 * tw + c) * M + i];
-      f[c] += v;
+  if (i < M) {
+    const int si = so.species(i);
+    const bool own = species[a] == si;
+    for (long long q = off[a] + g; q < off[a + 1]; q += kColGroups) {
+      const long long tw = twin[q];
+      if (own)
+        for (int c = 0; c < 3; c++) f[c] += FK[(3 * q + c) * M + i];
+      if (tw >= 0 && species[nbr_j[q]] == si)
+        for (int c = 0; c < 3; c++) f[c] -= FK[(3 * tw + c) * M + i];
     }
   }
-  for (int c = 0; c < 3; c++) kern[(long long)i * ncol + 1 + 3 * a + c] = f[c];
+#pragma unroll
+  for (int c = 0; c < 3; c++) red[c][g][x] = f[c];
+  __syncthreads();
+  if (g < 3 && i < M) {
+    double s = 0.0;
+    for (int q = 0; q < kColGroups; q++) s += red[g][q][x];
+    kt[(1 + 3LL * a + g) * M + i] = s;
+  }
 }
 
-// mean_efs[o] = sum_i kern[i][o] alpha[i]
-__global__ void k_kern_t_alpha(int M, long long ncol, const double *__restrict__ kern,
-                               const double *__restrict__ alpha,
-                               double *__restrict__ out) {
-  long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= ncol) return;
-  double acc = 0.0;
-  for (int i = 0; i < M; i++) acc += kern[(long long)i * ncol + o] * alpha[i];
-  out[o] = acc;
+// The pairs grouped by their centre's species: with the atoms in species
+// order (perm), start[k] is the first place of atom perm[k]'s pairs,
+// inv[perm[k]] = k and spairs[s] the first place of species s (spairs[S] =
+// all pairs).  One block.
+__global__ void __launch_bounds__(1024)
+k_group_scan(int N, const int *__restrict__ perm, const int *__restrict__ species,
+             const long long *__restrict__ off, int S, int *__restrict__ start,
+             int *__restrict__ inv, int *__restrict__ spairs) {
+  __shared__ int wsum[32], cnt[kMaxSpecies], carry;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  if (t < kMaxSpecies) cnt[t] = 0;
+  if (t == 0) carry = 0;
+  __syncthreads();
+  for (int base = 0; base < N; base += 1024) {
+    const int k = base + t;
+    int n = 0;
+    if (k < N) {
+      const int a = perm[k];
+      n = (int)(off[a + 1] - off[a]);
+      inv[a] = k;
+      atomicAdd(&cnt[species[a]], n);
+    }
+    int x = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    int before = carry;
+    for (int q = 0; q < w; q++) before += wsum[q];
+    if (k < N) start[k] = before + x - n;
+    __syncthreads();
+    if (t == 1023) carry = before + x;
+    __syncthreads();
+  }
+  if (t == 0) {
+    int acc = 0;
+    for (int s = 0; s < S; s++) {
+      spairs[s] = acc;
+      acc += cnt[s];
+    }
+    spairs[S] = acc;
+  }
 }
 
-__global__ void k_rownorms(int M, int nd, const double *__restrict__ S,
-                           double *__restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M) return;
-  double acc = 0.0;
-  for (int q = 0; q < nd; q++) acc += S[(long long)i * nd + q] * S[(long long)i * nd + q];
-  out[i] = sqrt(acc);
+// rows[3 r + c] = 3 q + c for the pair q at place r of the grouped order: a
+// warp per atom.
+__global__ void k_group_rows(int N, const int *__restrict__ perm,
+                             const long long *__restrict__ off,
+                             const int *__restrict__ start,
+                             int *__restrict__ rows) {
+  const int k = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (k >= N) return;
+  const int a = perm[k];
+  const int q0 = (int)off[a], n = (int)(off[a + 1] - off[a]);
+  for (int e = threadIdx.x & 31; e < 3 * n; e += 32)
+    rows[3 * start[k] + e] = 3 * q0 + e;
+}
+
+// out (C x R) = in^T (in: R x C), 32 x 32 tiles.
+__global__ void k_transpose32(long long R, int C, const double *__restrict__ in,
+                              double *__restrict__ out) {
+  __shared__ double t[32][33];
+  const long long r0 = (long long)blockIdx.x * 32;
+  const int c0 = blockIdx.y * 32;
+  for (int k = threadIdx.y; k < 32; k += blockDim.y)
+    if (r0 + k < R && c0 + (int)threadIdx.x < C)
+      t[k][threadIdx.x] = in[(r0 + k) * C + c0 + threadIdx.x];
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += blockDim.y)
+    if (c0 + k < C && r0 + threadIdx.x < R)
+      out[(c0 + k) * R + r0 + threadIdx.x] = t[threadIdx.x][k];
 }
 
 }  // namespace
@@ -436,12 +454,16 @@ int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
     default: eval(std::integral_constant<int, 0>()); break;
   }
   FGB_LAUNCH_CHECK("k_pair_basis");
+  // threads: whole warps, n_d split evenly over the fewest passes
+  const int passes = ceil_div(p.n_d, kDTmax);
+  const int nt = 32 * ceil_div(ceil_div(p.n_d, passes), 32);
   const auto dervs = [&](auto pp) -> int {
     constexpr int K = decltype(pp)::value;
+    const size_t bytes = K * per + sizeof(double) * 3 * K * (nt + 1);
     FGB_CUDA(cudaFuncSetAttribute(k_b2_dervs<K>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(K * per)));
-    k_b2_dervs<K><<<ceil_div(P, K), kDT, K * per, st>>>(
+                                  (int)bytes));
+    k_b2_dervs<K><<<ceil_div(P, K), nt, bytes, st>>>(
         p, P, center.as<int>(), nl->nbr_j.as<int>(),
         nl->nbr_rel.as<double4_16a>(), d_species, basis.as<double>(), d_A,
         d_B2, d_dB2, d_force_dots);
@@ -469,6 +491,35 @@ extern "C" int fgb_envs_envs(const double *d_desc1, const double *d_norm1,
   }
   if (n1 == 0 || n2 == 0) return FGB_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    cs = cudaStreamCaptureStatusActive;   // unknown: do not synchronise
+  }
+  if (cs == cudaStreamCaptureStatusNone) {
+    oz::Sliced A(st), B(st);
+    DevBuf err(st);
+    const int v = oz::tile64(n1, n2);
+    int rc, h = 0;
+    if ((rc = err.ensure(sizeof(int)))) return rc;
+    FGB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+    if ((rc = oz::slice({n1, n_desc, oz::kTM, d_desc1, n_desc, nullptr,
+                         nullptr}, A, st, oz::kS64)) ||
+        (rc = oz::slice({n2, n_desc, oz::kTN64v[v], d_desc2, n_desc, nullptr,
+                         nullptr}, B, st, oz::kS64)) ||
+        (rc = oz::gemm_envs(A, B, d_norm1, d_norm2, sig2, power, d_kern,
+                            err.as<int>(), st)))
+      return rc;
+    FGB_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost,
+                             st));
+    FGB_CUDA(cudaStreamSynchronize(st));
+    if (h) {
+      set_error("fgb_envs_envs: a bounded device wait ran out");
+      return FGB_ETIMEOUT;
+    }
+    return FGB_OK;
+  }
+  // a call being captured cannot read the products' time-out flag back
   dim3 g(ceil_div(n2, BN), ceil_div(n1, BM));
   k_envs_envs<<<g, GT, 0, st>>>(n1, n2, n_desc, d_desc1, d_norm1, d_desc2,
                                 d_norm2, sig2, power, d_kern);
@@ -502,13 +553,14 @@ extern "C" int fgb_b2_forward_dervs(fgb_b2_t b2, fgb_nlist_t nl,
 }
 
 namespace fgb {
-// envs_struc for one structure into d_kern; B2/norms of the structure are
-// left in ws (for the plain prediction's variance stage).
+// envs_struc for one structure, transposed: d_kt [(1 + 3N + 6) x M]; B2,
+// norms and stored gradients of the structure are left in ws.  The dots with
+// the sparse rows are exact kS64-slice products (ozaki.cu), whose epilogues
+// write the cosines and the force-kernel values.
 int envs_struc_impl(const B2Params &p, double sigma, double power,
-                           const int *h_counts, const double *d_sparse,
-                           fgb_nlist_s *nl, const int *d_species,
-                           double *d_kern, fgb_workspace &ws,
-                           cudaStream_t st) {
+                    const int *h_counts, const double *d_sparse,
+                    fgb_nlist_s *nl, const int *d_species, double *d_kt,
+                    fgb_workspace &ws, cudaStream_t st) {
   if (nl->n_struc != 1) {
     set_error("envs_struc needs a single-structure neighbour list");
     return FGB_EINVAL;
@@ -516,60 +568,60 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
   const int N = nl->n_atoms, S = p.n_species, nd = p.n_d;
   const long long P = nl->n_pairs;
   int rc;
-  if ((rc = check_species(d_species, N, S, ws.flag, st))) return rc;
-  std::vector<int> off(S + 1, 0);
-  for (int s = 0; s < S; s++) off[s + 1] = off[s] + h_counts[s];
-  const int M = off[S];
+  SparseOffsets so;
+  so.n = S;
+  so.o[0] = 0;
+  for (int s = 0; s < S; s++) so.o[s + 1] = so.o[s] + h_counts[s];
+  const int M = so.o[S];
   const long long ncol = 1 + 3LL * N + 6;
-  if (M == 0) return FGB_OK;
-  FGB_CUDA(cudaMemsetAsync(d_kern, 0, sizeof(double) * M * ncol, st));
-  if (N == 0) return FGB_OK;
-  if ((rc = ws.A.ensure(sizeof(double) * ((size_t)N * p.n_A + 1))) ||
+  if ((rc = ws.ozerr.ensure(sizeof(int)))) return rc;
+  FGB_CUDA(cudaMemsetAsync(ws.ozerr.p, 0, sizeof(int), st));
+  if (M == 0) return check_species(d_species, N, S, ws.flag, st);
+  if (N == 0) {
+    FGB_CUDA(cudaMemsetAsync(d_kt, 0, sizeof(double) * M * ncol, st));
+    return FGB_OK;
+  }
+  std::vector<int> counts;
+  bool pending = false;
+  if ((rc = species_permutation_start(S, ws, d_species, N, counts, st, nullptr,
+                                      pending)) ||
+      (rc = ws.start.ensure(sizeof(int) * (2 * (size_t)N + S + 1))) ||
+      (rc = ws.rows.ensure(sizeof(int) * (3 * (size_t)P + 1))) ||
+      (rc = ws.A.ensure(sizeof(double) * ((size_t)N * p.n_A + 1))) ||
       (rc = ws.B2.ensure(sizeof(double) * ((size_t)N * nd + 1))) ||
       (rc = ws.norms.ensure(sizeof(double) * (N + 1))) ||
+      (rc = ws.rowmax.ensure(sizeof(double) * (N + 1))) ||
       (rc = ws.dB2.ensure(sizeof(double) * ((size_t)3 * P * nd + 1))) ||
       (rc = ws.fdots.ensure(sizeof(double) * (3 * P + 1))) ||
       (rc = ws.kern.ensure(sizeof(double) * ((size_t)3 * P * M + 1))) ||
-      (rc = ws.var.ensure(sizeof(double) * (M + 1))) ||
-      (rc = ws.pos.ensure(sizeof(int) * (P + 1))) ||
-      (rc = ws.perm.ensure(sizeof(int) * (N + 1))) ||
-      (rc = ws.flags.ensure(sizeof(int) * (N + 1))) ||
-      (rc = ws.scal.ensure(sizeof(int) * (3 * P + 1))))
+      (rc = ws.snorm.ensure(sizeof(double) * (3 * (size_t)M + 1))))
     return rc;
+  double *snorm = ws.snorm.as<double>();
+  double2 *sinv = reinterpret_cast<double2 *>(snorm + M + (M & 1));
+  // the forward takes any species value; a species out of range is found
+  // next, before anything is indexed by it
   if ((rc = launch_b2_forward(p, nl, d_species, ws.A.as<double>(),
-                              ws.B2.as<double>(), ws.norms.as<double>(), st)))
+                              ws.B2.as<double>(), ws.norms.as<double>(), st,
+                              false, ws.rowmax.as<double>())) ||
+      (rc = oz::row_inverse(M, nd, d_sparse, snorm, sinv, st)) ||
+      (pending && (rc = species_permutation_finish(S, ws, counts))))
     return rc;
+  const long long *off = nl->offsets.as<long long>();
+  const int *perm = ws.perm.as<int>();
+  int *start = ws.start.as<int>(), *inv = start + N, *dsp = inv + N;
+  k_group_scan<<<1, 1024, 0, st>>>(N, perm, d_species, off, S, start, inv, dsp);
+  FGB_LAUNCH_CHECK("k_group_scan");
+  int *spairs = ws.counts.h + kMaxSpecies + 1;
+  FGB_CUDA(cudaMemcpyAsync(spairs, dsp, sizeof(int) * (S + 1),
+                           cudaMemcpyDeviceToHost, st));
+  if (ws.counts.ev) FGB_CUDA(cudaEventRecord(ws.counts.ev, st));
+  k_group_rows<<<ceil_div((long long)N * 32, 128), 128, 0, st>>>(
+      N, perm, off, start, ws.rows.as<int>());
+  FGB_LAUNCH_CHECK("k_group_rows");
   if ((rc = launch_b2_dervs(p, nl, d_species, ws.A.as<double>(),
                             ws.B2.as<double>(), ws.dB2.as<double>(),
                             ws.fdots.as<double>(), ws.pos, ws.basis, st)))
     return rc;
-  // host-side species permutation and pair rows (plain path: sync is fine)
-  std::vector<int> hs(N);
-  std::vector<long long> hoff(N + 1);
-  FGB_CUDA(cudaMemcpyAsync(hs.data(), d_species, sizeof(int) * N,
-                           cudaMemcpyDeviceToHost, st));
-  FGB_CUDA(cudaMemcpyAsync(hoff.data(), nl->offsets.p,
-                           sizeof(long long) * (N + 1), cudaMemcpyDeviceToHost,
-                           st));
-  FGB_CUDA(cudaStreamSynchronize(st));
-  std::vector<int> perm, inv(N), rows;
-  std::vector<int> sbase(S + 1, 0);
-  for (int s = 0; s < S; s++) {
-    sbase[s] = (int)perm.size();
-    for (int a = 0; a < N; a++)
-      if (hs[a] == s) { inv[a] = (int)perm.size() - sbase[s]; perm.push_back(a); }
-  }
-  sbase[S] = N;
-  FGB_CUDA(cudaMemcpyAsync(ws.perm.p, perm.data(), sizeof(int) * N,
-                           cudaMemcpyHostToDevice, st));
-  FGB_CUDA(cudaMemcpyAsync(ws.flags.p, inv.data(), sizeof(int) * N,
-                           cudaMemcpyHostToDevice, st));
-  DevBuf snorm, dots, rowsd;
-  if ((rc = snorm.ensure(sizeof(double) * (M + 1)))) return rc;
-  k_rownorms<<<ceil_div(M, 128), 128, 0, st>>>(M, nd, d_sparse,
-                                               snorm.as<double>());
-  FGB_LAUNCH_CHECK("k_rownorms");
-  FGB_CUDA(cudaMemsetAsync(ws.kern.p, 0, sizeof(double) * 3 * P * M, st));
   const double sig2 = sigma * sigma;
   // chunks of the energy (atoms) and stress (pairs) sums: at least 32 atoms
   // or pairs each and at most 128 chunks
@@ -580,56 +632,94 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
     return rc;
   double *spart = ws.part.as<double>() + (size_t)M * nce;
   FGB_CUDA(cudaMemsetAsync(ws.part.p, 0, sizeof(double) * (size_t)M * nce, st));
+  if (ws.counts.ev) FGB_CUDA(cudaEventSynchronize(ws.counts.ev));
+  constexpr int kRows = 65536;   // gradient rows sliced at a time
+  int base = 0;
   for (int s = 0; s < S; s++) {
-    const int Ns = sbase[s + 1] - sbase[s], Ms = h_counts[s];
+    const int Ns = counts[s], Ms = h_counts[s], k0 = base;
+    base += Ns;
     if (Ns == 0 || Ms == 0) continue;
-    const double *Ss = d_sparse + (size_t)off[s] * nd;
-    const int *perm_s = ws.perm.as<int>() + sbase[s];
-    if ((rc = dots.ensure(sizeof(double) * (size_t)Ns * Ms))) return rc;
-    dim3 g1(ceil_div(Ms, BN), ceil_div(Ns, BM));
-    k_dots<<<g1, GT, 0, st>>>(Ns, Ms, nd, ws.B2.as<double>(), perm_s, Ss,
-                              dots.as<double>());
-    FGB_LAUNCH_CHECK("k_dots");
+    const int *perm_s = perm + k0;
+    const int R = 3 * (spairs[s + 1] - spairs[s]);
+    const int vc = oz::tile64(Ns, Ms);
+    const int vf = oz::tile64(std::min(std::max(R, 1), kRows), Ms);
+    for (int v = 0; v < 2; v++)
+      if ((v == vc || (v == vf && R > 0)) &&
+          (rc = oz::slice({Ms, nd, oz::kTN64v[v],
+                           d_sparse + (size_t)so.o[s] * nd, nd, nullptr,
+                           nullptr},
+                          ws.ozSp[v], st, oz::kS64)))
+        return rc;
+    if ((rc = ws.dots.ensure(sizeof(double) * (size_t)Ns * Ms)) ||
+        (rc = oz::slice({Ns, nd, oz::kTM, ws.B2.as<double>(), nd, perm_s,
+                         nullptr, ws.rowmax.as<double>()},
+                        ws.ozA, st, oz::kS64)) ||
+        (rc = oz::gemm_cosine(ws.ozA, ws.ozSp[vc], perm_s,
+                              ws.norms.as<double>(), sinv + so.o[s],
+                              snorm + so.o[s], ws.dots.as<double>(),
+                              ws.ozerr.as<int>(), st)))
+      return rc;
     k_energy_part<<<dim3(ceil_div(Ms, kColRows), ceil_div(Ns, eper)),
                     kColRows * kColGroups, 0, st>>>(
-        Ns, Ms, eper, dots.as<double>(), perm_s, ws.norms.as<double>(),
-        snorm.as<double>() + off[s], sig2, power,
-        ws.part.as<double>() + off[s], M);
+        Ns, Ms, eper, ws.dots.as<double>(), perm_s, ws.norms.as<double>(),
+        snorm + so.o[s], sig2, power, ws.part.as<double>() + so.o[s], M);
     FGB_LAUNCH_CHECK("k_energy_part");
-    rows.clear();
-    for (int k = sbase[s]; k < sbase[s + 1]; k++) {
-      int a = perm[k];
-      for (long long q = hoff[a]; q < hoff[a + 1]; q++)
-        for (int c = 0; c < 3; c++) rows.push_back((int)(3 * q + c));
+    for (int r0 = 0; r0 < R; r0 += kRows) {
+      const int Rc = std::min(kRows, R - r0);
+      const int *rows = ws.rows.as<int>() + 3LL * spairs[s] + r0;
+      oz::ForceKernelArgs fk;
+      fk.rows = rows;
+      fk.center = ws.pos.as<int>();
+      fk.crow = inv;
+      fk.crow0 = k0;   // inv is the place among all species
+      fk.cosine = ws.dots.as<double>();
+      fk.d_norm = ws.norms.as<double>();
+      fk.fdots = ws.fdots.as<double>();
+      fk.s_norm = snorm + so.o[s];
+      fk.s_inv = sinv + so.o[s];
+      fk.sig2 = sig2;
+      fk.power = power;
+      fk.FK = ws.kern.as<double>();
+      fk.c_s = so.o[s];
+      fk.M = M;
+      if ((rc = oz::slice({Rc, nd, oz::kTM, ws.dB2.as<double>(), nd, rows,
+                           nullptr},
+                          ws.ozK, st, oz::kS64)) ||
+          (rc = oz::gemm_force_kernel(ws.ozK, ws.ozSp[vf], fk,
+                                      ws.ozerr.as<int>(), st)))
+        return rc;
     }
-    const int R = (int)rows.size();
-    if (R == 0) continue;
-    if ((rc = rowsd.ensure(sizeof(int) * R))) return rc;
-    FGB_CUDA(cudaMemcpyAsync(rowsd.p, rows.data(), sizeof(int) * R,
-                             cudaMemcpyHostToDevice, st));
-    dim3 g2(ceil_div(Ms, BN), ceil_div(R, BM));
-    k_force_kernel<<<g2, GT, 0, st>>>(
-        R, Ms, nd, ws.dB2.as<double>(), rowsd.as<int>(), Ss, ws.pos.as<int>(),
-        ws.flags.as<int>(), dots.as<double>(), ws.norms.as<double>(),
-        snorm.as<double>() + off[s], ws.fdots.as<double>(), sig2, power,
-        off[s], M, ws.kern.as<double>());
-    FGB_LAUNCH_CHECK("k_force_kernel");
-    FGB_CUDA(cudaStreamSynchronize(st));   // rows buffer reused next species
   }
-  k_force_cols<<<ceil_div((long long)M * N, 128), 128, 0, st>>>(
-      M, N, nl->offsets.as<long long>(), nl->nbr_twin.as<long long>(),
-      ws.kern.as<double>(), ncol, d_kern);
+  k_force_cols<<<dim3(N, ceil_div(M, kColRows)), kColRows * kColGroups, 0,
+                 st>>>(
+      M, N, so, off, nl->nbr_j.as<int>(), nl->nbr_twin.as<long long>(),
+      d_species, ws.kern.as<double>(), d_kt);
   FGB_LAUNCH_CHECK("k_force_cols");
   if (P > 0) {
     k_stress_part<<<dim3(ceil_div(M, kColRows), ncs), kColRows * kColGroups, 0,
-                    st>>>(M, P, sper, nl->nbr_rel.as<double4_16a>(),
-                          ws.kern.as<double>(), spart);
+                    st>>>(M, P, sper, so, nl->nbr_rel.as<double4_16a>(),
+                          ws.pos.as<int>(), d_species, ws.kern.as<double>(),
+                          spart);
     FGB_LAUNCH_CHECK("k_stress_part");
   }
-  k_col_final<<<dim3(ceil_div(M, 128), 7), 128, 0, st>>>(
-      M, nce, ncs, ws.part.as<double>(), spart, 1.0 / nl->h_volume[0], N, ncol,
-      d_kern);
+  k_col_final<<<dim3(ceil_div(M, kColRows), 7), kColRows * kColGroups, 0, st>>>(
+      M, nce, ncs, ws.part.as<double>(), spart, 1.0 / nl->h_volume[0], N, d_kt);
   FGB_LAUNCH_CHECK("k_col_final");
+  return FGB_OK;
+}
+
+// The tensor-core time-out flag of the products above, after the stream's
+// work (synchronises).
+int sliced_finish(fgb_workspace &ws, cudaStream_t st, const char *what) {
+  int h = 0;
+  if (ws.ozerr.p)
+    FGB_CUDA(cudaMemcpyAsync(&h, ws.ozerr.p, sizeof(int),
+                             cudaMemcpyDeviceToHost, st));
+  FGB_CUDA(cudaStreamSynchronize(st));
+  if (h) {
+    set_error("%s: a bounded device wait ran out", what);
+    return FGB_ETIMEOUT;
+  }
   return FGB_OK;
 }
 }  // namespace fgb
@@ -642,12 +732,24 @@ extern "C" int fgb_envs_struc(fgb_b2_t b2, double sigma, double power,
     set_error("fgb_envs_struc: invalid arguments");
     return FGB_EINVAL;
   }
-  fgb_workspace ws;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = envs_struc_impl(b2->p, sigma, power, h_counts, d_sparse, nl,
-                           d_species, d_kern, ws, st);
-  if (!rc) FGB_CUDA(cudaStreamSynchronize(st));
-  return rc;
+  fgb_workspace ws;
+  ws.scratch_on(st);
+  long long M = 0;
+  for (int s = 0; s < b2->p.n_species; s++) M += h_counts[s];
+  const long long ncol = 1 + 3LL * nl->n_atoms + 6;
+  DevBuf kt(st);
+  int rc;
+  if ((rc = kt.ensure(sizeof(double) * ((size_t)M * ncol + 1))) ||
+      (rc = envs_struc_impl(b2->p, sigma, power, h_counts, d_sparse, nl,
+                            d_species, kt.as<double>(), ws, st)))
+    return rc;
+  if (M > 0) {
+    k_transpose32<<<dim3(ceil_div(ncol, 32), ceil_div(M, 32)), dim3(32, 8), 0,
+                    st>>>(ncol, (int)M, kt.as<double>(), d_kern);
+    FGB_LAUNCH_CHECK("k_transpose32");
+  }
+  return sliced_finish(ws, st, "envs_struc");
 }
 
 extern "C" int fgb_predict_plain(fgb_model_t m, fgb_nlist_t nl,
@@ -666,15 +768,14 @@ extern "C" int fgb_predict_plain(fgb_model_t m, fgb_nlist_t nl,
   const int N = nl->n_atoms, M = m->M;
   const long long ncol = 1 + 3LL * N + 6;
   int rc;
-  DevBuf kern;
-  if ((rc = kern.ensure(sizeof(double) * ((size_t)M * ncol + 1)))) return rc;
+  DevBuf kt(st);
+  if ((rc = kt.ensure(sizeof(double) * ((size_t)M * ncol + 1)))) return rc;
   if ((rc = envs_struc_impl(m->b2, m->sigma, m->power, m->h_counts.data(),
                             m->Sraw.as<double>(), nl, d_species,
-                            kern.as<double>(), m->ws, st)))
+                            kt.as<double>(), m->ws, st)) ||
+      (rc = launch_kt_alpha(M, ncol, kt.as<double>(), m->alpha.as<double>(),
+                            d_mean_efs, st)))
     return rc;
-  k_kern_t_alpha<<<ceil_div(ncol, 128), 128, 0, st>>>(
-      M, ncol, kern.as<double>(), m->alpha.as<double>(), d_mean_efs);
-  FGB_LAUNCH_CHECK("k_kern_t_alpha");
   if (d_local_var && N > 0) {
     // local variances: envs_envs(structure, sparse) then |L_inv k|^2
     // (sparse_gp.cpp:116-133), on the B2 values left in the workspace.
@@ -687,8 +788,7 @@ extern "C" int fgb_predict_plain(fgb_model_t m, fgb_nlist_t nl,
     FGB_CUDA(cudaMemcpyAsync(d_local_var, m->ws.var.p, sizeof(double) * N,
                              cudaMemcpyDeviceToDevice, st));
   }
-  FGB_CUDA(cudaStreamSynchronize(st));
-  return FGB_OK;
+  return sliced_finish(m->ws, st, "fgb_predict_plain");
 }
 
 // ------------------------------------------------------------ QR solve

@@ -165,21 +165,14 @@ __global__ void k_variance_final(int M, int ntiles, const double *__restrict__ p
   var[atom] = kself - s * scale;
 }
 
-__global__ void k_transpose_rm(int R, int C, const double *__restrict__ in,
-                               double *__restrict__ out) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)R * C) return;
-  int r = (int)(idx / C), c = (int)(idx % C);
-  out[(long long)c * R + r] = in[idx];
-}
-
-__global__ void k_sum_parts(int M, int ntiles, const double *__restrict__ part,
+// out[m] = sum of the row's partial slots (fixed order, row_slots_sum)
+__global__ void k_sum_parts(int M, int nslots, const double *__restrict__ part,
                             double *__restrict__ out) {
-  int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  double s = 0.0;
-  for (int t = 0; t < ntiles; t++) s += part[(long long)m * ntiles + t];
-  out[m] = s;
+  const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int m = (int)(gt / kRowLanes), q = (int)(gt % kRowLanes);
+  if (m >= M) return;   // whole lane groups
+  const double s = row_slots_sum(part, m, nslots, q);
+  if (q == 0) out[m] = s;
 }
 
 // variance_efs = K_self - Q_self + V_SOR (sparse_gp.cpp:726)
@@ -190,14 +183,34 @@ __global__ void k_dtc_combine(long long n, const double *__restrict__ kself,
   if (i < n) v[i] = kself[i] - q[i] + v[i];
 }
 
+// out[o] = K^T row o . alpha: a warp per output.  The terms cancel (|alpha|
+// up to 1e6 against energies of eV), so products and sums keep their errors
+// in a second word.
 __global__ void k_kt_alpha(int M, long long ncol, const double *__restrict__ KT,
                            const double *__restrict__ alpha,
                            double *__restrict__ out) {
-  long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long o = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (o >= ncol) return;
-  double acc = 0.0;
-  for (int i = 0; i < M; i++) acc += KT[o * M + i] * alpha[i];
-  out[o] = acc;
+  double acc = 0.0, err = 0.0;
+  const auto add = [&](double b, double b_err) {
+    const double s = __dadd_rn(acc, b), bb = __dadd_rn(s, -acc);
+    const double e = __dadd_rn(__dadd_rn(acc, -__dadd_rn(s, -bb)),
+                               __dadd_rn(b, -bb));
+    acc = s;
+    err = __dadd_rn(err, __dadd_rn(e, b_err));
+  };
+  for (int i = lane; i < M; i += 32) {
+    const double x = KT[o * M + i], a = alpha[i], p = __dmul_rn(x, a);
+    add(p, __fma_rn(x, a, -p));
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const double b = __shfl_down_sync(0xffffffffu, acc, off);
+    const double b_err = __shfl_down_sync(0xffffffffu, err, off);
+    add(b, b_err);
+  }
+  if (lane == 0) out[o] = acc + err;
 }
 
 __global__ void k_check_species(int n, const int *__restrict__ species, int ns,
@@ -291,13 +304,10 @@ k_species_scatter(int n, const int *__restrict__ species, int ns,
 
 }  // namespace
 
-int launch_row_energy(int Mr, int Ms, const double *Kmat, const double *alpha,
-                      const int *perm, double *e_rows, double *e_atom,
-                      cudaStream_t st) {
-  StageTimer _pt(kStRowEnergy, st);
-  k_row_energy<<<ceil_div((long long)Mr * 32, 256), 256, 0, st>>>(
-      Mr, Ms, Kmat, alpha, perm, e_rows, e_atom);
-  FGB_LAUNCH_CHECK("k_row_energy");
+int launch_kt_alpha(int M, long long ncol, const double *KT,
+                    const double *alpha, double *out, cudaStream_t st) {
+  k_kt_alpha<<<ceil_div(ncol * 32, 128), 128, 0, st>>>(M, ncol, KT, alpha, out);
+  FGB_LAUNCH_CHECK("k_kt_alpha");
   return FGB_OK;
 }
 
@@ -310,16 +320,6 @@ int launch_variance_final(int Mr, int ntiles, const double *part,
       ceil_div((long long)Mr * kRowLanes, 128), 128, 0, st>>>(
       Mr, ntiles, part, perm, norms, sig2, xi, scale, var);
   FGB_LAUNCH_CHECK("k_variance_final");
-  return FGB_OK;
-}
-
-int launch_variance_fp64(int Mr, int R, int Ms, const double *Kmat,
-                         const double *Lp, double *part, int ntiles,
-                         cudaStream_t st) {
-  StageTimer _pt(kStVarianceGemm, st);
-  dim3 g3(ntiles, ceil_div(Mr, BM));
-  k_variance_gemm<<<g3, GT, 0, st>>>(Mr, R, Ms, Kmat, Lp, part, ntiles);
-  FGB_LAUNCH_CHECK("k_variance_gemm");
   return FGB_OK;
 }
 
@@ -400,14 +400,16 @@ int species_permutation_start(int S, fgb_workspace &ws, const int *d_species,
   FGB_LAUNCH_CHECK("k_species_scatter");
   if (h_species) return FGB_OK;   // counted and checked above
   fgb_pinned_counts &pc = ws.counts;
+  if (!pc.h && pc.pageable) pc.h = pc.host;
   if (!pc.h)
     FGB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&pc.h),
-                           sizeof(int) * (kMaxSpecies + 1),
+                           sizeof(int) * fgb_pinned_counts::kInts,
                            cudaHostAllocDefault));
-  if (!pc.ev) FGB_CUDA(cudaEventCreateWithFlags(&pc.ev, cudaEventDisableTiming));
+  if (!pc.ev && !pc.pageable)
+    FGB_CUDA(cudaEventCreateWithFlags(&pc.ev, cudaEventDisableTiming));
   FGB_CUDA(cudaMemcpyAsync(pc.h, tot, sizeof(int) * (S + 1),
                            cudaMemcpyDeviceToHost, st));
-  FGB_CUDA(cudaEventRecord(pc.ev, st));
+  if (pc.ev) FGB_CUDA(cudaEventRecord(pc.ev, st));
   pending = true;
   return FGB_OK;
 }
@@ -415,7 +417,7 @@ int species_permutation_start(int S, fgb_workspace &ws, const int *d_species,
 int species_permutation_finish(int S, fgb_workspace &ws,
                                std::vector<int> &counts) {
   const fgb_pinned_counts &pc = ws.counts;
-  FGB_CUDA(cudaEventSynchronize(pc.ev));
+  if (pc.ev) FGB_CUDA(cudaEventSynchronize(pc.ev));
   if (pc.h[S]) {
     set_error("species must lie in [0, %d)", S);
     return FGB_EINVAL;
@@ -947,7 +949,109 @@ extern "C" int fgb_model_set_R_inv(fgb_model_t m, const double *h_R_inv) {
     FGB_CUDA(cudaMemcpy(m->RinvT.p, t.data(), sizeof(double) * (size_t)M * M,
                         cudaMemcpyHostToDevice));
   m->has_rinv = true;
+  m->oz64R_ready[0] = m->oz64R_ready[1] = false;
   return FGB_OK;
+}
+
+// out[o] = |row o of K^T T|^2 for K^T (ncol x M, sliced in kt) and the lower
+// triangular B operand (row-major, M x M; its slices kept in `B` per model).
+static int solved_variance(fgb_model_s *m, const oz::Sliced &kt,
+                           const oz::Sliced &B, long long ncol, DevBuf &part,
+                           double *out, cudaStream_t st) {
+  int rc;
+  const int slots = B.RP / 16;
+  if ((rc = part.ensure(sizeof(double) * ((size_t)ncol * slots + 1))) ||
+      (rc = oz::gemm_rowsq(kt, B, true, part.as<double>(),
+                           m->ws.ozerr.as<int>(), st)))
+    return rc;
+  k_sum_parts<<<ceil_div(ncol * kRowLanes, 128), 128, 0, st>>>(
+      (int)ncol, slots, part.as<double>(), out);
+  FGB_LAUNCH_CHECK("k_sum_parts");
+  return FGB_OK;
+}
+
+// The M x M lower-triangular matrix `src` of the model as a kS64-slice B
+// operand for products with ncol rows, sliced once per tile height.
+static int solved_operand(const DevBuf &src, int M, int v, oz::Sliced *out,
+                          bool *ready, cudaStream_t st) {
+  if (ready[v]) return FGB_OK;
+  const int rc = oz::slice({M, M, oz::kTN64v[v], src.as<double>(), M, nullptr,
+                            nullptr},
+                           out[v], st, oz::kS64);
+  if (rc == FGB_OK) ready[v] = true;
+  return rc;
+}
+
+// Mean and, with `dtc`, the DTC (else the SOR) variances of one structure.
+static int predict_solved(fgb_model_s *m, fgb_nlist_s *nl, const int *d_species,
+                          double *d_mean_efs, double *d_variance_efs, bool dtc,
+                          const char *what, cudaStream_t st) {
+  if (!m->solved || !m->has_rinv) {
+    set_error("L_inv must be up to date to make predictions. Please call "
+              "update_matrices_QR and try again.");
+    return FGB_ESTALE;
+  }
+  const int N = nl->n_atoms, M = m->M;
+  const long long ncol = 1 + 3LL * N + 6;
+  if (ncol > (1LL << 30)) { set_error("%s: structure too large", what); return FGB_EINVAL; }
+  int rc;
+  DevBuf kt(st), part(st), kself(st), q(st);
+  oz::Sliced kts(st);
+  if ((rc = kt.ensure(sizeof(double) * ((size_t)M * ncol + 1)))) return rc;
+  if (dtc && !m->lfull_ready && M > 0) {
+    if ((rc = m->Lfull.ensure(sizeof(double) * (size_t)M * M))) return rc;
+    FGB_CUDA(cudaMemcpy(m->Lfull.p, m->h_L_inv.data(),
+                        sizeof(double) * (size_t)M * M, cudaMemcpyHostToDevice));
+    m->lfull_ready = true;
+    m->oz64Lfull_ready[0] = m->oz64Lfull_ready[1] = false;
+  }
+  if ((rc = envs_struc_impl(m->b2, m->sigma, m->power, m->h_counts.data(),
+                            m->Sraw.as<double>(), nl, d_species,
+                            kt.as<double>(), m->ws, st)))
+    return rc;
+  if (dtc) {
+    // K_self from the descriptors and stored gradients envs_struc left in
+    // the workspace (it computes them only when M > 0 and N > 0)
+    if ((rc = kself.ensure(sizeof(double) * ncol)) ||
+        (rc = q.ensure(sizeof(double) * ncol)) ||
+        (rc = self_kernel_impl(m->b2, m->sigma, m->power, nl, d_species,
+                               kself.as<double>(), m->ws, st, M > 0)))
+      return rc;
+  }
+  if (M == 0) {
+    FGB_CUDA(cudaMemsetAsync(d_mean_efs, 0, sizeof(double) * ncol, st));
+    if (dtc)
+      FGB_CUDA(cudaMemcpyAsync(d_variance_efs, kself.p, sizeof(double) * ncol,
+                               cudaMemcpyDeviceToDevice, st));
+    else
+      FGB_CUDA(cudaMemsetAsync(d_variance_efs, 0, sizeof(double) * ncol, st));
+    FGB_CUDA(cudaStreamSynchronize(st));
+    return FGB_OK;
+  }
+  const int v = oz::tile64((int)ncol, M);
+  if ((rc = launch_kt_alpha(M, ncol, kt.as<double>(), m->alpha.as<double>(),
+                            d_mean_efs, st)) ||
+      (rc = oz::slice({(int)ncol, M, oz::kTM, kt.as<double>(), M, nullptr,
+                       nullptr},
+                      kts, st, oz::kS64)) ||
+      // diag(K^T Sigma K) = column sums of (R_inv^T K)^2, with the lower
+      // factor R_inv^T (sparse_gp.cpp:689-691, 724)
+      (rc = solved_operand(m->RinvT, M, v, m->oz64R, m->oz64R_ready, st)) ||
+      (rc = solved_variance(m, kts, m->oz64R[v], ncol, part, d_variance_efs,
+                            st)))
+    return rc;
+  if (dtc) {
+    // diag(K^T Kuu^-1 K) = column sums of (L_inv K)^2 (sparse_gp.cpp:723)
+    if ((rc = solved_operand(m->Lfull, M, v, m->oz64Lfull, m->oz64Lfull_ready,
+                             st)) ||
+        (rc = solved_variance(m, kts, m->oz64Lfull[v], ncol, part,
+                              q.as<double>(), st)))
+      return rc;
+    k_dtc_combine<<<ceil_div(ncol, 256), 256, 0, st>>>(
+        ncol, kself.as<double>(), q.as<double>(), d_variance_efs);
+    FGB_LAUNCH_CHECK("k_dtc_combine");
+  }
+  return sliced_finish(m->ws, st, what);
 }
 
 extern "C" int fgb_predict_sor(fgb_model_t m, fgb_nlist_t nl,
@@ -957,51 +1061,8 @@ extern "C" int fgb_predict_sor(fgb_model_t m, fgb_nlist_t nl,
     set_error("fgb_predict_sor: invalid arguments");
     return FGB_EINVAL;
   }
-  if (!m->solved || !m->has_rinv) {
-    set_error("L_inv must be up to date to make predictions. Please call "
-              "update_matrices_QR and try again.");
-    return FGB_ESTALE;
-  }
-  cudaStream_t st = (cudaStream_t)stream;
-  const int N = nl->n_atoms, M = m->M;
-  const long long ncol = 1 + 3LL * N + 6;
-  if (ncol > (1LL << 30)) { set_error("fgb_predict_sor: structure too large"); return FGB_EINVAL; }
-  int rc;
-  DevBuf kern, kt, part;
-  const int ntiles = ceil_div(M, BN);
-  if ((rc = kern.ensure(sizeof(double) * ((size_t)M * ncol + 1))) ||
-      (rc = kt.ensure(sizeof(double) * ((size_t)M * ncol + 1))) ||
-      (rc = part.ensure(sizeof(double) * ((size_t)ncol * ntiles + 1))))
-    return rc;
-  if ((rc = envs_struc_impl(m->b2, m->sigma, m->power, m->h_counts.data(),
-                            m->Sraw.as<double>(), nl, d_species,
-                            kern.as<double>(), m->ws, st)))
-    return rc;
-  if (M == 0) {
-    FGB_CUDA(cudaMemsetAsync(d_mean_efs, 0, sizeof(double) * ncol, st));
-    FGB_CUDA(cudaMemsetAsync(d_variance_efs, 0, sizeof(double) * ncol, st));
-    return FGB_OK;
-  }
-  k_transpose_rm<<<ceil_div((long long)M * ncol, 256), 256, 0, st>>>(
-      M, (int)ncol, kern.as<double>(), kt.as<double>());
-  FGB_LAUNCH_CHECK("k_transpose_rm");
-  k_kt_alpha<<<ceil_div(ncol, 128), 128, 0, st>>>(M, ncol, kt.as<double>(),
-                                                  m->alpha.as<double>(),
-                                                  d_mean_efs);
-  FGB_LAUNCH_CHECK("k_kt_alpha");
-  // V = K^T R_inv = K^T (R_inv^T)^T: the triangular NT GEMM with the lower
-  // factor R_inv^T; variance_efs = row sums of V^2 (sparse_gp.cpp:689-691).
-  dim3 g(ntiles, ceil_div(ncol, BM));
-  k_variance_gemm<<<g, GT, 0, st>>>((int)ncol, M, M, kt.as<double>(),
-                                    m->RinvT.as<double>(), part.as<double>(),
-                                    ntiles);
-  FGB_LAUNCH_CHECK("k_variance_gemm");
-  k_sum_parts<<<ceil_div(ncol, 128), 128, 0, st>>>((int)ncol, ntiles,
-                                                   part.as<double>(),
-                                                   d_variance_efs);
-  FGB_LAUNCH_CHECK("k_sum_parts");
-  FGB_CUDA(cudaStreamSynchronize(st));
-  return FGB_OK;
+  return predict_solved(m, nl, d_species, d_mean_efs, d_variance_efs, false,
+                        "fgb_predict_sor", (cudaStream_t)stream);
 }
 
 extern "C" int fgb_predict_dtc(fgb_model_t m, fgb_nlist_t nl,
@@ -1011,75 +1072,6 @@ extern "C" int fgb_predict_dtc(fgb_model_t m, fgb_nlist_t nl,
     set_error("fgb_predict_dtc: invalid arguments");
     return FGB_EINVAL;
   }
-  if (!m->solved || !m->has_rinv) {
-    set_error("L_inv must be up to date to make predictions. Please call "
-              "update_matrices_QR and try again.");
-    return FGB_ESTALE;
-  }
-  cudaStream_t st = (cudaStream_t)stream;
-  const int N = nl->n_atoms, M = m->M;
-  const long long ncol = 1 + 3LL * N + 6;
-  if (ncol > (1LL << 30)) { set_error("fgb_predict_dtc: structure too large"); return FGB_EINVAL; }
-  int rc;
-  if (!m->lfull_ready && M > 0) {
-    if ((rc = m->Lfull.ensure(sizeof(double) * (size_t)M * M))) return rc;
-    FGB_CUDA(cudaMemcpy(m->Lfull.p, m->h_L_inv.data(),
-                        sizeof(double) * (size_t)M * M, cudaMemcpyHostToDevice));
-    m->lfull_ready = true;
-  }
-  DevBuf kern, kt, part, kself, q;
-  const int ntiles = ceil_div(M, BN);
-  if ((rc = kern.ensure(sizeof(double) * ((size_t)M * ncol + 1))) ||
-      (rc = kt.ensure(sizeof(double) * ((size_t)M * ncol + 1))) ||
-      (rc = part.ensure(sizeof(double) * ((size_t)ncol * ntiles + 1))) ||
-      (rc = kself.ensure(sizeof(double) * ncol)) ||
-      (rc = q.ensure(sizeof(double) * ncol)))
-    return rc;
-  if ((rc = envs_struc_impl(m->b2, m->sigma, m->power, m->h_counts.data(),
-                            m->Sraw.as<double>(), nl, d_species,
-                            kern.as<double>(), m->ws, st)))
-    return rc;
-  // K_self from the descriptors and stored gradients envs_struc left in the
-  // workspace (envs_struc_impl computes them only when M > 0 and N > 0)
-  if ((rc = self_kernel_impl(m->b2, m->sigma, m->power, nl, d_species,
-                             kself.as<double>(), m->ws, st, M > 0)))
-    return rc;
-  if (M == 0) {
-    FGB_CUDA(cudaMemsetAsync(d_mean_efs, 0, sizeof(double) * ncol, st));
-    FGB_CUDA(cudaMemcpyAsync(d_variance_efs, kself.p, sizeof(double) * ncol,
-                             cudaMemcpyDeviceToDevice, st));
-    FGB_CUDA(cudaStreamSynchronize(st));
-    return FGB_OK;
-  }
-  k_transpose_rm<<<ceil_div((long long)M * ncol, 256), 256, 0, st>>>(
-      M, (int)ncol, kern.as<double>(), kt.as<double>());
-  FGB_LAUNCH_CHECK("k_transpose_rm");
-  k_kt_alpha<<<ceil_div(ncol, 128), 128, 0, st>>>(M, ncol, kt.as<double>(),
-                                                  m->alpha.as<double>(),
-                                                  d_mean_efs);
-  FGB_LAUNCH_CHECK("k_kt_alpha");
-  dim3 g(ntiles, ceil_div(ncol, BM));
-  // diag(K^T Kuu^-1 K) = column sums of (L_inv K)^2 (sparse_gp.cpp:723)
-  k_variance_gemm<<<g, GT, 0, st>>>((int)ncol, M, M, kt.as<double>(),
-                                    m->Lfull.as<double>(), part.as<double>(),
-                                    ntiles);
-  FGB_LAUNCH_CHECK("k_variance_gemm");
-  k_sum_parts<<<ceil_div(ncol, 128), 128, 0, st>>>((int)ncol, ntiles,
-                                                   part.as<double>(),
-                                                   q.as<double>());
-  FGB_LAUNCH_CHECK("k_sum_parts");
-  // diag(K^T Sigma K) = column sums of (R_inv^T K)^2 (sparse_gp.cpp:724)
-  k_variance_gemm<<<g, GT, 0, st>>>((int)ncol, M, M, kt.as<double>(),
-                                    m->RinvT.as<double>(), part.as<double>(),
-                                    ntiles);
-  FGB_LAUNCH_CHECK("k_variance_gemm");
-  k_sum_parts<<<ceil_div(ncol, 128), 128, 0, st>>>((int)ncol, ntiles,
-                                                   part.as<double>(),
-                                                   d_variance_efs);
-  FGB_LAUNCH_CHECK("k_sum_parts");
-  k_dtc_combine<<<ceil_div(ncol, 256), 256, 0, st>>>(
-      ncol, kself.as<double>(), q.as<double>(), d_variance_efs);
-  FGB_LAUNCH_CHECK("k_dtc_combine");
-  FGB_CUDA(cudaStreamSynchronize(st));
-  return FGB_OK;
+  return predict_solved(m, nl, d_species, d_mean_efs, d_variance_efs, true,
+                        "fgb_predict_dtc", (cudaStream_t)stream);
 }
