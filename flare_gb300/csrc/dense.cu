@@ -7,9 +7,9 @@
 // Matrices are row-major.  The O(M^3) work runs as FP64-level products on
 // the tensor cores (ozaki.cu: 9 exact BF16 slices, exact integer sums, one
 // rounding; about 35x this GPU's FP64 DGEMM rate); the O(M nb^2) work on
-// diagonal blocks of nb = 128 runs in shared memory, one CTA per block:
+// diagonal blocks of nb = 128 in shared memory:
 //   Cholesky, right-looking by block columns: factor the diagonal block
-//     and invert it (k_potrf_block), L21 = A21 L11^-T as a product with
+//     and invert it (k_potrf_cluster), L21 = A21 L11^-T as a product with
 //     that inverse, then the trailing update A22 -= L21 L21^T;
 //   lower-triangular inverse, recursive: X = [X11 0; X21 X22] with X11,
 //     X22 the inverses of the diagonal halves (leaves of nb inverted by
@@ -32,57 +32,227 @@ namespace {
 constexpr int kNB = 128;          // diagonal block
 constexpr int kBlockThreads = 512;
 
-// Cholesky of one kb x kb diagonal block (kb <= kNB) in shared memory,
-// lower factor written back over A (upper part zeroed), and its inverse
-// into X (ld kb; thread j owns column j, forward substitution).  A leading
-// minor that is not positive sets *info = first bad row + 1 (global index
-// base + j + 1) and the block stops.
-__global__ void __launch_bounds__(kBlockThreads)
-k_potrf_block(int kb, double *__restrict__ A, long long lda,
-              double *__restrict__ X, int base, int *__restrict__ info) {
-  extern __shared__ double sh[];   // kb x kb
-  __shared__ int bad;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
-  for (int idx = tid; idx < kb * kb; idx += nt) {
-    const int i = idx / kb, j = idx - i * kb;
-    sh[idx] = j <= i ? A[(long long)i * lda + j] : 0.0;
-  }
-  if (tid == 0) bad = 0;
+// ------------------------------------------------- diagonal block, cluster
+// Cholesky factor of a kb x kb diagonal block (kb <= kNB) and the factor's
+// inverse, by a cluster of kCl CTAs.  An SM makes two FP64 multiply-adds a
+// clock, so one CTA needs at least 180 us for the 700,000 of a 128-block
+// (and took 820 us, with three barriers a column and the inverse by one
+// thread a column); eight CTAs share them (CLUSTER_US us).  Blocked by kIB =
+// 32 columns:
+//   every CTA factors and inverts the 32 x 32 diagonal block for itself (the
+//     chain of 32 pivots; identical results, so no exchange), warps 0-3 with
+//     the columns k = w mod 4, lanes the rows, warps 4-7 the inverse's rows;
+//   the rows below, dealt out cyclically, become L21 = A21 X^T;
+//   their trailing updates need all of L21: through global memory (L2 loads)
+//     between cluster barriers.
+// The inverse's columns are then independent: each CTA solves for its own
+// (cyclic) by the 32 x 32 inverses and products with L, reading A from L2.
+// Pivots: y = 1/sqrt(d) from the FP32 estimate by one third-order step of
+// the Householder iteration y (1 + e/2 + 3 e^2/8), e = 1 - d y^2 (22 bits
+// become more than 60 before rounding); L_kk = d y, columns times y.
+constexpr int kIB = 32, kCl = 8, kClT = 256;
+constexpr int kLd = kIB + 1;
+// shared doubles: diagonal blocks L and X, the panel, own columns of X, own
+// rows staged, exchange vectors
+constexpr int kClSmem = (kNB / kIB) * kIB * kLd + kIB * kLd + kNB * kLd +
+                        kNB * (kNB / kCl + 1) + (kNB / kCl) * kLd + 5 * kIB;
+
+__device__ __forceinline__ void cluster_barrier() {
   __syncthreads();
-  for (int j = 0; j < kb; j++) {
-    const double d = sh[j * kb + j];
-    if (tid == 0 && !(d > 0.0)) {
-      bad = 1;
-      atomicCAS(info, 0, base + j + 1);
+  asm volatile("barrier.cluster.arrive.release;\n"
+               "barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void inverse_barrier() {   // warps 4-7
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+}
+__device__ __forceinline__ double rsqrt64(double d) {
+  int e2 = 0;
+  if (!(d > 1e-30 && d < 1e30)) {
+    // into the FP32 range by an even power of two
+    e2 = ((int)((__double_as_longlong(d) >> 52) & 0x7FF) - 1023) & ~1;
+    d = scalbn(d, -e2);
+  }
+  double y = (double)rsqrtf((float)d);
+  const double t = d * y, e = fma(-t, y, 1.0);
+  y = fma(y * e, fma(0.375, e, 0.5), y);
+  return e2 ? scalbn(y, -e2 / 2) : y;
+}
+
+// The jb x jb block D (ld kLd, lower) becomes its factor and X its inverse
+// (both lower, zero above); returns 0 or 1 + the first bad pivot.  Rows and
+// columns past jb are treated as the identity.
+__device__ int factor_block32(int jb, double *D, double *X, double *ex,
+                              int *flag) {
+  const int t = threadIdx.x, w = (t >> 5) & 3, lane = t & 31;
+  const bool inv = t >= 128;
+  // exchange vectors, two of each: the next step's are written while this
+  // step's are still read
+  double *const cols[2] = {ex, ex + kIB}, *const xrs[2] = {ex + 2 * kIB,
+                                                           ex + 3 * kIB};
+  double *const piv = ex + 4 * kIB;
+  // v[q]: factor warps: a[lane][4 q + w]; inverse warps: sum for row 4 q + w,
+  // column lane
+  double v[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) v[q] = inv ? 0.0 : D[lane * kLd + 4 * q + w];
+  if (t == 0) *flag = 0;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kIB; k++) {
+    const int own = k & 3, qk = k >> 2;
+    double *col = cols[k & 1], *xr = xrs[k & 1];
+    if (!inv && w == own) {
+      const double d = __shfl_sync(0xffffffffu, v[qk], k);
+      double y = 1.0;
+      if (d > 0.0) y = rsqrt64(d);
+      else if (lane == 0 && *flag == 0) *flag = k + 1;
+      const double l = lane == k ? d * y : v[qk] * y;
+      v[qk] = l;
+      col[lane] = lane >= k ? l : 0.0;
+      if (lane == 0) piv[k & 1] = y;
     }
     __syncthreads();
-    if (bad) break;
-    const double ljj = sqrt(d);
-    for (int i = j + 1 + tid; i < kb; i += nt) sh[i * kb + j] /= ljj;
-    __syncthreads();
-    if (tid == 0) sh[j * kb + j] = ljj;
-    for (int i = j + 1 + warp; i < kb; i += nw) {
-      const double lij = sh[i * kb + j];
-      for (int k = j + 1 + lane; k <= i; k += 32)
-        sh[i * kb + k] -= lij * sh[k * kb + j];
+    if (!inv) {
+      const double li = col[lane];
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (4 * q + w > k) v[q] = fma(-li, col[4 * q + w], v[q]);
+    } else {
+      if (w == own) {
+        const double x = piv[k & 1] * ((lane == k ? 1.0 : 0.0) - v[qk]);
+        v[qk] = x;
+        xr[lane] = x;
+      }
+      inverse_barrier();
+      const double x = xr[lane];
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (4 * q + w > k) v[q] = fma(col[4 * q + w], x, v[q]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const int c = 4 * q + w;
+    if (!inv) D[lane * kLd + c] = c <= lane ? v[q] : 0.0;
+    else X[c * kLd + lane] = lane <= c ? v[q] : 0.0;
+  }
+  __syncthreads();
+  return *flag && *flag <= jb ? *flag : 0;
+}
+
+__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClT)
+k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
+                double *__restrict__ X, long long ldx, int base,
+                int *__restrict__ info) {
+  extern __shared__ double sh[];
+  double *XD = sh;                                   // diagonal inverses
+  double *D = XD + (kNB / kIB) * kIB * kLd;
+  double *P = D + kIB * kLd;                         // panel rows, then L rows
+  double *C = P + kNB * kLd;                         // own columns of X
+  double *R = C + kNB * (kNB / kCl + 1);             // own rows of A21
+  double *ex = R + (kNB / kCl) * kLd;
+  __shared__ int flag;
+  const int t = threadIdx.x, rank = blockIdx.x % kCl;
+  for (int j0 = 0; j0 < kb; j0 += kIB) {
+    const int jb = min(kIB, kb - j0);
+    double *Xd = XD + (j0 / kIB) * kIB * kLd;
+    for (int e = t; e < kIB * kIB; e += kClT) {
+      const int i = e / kIB, j = e % kIB;
+      double x = i == j ? 1.0 : 0.0;
+      if (i < jb && j <= i) x = __ldcg(A + (long long)(j0 + i) * lda + j0 + j);
+      D[i * kLd + j] = x;
     }
     __syncthreads();
-  }
-  if (bad) return;
-  for (int idx = tid; idx < kb * kb; idx += nt) {
-    const int i = idx / kb, j = idx - i * kb;
-    A[(long long)i * lda + j] = j <= i ? sh[idx] : 0.0;
-  }
-  // X = L^-1: column j by forward substitution
-  for (int j = tid; j < kb; j += nt) {
-    for (int i = 0; i < j; i++) X[(long long)i * kb + j] = 0.0;
-    X[(long long)j * kb + j] = 1.0 / sh[j * kb + j];
-    for (int i = j + 1; i < kb; i++) {
+    const int bad = factor_block32(jb, D, Xd, ex, &flag);
+    if (bad) {   // the same in every CTA: all leave here
+      if (rank == 0 && t == 0) atomicCAS(info, 0, base + j0 + bad);
+      return;
+    }
+    // own rows of the panel: every kCl-th row below the block
+    const int r0 = j0 + kIB, m = kb - r0;
+    const int nown = m > rank ? (m - rank + kCl - 1) / kCl : 0;
+    for (int e = t; e < nown * kIB; e += kClT)
+      R[(e / kIB) * kLd + e % kIB] =
+          __ldcg(A + (long long)(r0 + rank + kCl * (e / kIB)) * lda + j0 + e % kIB);
+    // every CTA has read the diagonal block and this panel's rows are its
+    // own: after this barrier the factor may replace them
+    cluster_barrier();
+    if (rank == 0)
+      for (int e = t; e < kIB * kIB; e += kClT) {
+        const int i = e / kIB, j = e % kIB;
+        if (i < jb && j < jb)
+          A[(long long)(j0 + i) * lda + j0 + j] = D[i * kLd + j];
+      }
+    __syncthreads();
+    for (int e = t; e < nown * kIB; e += kClT) {
+      const int q = e / kIB, c = e % kIB;
       double s = 0.0;
-      for (int k = j; k < i; k++) s += sh[i * kb + k] * X[(long long)k * kb + j];
-      X[(long long)i * kb + j] = -s / sh[i * kb + i];
+      for (int k = 0; k <= c; k++) s = fma(R[q * kLd + k], Xd[c * kLd + k], s);
+      A[(long long)(r0 + rank + kCl * q) * lda + j0 + c] = s;
     }
+    if (m <= 0) break;
+    cluster_barrier();
+    for (int e = t; e < m * kIB; e += kClT)
+      P[(e / kIB) * kLd + e % kIB] =
+          __ldcg(A + (long long)(r0 + e / kIB) * lda + j0 + e % kIB);
+    __syncthreads();
+    for (int e = t; e < nown * m; e += kClT) {
+      const int q = e / m, c = e - q * m, i = rank + kCl * q;
+      if (c > i) continue;
+      double s = 0.0;
+#pragma unroll 8
+      for (int k = 0; k < kIB; k++) s = fma(P[i * kLd + k], P[c * kLd + k], s);
+      double *a = A + (long long)(r0 + i) * lda + r0 + c;
+      *a = __ldcg(a) - s;
+    }
+    cluster_barrier();
+  }
+  cluster_barrier();   // all of L is written
+  // columns c = rank mod kCl of X, 32 rows at a time; column slot s holds
+  // column rank + kCl s, four slots to a block of 32 columns
+  constexpr int kOwn = kNB / kCl, kCLd = kOwn + 1, kPerBlk = kIB / kCl;
+  for (int i0 = 0; i0 < kb; i0 += kIB) {
+    const int ib = i0 / kIB, rows = min(kIB, kb - i0);
+    const int act = kPerBlk * (ib + 1);      // columns with entries here
+    // S = E - sum_k L_ik X_k, 32 columns of L at a time
+    double s[2] = {0.0, 0.0};                // up to 512 outputs, 2 a thread
+    for (int k0 = 0; k0 < i0; k0 += kIB) {
+      __syncthreads();
+      for (int e = t; e < rows * kIB; e += kClT)
+        P[(e / kIB) * kLd + e % kIB] =
+            __ldcg(A + (long long)(i0 + e / kIB) * lda + k0 + e % kIB);
+      __syncthreads();
+#pragma unroll
+      for (int o = 0; o < 2; o++) {
+        const int e = t + o * kClT, r = e % kIB, c = e / kIB;
+        if (c < act && k0 / kIB >= c / kPerBlk && r < rows)
+#pragma unroll 8
+          for (int k = 0; k < kIB; k++)
+            s[o] = fma(P[r * kLd + k], C[(k0 + k) * kCLd + c], s[o]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < 2; o++) {   // S into the panel (rows x columns)
+      const int e = t + o * kClT, r = e % kIB, c = e / kIB;
+      if (c < act)
+        P[r * kLd + c] =
+            (c / kPerBlk == ib && rank + kCl * c == i0 + r ? 1.0 : 0.0) - s[o];
+    }
+    __syncthreads();
+    const double *Xd = XD + ib * kIB * kLd;
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+      const int e = t + o * kClT, r = e % kIB, c = e / kIB;
+      if (c >= kOwn || rank + kCl * c >= kb || r >= rows) continue;
+      double x = 0.0;
+      if (c < act)
+        for (int k = 0; k <= r; k++) x = fma(Xd[r * kLd + k], P[k * kLd + c], x);
+      C[(i0 + r) * kCLd + c] = x;
+      X[(long long)(i0 + r) * ldx + rank + kCl * c] = x;
+    }
+    __syncthreads();
   }
 }
 
@@ -110,6 +280,17 @@ k_trtri_block(int M, const double *__restrict__ L, long long ldl,
       for (int k = j; k < i; k++) s += sh[i * kb + k] * Xb[(long long)k * ldx + j];
       Xb[(long long)i * ldx + j] = -s / sh[i * kb + i];
     }
+  }
+}
+
+// The diagonal blocks of the M x M matrix X from D (nblk x kNB x kNB).
+__global__ void k_put_blocks(int M, const double *__restrict__ D,
+                             double *__restrict__ X, long long ldx) {
+  const int b0 = blockIdx.x * kNB, kb = min(kNB, M - b0);
+  const double *d = D + (size_t)blockIdx.x * kNB * kNB;
+  for (int i = threadIdx.x / kNB; i < kb; i += blockDim.x / kNB) {
+    const int j = threadIdx.x % kNB;
+    if (j < kb) X[(long long)(b0 + i) * ldx + b0 + j] = d[i * kNB + j];
   }
 }
 
@@ -156,7 +337,7 @@ __global__ void k_build_At(int M, int nl, const double *__restrict__ Kuf,
   if (c == 0) b[r] = r < nl ? sqrt(noise[r]) * y[r] : 0.0;
 }
 
-// Per-block partial sums of squares (fixed order), then one block adds them.
+// Per-block partial sums of squares (fixed order), then each block adds them.
 __global__ void k_sumsq_part(long long n, const double *__restrict__ x,
                              double *__restrict__ part) {
   __shared__ double red[256];
@@ -178,35 +359,52 @@ __global__ void k_sumsq_part(long long n, const double *__restrict__ x,
 __global__ void k_add_shift(int M, double *__restrict__ A, long long lda,
                             const double *__restrict__ part, int nparts,
                             double factor) {
-  __shared__ double tot;
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int k = 0; k < nparts; k++) t += part[k];
-    tot = t * factor;
-  }
+  __shared__ double red[256];
+  double v = 0.0;
+  for (int k = threadIdx.x; k < nparts; k += 256) v += part[k];
+  red[threadIdx.x] = v;
   __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncthreads();
+  }
+  const double tot = red[0] * factor;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M;
        i += gridDim.x * blockDim.x)
     A[(long long)i * lda + i] += tot;
 }
 
-// y[j] = sum_r Q[r][j] b[r] for Q (n x M, row-major): 32 columns per block
-// (lane = column), 8 row groups, fixed-order sums.
+// part[ch][j] = sum of Q[r][j] b[r] over the chunk's rows (Q n x M,
+// row-major): 32 columns per block (lane = column), 8 row groups, fixed-order
+// sums; k_gemv_t_final adds the chunks.
+constexpr int kGemvChunks = 32;
 __global__ void k_gemv_t(long long n, int M, const double *__restrict__ Q,
-                         const double *__restrict__ b, double *__restrict__ y) {
+                         const double *__restrict__ b,
+                         double *__restrict__ part) {
   __shared__ double red[8][33];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
+  const long long per = (n + kGemvChunks - 1) / kGemvChunks;
+  const long long r1 = min(n, (blockIdx.y + 1) * per);
   double s = 0.0;
   if (j < M)
-    for (long long r = g; r < n; r += 8) s += Q[r * M + j] * b[r];
+    for (long long r = blockIdx.y * per + g; r < r1; r += 8)
+      s += Q[r * M + j] * b[r];
   red[g][lane] = s;
   __syncthreads();
   if (g == 0 && j < M) {
     double t = 0.0;
     for (int k = 0; k < 8; k++) t += red[k][lane];
-    y[j] = t;
+    part[(long long)blockIdx.y * M + j] = t;
   }
+}
+__global__ void k_gemv_t_final(int M, const double *__restrict__ part,
+                               double *__restrict__ y) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= M) return;
+  double t = 0.0;
+  for (int k = 0; k < kGemvChunks; k++) t += part[(long long)k * M + j];
+  y[j] = t;
 }
 
 int transpose(int rows, int cols, const double *in, long long ldi, double *out,
@@ -220,32 +418,57 @@ int transpose(int rows, int cols, const double *in, long long ldi, double *out,
 
 // Scratch of one factorisation: slices of the two operands and the
 // tensor-core GEMM's time-out flag.
+// A factorisation's diagonal-block inverses (nblk x kNB x kNB) are kept
+// for the triangular inverse that follows; info[f] is factorisation f's
+// first bad pivot (1-based; 0: none).
+constexpr int kMaxFactors = 4;
 struct Work {
   oz::Sliced A, B;
-  DevBuf err, t1, t2;
+  DevBuf err, t1, t2, dinv, info;
+  explicit Work(cudaStream_t st)
+      : A(st), B(st), err(st), t1(st), t2(st), dinv(st), info(st) {}
+  int start(cudaStream_t st) {
+    int rc;
+    if ((rc = err.ensure(sizeof(int))) ||
+        (rc = info.ensure(sizeof(int) * kMaxFactors)))
+      return rc;
+    FGB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+    FGB_CUDA(cudaMemsetAsync(info.p, 0, sizeof(int) * kMaxFactors, st));
+    return FGB_OK;
+  }
 };
 
 // C (m x n, ldc) = a A B^T + b C with A (m x k, lda) and B (n x k, ldb) at
 // FP64 level on the tensor cores.
 int gemm_nt(int m, int n, int k, const double *A, long long lda,
             const double *B, long long ldb, double *C, long long ldc,
-            double a, double b, Work &w, cudaStream_t st) {
+            double a, double b, Work &w, cudaStream_t st, bool lower = false) {
   if (m == 0 || n == 0) return FGB_OK;
   int rc;
   if ((rc = oz::slice({m, k, oz::kTM, A, lda, nullptr, nullptr}, w.A, st)) ||
       (rc = oz::slice({n, k, oz::kTN, B, ldb, nullptr, nullptr}, w.B, st)))
     return rc;
-  return oz::gemm_axpby(w.A, w.B, C, ldc, a, b, w.err.as<int>(), st);
+  return oz::gemm_axpby(w.A, w.B, C, ldc, a, b, w.err.as<int>(), st, lower);
 }
 
+// Waits for the stream and reports the first factorisation that met a bad
+// pivot, then a product whose bounded wait ran out.
 int finish(Work &w, cudaStream_t st, const char *what) {
-  int h = 0;
+  int h = 0, info[kMaxFactors] = {};
   FGB_CUDA(cudaMemcpyAsync(&h, w.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  FGB_CUDA(cudaMemcpyAsync(info, w.info.p, sizeof(info), cudaMemcpyDeviceToHost,
+                           st));
   FGB_CUDA(cudaStreamSynchronize(st));
   if (h) {
     set_error("%s: a bounded device wait ran out", what);
     return FGB_ETIMEOUT;
   }
+  for (int f : info)
+    if (f) {
+      set_error("Cholesky of Kuu + jitter failed (leading minor %d not "
+                "positive definite)", f);
+      return FGB_EINVAL;
+    }
   return FGB_OK;
 }
 
@@ -284,56 +507,84 @@ int trtri_rec(int lo, int n, const double *L, long long ldl, double *X,
                  0.0, w, st);
 }
 
-}  // namespace
-
 // Lower Cholesky factor of the symmetric M x M matrix A (row-major; the
-// lower triangle is read), in place (strict upper part zeroed).
-int cholesky(int M, double *A, long long lda, cudaStream_t st) {
-  if (M == 0) return FGB_OK;
-  Work w;
-  DevBuf info, Tinv;
+// lower triangle is read), in place (strict upper part zeroed); the diagonal
+// blocks' inverses into w.dinv, a bad pivot into info[f].
+int factor(int M, double *A, long long lda, int f, Work &w, cudaStream_t st) {
   int rc;
-  if ((rc = w.err.ensure(sizeof(int))) || (rc = info.ensure(sizeof(int))) ||
-      (rc = Tinv.ensure(sizeof(double) * kNB * kNB)))
+  const int nblk = ceil_div(M, kNB);
+  if ((rc = w.dinv.ensure(sizeof(double) * (size_t)nblk * kNB * kNB)))
     return rc;
-  FGB_CUDA(cudaMemsetAsync(w.err.p, 0, sizeof(int), st));
-  FGB_CUDA(cudaMemsetAsync(info.p, 0, sizeof(int), st));
-  FGB_CUDA(cudaFuncSetAttribute(k_potrf_block,
+  constexpr int kSmem = (int)sizeof(double) * kClSmem;
+  FGB_CUDA(cudaFuncSetAttribute(k_potrf_cluster,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                smem_for(kNB)));
+                                kSmem));
   for (int k0 = 0; k0 < M; k0 += kNB) {
     const int kb = std::min(kNB, M - k0);
     double *A11 = A + (long long)k0 * lda + k0;
-    k_potrf_block<<<1, kBlockThreads, smem_for(kb), st>>>(
-        kb, A11, lda, Tinv.as<double>(), k0, info.as<int>());
-    FGB_LAUNCH_CHECK("k_potrf_block");
+    double *X = w.dinv.as<double>() + (size_t)(k0 / kNB) * kNB * kNB;
+    k_potrf_cluster<<<kCl, kClT, kSmem, st>>>(kb, A11, lda, X, kNB, k0,
+                                              w.info.as<int>() + f);
+    FGB_LAUNCH_CHECK("k_potrf_cluster");
     const int r = M - k0 - kb;
     if (r == 0) break;
     double *A21 = A + (long long)(k0 + kb) * lda + k0;
     double *A22 = A + (long long)(k0 + kb) * lda + k0 + kb;
-    // L21 = A21 L11^-T, in place (the product reads slices of A21)
-    if ((rc = gemm_nt(r, kb, kb, A21, lda, Tinv.as<double>(), kb, A21, lda,
-                      1.0, 0.0, w, st)))
-      return rc;
-    // A22 -= L21 L21^T (the whole square; the strict upper part is zeroed
-    // at the end)
-    if ((rc = gemm_nt(r, r, kb, A21, lda, A21, lda, A22, lda, -1.0, 1.0, w,
-                      st)))
+    // L21 = A21 L11^-T, in place (the product reads slices of A21), then
+    // A22 -= L21 L21^T (lower tiles)
+    if ((rc = gemm_nt(r, kb, kb, A21, lda, X, kNB, A21, lda, 1.0, 0.0, w,
+                      st)) ||
+        (rc = gemm_nt(r, r, kb, A21, lda, A21, lda, A22, lda, -1.0, 1.0, w,
+                      st, true)))
       return rc;
   }
   k_zero_strict_upper<<<ceil_div((long long)M * M, 256), 256, 0, st>>>(M, A,
                                                                        lda);
   FGB_LAUNCH_CHECK("k_zero_strict_upper");
-  int hinfo = 0;
-  FGB_CUDA(cudaMemcpyAsync(&hinfo, info.p, sizeof(int), cudaMemcpyDeviceToHost,
-                           st));
-  if ((rc = finish(w, st, "Cholesky"))) return rc;
-  if (hinfo) {
-    set_error("Cholesky of Kuu + jitter failed (leading minor %d not "
-              "positive definite)", hinfo);
-    return FGB_EINVAL;
-  }
   return FGB_OK;
+}
+
+// X = L^-1 of the factor just made (diagonal inverses from w.dinv) or, with
+// `own`, of any lower-triangular L; X's strict upper part zeroed.
+int invert(int M, const double *L, long long ldl, double *X, long long ldx,
+           bool own, Work &w, cudaStream_t st) {
+  k_zero_strict_upper<<<ceil_div((long long)M * M, 256), 256, 0, st>>>(M, X,
+                                                                       ldx);
+  FGB_LAUNCH_CHECK("k_zero_strict_upper");
+  if (own) {
+    FGB_CUDA(cudaFuncSetAttribute(k_trtri_block,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  smem_for(kNB)));
+    k_trtri_block<<<ceil_div(M, kNB), kBlockThreads,
+                    smem_for(std::min(M, kNB)), st>>>(M, L, ldl, X, ldx);
+    FGB_LAUNCH_CHECK("k_trtri_block");
+  } else {
+    k_put_blocks<<<ceil_div(M, kNB), 256, 0, st>>>(M, w.dinv.as<double>(), X,
+                                                   ldx);
+    FGB_LAUNCH_CHECK("k_put_blocks");
+  }
+  return trtri_rec(0, M, L, ldl, X, ldx, w, st);
+}
+
+}  // namespace
+
+// L = chol(A) in place and X = L^-1 (SparseGP's Kuu + jitter).
+int cholesky_inverse(int M, double *A, double *X, cudaStream_t st) {
+  if (M == 0) return FGB_OK;
+  Work w(st);
+  int rc;
+  if ((rc = w.start(st)) || (rc = factor(M, A, M, 0, w, st)) ||
+      (rc = invert(M, A, M, X, M, false, w, st)))
+    return rc;
+  return finish(w, st, "Cholesky");
+}
+
+int cholesky(int M, double *A, long long lda, cudaStream_t st) {
+  if (M == 0) return FGB_OK;
+  Work w(st);
+  int rc;
+  if ((rc = w.start(st)) || (rc = factor(M, A, lda, 0, w, st))) return rc;
+  return finish(w, st, "Cholesky");
 }
 
 // X = L^-1 for a lower-triangular M x M matrix L (row-major; X's strict
@@ -341,20 +592,10 @@ int cholesky(int M, double *A, long long lda, cudaStream_t st) {
 int trtri_lower(int M, const double *L, long long ldl, double *X,
                 long long ldx, cudaStream_t st) {
   if (M == 0) return FGB_OK;
-  Work w;
+  Work w(st);
   int rc;
-  if ((rc = w.err.ensure(sizeof(int)))) return rc;
-  FGB_CUDA(cudaMemsetAsync(w.err.p, 0, sizeof(int), st));
-  k_zero_strict_upper<<<ceil_div((long long)M * M, 256), 256, 0, st>>>(M, X,
-                                                                       ldx);
-  FGB_LAUNCH_CHECK("k_zero_strict_upper");
-  FGB_CUDA(cudaFuncSetAttribute(k_trtri_block,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                smem_for(kNB)));
-  k_trtri_block<<<ceil_div(M, kNB), kBlockThreads, smem_for(std::min(M, kNB)),
-                  st>>>(M, L, ldl, X, ldx);
-  FGB_LAUNCH_CHECK("k_trtri_block");
-  if ((rc = trtri_rec(0, M, L, ldl, X, ldx, w, st))) return rc;
+  if ((rc = w.start(st)) || (rc = invert(M, L, ldl, X, ldx, true, w, st)))
+    return rc;
   return finish(w, st, "triangular inverse");
 }
 
@@ -363,11 +604,10 @@ int trtri_lower(int M, const double *L, long long ldl, double *X,
 int sym_product(int M, const double *A, bool transpose_first, double *C,
                 cudaStream_t st) {
   if (M == 0) return FGB_OK;
-  Work w;
-  DevBuf At;
+  Work w(st);
+  DevBuf At(st);
   int rc;
-  if ((rc = w.err.ensure(sizeof(int)))) return rc;
-  FGB_CUDA(cudaMemsetAsync(w.err.p, 0, sizeof(int), st));
+  if ((rc = w.start(st))) return rc;
   const double *op = A;
   if (transpose_first) {
     if ((rc = At.ensure(sizeof(double) * (size_t)M * M))) return rc;
@@ -391,20 +631,20 @@ int sym_product(int M, const double *A, bool transpose_first, double *C,
 // read; b has n entries.
 int cholqr_solve(int M, long long n, double *At, const double *b,
                  double *R_inv, double *Qtb, cudaStream_t st) {
-  Work w;
-  DevBuf G, X[3], A0, Q, Qt, part, P;
+  Work w(st);
+  DevBuf G(st), X[3] = {DevBuf(st), DevBuf(st), DevBuf(st)}, A0(st), Q(st),
+         Qt(st), part(st), P(st);
   int rc;
   const size_t MM = (size_t)M * M, nM = (size_t)n * M;
-  if ((rc = w.err.ensure(sizeof(int))) || (rc = G.ensure(sizeof(double) * MM)) ||
+  if ((rc = w.start(st)) || (rc = G.ensure(sizeof(double) * MM)) ||
       (rc = X[0].ensure(sizeof(double) * MM)) ||
       (rc = X[1].ensure(sizeof(double) * MM)) ||
       (rc = X[2].ensure(sizeof(double) * MM)) ||
       (rc = P.ensure(sizeof(double) * MM)) ||
       (rc = A0.ensure(sizeof(double) * nM)) ||
       (rc = Q.ensure(sizeof(double) * nM)) ||
-      (rc = part.ensure(sizeof(double) * 1024)))
+      (rc = part.ensure(sizeof(double) * std::max(1024, kGemvChunks * M))))
     return rc;
-  FGB_CUDA(cudaMemsetAsync(w.err.p, 0, sizeof(int), st));
   if (n > (long long)INT32_MAX) {
     set_error("update_matrices_QR: %lld rows exceed the product kernels' "
               "limit", n);
@@ -419,7 +659,7 @@ int cholqr_solve(int M, long long n, double *At, const double *b,
   const double *Tprev = At;   // Q_prev^T (M x n)
   for (int pass = 0; pass < 3; pass++) {
     if ((rc = gemm_nt(M, M, ni, Tprev, n, Tprev, n, G.as<double>(), M, 1.0,
-                      0.0, w, st)))
+                      0.0, w, st, true)))
       return rc;
     if (pass == 0) {
       const int nparts = 1024;
@@ -430,8 +670,9 @@ int cholqr_solve(int M, long long n, double *At, const double *b,
           M, G.as<double>(), M, part.as<double>(), nparts, shift);
       FGB_LAUNCH_CHECK("k_add_shift");
     }
-    if ((rc = cholesky(M, G.as<double>(), M, st)) ||
-        (rc = trtri_lower(M, G.as<double>(), M, X[pass].as<double>(), M, st)))
+    if ((rc = factor(M, G.as<double>(), M, pass, w, st)) ||
+        (rc = invert(M, G.as<double>(), M, X[pass].as<double>(), M, false, w,
+                     st)))
       return rc;
     // Q_pass = Q_prev R_pass^-1 = Q_prev X_pass^T (X = L^-1, R = L^T)
     if ((rc = gemm_nt(ni, M, M, Qprev, M, X[pass].as<double>(), M,
@@ -447,8 +688,11 @@ int cholqr_solve(int M, long long n, double *At, const double *b,
     }
   }
   // Q^T b with the final Q
-  k_gemv_t<<<ceil_div(M, 32), 256, 0, st>>>(n, M, Q.as<double>(), b, Qtb);
+  k_gemv_t<<<dim3(ceil_div(M, 32), kGemvChunks), 256, 0, st>>>(
+      n, M, Q.as<double>(), b, part.as<double>());
   FGB_LAUNCH_CHECK("k_gemv_t");
+  k_gemv_t_final<<<ceil_div(M, 256), 256, 0, st>>>(M, part.as<double>(), Qtb);
+  FGB_LAUNCH_CHECK("k_gemv_t_final");
   // R^-1 = R0^-1 R1^-1 R2^-1 = (X2 X1 X0)^T
   double *T1 = G.as<double>();
   if ((rc = transpose(M, M, X[1].as<double>(), M, T1, M, st)) ||

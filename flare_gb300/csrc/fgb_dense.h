@@ -7,6 +7,8 @@ namespace dense {
 // Lower Cholesky factor of a symmetric M x M row-major matrix, in place
 // (strict upper part zeroed); FGB_EINVAL if not positive definite.
 int cholesky(int M, double *A, long long lda, cudaStream_t st);
+// L = chol(A) in place, as above, and X = L^-1 (strict upper zeroed).
+int cholesky_inverse(int M, double *A, double *X, cudaStream_t st);
 // X = L^-1 for a lower-triangular M x M row-major L (strict upper of X
 // zeroed); L and X distinct.
 int trtri_lower(int M, const double *L, long long ldl, double *X,

@@ -105,8 +105,10 @@ int gemm_store(const Sliced &A, const Sliced &B, double *C, long long ldc,
                int *err, cudaStream_t st);
 // C = a (A B^T) + b C in FP64 from kS-slice operands (b = 0: C is only
 // written), the same exact integer sums and one rounding of the product.
+// lower: only C's lower triangle is wanted (tiles above it are skipped).
 int gemm_axpby(const Sliced &A, const Sliced &B, double *C, long long ldc,
-               double a, double b, int *err, cudaStream_t st);
+               double a, double b, int *err, cudaStream_t st,
+               bool lower = false);
 // B tile height (index into kTN64v) of a kS64-slice product.
 int tile64(int rows, int cols);
 // Products of kS64-slice operands (B tiles of kTN64v rows) for the

@@ -497,6 +497,13 @@ __global__ void k_wait_expiry(long long limit, int *__restrict__ err,
   __syncthreads();
 }
 
+// Column tiles of row tile mt with a column at or left of its last row.
+template <int TN>
+__host__ __device__ constexpr int lower_tiles(int mt, int NTt) {
+  const int w = ((mt + 1) * kTM - 1) / TN + 1;
+  return w < NTt ? w : NTt;
+}
+
 // Persistent, warp-specialised GEMM: one CTA per SM walks the tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ... (B tiles fastest).
 //   warp 0, lane 0  streams chunks into the shared-memory ring: a stage is
@@ -528,8 +535,8 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
           int SA, const __nv_bfloat16 *__restrict__ Asl,
           const double *__restrict__ Ascale,
           const __nv_bfloat16 *__restrict__ Bsl,
-          const double *__restrict__ Bscale, int tri, Epi epi,
-          int *__restrict__ err) {
+          const double *__restrict__ Bscale, int tri, int lower, int ntiles,
+          Epi epi, int *__restrict__ err) {
   constexpr int S = C::S, TN = C::TN, NST = C::STAGES, NCH = C::WCOLS / 16;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t *bar_load = reinterpret_cast<uint64_t *>(smem + NST * C::Stage);
@@ -541,7 +548,6 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
   long long *issued = reinterpret_cast<long long *>(tmem_slot + 2);
   long long *consumed = issued + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ntiles = MT * NTt;
   const int KCH = KP / kKC;
 
   if (warp == 0) {
@@ -571,7 +577,15 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
   // operand in L2), with the column order rotated by the row tile: a
   // persistent CTA's tiles t, t + grid, ... then visit every column tile
   // instead of a few (with a triangular B the column tiles differ in cost).
+  // lower: only the tiles that reach the diagonal or lie below it (row tile
+  // mt has lower_tiles(mt) of them).
   auto tile_rc = [&](int t, int &mt, int &nt) {
+    if (lower) {
+      mt = 0;
+      for (int w; t >= (w = lower_tiles<TN>(mt, NTt)); t -= w) mt++;
+      nt = t;
+      return;
+    }
     mt = fdiv(t, divNT);
     const int rot = mt - fdiv(mt, divNT) * NTt;
     nt = t - mt * NTt + rot;
@@ -911,7 +925,7 @@ int slice(const SliceSpec &sp, Sliced &out, cudaStream_t st, int S) {
 
 template <class C, class Epi>
 static int gemm_c(const Sliced &A, const Sliced &B, bool tri, const Epi &epi,
-                  int *err, cudaStream_t st) {
+                  int *err, cudaStream_t st, bool lower = false) {
   // A may carry more (less significant) slices than the product uses
   if (A.K != B.K || A.KP != B.KP || A.TR != kTM || B.TR != C::TN ||
       A.S < C::S || B.S != C::S) {
@@ -926,12 +940,17 @@ static int gemm_c(const Sliced &A, const Sliced &B, bool tri, const Epi &epi,
   FGB_CUDA(cudaGetDevice(&dev));
   FGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int MT = A.RP / kTM, NTt = B.RP / C::TN;
-  const int grid = std::max(1, std::min(MT * NTt, sms));
+  int ntiles = MT * NTt;
+  if (lower) {
+    ntiles = 0;
+    for (int mt = 0; mt < MT; mt++) ntiles += lower_tiles<C::TN>(mt, NTt);
+  }
+  const int grid = std::max(1, std::min(ntiles, sms));
   k_oz_gemm<C, Epi><<<grid, C::THREADS, C::Smem, st>>>(
       A.rows, B.rows, A.K, A.KP, MT, NTt, make_fastdiv(NTt), A.S,
       A.q.as<__nv_bfloat16>(),
       A.scale.as<double>(), B.q.as<__nv_bfloat16>(), B.scale.as<double>(),
-      tri ? 1 : 0, epi, err);
+      tri ? 1 : 0, lower ? 1 : 0, ntiles, epi, err);
   FGB_LAUNCH_CHECK("k_oz_gemm");
   return FGB_OK;
 }
@@ -957,8 +976,10 @@ int gemm_store(const Sliced &A, const Sliced &B, double *C, long long ldc,
 }
 
 int gemm_axpby(const Sliced &A, const Sliced &B, double *C, long long ldc,
-               double a, double b, int *err, cudaStream_t st) {
-  return gemm(A, B, false, EpiAxpby{C, ldc, B.rows, a, b}, err, st);
+               double a, double b, int *err, cudaStream_t st, bool lower) {
+  const EpiAxpby epi{C, ldc, B.rows, a, b};
+  if (B.TR == 32) return gemm_c<CfgF64n>(A, B, false, epi, err, st, lower);
+  return gemm_c<CfgF64>(A, B, false, epi, err, st, lower);
 }
 
 int gemm_f32(const Sliced &A, const Sliced &B, float *Y, long long ldy,

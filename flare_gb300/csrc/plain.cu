@@ -846,7 +846,7 @@ extern "C" int fgb_solve_qr(int M, int n_labels, const double *d_Kuu,
   cudaStream_t st = (cudaStream_t)stream;
   const long long rows = (long long)n_labels + M;
   int rc = FGB_OK;
-  DevBuf L, At, b, Qtb, Rinv;
+  DevBuf L(st), At(st), b(st), Qtb(st), Rinv(st);
   double *R_inv = d_R_inv;
   if ((rc = L.ensure(sizeof(double) * (size_t)M * M)) ||
       (rc = At.ensure(sizeof(double) * (size_t)rows * M)) ||
@@ -861,8 +861,7 @@ extern "C" int fgb_solve_qr(int M, int n_labels, const double *d_Kuu,
                            cudaMemcpyDeviceToDevice, st));
   k_add_diag<<<ceil_div(M, 256), 256, 0, st>>>(M, L.as<double>(), jitter);
   FGB_LAUNCH_CHECK("k_add_diag");
-  if ((rc = dense::cholesky(M, L.as<double>(), M, st)) ||
-      (rc = dense::trtri_lower(M, L.as<double>(), M, d_L_inv, M, st)) ||
+  if ((rc = dense::cholesky_inverse(M, L.as<double>(), d_L_inv, st)) ||
       (rc = dense::build_At(M, n_labels, d_Kuf, d_noise, d_y, L.as<double>(),
                             At.as<double>(), b.as<double>(), st)) ||
       (rc = dense::cholqr_solve(M, rows, At.as<double>(), b.as<double>(),
