@@ -34,10 +34,11 @@ constexpr int kBlockThreads = 512;
 
 // ------------------------------------------------- diagonal block, cluster
 // Cholesky factor of a kb x kb diagonal block (kb <= kNB) and the factor's
-// inverse, by a cluster of kCl CTAs.  An SM makes two FP64 multiply-adds a
+// inverse, by a cluster of kCl = 16 CTAs.  An SM makes two FP64 multiply-adds a
 // clock, so one CTA needs at least 180 us for the 700,000 of a 128-block
 // (and took 820 us, with three barriers a column and the inverse by one
-// thread a column); eight CTAs share them (CLUSTER_US us).  Blocked by kIB =
+// thread a column); sixteen CTAs share them in 124 us (eight: 164), of
+// which the four pivot chains below are 80.  Blocked by kIB =
 // 32 columns:
 //   every CTA factors and inverts the 32 x 32 diagonal block for itself (the
 //     chain of 32 pivots; identical results, so no exchange), warps 0-3 with
@@ -47,35 +48,95 @@ constexpr int kBlockThreads = 512;
 //     between cluster barriers.
 // The inverse's columns are then independent: each CTA solves for its own
 // (cyclic) by the 32 x 32 inverses and products with L, reading A from L2.
-// Pivots: y = 1/sqrt(d) from the FP32 estimate by one third-order step of
-// the Householder iteration y (1 + e/2 + 3 e^2/8), e = 1 - d y^2 (22 bits
-// become more than 60 before rounding); L_kk = d y, columns times y.
-constexpr int kIB = 32, kCl = 8, kClT = 256;
+// Pivots: y = 1/sqrt(d) from the hardware's estimate (about 20 bits) by one
+// third-order step of the Householder iteration y (1 + e/2 + 3 e^2/8), e = 1
+// - d y^2; L_kk = d y, columns times y.
+constexpr int kIB = 32, kCl = 16, kClT = 256;
 constexpr int kLd = kIB + 1;
 // shared doubles: diagonal blocks L and X, the panel, own columns of X, own
 // rows staged, exchange vectors
 constexpr int kClSmem = (kNB / kIB) * kIB * kLd + kIB * kLd + kNB * kLd +
-                        kNB * (kNB / kCl + 1) + (kNB / kCl) * kLd + 5 * kIB;
+                        kNB * (kNB / kCl + 1) + (kNB / kCl) * kLd + 6 * kIB + 4;
 
 __device__ __forceinline__ void cluster_barrier() {
   __syncthreads();
   asm volatile("barrier.cluster.arrive.release;\n"
                "barrier.cluster.wait.acquire;" ::: "memory");
 }
-__device__ __forceinline__ void inverse_barrier() {   // warps 4-7
-  asm volatile("bar.sync 1, 128;" ::: "memory");
+template <int ID, int N>
+__device__ __forceinline__ void bar_sync() {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+template <int ID, int N>
+__device__ __forceinline__ void bar_arrive() {
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
 }
 __device__ __forceinline__ double rsqrt64(double d) {
-  int e2 = 0;
-  if (!(d > 1e-30 && d < 1e30)) {
-    // into the FP32 range by an even power of two
-    e2 = ((int)((__double_as_longlong(d) >> 52) & 0x7FF) - 1023) & ~1;
-    d = scalbn(d, -e2);
-  }
-  double y = (double)rsqrtf((float)d);
+  if (!(d > 1e-290 && d < 1e290)) return rsqrt(d);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double t = d * y, e = fma(-t, y, 1.0);
-  y = fma(y * e, fma(0.375, e, 0.5), y);
-  return e2 ? scalbn(y, -e2 / 2) : y;
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// Column k of the factor from its updated values v (a lane per row): scaled
+// by the pivot's 1/sqrt, written to col, the pivot's y to *piv.
+__device__ __forceinline__ double pivot_column(int k, double v, double *col,
+                                               double *piv, int *flag) {
+  const int lane = threadIdx.x & 31;
+  const double d = __shfl_sync(0xffffffffu, v, k);
+  double y = 1.0;
+  if (d > 0.0) y = rsqrt64(d);
+  else if (lane == 0 && *flag == 0) *flag = k + 1;
+  const double l = lane == k ? d * y : v * y;
+  col[lane] = lane >= k ? l : 0.0;
+  if (lane == 0) *piv = y;
+  return l;
+}
+
+// The step of column K in factor_block32 (a template, so that the barrier
+// ids are constants).  Column K + 1's warp brings that column up to date
+// first, writes it and only arrives at the barrier that its readers wait at:
+// its other updates follow while they go on.  Chain of a step: one update,
+// the pivot (5 dependent FP64 instructions), the exchange.
+template <int K>
+__device__ __forceinline__ void factor_step(double (&v)[8], double *ex,
+                                            int *flag) {
+  const int t = threadIdx.x, w = (t >> 5) & 3, lane = t & 31;
+  const bool inv = t >= 128;
+  // four exchange columns in turn: a buffer is rewritten four steps on, after
+  // a barrier that every reader has passed
+  double *col = ex + (K & 3) * kIB, *piv = ex + 6 * kIB;
+  constexpr int own = K & 3;
+  if (inv || w != own) bar_sync<1 + (K & 3), kClT>();
+  if (!inv) {
+    const double li = col[lane];
+    constexpr int n1 = K + 1, o1 = n1 & 3, q1 = n1 >> 2;
+    if (n1 < kIB && w == o1) {
+      v[q1 & 7] = fma(-li, col[n1 & 31], v[q1 & 7]);
+      v[q1 & 7] = pivot_column(n1, v[q1 & 7], ex + o1 * kIB, piv + o1, flag);
+      bar_arrive<1 + o1, kClT>();
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (4 * q + w > K && !(w == o1 && q == q1))
+        v[q] = fma(-li, col[4 * q + w], v[q]);
+  } else {
+    double *xr = ex + (4 + (K & 1)) * kIB;
+    constexpr int qk = K >> 2;
+    if (w == own) {
+      const double x = piv[own] * ((lane == K ? 1.0 : 0.0) - v[qk]);
+      v[qk] = x;
+      xr[lane] = x;
+    }
+    bar_sync<5, 128>();
+    const double x = xr[lane];
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (4 * q + w > K) v[q] = fma(col[4 * q + w], x, v[q]);
+  }
+  if constexpr (K + 1 < kIB) factor_step<K + 1>(v, ex, flag);
 }
 
 // The jb x jb block D (ld kLd, lower) becomes its factor and X its inverse
@@ -85,11 +146,6 @@ __device__ int factor_block32(int jb, double *D, double *X, double *ex,
                               int *flag) {
   const int t = threadIdx.x, w = (t >> 5) & 3, lane = t & 31;
   const bool inv = t >= 128;
-  // exchange vectors, two of each: the next step's are written while this
-  // step's are still read
-  double *const cols[2] = {ex, ex + kIB}, *const xrs[2] = {ex + 2 * kIB,
-                                                           ex + 3 * kIB};
-  double *const piv = ex + 4 * kIB;
   // v[q]: factor warps: a[lane][4 q + w]; inverse warps: sum for row 4 q + w,
   // column lane
   double v[8];
@@ -97,39 +153,11 @@ __device__ int factor_block32(int jb, double *D, double *X, double *ex,
   for (int q = 0; q < 8; q++) v[q] = inv ? 0.0 : D[lane * kLd + 4 * q + w];
   if (t == 0) *flag = 0;
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kIB; k++) {
-    const int own = k & 3, qk = k >> 2;
-    double *col = cols[k & 1], *xr = xrs[k & 1];
-    if (!inv && w == own) {
-      const double d = __shfl_sync(0xffffffffu, v[qk], k);
-      double y = 1.0;
-      if (d > 0.0) y = rsqrt64(d);
-      else if (lane == 0 && *flag == 0) *flag = k + 1;
-      const double l = lane == k ? d * y : v[qk] * y;
-      v[qk] = l;
-      col[lane] = lane >= k ? l : 0.0;
-      if (lane == 0) piv[k & 1] = y;
-    }
-    __syncthreads();
-    if (!inv) {
-      const double li = col[lane];
-#pragma unroll
-      for (int q = 0; q < 8; q++)
-        if (4 * q + w > k) v[q] = fma(-li, col[4 * q + w], v[q]);
-    } else {
-      if (w == own) {
-        const double x = piv[k & 1] * ((lane == k ? 1.0 : 0.0) - v[qk]);
-        v[qk] = x;
-        xr[lane] = x;
-      }
-      inverse_barrier();
-      const double x = xr[lane];
-#pragma unroll
-      for (int q = 0; q < 8; q++)
-        if (4 * q + w > k) v[q] = fma(col[4 * q + w], x, v[q]);
-    }
+  if (!inv && w == 0) {
+    v[0] = pivot_column(0, v[0], ex, ex + 6 * kIB, flag);
+    bar_arrive<1, kClT>();
   }
+  factor_step<0>(v, ex, flag);
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 8; q++) {
@@ -197,14 +225,15 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
       P[(e / kIB) * kLd + e % kIB] =
           __ldcg(A + (long long)(r0 + e / kIB) * lda + j0 + e % kIB);
     __syncthreads();
-    for (int e = t; e < nown * m; e += kClT) {
-      const int q = e / m, c = e - q * m, i = rank + kCl * q;
-      if (c > i) continue;
-      double s = 0.0;
+    for (int q = t >> 5; q < nown; q += kClT / 32) {   // a warp per row
+      const int i = rank + kCl * q;
+      for (int c = t & 31; c <= i; c += 32) {
+        double s = 0.0;
 #pragma unroll 8
-      for (int k = 0; k < kIB; k++) s = fma(P[i * kLd + k], P[c * kLd + k], s);
-      double *a = A + (long long)(r0 + i) * lda + r0 + c;
-      *a = __ldcg(a) - s;
+        for (int k = 0; k < kIB; k++) s = fma(P[i * kLd + k], P[c * kLd + k], s);
+        double *a = A + (long long)(r0 + i) * lda + r0 + c;
+        *a = __ldcg(a) - s;
+      }
     }
     cluster_barrier();
   }
@@ -216,7 +245,8 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
     const int ib = i0 / kIB, rows = min(kIB, kb - i0);
     const int act = kPerBlk * (ib + 1);      // columns with entries here
     // S = E - sum_k L_ik X_k, 32 columns of L at a time
-    double s[2] = {0.0, 0.0};                // up to 512 outputs, 2 a thread
+    constexpr int kOut = kIB * kOwn / kClT;  // outputs a thread
+    double s[kOut] = {};
     for (int k0 = 0; k0 < i0; k0 += kIB) {
       __syncthreads();
       for (int e = t; e < rows * kIB; e += kClT)
@@ -224,7 +254,7 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
             __ldcg(A + (long long)(i0 + e / kIB) * lda + k0 + e % kIB);
       __syncthreads();
 #pragma unroll
-      for (int o = 0; o < 2; o++) {
+      for (int o = 0; o < kOut; o++) {
         const int e = t + o * kClT, r = e % kIB, c = e / kIB;
         if (c < act && k0 / kIB >= c / kPerBlk && r < rows)
 #pragma unroll 8
@@ -234,7 +264,7 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
     }
     __syncthreads();
 #pragma unroll
-    for (int o = 0; o < 2; o++) {   // S into the panel (rows x columns)
+    for (int o = 0; o < kOut; o++) {   // S into the panel (rows x columns)
       const int e = t + o * kClT, r = e % kIB, c = e / kIB;
       if (c < act)
         P[r * kLd + c] =
@@ -243,7 +273,7 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
     __syncthreads();
     const double *Xd = XD + ib * kIB * kLd;
 #pragma unroll
-    for (int o = 0; o < 2; o++) {
+    for (int o = 0; o < kOut; o++) {
       const int e = t + o * kClT, r = e % kIB, c = e / kIB;
       if (c >= kOwn || rank + kCl * c >= kb || r >= rows) continue;
       double x = 0.0;
@@ -446,7 +476,8 @@ int gemm_nt(int m, int n, int k, const double *A, long long lda,
   if (m == 0 || n == 0) return FGB_OK;
   int rc;
   if ((rc = oz::slice({m, k, oz::kTM, A, lda, nullptr, nullptr}, w.A, st)) ||
-      (rc = oz::slice({n, k, oz::kTN, B, ldb, nullptr, nullptr}, w.B, st)))
+      (rc = oz::slice({n, k, oz::kTN64v[oz::tile64(m, n)], B, ldb, nullptr,
+                       nullptr}, w.B, st)))
     return rc;
   return oz::gemm_axpby(w.A, w.B, C, ldc, a, b, w.err.as<int>(), st, lower);
 }
@@ -519,6 +550,9 @@ int factor(int M, double *A, long long lda, int f, Work &w, cudaStream_t st) {
   FGB_CUDA(cudaFuncSetAttribute(k_potrf_cluster,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSmem));
+  FGB_CUDA(cudaFuncSetAttribute(k_potrf_cluster,
+                                cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                1));
   for (int k0 = 0; k0 < M; k0 += kNB) {
     const int kb = std::min(kNB, M - k0);
     double *A11 = A + (long long)k0 * lda + k0;

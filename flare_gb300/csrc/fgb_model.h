@@ -38,7 +38,7 @@ struct fgb_workspace {
   // stored-gradient form: pairs grouped by species, basis values, gradients,
   // cosines, force kernel, sparse norms and slices
   fgb::DevBuf start, rows, basis, dB2, fdots, dots, kern, snorm;
-  fgb::oz::Sliced ozSp[2];
+  fgb::oz::Sliced ozSp[fgb::oz::kTiles64];
   // tensor-core paths: sliced rows, kernel matrix and (FP64 path) adjoint
   // weights of one row chunk
   fgb::oz::Sliced ozA, ozK, ozW;
@@ -50,9 +50,12 @@ struct fgb_workspace {
     for (fgb::DevBuf *b :
          {&perm, &flags, &pos, &scal, &flag, &A, &B2, &norms, &rowmax, &part,
           &start, &rows, &basis, &dB2, &fdots, &dots, &kern, &snorm, &ozerr,
-          &ozA.q, &ozA.scale, &ozK.q, &ozK.scale, &ozSp[0].q, &ozSp[0].scale,
-          &ozSp[1].q, &ozSp[1].scale})
+          &ozA.q, &ozA.scale, &ozK.q, &ozK.scale})
       b->on(st);
+    for (fgb::oz::Sliced &s : ozSp) {
+      s.q.on(st);
+      s.scale.on(st);
+    }
   }
 };
 
@@ -81,8 +84,9 @@ struct fgb_model_s {
   fgb::DevBuf Lfull;    // L_inv (M x M, lower triangular) for DTC, on demand
   bool lfull_ready = false;
   // R_inv^T and L_inv as kS64-slice B operands (SOR and DTC variances)
-  fgb::oz::Sliced oz64R[2], oz64Lfull[2];
-  bool oz64R_ready[2] = {}, oz64Lfull_ready[2] = {};
+  fgb::oz::Sliced oz64R[fgb::oz::kTiles64], oz64Lfull[fgb::oz::kTiles64];
+  bool oz64R_ready[fgb::oz::kTiles64] = {},
+       oz64Lfull_ready[fgb::oz::kTiles64] = {};
   fgb::DevBuf Bmap;     // mixed path: per species n_d x n_d FP32 folded matrix
   fgb::DevBuf Bfold;    // the folded matrices in FP64 (power 2), per species
   // the folded matrices in FP32-level slices (tensor-core force GEMM), one
@@ -110,8 +114,10 @@ struct fgb_model_s {
   // panels at kS64 slices, one set per B tile height (kTN64v), sliced the
   // first time each runs; largest |alpha| per species (the adjoint weights'
   // fixed scale); whether descriptors, alpha and L_inv are all finite
-  std::vector<std::unique_ptr<fgb::oz::Sliced>> oz64S[2], oz64ST[2], oz64L[2];
-  bool oz64S_ready[2] = {}, oz64ST_ready[2] = {}, oz64L_ready[2] = {};
+  std::vector<std::unique_ptr<fgb::oz::Sliced>> oz64S[fgb::oz::kTiles64],
+      oz64ST[fgb::oz::kTiles64], oz64L[fgb::oz::kTiles64];
+  bool oz64S_ready[fgb::oz::kTiles64] = {},
+       oz64ST_ready[fgb::oz::kTiles64] = {}, oz64L_ready[fgb::oz::kTiles64] = {};
   std::vector<double> alpha_max;
   bool finite = true;
   // slices of the kernel GEMM (9, 8 or 7) and of the variance GEMM (9, 8,

@@ -25,7 +25,8 @@ constexpr int kMaxK = 1472;
 // group then sums to at most 12288 * K.
 constexpr int kS64 = 10;
 constexpr int kMaxK64 = 1360;
-constexpr int kTN64v[2] = {48, 32};   // B tile heights of its products
+constexpr int kTiles64 = 3;
+constexpr int kTN64v[kTiles64] = {48, 32, 16};   // B tile heights of its products
 // FP32-level configuration (force GEMM of the mixed path): 4 slices, B tiles
 // of 128 rows; the biggest group (a + b = 5) sums to at most 6144 * K.
 constexpr int kSF32 = 4;
@@ -103,13 +104,13 @@ int gemm(const Sliced &A, const Sliced &B, bool tri, const Epi &epi, int *err,
 // one rounding.
 int gemm_store(const Sliced &A, const Sliced &B, double *C, long long ldc,
                int *err, cudaStream_t st);
-// C = a (A B^T) + b C in FP64 from kS-slice operands (b = 0: C is only
+// C = a (A B^T) + b C in FP64 from kS-slice operands (B tiles of kTN64v rows; b = 0: C is only
 // written), the same exact integer sums and one rounding of the product.
 // lower: only C's lower triangle is wanted (tiles above it are skipped).
 int gemm_axpby(const Sliced &A, const Sliced &B, double *C, long long ldc,
                double a, double b, int *err, cudaStream_t st,
                bool lower = false);
-// B tile height (index into kTN64v) of a kS64-slice product.
+// B tile height (index into kTN64v) of a kS64- or kS-slice product.
 int tile64(int rows, int cols);
 // Products of kS64-slice operands (B tiles of kTN64v rows) for the
 // stored-gradient form and the solved variances:

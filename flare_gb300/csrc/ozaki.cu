@@ -86,6 +86,7 @@ struct Cfg {
 };
 using CfgF64 = Cfg<kS, 48, kStages, kMaxK, 3>;
 using CfgF64n = Cfg<kS, 32, kStages, kMaxK, 2>;
+using CfgF64q = Cfg<kS, 16, 5, kMaxK, 1>;   // few output tiles
 // fewer slices: smaller stages, so a deeper ring fits; B tiles of 64 rows
 // take four epilogue warps per lane quarter (576 threads)
 constexpr int ring_depth(int S, int TN) {
@@ -93,7 +94,10 @@ constexpr int ring_depth(int S, int TN) {
 }
 template <int S, int TN>
 using CfgS = typename std::conditional<
-    S == kS, typename std::conditional<TN == 48, CfgF64, CfgF64n>::type,
+    S == kS,
+    typename std::conditional<
+        TN == 48, CfgF64,
+        typename std::conditional<TN == 32, CfgF64n, CfgF64q>::type>::type,
     Cfg<S, TN, ring_depth(S, TN), S == kS64 ? kMaxK64 : kMaxK,
         TN / 16>>::type;
 static_assert(CfgS<8, 48>::EW == 3 && CfgS<8, 32>::EW == 2 &&
@@ -961,6 +965,8 @@ int gemm_s(const Sliced &A, const Sliced &B, bool tri, const Epi &epi,
   if (B.TR == 32) return gemm_c<CfgS<S, 32>>(A, B, tri, epi, err, st);
   if constexpr (S < kS)
     if (B.TR == 64) return gemm_c<CfgS<S, 64>>(A, B, tri, epi, err, st);
+  if constexpr (S == kS64)
+    if (B.TR == 16) return gemm_c<CfgS<S, 16>>(A, B, tri, epi, err, st);
   return gemm_c<CfgS<S, 48>>(A, B, tri, epi, err, st);
 }
 
@@ -979,6 +985,7 @@ int gemm_axpby(const Sliced &A, const Sliced &B, double *C, long long ldc,
                double a, double b, int *err, cudaStream_t st, bool lower) {
   const EpiAxpby epi{C, ldc, B.rows, a, b};
   if (B.TR == 32) return gemm_c<CfgF64n>(A, B, false, epi, err, st, lower);
+  if (B.TR == 16) return gemm_c<CfgF64q>(A, B, false, epi, err, st, lower);
   return gemm_c<CfgF64>(A, B, false, epi, err, st, lower);
 }
 
@@ -1475,11 +1482,11 @@ int row_inverse(int M, int nd, const double *rows, double *norms, double2 *inv,
   return FGB_OK;
 }
 
-// The fewer rounds of tiles over the SMs weighted by a tile's time: a 48-row
-// tile takes 1.25 times a 32-row tile (2 x 1,000 sparse, n_d 680, the three
-// products of the FP64 path over both species: 500 atoms 417 us at 48 rows
-// against 335 at 32, 1,000 atoms 420 and 374, 1,500 atoms 426 and 480, 8,000
-// atoms 1,319 and 1,403).
+// The fewest rounds of tiles over the SMs, weighted by a tile's time: 48, 32
+// and 16 rows cost 20, 16 and 13 (2 x 1,000 sparse, n_d 680, the three
+// products of the FP64 path over both species: 64 atoms 397, 315 and 251 us;
+// 500 atoms 414, 327 and 272; 1,000 atoms 421, 371 and 450; 1,500 atoms 425,
+// 472 and 525; 4,000 atoms 824, 901 and 1,043).
 int tile64(int rows, int cols) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1487,9 +1494,16 @@ int tile64(int rows, int cols) {
           cudaSuccess)
     return 0;
   const long long mt = ceil_div(rows, kTM);
-  return 4 * ceil_div(mt * ceil_div(cols, kTN64v[1]), sms) <
-                 5 * ceil_div(mt * ceil_div(cols, kTN64v[0]), sms)
-             ? 1 : 0;
+  int best = 0, best_cost = 0;
+  for (int v = 0; v < kTiles64; v++) {
+    constexpr int kCost[kTiles64] = {20, 16, 13};
+    const int c = kCost[v] * ceil_div(mt * ceil_div(cols, kTN64v[v]), sms);
+    if (v == 0 || c < best_cost) {
+      best = v;
+      best_cost = c;
+    }
+  }
+  return best;
 }
 
 int gemm_cosine(const Sliced &A, const Sliced &B, const int *perm,

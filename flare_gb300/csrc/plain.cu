@@ -643,7 +643,7 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
     const int R = 3 * (spairs[s + 1] - spairs[s]);
     const int vc = oz::tile64(Ns, Ms);
     const int vf = oz::tile64(std::min(std::max(R, 1), kRows), Ms);
-    for (int v = 0; v < 2; v++)
+    for (int v = 0; v < oz::kTiles64; v++)
       if ((v == vc || (v == vf && R > 0)) &&
           (rc = oz::slice({Ms, nd, oz::kTN64v[v],
                            d_sparse + (size_t)so.o[s] * nd, nd, nullptr,

@@ -597,7 +597,7 @@ extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
   for (bool &r : m->ozS_ready) r = false;
   for (bool &r : m->ozL_ready) r = false;
   for (bool &r : m->ozB_ready) r = false;
-  for (int v = 0; v < 2; v++)
+  for (int v = 0; v < oz::kTiles64; v++)
     m->oz64S_ready[v] = m->oz64ST_ready[v] = m->oz64L_ready[v] = false;
   m->finite = true;
   for (int t = 0; t < M; t++) m->finite &= std::isfinite(snorm[t]);
@@ -949,7 +949,7 @@ extern "C" int fgb_model_set_R_inv(fgb_model_t m, const double *h_R_inv) {
     FGB_CUDA(cudaMemcpy(m->RinvT.p, t.data(), sizeof(double) * (size_t)M * M,
                         cudaMemcpyHostToDevice));
   m->has_rinv = true;
-  m->oz64R_ready[0] = m->oz64R_ready[1] = false;
+  for (bool &r : m->oz64R_ready) r = false;
   return FGB_OK;
 }
 
@@ -1003,7 +1003,7 @@ static int predict_solved(fgb_model_s *m, fgb_nlist_s *nl, const int *d_species,
     FGB_CUDA(cudaMemcpy(m->Lfull.p, m->h_L_inv.data(),
                         sizeof(double) * (size_t)M * M, cudaMemcpyHostToDevice));
     m->lfull_ready = true;
-    m->oz64Lfull_ready[0] = m->oz64Lfull_ready[1] = false;
+    for (bool &r : m->oz64Lfull_ready) r = false;
   }
   if ((rc = envs_struc_impl(m->b2, m->sigma, m->power, m->h_counts.data(),
                             m->Sraw.as<double>(), nl, d_species,
