@@ -215,11 +215,64 @@ __global__ void k_scan_add(TO *__restrict__ out, int n,
   if (i < n) out[i] += sums[blockIdx.x];
 }
 
+// The whole scan in one block, up to kScanOne elements: a thread takes
+// kScanOne / 1024 consecutive ones.  One launch instead of three (1,000
+// elements: 2.9 against 7.5 us; 32,000 were 36 us slower in one block).
+constexpr int kScanOne = 8 * kScanBlock;
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(kScanBlock)
+k_scan_one(const TI *__restrict__ in, TO *__restrict__ out, int n,
+           TO *__restrict__ total) {
+  __shared__ TO wsum[32];
+  constexpr int kPer = kScanOne / kScanBlock;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  // few elements stay with few warps
+  const int per = (n + kScanBlock - 1) / kScanBlock;
+  TO v[kPer], acc = 0;
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    const int i = t * per + k;
+    v[k] = k < per && i < n ? (TO)in[i] : (TO)0;
+    acc += v[k];
+  }
+  TO x = acc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const TO y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    TO s = wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const TO y = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += y;
+    }
+    wsum[lane] = s;
+  }
+  __syncthreads();
+  TO run = x - acc + (w ? wsum[w - 1] : (TO)0);
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    const int i = t * per + k;
+    if (k < per && i < n) out[i] = run;
+    run += v[k];
+  }
+  if (t == 0 && total) *total = wsum[31];
+}
+
 template <typename TI, typename TO>
 int scan_impl(const TI *d_in, TO *d_out, int n, TO *d_total, DevBuf &tmp,
               cudaStream_t st) {
   if (n <= 0) {
     if (d_total) FGB_CUDA(cudaMemsetAsync(d_total, 0, sizeof(TO), st));
+    return FGB_OK;
+  }
+  if (n <= kScanOne) {
+    k_scan_one<TI, TO><<<1, kScanBlock, 0, st>>>(d_in, d_out, n, d_total);
+    FGB_LAUNCH_CHECK("k_scan_one");
     return FGB_OK;
   }
   int nb = (n + kScanBlock - 1) / kScanBlock;
@@ -248,6 +301,11 @@ int scan_impl_raw(const TI *d_in, TO *d_out, int n, TO *d_total, TO *sums,
     if (d_total) FGB_CUDA(cudaMemsetAsync(d_total, 0, sizeof(TO), st));
     return FGB_OK;
   }
+  if (n <= kScanOne) {
+    k_scan_one<TI, TO><<<1, kScanBlock, 0, st>>>(d_in, d_out, n, d_total);
+    FGB_LAUNCH_CHECK("k_scan_one");
+    return FGB_OK;
+  }
   int nb = (n + kScanBlock - 1) / kScanBlock;
   if (nb > 4 * kScanBlock) {
     set_error("scan: %d elements exceed the two-level scan limit", n);
@@ -263,6 +321,8 @@ int scan_impl_raw(const TI *d_in, TO *d_out, int n, TO *d_total, TO *sums,
 }
 
 }  // namespace
+
+int scan_launches(int n) { return n <= 0 ? 0 : n <= kScanOne ? 1 : 3; }
 
 int scan_int_to_int_raw(const int *d_in, int *d_out, int n, int *d_total,
                         int *d_sums, cudaStream_t st) {

@@ -582,20 +582,24 @@ __global__ void k_forces(int n_atoms, const long long *__restrict__ offsets,
   }
 }
 
-// Per-structure energy and stress: fixed-order tree sums over the
-// structure's atoms.  One block per structure.
-__global__ void k_struct_reduce(int n_struc, const int *__restrict__ atom_off,
-                                const double *__restrict__ volume,
-                                const double *__restrict__ e_atom,
-                                const double *__restrict__ virial,
-                                double *__restrict__ energy,
-                                double *__restrict__ stress) {
+// Per-structure energy and stress: fixed-order tree sums over chunks of
+// kRedChunk atoms, a block per (structure, chunk); the chunks of a larger
+// structure are then added in order (k_struct_final).  The chunking follows
+// the structure's own atoms alone, so its sums do not depend on the batch.
+// One block for 97,556 atoms took 355 us, 48 blocks and the final sum 18.
+constexpr int kRedChunk = 2048;
+__global__ void __launch_bounds__(256)
+k_struct_reduce(const StrucGeom *__restrict__ geom,
+                const double *__restrict__ e_atom,
+                const double *__restrict__ virial, double *__restrict__ part,
+                double *__restrict__ energy, double *__restrict__ stress) {
   __shared__ double red[7][256];
-  int s = blockIdx.x;
-  if (s >= n_struc) return;
-  int t = threadIdx.x;
+  const int s = blockIdx.y, ch = blockIdx.x, t = threadIdx.x;
+  const int a0 = geom[s].atom0, na = geom[s].natoms;
+  if (ch > 0 && ch * kRedChunk >= na) return;
+  const int a1 = a0 + min(na, (ch + 1) * kRedChunk);
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int a = atom_off[s] + t; a < atom_off[s + 1]; a += blockDim.x) {
+  for (int a = a0 + ch * kRedChunk + t; a < a1; a += blockDim.x) {
     if (e_atom) acc[0] += e_atom[a];
     if (virial)
       for (int k = 0; k < 6; k++) acc[1 + k] += virial[6 * a + k];
@@ -607,11 +611,23 @@ __global__ void k_struct_reduce(int n_struc, const int *__restrict__ atom_off,
       for (int k = 0; k < 7; k++) red[k][t] += red[k][t + h];
     __syncthreads();
   }
-  if (t == 0) {
-    if (energy) energy[s] = red[0][0];
-    if (stress)
-      for (int k = 0; k < 6; k++) stress[6 * s + k] = -red[1 + k][0] / volume[s];
-  }
+  if (t >= 7) return;
+  if (na > kRedChunk) part[((long long)s * gridDim.x + ch) * 7 + t] = red[t][0];
+  else if (t == 0) { if (energy) energy[s] = red[0][0]; }
+  else if (stress) stress[6 * s + t - 1] = -red[t][0] / geom[s].volume;
+}
+
+__global__ void k_struct_final(const StrucGeom *__restrict__ geom, int maxch,
+                               const double *__restrict__ part,
+                               double *__restrict__ energy,
+                               double *__restrict__ stress) {
+  const int s = blockIdx.x, t = threadIdx.x, na = geom[s].natoms;
+  if (t >= 7 || na <= kRedChunk) return;
+  const int nch = (na + kRedChunk - 1) / kRedChunk;
+  double x = 0.0;
+  for (int c = 0; c < nch; c++) x += part[((long long)s * maxch + c) * 7 + t];
+  if (t == 0) { if (energy) energy[s] = x; }
+  else if (stress) stress[6 * s + t - 1] = -x / geom[s].volume;
 }
 
 }  // namespace
@@ -743,14 +759,32 @@ int launch_forces(const fgb_nlist_s *nl, const void *d_pair_grad, bool fp32,
   return FGB_OK;
 }
 
-int launch_struct_reduce(int n_struc, const int *d_atom_off,
-                         const double *d_volume, const double *d_e_atom,
+int launch_struct_reduce(const fgb_nlist_s *nl, const double *d_e_atom,
                          const double *d_virial, double *d_energy,
-                         double *d_stress, cudaStream_t st) {
-  k_struct_reduce<<<n_struc, 256, 0, st>>>(n_struc, d_atom_off, d_volume,
-                                           d_e_atom, d_virial, d_energy,
-                                           d_stress);
-  FGB_LAUNCH_CHECK("k_struct_reduce");
+                         double *d_stress, DevBuf &part, cudaStream_t st) {
+  int most = 0;
+  for (int s = 0; s < nl->n_struc; s++)
+    most = std::max(most, nl->h_atom_offsets[s + 1] - nl->h_atom_offsets[s]);
+  const int maxch = std::max(1, ceil_div(most, kRedChunk));
+  int rc;
+  if (maxch > 1 &&
+      (rc = part.ensure(sizeof(double) * 7 * (size_t)maxch * nl->n_struc)))
+    return rc;
+  // the grid's second dimension holds up to 65,535 structures
+  for (int s0 = 0; s0 < nl->n_struc; s0 += 65535) {
+    const int ns = std::min(65535, nl->n_struc - s0);
+    const StrucGeom *g = nl->geom.as<StrucGeom>() + s0;
+    double *p = maxch > 1 ? part.as<double>() + 7LL * maxch * s0 : nullptr;
+    double *e = d_energy ? d_energy + s0 : nullptr;
+    double *t = d_stress ? d_stress + 6LL * s0 : nullptr;
+    k_struct_reduce<<<dim3(maxch, ns), 256, 0, st>>>(g, d_e_atom, d_virial, p,
+                                                     e, t);
+    FGB_LAUNCH_CHECK("k_struct_reduce");
+    if (maxch > 1) {
+      k_struct_final<<<ns, 32, 0, st>>>(g, maxch, p, e, t);
+      FGB_LAUNCH_CHECK("k_struct_final");
+    }
+  }
   return FGB_OK;
 }
 

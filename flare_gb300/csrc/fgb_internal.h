@@ -78,6 +78,7 @@ int scan_int_to_int(const int *d_in, int *d_out, int n, int *d_total,
                     DevBuf &tmp, cudaStream_t st);
 int scan_int_to_ll(const int *d_in, long long *d_out, int n,
                    long long *d_total, DevBuf &tmp, cudaStream_t st);
+int scan_launches(int n);   // kernels one scan of n elements launches
 // Variants with caller-provided block sums (ceil(n/1024) + 1 elements).
 int scan_int_to_int_raw(const int *d_in, int *d_out, int n, int *d_total,
                         int *d_sums, cudaStream_t st);
@@ -151,6 +152,7 @@ struct fgb_nlist_s {
   // build copies back, whether n_pairs still waits for it, and a request
   // for a count pass (set by callers repeating a build that overflowed)
   long long last_slots = 0, min_slots = 0;
+  long long slots = 0;       // slots of the last build's list, 0: count pass
   int last_launches = 0;     // kernels the last build or rebuild launched
   long long *h_total = nullptr;
   bool total_pending = false;

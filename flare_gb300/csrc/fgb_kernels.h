@@ -24,10 +24,11 @@ int launch_b2_adjoint(const B2Params &p, const fgb_nlist_s *nl,
 // d_pair_grad as the adjoint wrote it (fp32: float3)
 int launch_forces(const fgb_nlist_s *nl, const void *d_pair_grad, bool fp32,
                   double *d_forces, double *d_virial, cudaStream_t st);
-int launch_struct_reduce(int n_struc, const int *d_atom_off,
-                         const double *d_volume, const double *d_e_atom,
+// Energies and stresses of the list's structures from per-atom energies and
+// virials; `part`: scratch for structures of more than one chunk of atoms.
+int launch_struct_reduce(const fgb_nlist_s *nl, const double *d_e_atom,
                          const double *d_virial, double *d_energy,
-                         double *d_stress, cudaStream_t st);
+                         double *d_stress, DevBuf &part, cudaStream_t st);
 
 // Stored forward-mode gradients (the reference's algorithm); scratch: each
 // pair's centre atom (left for the caller) and the pairs' basis values.

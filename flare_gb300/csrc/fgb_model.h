@@ -30,7 +30,8 @@ struct fgb_pinned_counts {
 struct fgb_workspace {
   fgb_pinned_counts counts;
   fgb::DevBuf perm, flags, pos, scal, scan_tmp, flag;
-  fgb::DevBuf A, B2, norms, e_atom, var, volume, atom_off;
+  fgb::DevBuf A, B2, norms, e_atom, var;
+  fgb::DevBuf redpart;  // chunk sums of structures above one chunk
   fgb::DevBuf rowmax;   // largest |B2| per row (tensor-core row scales)
   fgb::DevBuf gB2, pair_grad, forces, virial;
   fgb::DevBuf kmat, wmat, erows, part;

@@ -287,15 +287,8 @@ extern "C" int fgb_mapped_predict(fgb_mapped_t m, int n_struc,
       (rc = ws.pair_grad.ensure(sizeof(double3) * (P + 1))) ||
       (rc = ws.forces.ensure(sizeof(double) * (3 * (size_t)N + 1))) ||
       (rc = ws.virial.ensure(sizeof(double) * (6 * (size_t)N + 1))) ||
-      (rc = ws.volume.ensure(sizeof(double) * (n_struc + 1))) ||
-      (rc = ws.atom_off.ensure(sizeof(int) * (n_struc + 1))) ||
       (rc = ws.ozerr.ensure(sizeof(int))))
     return rc;
-  FGB_CUDA(cudaMemcpyAsync(ws.volume.p, m->nl.h_volume.data(),
-                           sizeof(double) * n_struc, cudaMemcpyHostToDevice, st));
-  FGB_CUDA(cudaMemcpyAsync(ws.atom_off.p, h_atom_offsets,
-                           sizeof(int) * (n_struc + 1), cudaMemcpyHostToDevice,
-                           st));
   FGB_CUDA(cudaMemsetAsync(ws.ozerr.p, 0, sizeof(int), st));
   if (N > 0) {
     FGB_CUDA(cudaMemsetAsync(ws.e_atom.p, 0, sizeof(double) * N, st));
@@ -380,10 +373,10 @@ extern "C" int fgb_mapped_predict(fgb_mapped_t m, int n_struc,
   }
   if ((want_e && d_energy) || (want_s && d_stress))
     if ((rc = launch_struct_reduce(
-             n_struc, ws.atom_off.as<int>(), ws.volume.as<double>(),
-             ws.e_atom.as<double>(),
+             &m->nl, ws.e_atom.as<double>(),
              want_grad ? ws.virial.as<double>() : nullptr,
-             want_e ? d_energy : nullptr, want_s ? d_stress : nullptr, st)))
+             want_e ? d_energy : nullptr, want_s ? d_stress : nullptr,
+             ws.redpart, st)))
       return rc;
   if (d_atom_energy && N > 0)
     FGB_CUDA(cudaMemcpyAsync(d_atom_energy, ws.e_atom.p, sizeof(double) * N,

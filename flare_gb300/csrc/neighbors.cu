@@ -69,8 +69,9 @@ __device__ __forceinline__ void image_offsets(const StrucGeom &g, int img,
 }
 
 // frac = (p * ct) * cdi ; f = frac - floor(frac); w = (f * cd) * cti
-__global__ void k_wrap_bin(int n, const double *__restrict__ pos,
-                           const int *__restrict__ atom_struct,
+// (also each atom's structure: the last whose first atom is not after it)
+__global__ void k_wrap_bin(int n, int n_struc, const double *__restrict__ pos,
+                           int *__restrict__ atom_struct,
                            const StrucGeom *__restrict__ geom,
                            double *__restrict__ wrapped, float4 *__restrict__ w32,
                            int *__restrict__ raw,
@@ -78,7 +79,14 @@ __global__ void k_wrap_bin(int n, const double *__restrict__ pos,
                            int *__restrict__ bin_count, int *__restrict__ flag) {
   int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
-  const StrucGeom &g = geom[atom_struct[a]];
+  int s_lo = 0, s_hi = n_struc;
+  while (s_hi - s_lo > 1) {
+    const int mid = (s_lo + s_hi) >> 1;
+    if (geom[mid].atom0 <= a) s_lo = mid;
+    else s_hi = mid;
+  }
+  atom_struct[a] = s_lo;
+  const StrucGeom &g = geom[s_lo];
   double p0 = pos[3 * a], p1 = pos[3 * a + 1], p2 = pos[3 * a + 2];
   double t[3], f[3], u[3];
 #pragma unroll
@@ -670,7 +678,6 @@ int fgb::nlist_build(fgb_nlist_s *nl, int n_struc, const int *h_atom_offsets,
   nl->h_cells.assign(h_cells, h_cells + 9 * n_struc);
   nl->h_volume.resize(n_struc);
   std::vector<StrucGeom> geom(n_struc);
-  std::vector<int> atom_struct(N);
   long long nbins = 0;
   double dmax = 0.0;   // atoms per unit volume, densest structure
   for (int s = 0; s < n_struc; s++) {
@@ -696,8 +703,6 @@ int fgb::nlist_build(fgb_nlist_s *nl, int n_struc, const int *h_atom_offsets,
     nl->h_volume[s] = geom[s].volume;
     dmax = std::max(dmax, geom[s].natoms / geom[s].volume);
     nbins += (long long)geom[s].nb[0] * geom[s].nb[1] * geom[s].nb[2];
-    for (int a = h_atom_offsets[s]; a < h_atom_offsets[s + 1]; a++)
-      atom_struct[a] = s;
   }
   if (nbins > (1 << 26)) {
     set_error("fgb_nlist_build: too many bins");
@@ -721,9 +726,6 @@ int fgb::nlist_build(fgb_nlist_s *nl, int n_struc, const int *h_atom_offsets,
     return rc;
   FGB_CUDA(cudaMemcpyAsync(nl->geom.p, geom.data(), sizeof(StrucGeom) * n_struc,
                            cudaMemcpyHostToDevice, st));
-  if (N > 0)
-    FGB_CUDA(cudaMemcpyAsync(nl->atom_struct.p, atom_struct.data(),
-                             sizeof(int) * N, cudaMemcpyHostToDevice, st));
   FGB_CUDA(cudaMemsetAsync(nl->bin_count.p, 0, sizeof(int) * (nbins + 1), st));
   FGB_CUDA(cudaMemsetAsync(nl->flag.p, 0, sizeof(int) * 4, st));
   const int T = 128;
@@ -735,10 +737,10 @@ int fgb::nlist_build(fgb_nlist_s *nl, int n_struc, const int *h_atom_offsets,
     return FGB_OK;
   }
   k_wrap_bin<<<ceil_div(N, T), T, 0, st>>>(
-      N, d_positions, nl->atom_struct.as<int>(), nl->geom.as<StrucGeom>(),
-      nl->wrapped.as<double>(), nl->wrapped32.as<float4>(),
-      nl->raw_bin.as<int>(), nl->home_bin.as<int>(),
-      nl->bin_slot.as<int>(), nl->bin_count.as<int>(), nl->flag.as<int>());
+      N, n_struc, d_positions, nl->atom_struct.as<int>(),
+      nl->geom.as<StrucGeom>(), nl->wrapped.as<double>(),
+      nl->wrapped32.as<float4>(), nl->raw_bin.as<int>(),
+      nl->home_bin.as<int>(), nl->bin_slot.as<int>(), nl->bin_count.as<int>(), nl->flag.as<int>());
   FGB_LAUNCH_CHECK("k_wrap_bin");
   if ((rc = scan_int_to_int(nl->bin_count.as<int>(), nl->bin_start.as<int>(),
                             (int)nbins, nl->bin_start.as<int>() + nbins,
@@ -763,7 +765,7 @@ int fgb::nlist_build(fgb_nlist_s *nl, int n_struc, const int *h_atom_offsets,
   const long long C = nl->count_pass ? 0 : single_pass_slots(nl, dmax, cutoff, N);
   if (C > 0) {
     const long long slots = (long long)N * C;
-    nl->last_slots = C;
+    nl->last_slots = nl->slots = C;
     if ((rc = nl->tmp_key.ensure(sizeof(unsigned long long) * (slots + 1))) ||
         (rc = nl->tmp_rel.ensure(sizeof(double4_16a) * (slots + 1))) ||
         (rc = nl->nbr_j.ensure(sizeof(int) * (slots + 1))) ||
@@ -803,7 +805,7 @@ int fgb::nlist_build(fgb_nlist_s *nl, int n_struc, const int *h_atom_offsets,
                              cudaMemcpyDeviceToHost, st));
     nl->n_pairs = slots;   // an upper bound until nlist_finish reads the count
     nl->total_pending = true;
-    nl->last_launches = 11;
+    nl->last_launches = 5 + scan_launches((int)nbins) + scan_launches(N);
     if (!check) return FGB_OK;
     FGB_CUDA(cudaMemcpyAsync(hflag, nl->flag.p, sizeof(int) * 4,
                              cudaMemcpyDeviceToHost, st));
@@ -834,9 +836,11 @@ int fgb::nlist_build(fgb_nlist_s *nl, int n_struc, const int *h_atom_offsets,
   }
   nl->n_pairs = P;
   nl->total_pending = false;
-  // wrap, bin scan (3), bin fill, count, pair scan (3), then fill, rank and
-  // twin when there are pairs; after an overflowed single pass its 6 more
-  nl->last_launches = 9 + (P > 0 ? 3 : 0) + (C > 0 ? 6 : 0);
+  nl->slots = 0;
+  // wrap, bin scan, bin fill, count, pair scan, then fill, rank and twin when
+  // there are pairs; after an overflowed single pass its more
+  nl->last_launches = 3 + scan_launches((int)nbins) + scan_launches(N) +
+                      (P > 0 ? 3 : 0) + (C > 0 ? 3 + scan_launches(N) : 0);
   if ((rc = nl->tmp_key.ensure(sizeof(unsigned long long) * (P + 1))) ||
       (rc = nl->tmp_rel.ensure(sizeof(double4_16a) * (P + 1))) ||
       (rc = nl->nbr_j.ensure(sizeof(int) * (P + 1))) ||
@@ -899,10 +903,11 @@ int nlist_rebuild_fixed(fgb_nlist_s *nl, const double *d_positions,
   nl->last_launches = 0;
   if (N == 0) return FGB_OK;
   k_wrap_bin<<<ceil_div(N, T), T, 0, st>>>(
-      N, d_positions, nl->atom_struct.as<int>(), nl->geom.as<StrucGeom>(),
-      nl->wrapped.as<double>(), nl->wrapped32.as<float4>(),
-      nl->raw_bin.as<int>(), nl->home_bin.as<int>(), nl->bin_slot.as<int>(),
-      nl->bin_count.as<int>(), nl->flag.as<int>());
+      N, nl->n_struc, d_positions, nl->atom_struct.as<int>(),
+      nl->geom.as<StrucGeom>(), nl->wrapped.as<double>(),
+      nl->wrapped32.as<float4>(), nl->raw_bin.as<int>(),
+      nl->home_bin.as<int>(), nl->bin_slot.as<int>(), nl->bin_count.as<int>(),
+      nl->flag.as<int>());
   FGB_LAUNCH_CHECK("k_wrap_bin");
   if ((rc = scan_int_to_int(nl->bin_count.as<int>(), nl->bin_start.as<int>(),
                             (int)nbins, nl->bin_start.as<int>() + nbins,
@@ -913,12 +918,30 @@ int nlist_rebuild_fixed(fgb_nlist_s *nl, const double *d_positions,
       nl->bin_start.as<int>(), nl->bin_atoms.as<int>());
   FGB_LAUNCH_CHECK("k_bin_fill");
   const long long NW = (long long)N * 32;
-  k_count<<<ceil_div(NW, T), T, 0, st>>>(
-      N, nl->atom_struct.as<int>(), nl->geom.as<StrucGeom>(),
-      nl->wrapped.as<double>(), nl->wrapped32.as<float4>(),
-      nl->raw_bin.as<int>(), nl->bin_start.as<int>(), nl->bin_atoms.as<int>(),
-      cutoff, nl->counts.as<int>());
-  FGB_LAUNCH_CHECK("k_count");
+  // after a single-pass build: pairs go to the atoms' slots again (more than
+  // those set flag[3], as more than cap do), with no count pass
+  const long long C = nl->slots;
+  if (C == 0) {
+    k_count<<<ceil_div(NW, T), T, 0, st>>>(
+        N, nl->atom_struct.as<int>(), nl->geom.as<StrucGeom>(),
+        nl->wrapped.as<double>(), nl->wrapped32.as<float4>(),
+        nl->raw_bin.as<int>(), nl->bin_start.as<int>(),
+        nl->bin_atoms.as<int>(), cutoff, nl->counts.as<int>());
+    FGB_LAUNCH_CHECK("k_count");
+  }
+  const auto fill = [&]() -> int {
+    k_fill<<<ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st>>>(
+        N, nl->atom_struct.as<int>(), nl->geom.as<StrucGeom>(),
+        nl->wrapped.as<double>(), nl->wrapped32.as<float4>(),
+        nl->raw_bin.as<int>(), nl->bin_start.as<int>(),
+        nl->bin_atoms.as<int>(), cutoff, nl->offsets.as<long long>(), C,
+        C ? nl->counts.as<int>() : nullptr,
+        nl->tmp_key.as<unsigned long long>(), nl->tmp_rel.as<double4_16a>(),
+        nl->flag.as<int>());
+    FGB_LAUNCH_CHECK("k_fill");
+    return FGB_OK;
+  };
+  if (C && (rc = fill())) return rc;
   if ((rc = scan_int_to_ll(nl->counts.as<int>(), nl->offsets.as<long long>(),
                            N, nl->offsets.as<long long>() + N, nl->scan_tmp,
                            st)))
@@ -926,17 +949,10 @@ int nlist_rebuild_fixed(fgb_nlist_s *nl, const double *d_positions,
   k_clamp_offsets<<<ceil_div(N + 1, T), T, 0, st>>>(
       N, cap, nl->offsets.as<long long>(), nl->flag.as<int>());
   FGB_LAUNCH_CHECK("k_clamp_offsets");
-  k_fill<<<ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st>>>(
-      N, nl->atom_struct.as<int>(), nl->geom.as<StrucGeom>(),
-      nl->wrapped.as<double>(), nl->wrapped32.as<float4>(),
-      nl->raw_bin.as<int>(), nl->bin_start.as<int>(), nl->bin_atoms.as<int>(),
-      cutoff, nl->offsets.as<long long>(), 0LL, nullptr,
-      nl->tmp_key.as<unsigned long long>(), nl->tmp_rel.as<double4_16a>(),
-      nl->flag.as<int>());
-  FGB_LAUNCH_CHECK("k_fill");
+  if (!C && (rc = fill())) return rc;
   k_rank_scatter<<<ceil_div(NW, T), T, 0, st>>>(
       N, nl->atom_struct.as<int>(), nl->geom.as<StrucGeom>(),
-      nl->offsets.as<long long>(), 0LL, nl->tmp_key.as<unsigned long long>(),
+      nl->offsets.as<long long>(), C, nl->tmp_key.as<unsigned long long>(),
       nl->tmp_rel.as<double4_16a>(), nl->nbr_j.as<int>(),
       nl->nbr_shift.as<int>(), nl->nbr_rel.as<double4_16a>());
   FGB_LAUNCH_CHECK("k_rank_scatter");
@@ -947,7 +963,8 @@ int nlist_rebuild_fixed(fgb_nlist_s *nl, const double *d_positions,
       nl->flag.as<int>());
   FGB_LAUNCH_CHECK("k_twin");
   nl->n_pairs = cap;   // an upper bound; the device offsets hold the count
-  nl->last_launches = 13;
+  nl->last_launches = 6 + (C ? 0 : 1) + scan_launches((int)nbins) +
+                      scan_launches(N);
   return FGB_OK;
 }
 
@@ -1110,7 +1127,6 @@ extern "C" int fgb_nlist_build_noalloc(const double *h_cell,
   }
   FGB_CUDA(cudaMemcpyAsync(d_geom, &geom, sizeof(StrucGeom),
                            cudaMemcpyHostToDevice, st));
-  FGB_CUDA(cudaMemsetAsync(atom_struct, 0, sizeof(int) * (N + 1), st));
   FGB_CUDA(cudaMemsetAsync(bin_count, 0, sizeof(int) * (nbins + 1), st));
   FGB_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * 4, st));
   if (N == 0) {
@@ -1118,8 +1134,8 @@ extern "C" int fgb_nlist_build_noalloc(const double *h_cell,
     return FGB_OK;
   }
   const int T = 128;
-  k_wrap_bin<<<ceil_div(N, T), T, 0, st>>>(N, d_positions, atom_struct, d_geom,
-                                           wrapped, w32, raw, home, slot,
+  k_wrap_bin<<<ceil_div(N, T), T, 0, st>>>(N, 1, d_positions, atom_struct,
+                                           d_geom, wrapped, w32, raw, home, slot,
                                            bin_count, flag);
   FGB_LAUNCH_CHECK("k_wrap_bin");
   if ((rc = scan_int_to_int_raw(bin_count, bin_start, (int)nbins,
