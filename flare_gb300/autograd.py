@@ -29,9 +29,9 @@ class SGPEnergy(torch.autograd.Function):
         S = len(structures)
         dev = positions.device
         d_sp = torch.from_numpy(sp).to(dev)
-        e = torch.zeros(S, dtype=torch.float64, device=dev)
-        f = torch.zeros((max(N, 1), 3), dtype=torch.float64, device=dev)
-        st = torch.zeros((S, 6), dtype=torch.float64, device=dev)
+        e = torch.empty(S, dtype=torch.float64, device=dev)
+        f = torch.empty((max(N, 1), 3), dtype=torch.float64, device=dev)
+        st = torch.empty((S, 6), dtype=torch.float64, device=dev)
         prec = _prec[precision or get_precision()]
         _lib.check(_lib.lib().fgb_predict(
             m.h, S, _lib.ptr(offsets), _lib.ptr(cells), _lib.ptr(positions),

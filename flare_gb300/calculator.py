@@ -53,6 +53,11 @@ def sort_variances(structure, variances):
     """calculator.py:188-206: species-sorted variances back to atom order."""
     assert len(variances) == structure.noa
     out = np.zeros(len(variances))
+    if isinstance(structure, Structure):
+        # the order needs the species alone, not the descriptors
+        order = structure.species_order()
+        out[order] = np.asarray(variances)[:len(order)]
+        return out
     dv = structure.descriptors[0]
     v = 0
     for s in range(dv.n_types):

@@ -261,6 +261,17 @@ class ClusterDescriptor:
 
 
 # ---------------------------------------------------------- structure
+def _species_int32(species):
+    """A species list as an int32 array; small non-negative codes go through
+    bytes (5 us per 1,000 against 35 for a list)."""
+    if type(species) in (list, tuple):
+        try:
+            return np.frombuffer(bytes(species), np.uint8).astype(np.int32)
+        except (TypeError, ValueError):
+            pass
+    return np.asarray(species, np.int32)
+
+
 class _NList:
     """Owner of an fgb_nlist_t handle."""
 
@@ -310,8 +321,8 @@ class Structure:
             dev = _device()
             self._dev = {
                 "pos": torch.from_numpy(self.positions).to(dev),
-                "species": torch.tensor(self.species, dtype=torch.int32,
-                                        device=dev),
+                "species": torch.from_numpy(
+                    _species_int32(self.species)).to(dev),
                 "offsets": np.array([0, self.noa], dtype=np.int32),
                 "cell": np.ascontiguousarray(self.cell.reshape(-1)),
             }
@@ -375,15 +386,22 @@ class Structure:
         check(lib().fgb_nlist_size(self.nlist().h, ctypes.byref(P), None))
         return P.value
 
+    def species_order(self, k=0):
+        """Atom indices in species order (species 0's atoms ascending, then
+        1's, ...) for descriptor calculator ``k``."""
+        sp = np.asarray(self.species)
+        S = self.descriptor_calculators[k].descriptor_settings[0]
+        return np.concatenate([np.nonzero(sp == s)[0] for s in range(S)])
+
     # ----------------------------------------------------- descriptors
     def b2_values(self, k=0):
         """(B2 [N x n_d], norms [N]) as device tensors, atom order."""
         calc = self.descriptor_calculators[k]
         d = self._inputs()
         dev = _device()
-        B = torch.zeros((max(self.noa, 1), calc.n_descriptors),
+        B = torch.empty((max(self.noa, 1), calc.n_descriptors),
                         dtype=torch.float64, device=dev)
-        nrm = torch.zeros(max(self.noa, 1), dtype=torch.float64, device=dev)
+        nrm = torch.empty(max(self.noa, 1), dtype=torch.float64, device=dev)
         check(lib().fgb_b2_forward(calc.handle, self.nlist().h, ptr(d["species"]),
                                    ptr(B), ptr(nrm), stream_ptr()), "B2")
         return B[:self.noa], nrm[:self.noa]
@@ -428,22 +446,25 @@ class Structure:
 def envs_envs_gpu(envs1, envs2, sigma, power):
     """envs_envs (normalized_dot_product.cpp:28-89) in FP64."""
     dev = _device()
-    K = torch.zeros((envs1.n_clusters, envs2.n_clusters), dtype=torch.float64,
-                    device=dev)
+    K = np.zeros((envs1.n_clusters, envs2.n_clusters))
     sig2 = sigma * sigma
     for s in range(envs1.n_types):
-        d1 = torch.from_numpy(np.ascontiguousarray(envs1.descriptors[s])).to(dev)
-        d2 = torch.from_numpy(np.ascontiguousarray(envs2.descriptors[s])).to(dev)
-        if d1.shape[0] == 0 or d2.shape[0] == 0:
+        m1, m2 = len(envs1.descriptors[s]), len(envs2.descriptors[s])
+        if m1 == 0 or m2 == 0:
             continue
-        n1 = torch.from_numpy(np.ascontiguousarray(
-            envs1.descriptor_norms[s], dtype=np.float64)).to(dev)
-        n2 = torch.from_numpy(np.ascontiguousarray(
-            envs2.descriptor_norms[s], dtype=np.float64)).to(dev)
-        blk = _kernel_block(d1, n1, d2, n2, sig2, power)
+        # rows and norms of both sets in one copy to the device
+        sets = [envs1] if envs2 is envs1 else [envs1, envs2]
+        flat = torch.from_numpy(np.concatenate(
+            [np.asarray(x, np.float64).reshape(-1) for e in sets
+             for x in (e.descriptors[s], e.descriptor_norms[s])])).to(dev)
+        nd = envs1.n_descriptors
+        d1, n1 = flat[:m1 * nd].view(m1, nd), flat[m1 * nd:m1 * (nd + 1)]
+        rest = flat[m1 * (nd + 1):] if len(sets) == 2 else flat
+        d2, n2 = rest[:m2 * nd].view(m2, nd), rest[m2 * nd:m2 * (nd + 1)]
         c1, c2 = envs1.cumulative_type_count[s], envs2.cumulative_type_count[s]
-        K[c1:c1 + d1.shape[0], c2:c2 + d2.shape[0]] = blk
-    return K.cpu().numpy()
+        K[c1:c1 + m1, c2:c2 + m2] = _kernel_block(d1, n1, d2, n2, sig2,
+                                                  power).cpu().numpy()
+    return K
 
 
 def _kernel_block(d1, n1, d2, n2, sig2, power):
@@ -472,7 +493,7 @@ def _envs_struc_device(envs, struc, sigma, power, k=0):
     M = int(counts.sum())
     ncol = 1 + 3 * struc.noa + 6
     dev = _device()
-    out = torch.zeros((M, ncol), dtype=torch.float64, device=dev)
+    out = torch.empty((M, ncol), dtype=torch.float64, device=dev)
     if M == 0:
         return out
     d_rows = torch.from_numpy(rows).to(dev)
@@ -858,9 +879,9 @@ class _Training:
         Kuf = torch.from_numpy(np.ascontiguousarray(self.Kuf)).to(dev)
         y = torch.from_numpy(np.ascontiguousarray(self.y)).to(dev)
         nv = torch.from_numpy(np.ascontiguousarray(self.noise_vector)).to(dev)
-        alpha = torch.zeros(M, dtype=torch.float64, device=dev)
-        Li = torch.zeros((M, M), dtype=torch.float64, device=dev)
-        Ri = torch.zeros((M, M), dtype=torch.float64, device=dev)
+        alpha = torch.empty(M, dtype=torch.float64, device=dev)
+        Li = torch.empty((M, M), dtype=torch.float64, device=dev)
+        Ri = torch.empty((M, M), dtype=torch.float64, device=dev)
         check(lib().fgb_solve_qr(M, int(self.n_labels), ptr(Kuu), ptr(Kuf),
                                  ptr(y), ptr(nv), float(self.Kuu_jitter),
                                  ptr(alpha), ptr(Li), ptr(Ri), stream_ptr()),
@@ -946,7 +967,7 @@ def pack_structures(structures):
                                            for s in structures]))
     pos = np.ascontiguousarray(np.concatenate([s.positions for s in structures]))
     sp = np.ascontiguousarray(np.concatenate(
-        [np.asarray(s.species, np.int32) for s in structures]))
+        [_species_int32(s.species) for s in structures]))
     return offsets, cells, pos, sp
 
 
@@ -1059,11 +1080,9 @@ class SparseGP(_Training):
         calcs = structures[0].descriptor_calculators
         models = self._device_models(calcs)
         offsets, cells, pos, sp = pack_structures(structures)
-        dev = _device()
+        _device()
         N = int(offsets[-1])
         S = len(structures)
-        d_pos = torch.from_numpy(pos).to(dev)
-        d_sp = torch.from_numpy(sp).to(dev)
         prec = _prec[precision or _default_precision[0]]
         cutoff = structures[0].cutoff
         for s in structures:
@@ -1072,14 +1091,12 @@ class SparseGP(_Training):
         out = None
         local_vars = []
         for m in models:
-            e = torch.zeros(S, dtype=torch.float64, device=dev)
-            f = torch.zeros((max(N, 1), 3), dtype=torch.float64, device=dev)
-            st = torch.zeros((S, 6), dtype=torch.float64, device=dev)
-            v = torch.zeros(max(N, 1), dtype=torch.float64, device=dev)
-            check(lib().fgb_predict(m.h, S, ptr(offsets), ptr(cells),
-                                    ptr(d_pos), ptr(d_sp), cutoff, int(want),
-                                    prec, ptr(e), ptr(f), ptr(st), ptr(v),
-                                    stream_ptr(stream)),
+            e, st = np.zeros(S), np.zeros((S, 6))
+            f, v = np.zeros((max(N, 1), 3)), np.zeros(max(N, 1))
+            check(lib().fgb_predict_host(m.h, S, ptr(offsets), ptr(cells),
+                                         ptr(pos), ptr(sp), cutoff, int(want),
+                                         prec, ptr(e), ptr(f), ptr(st), ptr(v),
+                                         stream_ptr(stream)),
                   "predict")
             if out is None:
                 out = [e, f, st]
@@ -1087,13 +1104,10 @@ class SparseGP(_Training):
                 out[0] += e
                 out[1] += f
                 out[2] += st
-            local_vars.append(v)
-        torch.cuda.current_stream().synchronize()
-        lv = [v.cpu().numpy()[:N] for v in local_vars]
-        return {"energy": out[0].cpu().numpy(),
-                "forces": out[1].cpu().numpy()[:N],
-                "stress": out[2].cpu().numpy(), "local_var": lv[0],
-                "local_vars": lv, "offsets": offsets}
+            local_vars.append(v[:N])
+        return {"energy": out[0], "forces": out[1][:N], "stress": out[2],
+                "local_var": local_vars[0], "local_vars": local_vars,
+                "offsets": offsets}
 
     def _predict_one(self, structure, want):
         r = self.predict_batch([structure], want)
@@ -1111,12 +1125,8 @@ class SparseGP(_Training):
         one array per kernel (each stored in its descriptor's
         species-sorted order, as the reference does)."""
         r = self._predict_one(structure, 0xF)
-        sp = np.asarray(structure.species)
-        out = []
-        for i, v in enumerate(r["local_vars"]):
-            S = structure.descriptor_calculators[i].descriptor_settings[0]
-            order = np.concatenate([np.nonzero(sp == s)[0] for s in range(S)])
-            out.append(v[order])
+        out = [v[structure.species_order(i)]
+               for i, v in enumerate(r["local_vars"])]
         structure.local_uncertainties = out
 
     def _stacked_kernel_matrix(self, structure):
@@ -1152,14 +1162,12 @@ class SparseGP(_Training):
         m = self._device_model(structure.descriptor_calculators)
         dev = _device()
         n_out = 1 + 3 * structure.noa + 6
-        mean = torch.zeros(n_out, dtype=torch.float64, device=dev)
-        var = torch.zeros(n_out, dtype=torch.float64, device=dev)
+        both = torch.empty((2, n_out), dtype=torch.float64, device=dev)
         d = structure._inputs()
         check(lib().fgb_predict_sor(m.h, structure.nlist().h, ptr(d["species"]),
-                                    ptr(mean), ptr(var), stream_ptr()),
+                                    ptr(both[0]), ptr(both[1]), stream_ptr()),
               "predict_SOR")
-        structure.mean_efs = mean.cpu().numpy()
-        structure.variance_efs = var.cpu().numpy()
+        structure.mean_efs, structure.variance_efs = both.cpu().numpy()
 
     def predict_DTC(self, structure):
         """sparse_gp.cpp:694-729: mean_efs and the DTC variances K_self -
@@ -1187,14 +1195,12 @@ class SparseGP(_Training):
         m = self._device_model(structure.descriptor_calculators)
         dev = _device()
         n_out = 1 + 3 * structure.noa + 6
-        mean = torch.zeros(n_out, dtype=torch.float64, device=dev)
-        var = torch.zeros(n_out, dtype=torch.float64, device=dev)
+        both = torch.empty((2, n_out), dtype=torch.float64, device=dev)
         d = structure._inputs()
         check(lib().fgb_predict_dtc(m.h, structure.nlist().h, ptr(d["species"]),
-                                    ptr(mean), ptr(var), stream_ptr()),
+                                    ptr(both[0]), ptr(both[1]), stream_ptr()),
               "predict_DTC")
-        structure.mean_efs = mean.cpu().numpy()
-        structure.variance_efs = var.cpu().numpy()
+        structure.mean_efs, structure.variance_efs = both.cpu().numpy()
 
     def mixed_plan(self, kernel_index=0):
         """The mixed path's precision plan for one kernel of this model:
@@ -1255,10 +1261,6 @@ class SparseGP(_Training):
     def compute_cluster_uncertainties(self, structure):
         """sparse_gp.cpp:94-139 (species-sorted variances)."""
         r = self.predict_batch([structure], _lib.FGB_WANT_LOCAL_VAR)
-        sp = np.asarray(structure.species)
-        out = []
-        for i, v in enumerate(r["local_vars"]):
-            S = structure.descriptor_calculators[i].descriptor_settings[0]
-            order = np.concatenate([np.nonzero(sp == s)[0] for s in range(S)])
-            out.append(v[order])
+        out = [v[structure.species_order(i)]
+               for i, v in enumerate(r["local_vars"])]
         return out

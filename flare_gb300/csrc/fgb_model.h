@@ -15,6 +15,7 @@
 struct fgb_pinned_counts {
   static constexpr int kInts = 2 * (fgb::kMaxSpecies + 1);
   int *h = nullptr;
+  int *status = nullptr;   // page-locked, 8 ints: a call's error flags
   cudaEvent_t ev = nullptr;
   bool pageable = false;
   int host[kInts] = {};
@@ -23,6 +24,7 @@ struct fgb_pinned_counts {
   fgb_pinned_counts &operator=(const fgb_pinned_counts &) = delete;
   ~fgb_pinned_counts() {
     if (h && !pageable) cudaFreeHost(h);
+    if (status) cudaFreeHost(status);
     if (ev) cudaEventDestroy(ev);
   }
 };
@@ -60,8 +62,20 @@ struct fgb_workspace {
   }
 };
 
+// Device inputs and outputs of a prediction from host memory, each one block
+// ([positions | species], [energies | stresses | variances | forces]), and
+// page-locked staging for small ones (one copy each way; larger ones are
+// copied from and to the caller's arrays).
 struct fgb_io {
-  fgb::DevBuf pos, species, energy, forces, stress, var;
+  static constexpr size_t kStage = 256 * 1024;   // bytes each way
+  fgb::DevBuf in, out;
+  unsigned char *stage = nullptr;   // 2 kStage: in, out
+  fgb_io() = default;
+  fgb_io(const fgb_io &) = delete;
+  fgb_io &operator=(const fgb_io &) = delete;
+  ~fgb_io() {
+    if (stage) cudaFreeHost(stage);
+  }
 };
 
 struct fgb_model_s {
@@ -169,6 +183,10 @@ struct PredictHostIO {
   const int *species = nullptr;
   double *energy = nullptr, *forces = nullptr, *stress = nullptr,
          *local_var = nullptr;
+  // the results' device block and its staging (null: copied one by one)
+  const void *block = nullptr;
+  void *stage = nullptr;
+  size_t bytes = 0;
 };
 
 // One batched prediction on device positions (predict.cu): the body of

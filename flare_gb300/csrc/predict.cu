@@ -895,7 +895,11 @@ int predict_impl(fgb_model_s *m, int n_struc, const int *h_atom_offsets,
       return rc;
   }
   if (fixed) return FGB_OK;
-  if (hio) {   // results to the host ahead of the one synchronisation below
+  // results to the host ahead of the one synchronisation below
+  if (hio && hio->stage) {
+    FGB_CUDA(cudaMemcpyAsync(hio->stage, hio->block, hio->bytes,
+                             cudaMemcpyDeviceToHost, st));
+  } else if (hio) {
     if (hio->energy && want_e)
       FGB_CUDA(cudaMemcpyAsync(hio->energy, d_energy, sizeof(double) * n_struc,
                                cudaMemcpyDeviceToHost, st));
@@ -910,7 +914,11 @@ int predict_impl(fgb_model_s *m, int n_struc, const int *h_atom_offsets,
                                sizeof(double) * N, cudaMemcpyDeviceToHost, st));
   }
   // deferred checks: neighbour-list consistency, tensor-core waits
-  int h[5] = {0, 0, 0, 0, 0};
+  if (!m->ws.counts.status)
+    FGB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&m->ws.counts.status),
+                           sizeof(int) * 8, cudaHostAllocDefault));
+  int *h = m->ws.counts.status;
+  h[4] = 0;
   FGB_CUDA(cudaMemcpyAsync(h, m->nl.flag.p, sizeof(int) * 4,
                            cudaMemcpyDeviceToHost, st));
   if (sliced)
@@ -961,19 +969,33 @@ extern "C" int fgb_predict_host(fgb_model_t m, int n_struc,
   cudaStream_t st = (cudaStream_t)stream;
   const int N = h_atom_offsets[n_struc];
   int rc;
-  if ((rc = m->io.pos.ensure(sizeof(double) * (3 * (size_t)N + 1))) ||
-      (rc = m->io.species.ensure(sizeof(int) * (N + 1))) ||
-      (rc = m->io.energy.ensure(sizeof(double) * (n_struc + 1))) ||
-      (rc = m->io.forces.ensure(sizeof(double) * (3 * (size_t)N + 1))) ||
-      (rc = m->io.stress.ensure(sizeof(double) * (6 * (size_t)n_struc + 1))) ||
-      (rc = m->io.var.ensure(sizeof(double) * (N + 1))))
+  const size_t in_pos = sizeof(double) * 3 * (size_t)N;
+  const size_t in_bytes = in_pos + sizeof(int) * (size_t)N;
+  const size_t S = n_struc;
+  const size_t out_bytes = sizeof(double) * (7 * S + 4 * (size_t)N);
+  fgb_io &io = m->io;
+  if ((rc = io.in.ensure(in_bytes + 16)) || (rc = io.out.ensure(out_bytes + 16)))
     return rc;
-  if (N > 0) {
-    FGB_CUDA(cudaMemcpyAsync(m->io.pos.p, h_positions, sizeof(double) * 3 * N,
+  const bool stage_in = in_bytes <= fgb_io::kStage,
+             stage_out = out_bytes <= fgb_io::kStage;
+  if ((stage_in || stage_out) && !io.stage)
+    FGB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&io.stage),
+                           2 * fgb_io::kStage, cudaHostAllocDefault));
+  double *d_pos = io.in.as<double>();
+  int *d_species = reinterpret_cast<int *>(d_pos + 3 * (size_t)N);
+  if (N > 0 && stage_in) {
+    std::memcpy(io.stage, h_positions, in_pos);
+    std::memcpy(io.stage + in_pos, h_species, in_bytes - in_pos);
+    FGB_CUDA(cudaMemcpyAsync(d_pos, io.stage, in_bytes, cudaMemcpyHostToDevice,
+                             st));
+  } else if (N > 0) {
+    FGB_CUDA(cudaMemcpyAsync(d_pos, h_positions, in_pos,
                              cudaMemcpyHostToDevice, st));
-    FGB_CUDA(cudaMemcpyAsync(m->io.species.p, h_species, sizeof(int) * N,
+    FGB_CUDA(cudaMemcpyAsync(d_species, h_species, in_bytes - in_pos,
                              cudaMemcpyHostToDevice, st));
   }
+  double *d_e = io.out.as<double>(), *d_s = d_e + S, *d_v = d_s + 6 * S,
+         *d_f = d_v + N;
   // species counted on the host (no read-back) and results copied back
   // before the prediction's final synchronisation
   PredictHostIO hio;
@@ -982,11 +1004,28 @@ extern "C" int fgb_predict_host(fgb_model_t m, int n_struc,
   hio.forces = h_forces;
   hio.stress = h_stress;
   hio.local_var = h_local_var;
-  return predict_impl(m, n_struc, h_atom_offsets, h_cells,
-                      m->io.pos.as<double>(), m->io.species.as<int>(), cutoff,
-                      want, precision, m->io.energy.as<double>(),
-                      m->io.forces.as<double>(), m->io.stress.as<double>(),
-                      m->io.var.as<double>(), st, nullptr, &hio);
+  unsigned char *out = io.stage + fgb_io::kStage;
+  if (stage_out) {
+    hio.block = d_e;
+    hio.stage = out;
+    hio.bytes = out_bytes;
+  }
+  if ((rc = predict_impl(m, n_struc, h_atom_offsets, h_cells, d_pos, d_species,
+                         cutoff, want, precision, d_e, d_f, d_s, d_v, st,
+                         nullptr, &hio)))
+    return rc;
+  if (stage_out) {
+    const double *r = reinterpret_cast<const double *>(out);
+    if (h_energy && (want & FGB_WANT_ENERGY))
+      std::memcpy(h_energy, r, sizeof(double) * S);
+    if (h_stress && (want & FGB_WANT_STRESS))
+      std::memcpy(h_stress, r + S, sizeof(double) * 6 * S);
+    if (h_local_var && (want & FGB_WANT_LOCAL_VAR))
+      std::memcpy(h_local_var, r + 7 * S, sizeof(double) * N);
+    if (h_forces && (want & FGB_WANT_FORCES))
+      std::memcpy(h_forces, r + 7 * S + N, sizeof(double) * 3 * N);
+  }
+  return FGB_OK;
 }
 
 extern "C" int fgb_model_set_R_inv(fgb_model_t m, const double *h_R_inv) {

@@ -379,16 +379,22 @@ def _run(handle_fn, structures):
     N, S = int(offsets[-1]), len(structures)
     d_pos = torch.from_numpy(pos).to(dev)
     d_sp = torch.from_numpy(sp).to(dev)
-    out = {"energy": torch.zeros(S, dtype=torch.float64, device=dev),
-           "forces": torch.zeros((max(N, 1), 3), dtype=torch.float64, device=dev),
-           "stress": torch.zeros((S, 6), dtype=torch.float64, device=dev),
-           "atom_energies": torch.zeros(max(N, 1), dtype=torch.float64, device=dev),
-           "local_var": torch.zeros(max(N, 1), dtype=torch.float64, device=dev)}
-    handle_fn(S, offsets, cells, d_pos, d_sp, out)
-    torch.cuda.current_stream().synchronize()
-    return {k: (v.cpu().numpy()[:N] if k in ("forces", "atom_energies",
-                                             "local_var") else v.cpu().numpy())
-            for k, v in out.items()}, offsets
+    # one block of results, copied back at once
+    n1 = max(N, 1)
+    shapes = {"energy": (S,), "stress": (S, 6), "forces": (n1, 3),
+              "atom_energies": (n1,), "local_var": (n1,)}
+    sizes = [int(np.prod(s)) for s in shapes.values()]
+    block = torch.empty(sum(sizes), dtype=torch.float64, device=dev)
+
+    def split(flat):
+        return {k: x.reshape(s) for (k, s), x in zip(
+            shapes.items(), (flat[e - n:e] for n, e in
+                             zip(sizes, np.cumsum(sizes).tolist())))}
+
+    handle_fn(S, offsets, cells, d_pos, d_sp, split(block))
+    r = split(block.cpu().numpy())
+    return {k: v[:N] if k in ("forces", "atom_energies", "local_var") else v
+            for k, v in r.items()}, offsets
 
 
 class MappedPotential:
@@ -471,16 +477,13 @@ class LocalStdFromFiles:
 
     def std(self, structures, precision="fp64"):
         offsets, cells, pos, sp = pack_structures(structures)
-        dev = _device()
+        _device()
         N, S = int(offsets[-1]), len(structures)
-        d_pos = torch.from_numpy(pos).to(dev)
-        d_sp = torch.from_numpy(sp).to(dev)
-        v = torch.zeros(max(N, 1), dtype=torch.float64, device=dev)
+        v = np.zeros(max(N, 1))
         prec = {"fp64": _lib.FGB_PREC_FP64, "mixed": _lib.FGB_PREC_MIXED}[precision]
-        check(lib().fgb_predict(self._model.h, S, ptr(offsets), ptr(cells),
-                                ptr(d_pos), ptr(d_sp), self.cutoff,
-                                _lib.FGB_WANT_LOCAL_VAR, prec, None, None,
-                                None, ptr(v), stream_ptr()), "LocalStdFromFiles")
-        torch.cuda.current_stream().synchronize()
-        var = v.cpu().numpy()[:N] / self.sigma ** 2
+        check(lib().fgb_predict_host(
+            self._model.h, S, ptr(offsets), ptr(cells), ptr(pos), ptr(sp),
+            self.cutoff, _lib.FGB_WANT_LOCAL_VAR, prec, None, None, None,
+            ptr(v), stream_ptr()), "LocalStdFromFiles")
+        var = v[:N] / self.sigma ** 2
         return np.sign(var) * np.sqrt(np.abs(var))
