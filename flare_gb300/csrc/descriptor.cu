@@ -67,7 +67,12 @@ __device__ __forceinline__ df finish(df a) {
 // Shared memory: A[nA] | g[kChunk*nmax] | Y[kChunk*nh] | sp[kChunk] | red,
 // in the compute type T: double (FP64 path) or df (double-float, the
 // mixed-precision path; the pair geometry arrives in FP64 and is split).
-template <typename T, int NC, int LC>
+// NS: threads per (species, lm) of the A contraction (NC / NS accumulators
+// each), more than one where few (species, lm) would leave most of the
+// block's threads idle (one species, l_max 3: 64 threads busy instead of 16;
+// 2,048 atoms, double-float: 35.7 -> 25 us).  A template, because the loops
+// over the accumulators of NS = 1 cost 5% with NS at run time.
+template <typename T, int NC, int LC, int NS>
 __global__ void __launch_bounds__(kChunk, 12)
 k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
              const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
@@ -112,9 +117,9 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
   const int si_raw = species[i];
   const bool si_ok = si_raw >= 0 && si_raw < ns;
   const int si = si_ok ? si_raw : 0;
-  T areg[NC > 0 ? NC : 1];
+  T areg[NC > 0 ? NC / NS : 1];
 #pragma unroll
-  for (int n = 0; n < (NC > 0 ? NC : 1); n++) areg[n] = T(0);
+  for (int n = 0; n < (NC > 0 ? NC / NS : 1); n++) areg[n] = T(0);
   if (!regA)
     for (int e = t; e < nA; e += blockDim.x) A[e] = T(0);
   const long long b = offsets[i], e_ = offsets[i + 1];
@@ -129,7 +134,10 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
       double rc = ok ? p.cutoffs[si * kMaxSpecies + sj] : 0.0;
       if (ok && r.x <= rc) {
         radial_eval<T, NC>(p, T(r.x), T(rc), sg + t * nm, (T *)nullptr);
-        ylm_eval<T, LC>(p.l_max, T(r.y), T(r.z), T(r.w), sy + t * nh, nullptr);
+        if constexpr (std::is_same<T, double>::value)
+          ylm_eval<T, LC>(p.l_max, r.y, r.z, r.w, sy + t * nh, nullptr, r.x);
+        else
+          ylm_eval<T, LC>(p.l_max, T(r.y), T(r.z), T(r.w), sy + t * nh, nullptr);
       } else {
         sj = -1;
       }
@@ -163,23 +171,27 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
       if (sj >= 0)
         sord[sbeg[sj] + (warp ? scnt[sj] : 0) + rank] = t;
       __syncthreads();
-      for (int it = t; it < S * NH; it += blockDim.x) {
-        const int s = it / NH, lm = it % NH;
-        T acc[NC];
+      constexpr int NP = NC / NS;
+      for (int it = t; it < S * NH * NS; it += blockDim.x) {
+        const int part = it % NS, e = it / NS;
+        const int s = e / NH, lm = e % NH;
+        T acc[NP];
 #pragma unroll
-        for (int n = 0; n < NC; n++) acc[n] = T(0);
+        for (int n = 0; n < NP; n++) acc[n] = T(0);
         for (int q = sbeg[s]; q < sbeg[s + 1]; q++) {
           const int pq = sord[q];
           const T y = sy[pq * NH + lm];
 #pragma unroll
-          for (int n = 0; n < NC; n++) mac(acc[n], sg[pq * NC + n], y);
+          for (int n = 0; n < NP; n++)
+            mac(acc[n], sg[pq * NC + part * NP + n], y);
         }
         if (regA) {
 #pragma unroll
-          for (int n = 0; n < NC; n++) areg[n] += finish(acc[n]);
+          for (int n = 0; n < NP; n++) areg[n] += finish(acc[n]);
         } else {
 #pragma unroll
-          for (int n = 0; n < NC; n++) A[(s * NC + n) * NH + lm] += finish(acc[n]);
+          for (int n = 0; n < NP; n++)
+            A[(s * NC + part * NP + n) * NH + lm] += finish(acc[n]);
         }
       }
     } else {
@@ -202,10 +214,13 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
     A = sy + (kChunk * nh - nA);
     if constexpr (kFixed) {
       constexpr int NH = (LC + 1) * (LC + 1);
-      if (t < p.n_species * NH) {
-        const int s = t / NH, lm = t % NH;
+      constexpr int NP = NC / NS;
+      if (t < p.n_species * NH * NS) {
+        const int part = t % NS, e = t / NS;
+        const int s = e / NH, lm = e % NH;
 #pragma unroll
-        for (int n = 0; n < NC; n++) A[(s * NC + n) * NH + lm] = areg[n];
+        for (int n = 0; n < NP; n++)
+          A[(s * NC + part * NP + n) * NH + lm] = areg[n];
       }
     }
     __syncthreads();
@@ -314,6 +329,99 @@ __device__ __forceinline__ float3 pair_out(float x, float y, float z) {
   return make_float3(x, y, z);
 }
 
+// dE/dr of one pair in FP64: dE/dr = e sum_lm d_lm Y_lm + sum_lm c_lm grad
+// Y_lm with c_lm = sum_n u[lm][n] g_n and d_lm = sum_n u[lm][n] dg_n.  The
+// sums over l run inside those over m, on the common factors of the
+// harmonics (l, +m) and (l, -m), and the projection onto the tangent plane is
+// applied once to the summed gradient: 6 multiply-adds for two harmonics
+// beside the 2 n_max of each instead of about 25 for each.  FP64 instructions
+// bound this kernel (84,000 pairs, n_max 8, l_max 4: 253 -> 191 us).
+template <int NC, int LC>
+__device__ __forceinline__ double3 pair_gradient64(
+    int Lrt, double r, double x, double y, double z,
+    const double *__restrict__ u, int nm_rt, const double *g,
+    const double *dg) {
+  constexpr int LA = LC > 0 ? LC : kMaxL;
+  const int L = LC > 0 ? LC : Lrt, nm = NC > 0 ? NC : nm_rt;
+  const double ir = 1.0 / r;
+  const double ux = x * ir, uy = y * ir, uz = z * ir;
+  double C[LA + 1], S[LA + 1];
+  C[0] = 1.0;
+  S[0] = 0.0;
+#pragma unroll
+  for (int m = 1; m <= L; m++) {
+    C[m] = ux * C[m - 1] - uy * S[m - 1];
+    S[m] = ux * S[m - 1] + uy * C[m - 1];
+  }
+  double qnext[LA + 2], qcur[LA + 2];   // Q_l^{m+1}, Q_l^m
+#pragma unroll
+  for (int l = 0; l <= L + 1; l++) qnext[l] = 0.0;
+  double orad = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
+#pragma unroll
+  for (int m = L; m >= 0; m--) {
+    double dfact;
+    dfact_const(m, dfact);
+#pragma unroll
+    for (int l = 0; l <= L; l++) qcur[l] = 0.0;
+    qcur[m] = dfact;
+    if (m + 1 <= L) qcur[m + 1] = (double)(2 * m + 1) * uz * dfact;
+#pragma unroll
+    for (int l = m + 2; l <= L; l++)
+      qcur[l] = div_int((double)(2 * l - 1) * uz * qcur[l - 1] -
+                            (double)(l + m - 1) * qcur[l - 2],
+                        l - m);
+    // sums over l of K Q c, K Q' c and K Q d for +m and -m
+    double t1 = 0.0, t2 = 0.0, w1 = 0.0, w2 = 0.0, v1 = 0.0, v2 = 0.0;
+#pragma unroll
+    for (int l = m; l <= L; l++) {
+      const double K = c_ylm_norm[l * (kMaxL + 1) + m];
+      const double qv = K * qcur[l], qd = K * qnext[l];
+      const double *up = u + (l * l + l + m) * nm;
+      double c = 0.0, d = 0.0;
+#pragma unroll
+      for (int n = 0; n < nm; n++) {
+        const double a = up[n];
+        c = fma(a, g[n], c);
+        d = fma(a, dg[n], d);
+      }
+      t1 = fma(qv, c, t1);
+      w1 = fma(qd, c, w1);
+      v1 = fma(qv, d, v1);
+      if (m > 0) {
+        const double *un = u + (l * l + l - m) * nm;
+        c = 0.0;
+        d = 0.0;
+#pragma unroll
+        for (int n = 0; n < nm; n++) {
+          const double a = un[n];
+          c = fma(a, g[n], c);
+          d = fma(a, dg[n], d);
+        }
+        t2 = fma(qv, c, t2);
+        w2 = fma(qd, c, w2);
+        v2 = fma(qv, d, v2);
+      }
+    }
+    if (m == 0) {
+      orad += v1;
+      g2 += w1;
+    } else {
+      t1 *= (double)m;
+      t2 *= (double)m;
+      g0 = fma(t1, C[m - 1], fma(t2, S[m - 1], g0));
+      g1 = fma(t2, C[m - 1], fma(-t1, S[m - 1], g1));
+      g2 = fma(w1, C[m], fma(w2, S[m], g2));
+      orad = fma(v1, C[m], fma(v2, S[m], orad));
+    }
+#pragma unroll
+    for (int l = 0; l <= L; l++) qnext[l] = qcur[l];
+  }
+  const double ug = ux * g0 + uy * g1 + uz * g2;
+  return make_double3(fma(orad, ux, (g0 - ux * ug) * ir),
+                      fma(orad, uy, (g1 - uy * ug) * ir),
+                      fma(orad, uz, (g2 - uz * ug) * ir));
+}
+
 // Atoms per block of the adjoint and its block size: ~42 pairs per atom,
 // so three atoms' pairs fill the 128 threads of the pair loop.
 // The 2l + 1 entries u[c][l^2 .. l^2 + 2l] (M = 2l + 1 at compile time),
@@ -373,6 +481,7 @@ __device__ void u_entries_any(const T *A, const T *wsrc, int nh, int nr,
 }
 
 constexpr int kAdjAtoms = 3;
+constexpr int kAdjFew = 608;   // four blocks on each of 152 SMs
 // Shared-memory values per atom of the adjoint: u and A (n_A each) and
 // optionally the dE/dB2 row, rounded up to whole groups of 4.
 __host__ __device__ constexpr int adj_atom_values(int nA, int nd_in_smem) {
@@ -385,10 +494,13 @@ constexpr int kAdjThreads = 128;
 // loads, recurrence chains): the FP32 kernel is held to 48 registers for
 // 10 blocks (40 warps) per SM.  On the alloy workload that measured 0.212
 // ms per 32k atoms, against 0.244 ms at 8 blocks (64 registers) and 0.232
-// ms at 12 (40 registers, more spilled values).
+// ms at 12 (40 registers, more spilled values).  The FP64 kernel, bound by
+// its FP64 instructions, takes 4 blocks (8,000 atoms: 650 us against 736 at 2,
+// 666 at 3 and 650 at 5).
 template <typename T, int NC, int LC>
-__global__ void __launch_bounds__(kAdjThreads, sizeof(T) == 4 ? 10 : 2)
-k_b2_adjoint(B2Params p, int n_atoms, const long long *__restrict__ offsets,
+__global__ void __launch_bounds__(kAdjThreads, sizeof(T) == 4 ? 10 : 4)
+k_b2_adjoint(B2Params p, int n_atoms, int apb,
+             const long long *__restrict__ offsets,
              const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
              const int *__restrict__ species, const double *__restrict__ A_in,
              const float *__restrict__ A_in32, const T *__restrict__ gB2,
@@ -396,9 +508,9 @@ k_b2_adjoint(B2Params p, int n_atoms, const long long *__restrict__ offsets,
              int w_in_smem) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *smem = reinterpret_cast<T *>(smem_raw);
-  const int i0 = blockIdx.x * kAdjAtoms;
+  const int i0 = blockIdx.x * apb;
   if (i0 >= n_atoms) return;
-  const int na = min(kAdjAtoms, n_atoms - i0);
+  const int na = min(apb, n_atoms - i0);
   constexpr int NA = NC > 0 ? NC : kMaxNmax;
   const int nh = LC > 0 ? (LC + 1) * (LC + 1) : p.n_harm;
   const int nm = NC > 0 ? NC : p.n_max;
@@ -494,38 +606,51 @@ k_b2_adjoint(B2Params p, int n_atoms, const long long *__restrict__ offsets,
               rz = as_compute(r.z, T(0)), rw = as_compute(r.w, T(0));
       radial_eval<T, NC>(p, rx, as_compute(rc, T(0)), g, dg);
       const T *us = u + sj * nm * nh;
-      T orad = T(0), ox = T(0), oy = T(0), oz = T(0);
-      ylm_visit<T, LC, true>(p.l_max, ry, rz, rw,
-                             [&](int idx, T v, T gx, T gy, T gz) {
-        T c = T(0), d = T(0);
-        const T *ul = us + idx * nm;
-        if constexpr (std::is_same<T, float>::value && NC > 0 && NC % 4 == 0) {
-          // n_max values of the harmonic in 16-byte loads (u rows start on
-          // 16-byte boundaries: per and n_max n_harm are whole 4-groups)
+      if constexpr (std::is_same<T, double>::value) {
+        out = pair_gradient64<NC, LC>(p.l_max, rx, ry, rz, rw, us, nm, g, dg);
+      } else {
+        T orad = T(0), ox = T(0), oy = T(0), oz = T(0);
+        ylm_visit<T, LC, true>(p.l_max, ry, rz, rw,
+                               [&](int idx, T v, T gx, T gy, T gz) {
+          T c = T(0), d = T(0);
+          const T *ul = us + idx * nm;
+          if constexpr (std::is_same<T, float>::value && NC > 0 && NC % 4 == 0) {
+            // n_max values of the harmonic in 16-byte loads (u rows start on
+            // 16-byte boundaries: per and n_max n_harm are whole 4-groups)
 #pragma unroll
-          for (int q = 0; q < NC / 4; q++) {
-            const float4 uv = reinterpret_cast<const float4 *>(ul)[q];
-            c += uv.x * g[4 * q];     d += uv.x * dg[4 * q];
-            c += uv.y * g[4 * q + 1]; d += uv.y * dg[4 * q + 1];
-            c += uv.z * g[4 * q + 2]; d += uv.z * dg[4 * q + 2];
-            c += uv.w * g[4 * q + 3]; d += uv.w * dg[4 * q + 3];
-          }
-        } else {
+            for (int q = 0; q < NC / 4; q++) {
+              const float4 uv = reinterpret_cast<const float4 *>(ul)[q];
+              c += uv.x * g[4 * q];     d += uv.x * dg[4 * q];
+              c += uv.y * g[4 * q + 1]; d += uv.y * dg[4 * q + 1];
+              c += uv.z * g[4 * q + 2]; d += uv.z * dg[4 * q + 2];
+              c += uv.w * g[4 * q + 3]; d += uv.w * dg[4 * q + 3];
+            }
+          } else if constexpr (std::is_same<T, float>::value && NC > 0 &&
+                               NC % 2 == 0) {
+            // 8-byte loads (per, n_max n_harm and n_max are even)
 #pragma unroll
-          for (int n = 0; n < nm; n++) {
-            const T uv = ul[n];
-            c += uv * g[n];
-            d += uv * dg[n];
+            for (int q = 0; q < NC / 2; q++) {
+              const float2 uv = reinterpret_cast<const float2 *>(ul)[q];
+              c += uv.x * g[2 * q];     d += uv.x * dg[2 * q];
+              c += uv.y * g[2 * q + 1]; d += uv.y * dg[2 * q + 1];
+            }
+          } else {
+#pragma unroll
+            for (int n = 0; n < nm; n++) {
+              const T uv = ul[n];
+              c += uv * g[n];
+              d += uv * dg[n];
+            }
           }
-        }
-        orad += d * v;
-        ox += c * gx;
-        oy += c * gy;
-        oz += c * gz;
-      });
-      const T ir = T(1) / rx;
-      out = pair_out(orad * (ry * ir) + ox, orad * (rz * ir) + oy,
-                     orad * (rw * ir) + oz);
+          orad += d * v;
+          ox += c * gx;
+          oy += c * gy;
+          oz += c * gz;
+        });
+        const T ir = T(1) / rx;
+        out = pair_out(orad * (ry * ir) + ox, orad * (rz * ir) + oy,
+                       orad * (rw * ir) + oz);
+      }
     }
     pair_grad[pp] = out;
   }
@@ -657,8 +782,18 @@ static void dispatch_nl(const B2Params &p, F &&f) {
 
 template <typename T, int NC, int LC>
 struct FwdK {
-  static constexpr auto fn = k_b2_forward<T, NC, LC>;
   static constexpr bool kFixed = NC > 0 && LC > 0;
+  static constexpr int kNH = (LC + 1) * (LC + 1);
+  // calls g with the kernel for S species: the most threads per (species,
+  // lm) that one block holds with A in registers
+  template <typename G>
+  static void with(int S, G &&g) {
+    if constexpr (kFixed && NC % 4 == 0 && 4 * kNH <= kChunk)
+      if (4 * S * kNH <= kChunk) return g(k_b2_forward<T, NC, LC, 4>);
+    if constexpr (kFixed && NC % 2 == 0 && 2 * kNH <= kChunk)
+      if (2 * S * kNH <= kChunk) return g(k_b2_forward<T, NC, LC, 2>);
+    g(k_b2_forward<T, NC, LC, 1>);
+  }
 };
 template <typename T, int NC, int LC>
 struct AdjK {
@@ -679,23 +814,29 @@ int launch_b2_forward(const B2Params &p, const fgb_nlist_s *nl,
   }
   cudaError_t e = cudaSuccess;
   auto go = [&](auto k) {
-    auto fn = decltype(k)::fn;
     // the specialised kernels keep A in registers when one (species, lm)
     // per thread covers it (the same test as in the kernel)
     const bool regA = decltype(k)::kFixed && p.n_species * p.n_harm <= kChunk &&
                       p.n_species * p.n_max <= kChunk;
     const size_t sm = b2_forward_smem(p, regA);
-    // all of the SM's unified memory as shared memory: twelve blocks of
-    // ~19 KB each
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm);
-    if (e != cudaSuccess) return;
-    fn<<<N, kChunk, sm, st>>>(p, N, nl->offsets.as<long long>(),
-                              nl->nbr_j.as<int>(), nl->nbr_rel.as<double4_16a>(),
-                              d_species, d_A, d_B2, d_norms, d_rowmax, d_A32);
+    const auto launch = [&](auto fn) {
+      // all of the SM's unified memory as shared memory: twelve blocks of
+      // ~19 KB each
+      e = cudaFuncSetAttribute(fn,
+                               cudaFuncAttributePreferredSharedMemoryCarveout,
+                               cudaSharedmemCarveoutMaxShared);
+      if (e != cudaSuccess) return;
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sm);
+      if (e != cudaSuccess) return;
+      fn<<<N, kChunk, sm, st>>>(p, N, nl->offsets.as<long long>(),
+                                nl->nbr_j.as<int>(),
+                                nl->nbr_rel.as<double4_16a>(), d_species, d_A,
+                                d_B2, d_norms, d_rowmax, d_A32);
+    };
+    // without A in registers (more radial values than threads) no split
+    if (regA) decltype(k)::with(p.n_species, launch);
+    else decltype(k)::with(kMaxSpecies * kChunk, launch);
   };
   if (dfloat) dispatch_nl<FwdK, df>(p, go);
   else dispatch_nl<FwdK, double>(p, go);
@@ -717,7 +858,11 @@ int launch_b2_adjoint(const B2Params &p, const fgb_nlist_s *nl,
     set_error("B2 adjoint needs %zu bytes of shared memory", sm);
     return FGB_EINVAL;
   }
-  const size_t smw = es * (size_t)adj_atom_values(p.n_A, p.n_d) * kAdjAtoms;
+  // few atoms: one a block, so that they reach all SMs (32 atoms FP64: 34 ->
+  // 30 us, 256 atoms FP32: 8.3 -> 7.6)
+  const int apb = N <= kAdjFew ? 1 : kAdjAtoms;
+  sm = es * (size_t)adj_atom_values(p.n_A, 0) * apb;
+  const size_t smw = es * (size_t)adj_atom_values(p.n_A, p.n_d) * apb;
   const int w_in_smem = smw <= 96 * 1024 ? 1 : 0;
   if (w_in_smem) sm = smw;
   cudaError_t e = cudaSuccess;
@@ -727,8 +872,8 @@ int launch_b2_adjoint(const B2Params &p, const fgb_nlist_s *nl,
                              (int)sm);
     if (e != cudaSuccess) return;
     using G = typename decltype(k)::type;   // dE/dB2 in the compute type
-    fn<<<ceil_div(N, kAdjAtoms), kAdjThreads, sm, st>>>(
-        p, N, nl->offsets.as<long long>(), nl->nbr_j.as<int>(),
+    fn<<<ceil_div(N, apb), kAdjThreads, sm, st>>>(
+        p, N, apb, nl->offsets.as<long long>(), nl->nbr_j.as<int>(),
         nl->nbr_rel.as<double4_16a>(), d_species, d_A,
         fp32 ? d_A32 : nullptr, static_cast<const G *>(d_gB2),
         static_cast<typename PairGrad<G>::type *>(d_pair_grad), w_in_smem);

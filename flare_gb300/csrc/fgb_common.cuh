@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
+#include <type_traits>
 
 #include "flaregb.h"
 
@@ -120,14 +121,20 @@ static_assert(kMaxL == 10, "the double-factorial and reciprocal tables");
 static __constant__ double c_dfact[kMaxL + 1] = {FGB_DFACT(FGB_AS_F64)};
 static __constant__ float c_dfact_f[kMaxL + 1] = {FGB_DFACT(FGB_AS_F32)};
 static __constant__ float c_dfact_lo[kMaxL + 1] = {FGB_DFACT(FGB_AS_F32_LO)};
+static __constant__ double c_inv[kNumInv] = {FGB_INV(FGB_AS_F64)};
 static __constant__ float c_inv_f[kNumInv] = {FGB_INV(FGB_AS_F32)};
 static __constant__ float c_inv_lo[kNumInv] = {FGB_INV(FGB_AS_F32_LO)};
 
 __device__ __forceinline__ void dfact_const(int m, double &v) { v = c_dfact[m]; }
 __device__ __forceinline__ void dfact_const(int m, float &v) { v = c_dfact_f[m]; }
-// x / k for a small positive integer k
+// x / k for a small positive integer k.  FP64: the product with 1/k rounded
+// to nearest and Markstein's correction step (P. W. Markstein, IBM J. Res.
+// Dev. 34, 1990), which rounds the quotient correctly: 3 FP64 instructions
+// where a division takes about ten.
 __device__ __forceinline__ double div_int(double x, int k) {
-  return x / (double)k;
+  const double inv = c_inv[k], q = x * inv;
+  if ((k & (k - 1)) == 0) return q;     // powers of two are exact
+  return fma(fma(-q, (double)k, x), inv, q);
 }
 __device__ __forceinline__ float div_int(float x, int k) {
   return x * c_inv_f[k];
@@ -340,11 +347,17 @@ __device__ __forceinline__ void radial_eval(const B2Params &p, T r, T rc,
 // m = L..0, l = m..L) with the Cartesian gradient when Grad (zeros
 // otherwise).  LC > 0 fixes l_max at compile time (loops unrolled, the
 // recurrence state kept in registers); LC = 0 takes Lrt.
+// rk > 0: the vector's length, known to the caller.
 template <typename T, int LC, bool Grad, typename Fn>
-__device__ __forceinline__ void ylm_visit(int Lrt, T x, T y, T z, Fn &&fn) {
+__device__ __forceinline__ void ylm_visit(int Lrt, T x, T y, T z, Fn &&fn,
+                                          double rk = 0.0) {
   constexpr int LA = LC > 0 ? LC : kMaxL;
   const int L = LC > 0 ? LC : Lrt;
-  T r = sqrt(x * x + y * y + z * z);
+  T r;
+  if constexpr (std::is_same<T, double>::value)
+    r = rk > 0.0 ? rk : sqrt(x * x + y * y + z * z);
+  else
+    r = sqrt(x * x + y * y + z * z);
   T ir = T(1) / r;
   T ux = x * ir, uy = y * ir, uz = z * ir;
   T C[LA + 1], S[LA + 1];
@@ -414,17 +427,18 @@ __device__ __forceinline__ void ylm_visit(int Lrt, T x, T y, T z, Fn &&fn) {
 // The harmonics into Y[] (and, if Yd != nullptr, the Cartesian gradient
 // into Yd[3*idx + k]).
 template <typename T, int LC = 0>
-__device__ __forceinline__ void ylm_eval(int L, T x, T y, T z, T *Y, T *Yd) {
+__device__ __forceinline__ void ylm_eval(int L, T x, T y, T z, T *Y, T *Yd,
+                                         double rk = 0.0) {
   if (Yd) {
     ylm_visit<T, LC, true>(L, x, y, z, [&](int idx, T v, T gx, T gy, T gz) {
       Y[idx] = v;
       Yd[3 * idx] = gx;
       Yd[3 * idx + 1] = gy;
       Yd[3 * idx + 2] = gz;
-    });
+    }, rk);
   } else {
     ylm_visit<T, LC, false>(L, x, y, z,
-                            [&](int idx, T v, T, T, T) { Y[idx] = v; });
+                            [&](int idx, T v, T, T, T) { Y[idx] = v; }, rk);
   }
 }
 

@@ -89,7 +89,8 @@ k_pair_basis(B2Params p, long long P, const int *__restrict__ center,
         y[(nh + idx) * P] = gx;
         y[(2 * nh + idx) * P] = gy;
         y[(3 * nh + idx) * P] = gz;
-      });
+      },
+      r.x);
 }
 
 // dB2 rows of PP consecutive pairs: dA in shared memory, then a thread per
