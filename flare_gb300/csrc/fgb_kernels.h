@@ -31,11 +31,13 @@ int launch_struct_reduce(const fgb_nlist_s *nl, const double *d_e_atom,
                          double *d_stress, DevBuf &part, cudaStream_t st);
 
 // Stored forward-mode gradients (the reference's algorithm); scratch: each
-// pair's centre atom (left for the caller) and the pairs' basis values.
+// pair's centre atom (left for the caller) and the pairs' basis values;
+// d_rowmax (optional): each gradient row's largest magnitude.
 int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
                     const int *d_species, const double *d_A, const double *d_B2,
                     double *d_dB2, double *d_force_dots, DevBuf &center,
-                    DevBuf &basis, cudaStream_t st);
+                    DevBuf &basis, cudaStream_t st,
+                    double *d_rowmax = nullptr);
 
 // The local-variance finish var = k_self - scale sum(part) (predict.cu).
 int launch_variance_final(int Mr, int ntiles, const double *part,

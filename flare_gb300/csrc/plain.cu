@@ -48,11 +48,13 @@ k_envs_envs(int M, int N, int K, const double *__restrict__ D1,
 // is nonzero only in block s_j:
 // dA_p[c][n][lm] = dg_n (x_c/r) Y_lm + g_n dY_lm/dx_c, and
 // dB2_p[c][(n1,n2,l)] = sum_m A[n1][lm] dA_p[c][n2][lm] + dA_p[c][n1][lm] A[n2][lm].
-// Two kernels over the flat pair list, both bound by FP64 instructions (64
-// cycles each per warp on an SM quarter), so the pairs are spread over all
-// SMs.  One block per atom that walked its pairs in series, one thread
-// evaluating each pair's basis, took 913 us for 108 FCC atoms (3,456 pairs,
-// n_d 144) where these take 78 us (k_pair_basis 15, k_b2_dervs 63).
+// Kernels over the flat pair list, bound by FP64 instructions (64 cycles each
+// per warp on an SM quarter), so the pairs are spread over all SMs.  One
+// block per atom that walked its pairs in series, one thread evaluating each
+// pair's basis, took 913 us for 108 FCC atoms (3,456 pairs, n_d 144) and a
+// thread per descriptor over eight pairs' rows 78 us (lanes of different l
+// and species blocks); these take 64 us (k_pair_basis 14, k_b2_dervs 38,
+// k_row_dots 12).
 constexpr int kBT = 32;   // pairs (threads) per block of k_pair_basis
 
 // Basis values of every pair, value-major so that neighbouring pairs are
@@ -93,96 +95,149 @@ k_pair_basis(B2Params p, long long P, const int *__restrict__ center,
       r.x);
 }
 
-// dB2 rows of PP consecutive pairs: dA in shared memory, then a thread per
-// descriptor q for all PP x 3 rows, and the rows' dots with B2 by a
-// fixed-order block sum.
+// Radial pairs (n1 <= n2) ordered for a neighbour of species s = blockIdx.x:
+// first those with both in its block of n_max (two products), then one in it
+// (one product), then none (zero rows); tab[s npair + rank] = n1 | n2 << 16.
+__global__ void k_derv_items(int nr, int nm, int npair, int *__restrict__ tab) {
+  const int s = blockIdx.x, lo = s * nm, hi = lo + nm, out = nr - nm;
+  const int two = nm * (nm + 1) / 2, one = nm * out;
+  int n1 = 0, first = 0;   // pairs of rows before n1
+  for (int pi = threadIdx.x; pi < npair; pi += blockDim.x) {
+    while (pi - first >= nr - n1) { first += nr - n1; n1++; }
+    const int n2 = n1 + pi - first;
+    const bool i1 = n1 >= lo && n1 < hi, i2 = n2 >= lo && n2 < hi;
+    // index among the columns outside the block
+    const int o1 = n1 < lo ? n1 : n1 - nm, o2 = n2 < lo ? n2 : n2 - nm;
+    int r;
+    if (i1 && i2) r = (n1 - lo) * nm - (n1 - lo) * (n1 - lo - 1) / 2 + n2 - n1;
+    else if (i1) r = two + (n1 - lo) * out + o2;
+    else if (i2) r = two + (n2 - lo) * out + o1;
+    else r = two + one + o1 * out - o1 * (o1 - 1) / 2 + o2 - o1;
+    tab[s * npair + r] = n1 | n2 << 16;
+  }
+}
+
+// dB2 rows of PP consecutive pairs: their dA and their centres' A in shared
+// memory (rows of odd length, so that the lanes' rows fall into different
+// banks), then a thread per (pair, radial pair) for its l_max + 1 values of
+// the three components, in k_derv_items' order so that a warp's threads do
+// the same number of products.
 constexpr int kDTmax = 256;
-template <int PP>
+template <int PP, int LC>
 __global__ void __launch_bounds__(kDTmax)
 k_b2_dervs(B2Params p, long long P, const int *__restrict__ center,
            const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
            const int *__restrict__ species, const double *__restrict__ basis,
-           const double *__restrict__ A_in, const double *__restrict__ B2_in,
-           double *__restrict__ dB2, double *__restrict__ fdots) {
-  extern __shared__ double dA[];   // PP x 3 x nm x nh | 3 PP x (threads + 1)
-  const int nA = p.n_A, nh = p.n_harm, nm = p.n_max, nr = p.n_rad,
-            L1 = p.l_max + 1, nd = p.n_d, nmh = nm * nh;
+           const int *__restrict__ tab, int npair,
+           const double *__restrict__ A_in, double *__restrict__ dB2) {
+  extern __shared__ double sm[];   // dA: PP x 3 x nm x ld | A: PP x nr x ld
+  const int L = LC > 0 ? LC : p.l_max, L1 = L + 1;
+  const int nh = L1 * L1, ld = nh | 1;
+  const int nm = p.n_max, nr = p.n_rad, nd = p.n_d, nmh = nm * nh;
   const long long p0 = (long long)blockIdx.x * PP;
+  const int np = (int)min((long long)PP, P - p0);
   const int t = threadIdx.x, nt = blockDim.x;
-  double *red = dA + PP * 3 * nmh;
-  int cen[PP], sj[PP];
-#pragma unroll
-  for (int k = 0; k < PP; k++) {
-    cen[k] = p0 + k < P ? center[p0 + k] : center[p0];
-    sj[k] = p0 + k < P ? species[nbr_j[p0 + k]] : -1;
+  double *dA = sm, *As = sm + PP * 3 * nm * ld;
+  __shared__ int s_slot[PP], s_sj[PP];
+  if (t < np) {
+    // pairs of one centre share the slot of the first
+    const int c = center[p0 + t];
+    int k = t;
+    while (k > 0 && center[p0 + k - 1] == c) k--;
+    s_slot[t] = k;
+    s_sj[t] = species[nbr_j[p0 + t]];
   }
-  for (int e = t; e < nmh; e += nt) {
-    const int n = e / nh, lm = e - n * nh;
-    const double *bn = basis + n * P + p0;
-    const double *by = basis + (2 * nm + lm) * P + p0;
-#pragma unroll
-    for (int k = 0; k < PP; k++) {
-      if (p0 + k >= P) break;
-      const double4_16a r = rel[p0 + k];
-      const double ir = 1.0 / r.x;
-      const double g = bn[k], dgy = bn[nm * P + k] * ir * by[k];
-      double *d = dA + k * 3 * nmh + e;
-      d[0] = fma(dgy, r.y, g * by[nh * P + k]);
-      d[nmh] = fma(dgy, r.z, g * by[2 * nh * P + k]);
-      d[2 * nmh] = fma(dgy, r.w, g * by[3 * nh * P + k]);
+  __syncthreads();
+  for (int k = 0; k < np; k++) {
+    const double4_16a r = rel[p0 + k];
+    const double ir = 1.0 / r.x;
+    for (int e = t; e < nmh; e += nt) {
+      const int n = e / nh, lm = e - n * nh;
+      const double *bn = basis + n * P + p0 + k;
+      const double *by = basis + (2 * nm + lm) * P + p0 + k;
+      const double g = bn[0], dgy = bn[nm * P] * ir * by[0];
+      double *d = dA + (k * 3 * nm + n) * ld + lm;
+      d[0] = fma(dgy, r.y, g * by[nh * P]);
+      d[nm * ld] = fma(dgy, r.z, g * by[2 * nh * P]);
+      d[2 * nm * ld] = fma(dgy, r.w, g * by[3 * nh * P]);
+    }
+    if (s_slot[k] == k) {
+      const double *A = A_in + (long long)center[p0 + k] * p.n_A;
+      for (int e = t; e < nr * nh; e += nt)
+        As[(k * nr + e / nh) * ld + e % nh] = A[e];
     }
   }
   __syncthreads();
-  double fd[3 * PP];
+  const int two = nm * (nm + 1) / 2, one = nm * (nr - nm);
+  int k = 0;
+  for (int f = t;; f += nt) {
+    while (k < np && f - k * npair >= npair) k++;
+    if (k >= np) break;
+    const int it = f - k * npair, sj = s_sj[k];
+    const int n12 = tab[sj * npair + it], n1 = n12 & 0xFFFF, n2 = n12 >> 16;
+    const int pidx = n1 * nr - n1 * (n1 - 1) / 2 + n2 - n1;
+    double *out = dB2 + 3 * (p0 + k) * nd + pidx * L1;
+    // product 1: dA of the column in the block, A of the other
+    const bool in1 = it < two || (n1 >= sj * nm && n1 < (sj + 1) * nm);
+    const int cin = in1 ? n1 : n2, cot = in1 ? n2 : n1;
+    const double *a = As + (s_slot[k] * nr + cot) * ld;
+    const double *d = dA + (k * 3 * nm + cin - sj * nm) * ld;
+    const double *b = As + (s_slot[k] * nr + cin) * ld;
+    const double *e = dA + (k * 3 * nm + cot - sj * nm) * ld;
 #pragma unroll
-  for (int k = 0; k < 3 * PP; k++) fd[k] = 0.0;
-  for (int q = t; q < nd; q += nt) {
-    const int l = q % L1;
-    int pidx = q / L1, n1 = 0;
-    while (pidx >= nr - n1) { pidx -= nr - n1; n1++; }
-    const int n2 = n1 + pidx, b1 = n1 / nm, b2 = n2 / nm;
-    const int o1 = n1 * nh + l * l, o2 = n2 * nh + l * l;
-    const int e1 = o1 - b1 * nmh, e2 = o2 - b2 * nmh;
-#pragma unroll
-    for (int k = 0; k < PP; k++) {
-      if (p0 + k >= P) break;
+    for (int l = 0; l <= L; l++) {
       double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-      const double *A = A_in + (long long)cen[k] * nA;
-      const double *d = dA + k * 3 * nmh;
-      if (b2 == sj[k])
-        for (int m = 0; m < 2 * l + 1; m++) {
-          const double a = A[o1 + m];
-          v0 = fma(a, d[e2 + m], v0);
-          v1 = fma(a, d[nmh + e2 + m], v1);
-          v2 = fma(a, d[2 * nmh + e2 + m], v2);
+      if (it < two + one) {
+#pragma unroll
+        for (int m = l * l; m < (l + 1) * (l + 1); m++) {
+          const double x = a[m];
+          v0 = fma(x, d[m], v0);
+          v1 = fma(x, d[nm * ld + m], v1);
+          v2 = fma(x, d[2 * nm * ld + m], v2);
         }
-      if (b1 == sj[k])
-        for (int m = 0; m < 2 * l + 1; m++) {
-          const double a = A[o2 + m];
-          v0 = fma(a, d[e1 + m], v0);
-          v1 = fma(a, d[nmh + e1 + m], v1);
-          v2 = fma(a, d[2 * nmh + e1 + m], v2);
-        }
-      const double b = B2_in[(long long)cen[k] * nd + q];
-      double *out = dB2 + 3 * (p0 + k) * nd + q;
-      out[0] = v0;
-      out[nd] = v1;
-      out[2 * (long long)nd] = v2;
-      fd[3 * k] = fma(v0, b, fd[3 * k]);
-      fd[3 * k + 1] = fma(v1, b, fd[3 * k + 1]);
-      fd[3 * k + 2] = fma(v2, b, fd[3 * k + 2]);
+        if (it < two)
+#pragma unroll
+          for (int m = l * l; m < (l + 1) * (l + 1); m++) {
+            const double x = b[m];
+            v0 = fma(x, e[m], v0);
+            v1 = fma(x, e[nm * ld + m], v1);
+            v2 = fma(x, e[2 * nm * ld + m], v2);
+          }
+      }
+      out[l] = v0;
+      out[nd + l] = v1;
+      out[2 * (long long)nd + l] = v2;
     }
   }
+}
+
+// Each gradient row's dot with its centre's B2 and its largest magnitude (the
+// tensor-core row scales): a warp per row.
+__global__ void __launch_bounds__(256)
+k_row_dots(long long rows, int nd, const int *__restrict__ center,
+           const double *__restrict__ dB2, const double *__restrict__ B2,
+           double *__restrict__ fdots, double *__restrict__ rowmax) {
+  const long long m = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (m >= rows) return;
+  const double *a = dB2 + m * nd, *b = B2 + (long long)center[m / 3] * nd;
+  double x = 0.0;
+  unsigned long long mx = 0;
+  for (int q = lane; q < nd; q += 32) {
+    const double v = a[q];
+    x = fma(v, b[q], x);
+    mx = max(mx, (unsigned long long)__double_as_longlong(v) &
+                     0x7FFFFFFFFFFFFFFFULL);
+  }
 #pragma unroll
-  for (int k = 0; k < 3 * PP; k++) red[k * (nt + 1) + t] = fd[k];
-  __syncthreads();
-  for (int k = t >> 5; k < 3 * PP; k += nt / 32) {
-    double x = 0.0;
-    for (int q = t & 31; q < nt; q += 32) x += red[k * (nt + 1) + q];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-      x += __shfl_down_sync(0xffffffffu, x, off);
-    if ((t & 31) == 0 && p0 + k / 3 < P) fdots[3 * p0 + k] = x;
+  for (int off = 16; off > 0; off >>= 1) {
+    x += __shfl_down_sync(0xffffffffu, x, off);
+    mx = max(mx, (unsigned long long)__shfl_down_sync(0xffffffffu,
+                                                      (long long)mx, off));
+  }
+  if (lane == 0) {
+    fdots[m] = x;
+    if (rowmax) rowmax[m] = __longlong_as_double((long long)mx);
   }
 }
 
@@ -416,64 +471,72 @@ __global__ void k_transpose32(long long R, int C, const double *__restrict__ in,
 int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
                     const int *d_species, const double *d_A, const double *d_B2,
                     double *d_dB2, double *d_force_dots, DevBuf &center,
-                    DevBuf &basis, cudaStream_t st) {
+                    DevBuf &basis, cudaStream_t st, double *d_rowmax) {
   const int N = nl->n_atoms;
   const long long P = nl->n_pairs;
   if (N == 0 || P == 0) return FGB_OK;
-  // dA of a pair: PP = 8 pairs a block while they leave room for two blocks
-  // on an SM, else 2
-  const size_t per = sizeof(double) * 3 * (size_t)p.n_max * p.n_harm;
-  const int PP = 8 * per <= 96 * 1024 ? 8 : 2;
   // descriptors whose A, B2 row and pair basis together exceed 200 KB are
   // refused by every stored-gradient entry point
-  const size_t sm = sizeof(double) * ((size_t)p.n_A + p.n_d + 2 * p.n_max +
-                                      4 * p.n_harm + 192) + per;
-  if (sm > 200 * 1024) {
-    set_error("stored-gradient form needs %zu bytes of shared memory", sm);
+  const size_t lim = sizeof(double) *
+                     ((size_t)p.n_A + p.n_d + 2 * p.n_max + 4 * p.n_harm + 192 +
+                      3 * (size_t)p.n_max * p.n_harm);
+  if (lim > 200 * 1024) {
+    set_error("stored-gradient form needs %zu bytes of shared memory", lim);
     return FGB_EINVAL;
   }
+  // dA and A of a pair: 4 pairs a block while that leaves room for four
+  // blocks on an SM, else one
+  const size_t per = sizeof(double) * (3 * (size_t)p.n_max + p.n_rad) *
+                     (p.n_harm | 1);
+  const int PP = 4 * per <= 48 * 1024 ? 4 : 1;
+  const int npair = p.n_rad * (p.n_rad + 1) / 2;
+  const size_t nbasis = (size_t)(2 * p.n_max + 4 * p.n_harm) * (size_t)P;
   int rc;
   if ((rc = center.ensure(sizeof(int) * P)) ||
-      (rc = basis.ensure(sizeof(double) * (2 * p.n_max + 4 * p.n_harm) *
-                         (size_t)P)))
+      (rc = basis.ensure(sizeof(double) * nbasis +
+                         sizeof(int) * (size_t)p.n_species * npair)))
     return rc;
+  int *tab = reinterpret_cast<int *>(basis.as<double>() + nbasis);
   k_pair_center<<<ceil_div((long long)N * 32, 128), 128, 0, st>>>(
       N, nl->offsets.as<long long>(), center.as<int>());
   FGB_LAUNCH_CHECK("k_pair_center");
-  const auto eval = [&](auto lc) {
-    k_pair_basis<decltype(lc)::value><<<ceil_div(P, kBT), kBT, 0, st>>>(
+  k_derv_items<<<p.n_species, 128, 0, st>>>(p.n_rad, p.n_max, npair, tab);
+  FGB_LAUNCH_CHECK("k_derv_items");
+  // threads: whole warps, the block's items split evenly over the fewest
+  // passes
+  const int items = PP * npair, passes = ceil_div(items, kDTmax);
+  const int nt = 32 * ceil_div(ceil_div(items, passes), 32);
+  const auto run = [&](auto pp, auto lc) -> int {
+    constexpr int K = decltype(pp)::value, LC = decltype(lc)::value;
+    k_pair_basis<LC><<<ceil_div(P, kBT), kBT, 0, st>>>(
         p, P, center.as<int>(), nl->nbr_j.as<int>(),
         nl->nbr_rel.as<double4_16a>(), d_species, basis.as<double>());
-  };
-  switch (p.l_max) {
-    case 1: eval(std::integral_constant<int, 1>()); break;
-    case 2: eval(std::integral_constant<int, 2>()); break;
-    case 3: eval(std::integral_constant<int, 3>()); break;
-    case 4: eval(std::integral_constant<int, 4>()); break;
-    case 5: eval(std::integral_constant<int, 5>()); break;
-    case 6: eval(std::integral_constant<int, 6>()); break;
-    default: eval(std::integral_constant<int, 0>()); break;
-  }
-  FGB_LAUNCH_CHECK("k_pair_basis");
-  // threads: whole warps, n_d split evenly over the fewest passes
-  const int passes = ceil_div(p.n_d, kDTmax);
-  const int nt = 32 * ceil_div(ceil_div(p.n_d, passes), 32);
-  const auto dervs = [&](auto pp) -> int {
-    constexpr int K = decltype(pp)::value;
-    const size_t bytes = K * per + sizeof(double) * 3 * K * (nt + 1);
-    FGB_CUDA(cudaFuncSetAttribute(k_b2_dervs<K>,
+    FGB_LAUNCH_CHECK("k_pair_basis");
+    FGB_CUDA(cudaFuncSetAttribute(k_b2_dervs<K, LC>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)bytes));
-    k_b2_dervs<K><<<ceil_div(P, K), nt, bytes, st>>>(
+                                  (int)(K * per)));
+    k_b2_dervs<K, LC><<<ceil_div(P, K), nt, K * per, st>>>(
         p, P, center.as<int>(), nl->nbr_j.as<int>(),
-        nl->nbr_rel.as<double4_16a>(), d_species, basis.as<double>(), d_A,
-        d_B2, d_dB2, d_force_dots);
+        nl->nbr_rel.as<double4_16a>(), d_species, basis.as<double>(), tab,
+        npair, d_A, d_dB2);
+    FGB_LAUNCH_CHECK("k_b2_dervs");
     return FGB_OK;
   };
-  if ((rc = PP == 8 ? dervs(std::integral_constant<int, 8>())
-                    : dervs(std::integral_constant<int, 2>())))
+  const auto with_l = [&](auto pp) -> int {
+    switch (p.l_max) {
+      case 1: return run(pp, std::integral_constant<int, 1>());
+      case 2: return run(pp, std::integral_constant<int, 2>());
+      case 3: return run(pp, std::integral_constant<int, 3>());
+      case 4: return run(pp, std::integral_constant<int, 4>());
+      default: return run(pp, std::integral_constant<int, 0>());
+    }
+  };
+  if ((rc = PP == 4 ? with_l(std::integral_constant<int, 4>())
+                    : with_l(std::integral_constant<int, 1>())))
     return rc;
-  FGB_LAUNCH_CHECK("k_b2_dervs");
+  k_row_dots<<<ceil_div(3 * P * 32, 256), 256, 0, st>>>(
+      3 * P, p.n_d, center.as<int>(), d_dB2, d_B2, d_force_dots, d_rowmax);
+  FGB_LAUNCH_CHECK("k_row_dots");
   return FGB_OK;
 }
 
@@ -593,7 +656,7 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
       (rc = ws.norms.ensure(sizeof(double) * (N + 1))) ||
       (rc = ws.rowmax.ensure(sizeof(double) * (N + 1))) ||
       (rc = ws.dB2.ensure(sizeof(double) * ((size_t)3 * P * nd + 1))) ||
-      (rc = ws.fdots.ensure(sizeof(double) * (3 * P + 1))) ||
+      (rc = ws.fdots.ensure(sizeof(double) * (6 * P + 1))) ||
       (rc = ws.kern.ensure(sizeof(double) * ((size_t)3 * P * M + 1))) ||
       (rc = ws.snorm.ensure(sizeof(double) * (3 * (size_t)M + 1))))
     return rc;
@@ -621,7 +684,8 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
   FGB_LAUNCH_CHECK("k_group_rows");
   if ((rc = launch_b2_dervs(p, nl, d_species, ws.A.as<double>(),
                             ws.B2.as<double>(), ws.dB2.as<double>(),
-                            ws.fdots.as<double>(), ws.pos, ws.basis, st)))
+                            ws.fdots.as<double>(), ws.pos, ws.basis, st,
+                            ws.fdots.as<double>() + 3 * P)))
     return rc;
   const double sig2 = sigma * sigma;
   // chunks of the energy (atoms) and stress (pairs) sums: at least 32 atoms
@@ -684,7 +748,7 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
       fk.c_s = so.o[s];
       fk.M = M;
       if ((rc = oz::slice({Rc, nd, oz::kTM, ws.dB2.as<double>(), nd, rows,
-                           nullptr},
+                           nullptr, ws.fdots.as<double>() + 3 * P},
                           ws.ozK, st, oz::kS64)) ||
           (rc = oz::gemm_force_kernel(ws.ozK, ws.ozSp[vf], fk,
                                       ws.ozerr.as<int>(), st)))
