@@ -57,6 +57,53 @@ __device__ __forceinline__ void mac(df &acc, df a, df b) {
   acc.hi = s;
   acc.lo = __fadd_rn(acc.lo, __fadd_rn(se, pe));
 }
+// Accumulators of two radial values that meet the same harmonic, and the
+// basis values in the layout they are read in.  FP64: the two values.
+// Double-float: packed FP32 pairs, (hi, hi) and (lo, lo), so that each
+// instruction of mac serves both (bit for bit the same sums; ny = -y).
+template <typename T> struct Duo {
+  T a, b;
+  __device__ __forceinline__ void zero() { a = b = T(0); }
+  __device__ __forceinline__ void mac2(const T *g, T y) {
+    mac(a, g[0], y);
+    mac(b, g[1], y);
+  }
+  __device__ __forceinline__ void get(T &x, T &z) const { x = a; z = b; }
+  __device__ __forceinline__ static void put(T *g, T x, T z) {
+    g[0] = x;
+    g[1] = z;
+  }
+};
+template <> struct Duo<df> {
+  dfm::f32x2 hi, lo;
+  __device__ __forceinline__ void zero() { hi = lo = 0; }
+  __device__ __forceinline__ void mac2(const df *g, df y) {
+    using namespace dfm;
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(g);
+    const f32x2 yh = pack2(y.hi, y.hi), yl = pack2(y.lo, y.lo);
+    // the products as scalar instructions: a packed one may be fused with
+    // the packed sums below, and then the sums are others
+    float g0, g1;
+    unpack2(v.x, g0, g1);
+    const float p0 = __fmul_rn(g0, y.hi), p1 = __fmul_rn(g1, y.hi);
+    const f32x2 p = pack2(p0, p1);
+    f32x2 pe = fma2(v.x, yh, pack2(-p0, -p1));
+    pe = fma2(v.x, yl, pe);
+    pe = fma2(v.y, yh, pe);
+    const f32x2 s = add2(hi, p);
+    const f32x2 bb = sub2(s, hi);
+    const f32x2 se = add2(sub2(hi, sub2(s, bb)), sub2(p, bb));
+    hi = s;
+    lo = add2(lo, add2(se, pe));
+  }
+  __device__ __forceinline__ void get(df &x, df &z) const {
+    dfm::unpack2(hi, x.hi, z.hi);
+    dfm::unpack2(lo, x.lo, z.lo);
+  }
+  __device__ __forceinline__ static void put(df *g, df x, df z) {
+    *reinterpret_cast<float4 *>(g) = make_float4(x.hi, z.hi, x.lo, z.lo);
+  }
+};
 __device__ __forceinline__ double finish(double a) { return a; }
 __device__ __forceinline__ df finish(df a) {
   df r;
@@ -133,7 +180,15 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
       const bool ok = si_ok && sj >= 0 && sj < ns;
       double rc = ok ? p.cutoffs[si * kMaxSpecies + sj] : 0.0;
       if (ok && r.x <= rc) {
-        radial_eval<T, NC>(p, T(r.x), T(rc), sg + t * nm, (T *)nullptr);
+        if constexpr (kFixed) {
+          T g[NC];
+          radial_eval<T, NC>(p, T(r.x), T(rc), g, (T *)nullptr);
+#pragma unroll
+          for (int n = 0; n < NC; n += 2)
+            Duo<T>::put(sg + t * NC + n, g[n], g[n + 1]);
+        } else {
+          radial_eval<T, NC>(p, T(r.x), T(rc), sg + t * nm, (T *)nullptr);
+        }
         if constexpr (std::is_same<T, double>::value)
           ylm_eval<T, LC>(p.l_max, r.y, r.z, r.w, sy + t * nh, nullptr, r.x);
         else
@@ -172,19 +227,23 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
         sord[sbeg[sj] + (warp ? scnt[sj] : 0) + rank] = t;
       __syncthreads();
       constexpr int NP = NC / NS;
+      static_assert(NP % 2 == 0, "radial values are summed in pairs");
       for (int it = t; it < S * NH * NS; it += blockDim.x) {
         const int part = it % NS, e = it / NS;
         const int s = e / NH, lm = e % NH;
-        T acc[NP];
+        Duo<T> duo[NP / 2];
 #pragma unroll
-        for (int n = 0; n < NP; n++) acc[n] = T(0);
+        for (int n = 0; n < NP / 2; n++) duo[n].zero();
         for (int q = sbeg[s]; q < sbeg[s + 1]; q++) {
           const int pq = sord[q];
           const T y = sy[pq * NH + lm];
 #pragma unroll
-          for (int n = 0; n < NP; n++)
-            mac(acc[n], sg[pq * NC + part * NP + n], y);
+          for (int n = 0; n < NP / 2; n++)
+            duo[n].mac2(sg + pq * NC + part * NP + 2 * n, y);
         }
+        T acc[NP];
+#pragma unroll
+        for (int n = 0; n < NP / 2; n++) duo[n].get(acc[2 * n], acc[2 * n + 1]);
         if (regA) {
 #pragma unroll
           for (int n = 0; n < NP; n++) areg[n] += finish(acc[n]);
