@@ -22,7 +22,8 @@ namespace fgb {
 
 namespace {
 
-constexpr int kChunk = 64;      // pairs per shared-memory chunk = block size
+constexpr int kChunk = 64;      // pairs per sum into A = block size
+constexpr int kHalf = kChunk / 2;
 
 __device__ __forceinline__ void decode_b2(int q, int L1, int nr, int &n1,
                                           int &n2, int &l) {
@@ -111,6 +112,13 @@ __device__ __forceinline__ df finish(df a) {
   return r;
 }
 
+// Shared-memory values with kHalf rows: the basis values of a half, later A
+// after the staged B2 row.
+__host__ __device__ inline int half_values(int nm, int nh, int nA, int nd) {
+  const int rows = kHalf * (nm + nh);
+  return rows > nA + nd ? rows : nA + nd;
+}
+
 // Shared memory: A[nA] | g[kChunk*nmax] | Y[kChunk*nh] | sp[kChunk] | red,
 // in the compute type T: double (FP64 path) or df (double-float, the
 // mixed-precision path; the pair geometry arrives in FP64 and is split).
@@ -119,7 +127,11 @@ __device__ __forceinline__ df finish(df a) {
 // block's threads idle (one species, l_max 3: 64 threads busy instead of 16;
 // 2,048 atoms, double-float: 35.7 -> 25 us).  A template, because the loops
 // over the accumulators of NS = 1 cost 5% with NS at run time.
-template <typename T, int NC, int LC, int NS>
+// ROWS: pairs with their basis values in shared memory at a time.  With
+// kHalf, the sums of a chunk run over its two halves, the block's first warp
+// evaluates a half's harmonics and the second its radial values (the same
+// sums over the same pairs in the same order).
+template <typename T, int NC, int LC, int NS, int ROWS>
 __global__ void __launch_bounds__(kChunk, 12)
 k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
              const int *__restrict__ nbr_j, const double4_16a *__restrict__ rel,
@@ -148,11 +160,13 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
   // buffer for the contraction (b2_forward_smem leaves A out)
   const bool regA = kFixed && p.n_species * nh <= kChunk &&
                     p.n_species * nm <= kChunk;
+  static_assert(ROWS == kChunk || (ROWS == kHalf && kFixed), "");
   T *A = reinterpret_cast<T *>(smem_raw);
   T *sg = regA ? A : A + nA;
-  T *sy = sg + kChunk * nm;
+  T *sy = sg + ROWS * nm;
   int *ssp = (int *)(sy + kChunk * nh);
-  T *red = (T *)(ssp + kChunk);
+  T *red = ROWS == kHalf ? sg + half_values(nm, nh, nA, p.n_d)
+                         : (T *)(ssp + kChunk);
   int *sord = (int *)(red + kChunk);      // chunk pairs, sorted by species
   int *scnt = sord + kChunk;              // [warp][species] counts
   int *sbeg = scnt + 2 * kMaxSpecies;     // species starts in sord
@@ -170,6 +184,69 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
   if (!regA)
     for (int e = t; e < nA; e += blockDim.x) A[e] = T(0);
   const long long b = offsets[i], e_ = offsets[i + 1];
+  if constexpr (ROWS == kHalf) {
+    __shared__ unsigned s_of[kMaxSpecies];   // the half's pairs of a species
+    constexpr int NH = (LC + 1) * (LC + 1), NP = NC / NS;
+    const int lane = t & 31, part = t % NS, s = t / NS / NH,
+              lm = t / NS % NH;
+    for (long long c0 = b; c0 < e_; c0 += kChunk) {
+      Duo<T> duo[NP / 2];
+#pragma unroll
+      for (int n = 0; n < NP / 2; n++) duo[n].zero();
+      const long long c1 = min(c0 + kChunk, e_);
+      for (long long h0 = c0; h0 < c1; h0 += kHalf) {
+        const long long pp = h0 + lane;
+        int sj = -1;
+        if (pp < e_) {
+          const int j = nbr_j[pp];
+          const double4_16a r = rel[pp];
+          sj = species[j];
+          const bool ok = si_ok && sj >= 0 && sj < ns;
+          const double rc = ok ? p.cutoffs[si * kMaxSpecies + sj] : 0.0;
+          if (!ok || !(r.x <= rc)) {
+            sj = -1;
+          } else if (t < kHalf) {
+            if constexpr (std::is_same<T, double>::value)
+              ylm_eval<T, LC>(p.l_max, r.y, r.z, r.w, sy + lane * NH, nullptr,
+                              r.x);
+            else
+              ylm_eval<T, LC>(p.l_max, T(r.y), T(r.z), T(r.w),
+                              sy + lane * NH, nullptr);
+          } else {
+            T g[NC];
+            radial_eval<T, NC>(p, T(r.x), T(rc), g, (T *)nullptr);
+#pragma unroll
+            for (int n = 0; n < NC; n += 2)
+              Duo<T>::put(sg + lane * NC + n, g[n], g[n + 1]);
+          }
+        }
+        if (t >= kHalf) {
+          __syncwarp();
+          for (int q = 0; q < ns; q++) {
+            const unsigned m = __ballot_sync(0xffffffffu, sj == q);
+            if (lane == 0) s_of[q] = m;
+          }
+        }
+        __syncthreads();
+        if (s < ns)
+          for (unsigned m = s_of[s]; m; m &= m - 1) {
+            const int pq = __ffs(m) - 1;
+            const T y = sy[pq * NH + lm];
+#pragma unroll
+            for (int n = 0; n < NP / 2; n++)
+              duo[n].mac2(sg + pq * NC + part * NP + 2 * n, y);
+          }
+        __syncthreads();
+      }
+#pragma unroll
+      for (int n = 0; n < NP / 2; n++) {
+        T x, z;
+        duo[n].get(x, z);
+        areg[2 * n] += finish(x);
+        areg[2 * n + 1] += finish(z);
+      }
+    }
+  } else
   for (long long c0 = b; c0 < e_; c0 += kChunk) {
     long long pp = c0 + t;
     int sj = -1;
@@ -270,7 +347,8 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
   if (regA) {
     // the Y buffer is free after the last chunk (synchronised above); A
     // takes its end, clear of the B2 row staged from the start of g
-    A = sy + (kChunk * nh - nA);
+    A = ROWS == kHalf ? sg + half_values(nm, nh, nA, p.n_d) - nA
+                      : sy + (kChunk * nh - nA);
     if constexpr (kFixed) {
       constexpr int NH = (LC + 1) * (LC + 1);
       constexpr int NP = NC / NS;
@@ -298,7 +376,8 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
     // decoding per value); the row is staged in the basis-value buffers and
     // written with coalesced stores when it fits there.
     constexpr int L1c = LC + 1, NH = (LC + 1) * (LC + 1);
-    const bool stage = nd <= kChunk * (nm + nh) - (regA ? nA : 0);
+    const bool stage =
+        ROWS == kHalf || nd <= kChunk * (nm + nh) - (regA ? nA : 0);
     T *out_s = sg;
     const int npair = nr * (nr + 1) / 2;
     for (int pi = t; pi < npair; pi += blockDim.x) {
@@ -816,7 +895,10 @@ __global__ void k_struct_final(const StrucGeom *__restrict__ geom, int maxch,
 
 }  // namespace
 
-size_t b2_forward_smem(const B2Params &p, bool regA) {
+size_t b2_forward_smem(const B2Params &p, bool regA, bool half) {
+  if (half)   // values | reduction
+    return sizeof(double) * (half_values(p.n_max, p.n_harm, p.n_A, p.n_d) +
+                             kChunk / 32);
   // A (unless it stays in registers and is laid over Y) | g | Y | pair
   // species | reduction | species-sorted pair order and per-warp species
   // counts (2 x kMaxSpecies) and starts (kMaxSpecies + 1)
@@ -843,15 +925,24 @@ template <typename T, int NC, int LC>
 struct FwdK {
   static constexpr bool kFixed = NC > 0 && LC > 0;
   static constexpr int kNH = (LC + 1) * (LC + 1);
+  // Half the rows where whole chunks leave room for fewer than the kernel's
+  // twelve blocks in the SM's shared memory.  n_max 10, l_max 6 (30 KB, seven
+  // blocks; 97,556 atoms, double-float): 2,038 us whole, 1,756 half.  n_max 8,
+  // l_max 4 (17 KB): 417 us whole, 453 half, the harmonics of a half being
+  // the longer wait.
+  static constexpr int HROWS =
+      kFixed && 12 * 8 * kChunk * (NC + kNH) > 227 * 1024 ? kHalf : kChunk;
   // calls g with the kernel for S species: the most threads per (species,
   // lm) that one block holds with A in registers
   template <typename G>
   static void with(int S, G &&g) {
     if constexpr (kFixed && NC % 4 == 0 && 4 * kNH <= kChunk)
-      if (4 * S * kNH <= kChunk) return g(k_b2_forward<T, NC, LC, 4>);
+      if (4 * S * kNH <= kChunk) return g(k_b2_forward<T, NC, LC, 4, HROWS>);
     if constexpr (kFixed && NC % 2 == 0 && 2 * kNH <= kChunk)
-      if (2 * S * kNH <= kChunk) return g(k_b2_forward<T, NC, LC, 2>);
-    g(k_b2_forward<T, NC, LC, 1>);
+      if (2 * S * kNH <= kChunk) return g(k_b2_forward<T, NC, LC, 2, HROWS>);
+    if constexpr (kFixed && kNH <= kChunk)
+      if (S * kNH <= kChunk) return g(k_b2_forward<T, NC, LC, 1, HROWS>);
+    g(k_b2_forward<T, NC, LC, 1, kChunk>);
   }
 };
 template <typename T, int NC, int LC>
@@ -877,7 +968,8 @@ int launch_b2_forward(const B2Params &p, const fgb_nlist_s *nl,
     // per thread covers it (the same test as in the kernel)
     const bool regA = decltype(k)::kFixed && p.n_species * p.n_harm <= kChunk &&
                       p.n_species * p.n_max <= kChunk;
-    const size_t sm = b2_forward_smem(p, regA);
+    const size_t sm = b2_forward_smem(
+        p, regA, regA && decltype(k)::HROWS == kHalf);
     const auto launch = [&](auto fn) {
       // all of the SM's unified memory as shared memory: twelve blocks of
       // ~19 KB each

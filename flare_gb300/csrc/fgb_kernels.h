@@ -4,7 +4,8 @@
 
 namespace fgb {
 
-size_t b2_forward_smem(const B2Params &p, bool regA = false);
+size_t b2_forward_smem(const B2Params &p, bool regA = false,
+                       bool half = false);
 // dfloat: compute in double-float (mixed-precision path) instead of FP64;
 // d_rowmax (optional): each row's largest |B2| as written
 // d_A32 (double-float forward only): A written in FP32 instead of d_A, for
