@@ -475,9 +475,10 @@ int gemm_nt(int m, int n, int k, const double *A, long long lda,
             double a, double b, Work &w, cudaStream_t st, bool lower = false) {
   if (m == 0 || n == 0) return FGB_OK;
   int rc;
-  if ((rc = oz::slice({m, k, oz::kTM, A, lda, nullptr, nullptr}, w.A, st)) ||
-      (rc = oz::slice({n, k, oz::kTN64v[oz::tile64(m, n)], B, ldb, nullptr,
-                       nullptr}, w.B, st)))
+  if ((rc = oz::slice_pair(
+           {m, k, oz::kTM, A, lda, nullptr, nullptr}, w.A,
+           {n, k, oz::kTN64v[oz::tile64(m, n)], B, ldb, nullptr, nullptr}, w.B,
+           st)))
     return rc;
   return oz::gemm_axpby(w.A, w.B, C, ldc, a, b, w.err.as<int>(), st, lower);
 }

@@ -89,6 +89,10 @@ int prepare(int rows, int K, int TR, int S, Sliced &out);
 // Slice rows into S = kS64 (FP64 path), kS (FP64-level), 8, 7 or 6 (the mixed path's kernel
 // and variance GEMMs) or kSF32 (FP32-level) digits.
 int slice(const SliceSpec &sp, Sliced &out, cudaStream_t st, int S = kS);
+// Both operands of a kS-slice product (no perm, rownorm or rowmax) in one
+// launch; the same rows are taken apart once.
+int slice_pair(const SliceSpec &a, Sliced &A, const SliceSpec &b, Sliced &B,
+               cudaStream_t st);
 
 // Product of S-slice operands (S = 10, 9, 8, 7 or 6; B.S == S, A.S >= S); the
 // tile shape follows B.TR (one of kTNF64v).

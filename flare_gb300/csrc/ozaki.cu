@@ -17,7 +17,7 @@
 //                    sparse GP (energy 4e-12 eV/atom, std 4e-13 against FP64)
 //   S = 4, TN = 128: FP32-level (2^-24); the alpha-folded force GEMM
 //
-// Data movement: slices are written by k_oz_slice8 directly in the tensor
+// Data movement: slices are written by k_oz_slice directly in the tensor
 // core's no-swizzle K-major canonical layout (8 x 16-byte core matrices),
 // tiled so that the S slices of every (row tile, 16-wide k chunk) are one
 // contiguous block.  One thread streams each chunk with two cp.async.bulk
@@ -310,35 +310,13 @@ __device__ __forceinline__ void store_digits8(long long (&X)[8],
   }
 }
 
-// Row scales: 2^e with e from the row's largest magnitude (after the
-// optional division by the row norm), one warp per row; rows past R and
-// empty rows get 2^0.  Written to `scale` for k_oz_slice8.
-__global__ void __launch_bounds__(256)
-k_oz_rowscale(int R, int K, int RP, const double *__restrict__ src,
-              long long ld, const int *__restrict__ perm,
-              const double *__restrict__ rownorm, double thresh,
-              double *__restrict__ scale) {
-  const int m = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (m >= RP) return;
-  bool valid = m < R;
-  long long row = 0;
-  double inv = 1.0;
-  if (valid) {
-    row = perm ? (long long)perm[m] : (long long)m;
-    if (rownorm) {
-      const double n = rownorm[row];
-      if (n >= thresh) inv = 1.0 / n;
-      else valid = false;
-    }
-  }
+// The scale of a row of K values (each times `inv`): 2^e with e from its
+// largest magnitude, 2^0 for an empty row; by the lanes of one warp.
+__device__ __forceinline__ double row_scale(int K, const double *sr, double inv) {
   unsigned long long mb = 0;
-  if (valid) {
-    const double *sr = src + row * ld;
-    for (int k = lane; k < K; k += 32)
-      mb = max(mb, (unsigned long long)__double_as_longlong(sr[k]) &
-                       0x7FFFFFFFFFFFFFFFULL);
-  }
+  for (int k = threadIdx.x & 31; k < K; k += 32)
+    mb = max(mb, (unsigned long long)__double_as_longlong(sr[k]) &
+                     0x7FFFFFFFFFFFFFFFULL);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1)
     mb = max(mb, (unsigned long long)__shfl_xor_sync(0xffffffffu, (long long)mb, off));
@@ -347,62 +325,19 @@ k_oz_rowscale(int R, int K, int RP, const double *__restrict__ src,
   // an infinity or NaN in the row: scale +inf, which makes every product of
   // the row NaN at kS64 slices
   const bool bad = mb >= 0x7FF0000000000000ULL;
-  if (lane == 0)
-    scale[m] = bad ? __longlong_as_double(0x7FF0000000000000LL) : ldexp(1.0, e);
+  return bad ? __longlong_as_double(0x7FF0000000000000LL) : ldexp(1.0, e);
 }
 
-// The same scales from each source row's largest |value| given up front
-// (`rowmax`, indexed like the source rows): a thread per row.
-__global__ void k_oz_scale_from_max(int R, int RP, const int *__restrict__ perm,
-                                    const double *__restrict__ rownorm,
-                                    double thresh,
-                                    const double *__restrict__ rowmax,
-                                    double *__restrict__ scale) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= RP) return;
-  double mx = 0.0;
-  if (m < R) {
-    const long long row = perm ? (long long)perm[m] : (long long)m;
-    double inv = 1.0;
-    bool valid = true;
-    if (rownorm) {
-      const double n = rownorm[row];
-      if (n >= thresh) inv = 1.0 / n;
-      else valid = false;
-    }
-    if (valid) mx = rowmax[row] * inv;
-  }
-  const int e = mx > 0.0 ? ilogb(mx) + 1 : 0;
-  scale[m] = ldexp(1.0, e);
-}
-
-// Row slicing: each row scaled to (-1, 1) by its power of two 2^e
-// (k_oz_rowscale), the scaled value y taken as the integer X = rn(y 2^(6S))
-// (exact for |y| >= 2^-1 of the row's top binade, rounded at 2^(-6S) below
-// that) and its S balanced base-64 digits stored (store_digits8).  A warp
-// takes 8 rows (one core-matrix row group) and one part of kSlicePart
-// columns, 32 consecutive k at a time, lane = row + 8 x (k group of 8), so
-// that the 16-byte row pieces a store instruction writes for one slice are
-// two contiguous 256-byte blocks (one 16-k chunk each) rather than 32
-// scattered pieces; the parts let a few thousand rows fill the GPU.  A warp
-// spends about 3 us in each 32-column step (1,500 instructions a lane), so
-// few rows take parts of one step (slice_s).
-constexpr int kSlicePart = 128;
-static_assert(kSlicePart % 32 == 0, "a part is whole 32-column steps");
-template <int S>
+// Row scales (after the optional division by the row norm), one warp per
+// row; rows past R and empty rows get 2^0.  For k_oz_slice where its blocks
+// would read each row many times (slice_op).
 __global__ void __launch_bounds__(256)
-k_oz_slice8(int R, int K, int RP, int KP, int TR, int npart, int ncols,
-            const double *__restrict__ src, long long ld, int vec,
-            const int *__restrict__ perm, const double *__restrict__ rownorm,
-            double thresh, __nv_bfloat16 *__restrict__ out,
-            const double *__restrict__ scale) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int part = (int)(gw % npart);
-  const int m0 = (int)(gw / npart) * 8;
-  if (m0 >= RP) return;
-  const int r = lane & 7, g = lane >> 3;
-  const int m = m0 + r;
+k_oz_rowscale(int R, int K, int RP, const double *__restrict__ src,
+              long long ld, const int *__restrict__ perm,
+              const double *__restrict__ rownorm, double thresh,
+              double *__restrict__ scale) {
+  const int m = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (m >= RP) return;
   bool valid = m < R;
   long long row = 0;
   double inv = 1.0;
@@ -414,11 +349,93 @@ k_oz_slice8(int R, int K, int RP, int KP, int TR, int npart, int ncols,
       else valid = false;
     }
   }
-  const double *sr = src + row * ld;
-  const int e = pow2_exp(scale[m]);
-  const size_t stride = (size_t)TR * kKC;
-  const int kend = min(KP, (part + 1) * ncols);
-  for (int k0 = part * ncols + g * 8; k0 < kend; k0 += 32) {
+  const double x = row_scale(valid ? K : 0, src + row * ld, inv);
+  if ((threadIdx.x & 31) == 0) scale[m] = x;
+}
+
+constexpr int kSliceWarps = 4;
+// Where a row's scale comes from.
+enum { kScaleRows, kScaleMax, kScaleGiven };
+// One operand of k_oz_slice, and optionally a second layout of the same rows.
+struct SliceOp {
+  int R, K, RP, KP, TR, ncols, nparts, mode, vec;
+  const double *src;
+  long long ld;
+  const int *perm;
+  const double *rownorm, *rowmax;
+  __nv_bfloat16 *out, *out2;   // out2: rows in tiles of TR2, or null
+  double *scale, *scale2;
+  int RP2, TR2;
+};
+
+// Row slicing: each row scaled to (-1, 1) by its power of two 2^e, the
+// scaled value y taken as the integer X = rn(y 2^(6S)) (exact for |y| >=
+// 2^-1 of the row's top binade, rounded at 2^(-6S) below that) and its S
+// balanced base-64 digits stored (store_digits8).  A block takes 8 rows (one
+// core-matrix row group) and ncols columns, a warp 32 consecutive k at a
+// time, lane = row + 8 x (k group of 8), so that the 16-byte row pieces a
+// store instruction writes for one slice are two contiguous 256-byte blocks
+// (one 16-k chunk each) rather than 32 scattered pieces.
+// The scale: kScaleRows, the block reads its rows whole for their largest
+// magnitude; kScaleMax, that is given (`rowmax`, indexed like the source
+// rows); kScaleGiven, k_oz_rowscale has written it.  Blocks past nblk_a take
+// the second operand (PAIR).  A warp spends 3 us in a 32-column step and a
+// launch about as long, so the products of a solve (1,200 sparse rows: 152
+// products, mostly of 128 columns) are bound by launches: four for each
+// product's operands took 2.99 ms, one takes 1.56.
+template <int S, bool PAIR>
+__global__ void __launch_bounds__(kSliceWarps * 32)
+k_oz_slice(const __grid_constant__ SliceOp oa, const __grid_constant__ SliceOp ob,
+           int nblk_a, double thresh) {
+  const bool second = PAIR && (int)blockIdx.x >= nblk_a;
+  const SliceOp &o = second ? ob : oa;
+  const int part = blockIdx.y;
+  if (part >= o.nparts) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = ((int)blockIdx.x - (second ? nblk_a : 0)) * 8;
+  const int r = lane & 7, g = lane >> 3;
+  const int m = m0 + r;
+  const int R = o.R, K = o.K, KP = o.KP;
+  bool valid = m < R;
+  long long row = 0;
+  double inv = 1.0;
+  if (valid) {
+    row = o.perm ? (long long)o.perm[m] : (long long)m;
+    if (o.rownorm) {
+      const double n = o.rownorm[row];
+      if (n >= thresh) inv = 1.0 / n;
+      else valid = false;
+    }
+  }
+  double sc;
+  if (o.mode == kScaleRows) {
+    __shared__ double s_scale[8];
+    for (int q = warp; q < 8; q += kSliceWarps) {
+      const long long rq = __shfl_sync(0xffffffffu, row, q);
+      const bool vq = __shfl_sync(0xffffffffu, (int)valid, q);
+      const double iq = __shfl_sync(0xffffffffu, inv, q);
+      const double x = row_scale(vq ? K : 0, o.src + rq * o.ld, iq);
+      if (lane == 0) s_scale[q] = x;
+    }
+    __syncthreads();
+    sc = s_scale[r];
+  } else if (o.mode == kScaleMax) {
+    const double mx = valid ? o.rowmax[row] * inv : 0.0;
+    sc = ldexp(1.0, mx > 0.0 ? ilogb(mx) + 1 : 0);
+  } else {
+    sc = !PAIR || m < o.RP ? o.scale[m] : 1.0;
+  }
+  if (part == 0 && threadIdx.x < 8) {
+    if ((!PAIR || m < o.RP) && o.mode != kScaleGiven) o.scale[m] = sc;
+    if (PAIR && m < o.RP2) o.scale2[m] = sc;
+  }
+  const double *sr = o.src + row * o.ld;
+  const int e = pow2_exp(sc), TR = o.TR;
+  const bool vec = o.vec, scaled = o.rownorm;
+  __nv_bfloat16 *out = o.out;
+  const int kend = min(KP, (part + 1) * o.ncols);
+  for (int k0 = part * o.ncols + warp * 32 + g * 8; k0 < kend;
+       k0 += kSliceWarps * 32) {
     // the lane's 8 values: four 16-byte loads when the source rows allow
     // (vec: 16-byte aligned rows) and all 8 lie inside the row
     double v[8];
@@ -438,10 +455,15 @@ k_oz_slice8(int R, int K, int RP, int KP, int TR, int npart, int ncols,
     for (int j = 0; j < 8; j++) {
       const int k = k0 + j;
       X[j] = (valid && k < K)
-                 ? fixed_rn(rownorm ? v[j] * inv : v[j], kBeta * S - e)
+                 ? fixed_rn(scaled ? v[j] * inv : v[j], kBeta * S - e)
                  : 0;
     }
-    store_digits8<S>(X, out + tiled_index<S>(m, k0, KP, TR), stride);
+    if (!PAIR || m < o.RP)
+      store_digits8<S>(X, out + tiled_index<S>(m, k0, KP, TR),
+                       (size_t)TR * kKC);
+    if (PAIR && m < o.RP2)
+      store_digits8<S>(X, o.out2 + tiled_index<S>(m, k0, KP, o.TR2),
+                       (size_t)o.TR2 * kKC);
   }
 }
 
@@ -881,38 +903,75 @@ int prepare(int rows, int K, int TR, int S, Sliced &out) {
   return FGB_OK;
 }
 
+// The launch of one operand: its layout, the parts of its rows and where the
+// scales come from.
 template <int S>
-static int slice_s(const SliceSpec &sp, Sliced &out, cudaStream_t st) {
+static int slice_op(const SliceSpec &sp, Sliced &out, SliceOp &o,
+                    cudaStream_t st) {
   int rc;
   if ((rc = prepare(sp.rows, sp.K, sp.TR, S, out))) return rc;
+  // 16-byte loads need every row start 16-byte aligned
+  const int vec = (sp.ld % 2 == 0 &&
+                   reinterpret_cast<uintptr_t>(sp.src) % 16 == 0) ? 1 : 0;
+  // four 32-column steps a warp, or one while that would leave SMs with
+  // fewer than 8 warps (256 rows x 144: 10.8 against 5.1 us; 16,000 x 680
+  // the same 54 us in either form)
+  constexpr int kStep = 32 * kSliceWarps;
+  const bool few = (long long)(out.RP / 8) * kSliceWarps *
+                       ceil_div(out.KP, 4 * kStep) < 8 * 152;
+  int ncols = few ? kStep : 4 * kStep;
+  while (ceil_div(out.KP, ncols) > 65535) ncols *= 2;   // the grid's y limit
+  o = {sp.rows, sp.K, out.RP, out.KP, sp.TR, ncols, ceil_div(out.KP, ncols),
+       kScaleRows, vec, sp.src, sp.ld, sp.perm, sp.rownorm, sp.rowmax,
+       out.q.as<__nv_bfloat16>(), nullptr, out.scale.as<double>(), nullptr,
+       0, 0};
+  // a block that finds the scales reads its rows whole: in many parts of
+  // long rows that is more than a pass of its own
   if (sp.rowmax) {
-    k_oz_scale_from_max<<<ceil_div(out.RP, 256), 256, 0, st>>>(
-        sp.rows, out.RP, sp.perm, sp.rownorm, kEmptyThresh, sp.rowmax,
-        out.scale.as<double>());
-    FGB_LAUNCH_CHECK("k_oz_scale_from_max");
-  } else {
+    o.mode = kScaleMax;
+  } else if (o.nparts > 1 && !(few && sp.K <= 2048)) {
+    o.mode = kScaleGiven;
     k_oz_rowscale<<<ceil_div((long long)out.RP * 32, 256), 256, 0, st>>>(
         sp.rows, sp.K, out.RP, sp.src, sp.ld, sp.perm, sp.rownorm,
         kEmptyThresh, out.scale.as<double>());
     FGB_LAUNCH_CHECK("k_oz_rowscale");
   }
-  // parts of one step while the 128-column parts would leave SMs with fewer
-  // than 8 warps (256 rows x 144: 10.8 against 5.1 us; 16,000 x 680
-  // the same 54 us in either form)
-  const int ncols =
-      (long long)(out.RP / 8) * ceil_div(out.KP, kSlicePart) < 8 * 152
-          ? 32 : kSlicePart;
-  const int nparts = ceil_div(out.KP, ncols);
-  const long long threads = (long long)(out.RP / 8) * nparts * 32;  // RP % 8 == 0
-  // 16-byte loads need every row start 16-byte aligned
-  const int vec = (sp.ld % 2 == 0 &&
-                   reinterpret_cast<uintptr_t>(sp.src) % 16 == 0) ? 1 : 0;
-  k_oz_slice8<S><<<ceil_div(threads, 256), 256, 0, st>>>(
-      sp.rows, sp.K, out.RP, out.KP, sp.TR, nparts, ncols, sp.src, sp.ld, vec,
-      sp.perm, sp.rownorm, kEmptyThresh, out.q.as<__nv_bfloat16>(),
-      out.scale.as<double>());
-  FGB_LAUNCH_CHECK("k_oz_slice8");
   return FGB_OK;
+}
+
+template <int S, bool PAIR>
+static int launch_slice(const SliceOp &a, const SliceOp *b, cudaStream_t st) {
+  const int na = std::max(a.RP, a.RP2) / 8, nb = b ? b->RP / 8 : 0;   // RP % 8 == 0
+  const dim3 grid(na + nb, std::max(a.nparts, b ? b->nparts : 1));
+  k_oz_slice<S, PAIR><<<grid, kSliceWarps * 32, 0, st>>>(a, b ? *b : a, na,
+                                                         kEmptyThresh);
+  FGB_LAUNCH_CHECK("k_oz_slice");
+  return FGB_OK;
+}
+
+template <int S>
+static int slice_s(const SliceSpec &sp, Sliced &out, cudaStream_t st) {
+  SliceOp o;
+  const int rc = slice_op<S>(sp, out, o, st);
+  return rc ? rc : launch_slice<S, false>(o, nullptr, st);
+}
+
+int slice_pair(const SliceSpec &a, Sliced &A, const SliceSpec &b, Sliced &B,
+               cudaStream_t st) {
+  SliceOp oa, ob;
+  int rc;
+  if ((rc = slice_op<kS>(a, A, oa, st))) return rc;
+  if (a.src == b.src && a.rows == b.rows && a.K == b.K && a.ld == b.ld) {
+    // the same rows: their digits once, in both layouts
+    if ((rc = prepare(b.rows, b.K, b.TR, kS, B))) return rc;
+    oa.out2 = B.q.as<__nv_bfloat16>();
+    oa.scale2 = B.scale.as<double>();
+    oa.RP2 = B.RP;
+    oa.TR2 = B.TR;
+    return launch_slice<kS, true>(oa, nullptr, st);
+  }
+  if ((rc = slice_op<kS>(b, B, ob, st))) return rc;
+  return launch_slice<kS, true>(oa, &ob, st);
 }
 
 int slice(const SliceSpec &sp, Sliced &out, cudaStream_t st, int S) {
