@@ -34,29 +34,31 @@ constexpr int kBlockThreads = 512;
 
 // ------------------------------------------------- diagonal block, cluster
 // Cholesky factor of a kb x kb diagonal block (kb <= kNB) and the factor's
-// inverse, by a cluster of kCl = 16 CTAs.  An SM makes two FP64 multiply-adds a
-// clock, so one CTA needs at least 180 us for the 700,000 of a 128-block
-// (and took 820 us, with three barriers a column and the inverse by one
-// thread a column); sixteen CTAs share them in 124 us (eight: 164), of
-// which the four pivot chains below are 80.  Blocked by kIB =
-// 32 columns:
-//   every CTA factors and inverts the 32 x 32 diagonal block for itself (the
-//     chain of 32 pivots; identical results, so no exchange), warps 0-3 with
-//     the columns k = w mod 4, lanes the rows, warps 4-7 the inverse's rows;
-//   the rows below, dealt out cyclically, become L21 = A21 X^T;
+// inverse, by a cluster of kCl = 16 CTAs.  An SM finishes an FP64 warp
+// instruction every 16 cycles and a warp one of its own every 64, dependent
+// or not, so one CTA needs at least 180 us for the 700,000 multiply-adds of a
+// 128-block (and took 820 us, with three barriers a column and the inverse
+// by one thread a column).  Sixteen CTAs, blocked by kIB = 32 columns:
+//   every CTA factors the 32 x 32 diagonal block for itself (the chain of 32
+//     pivots; identical results, so no exchange);
+//   the rows below and the 32 rows of the identity, which become the block's
+//     inverse, are dealt out cyclically, a warp solving for a row;
 //   their trailing updates need all of L21: through global memory (L2 loads)
 //     between cluster barriers.
-// The inverse's columns are then independent: each CTA solves for its own
-// (cyclic) by the 32 x 32 inverses and products with L, reading A from L2.
-// Pivots: y = 1/sqrt(d) from the hardware's estimate (about 20 bits) by one
-// third-order step of the Householder iteration y (1 + e/2 + 3 e^2/8), e = 1
-// - d y^2; L_kk = d y, columns times y.
-constexpr int kIB = 32, kCl = 16, kClT = 256;
+// The rest of the inverse follows in k_potrf_inverse.
+// 72 us a 128-block and 8 for k_potrf_inverse; of the 72, 45 are the four
+// chains of 32 pivots (720 cycles each: five dependent FP64 instructions of
+// 66, the exchange between warps 140, the division's estimate and the stores)
+// and 9 the cluster's barriers.  With the 32 x 32 inverses beside the pivots in
+// every CTA, square roots on the chain and the rest of the inverse in the
+// cluster it took 118 us (1,190 cycles a pivot).
+constexpr int kIB = 32, kCl = 16, kClT = 256, kClW = kClT / 32;
+// warps that factor a block: as many as the FP64 unit serves in the 64 cycles
+// of one instruction, so that the pivot's never wait behind the updates
+constexpr int kFW = 4, kFT = 32 * kFW;
 constexpr int kLd = kIB + 1;
-// shared doubles: diagonal blocks L and X, the panel, own columns of X, own
-// rows staged, exchange vectors
-constexpr int kClSmem = (kNB / kIB) * kIB * kLd + kIB * kLd + kNB * kLd +
-                        kNB * (kNB / kCl + 1) + (kNB / kCl) * kLd + 6 * kIB + 4;
+// shared doubles: the panel, the block's columns V and U, 1/sqrt(pivot)
+constexpr int kClSmem = (kNB - kIB) * kLd + 2 * kIB * kIB + kIB;
 
 __device__ __forceinline__ void cluster_barrier() {
   __syncthreads();
@@ -71,102 +73,99 @@ template <int ID, int N>
 __device__ __forceinline__ void bar_arrive() {
   __threadfence_block();
   asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
+  __syncwarp();
+}
+// d positive and far from the ends of the exponent range, by its upper word
+// (an FP64 comparison takes an FP64 instruction's time).
+__device__ __forceinline__ bool ordinary(double d) {
+  return (unsigned)(__double2hiint(d) >> 20) - 60u < 1920u;
+}
+// From the hardware's estimates y (about 20 bits) by one third-order step of
+// the Householder iteration: 1/d, y (1 + e + e^2) with e = 1 - d y;
+// 1/sqrt(d), y (1 + e/2 + 3 e^2/8) with e = 1 - d y^2.
+__device__ __forceinline__ double rcp64(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 __device__ __forceinline__ double rsqrt64(double d) {
-  if (!(d > 1e-290 && d < 1e290)) return rsqrt(d);
+  if (!ordinary(d)) return rsqrt(d);
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double t = d * y, e = fma(-t, y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
-// Column k of the factor from its updated values v (a lane per row): scaled
-// by the pivot's 1/sqrt, written to col, the pivot's y to *piv.
-__device__ __forceinline__ double pivot_column(int k, double v, double *col,
-                                               double *piv, int *flag) {
+// v / d where the estimate does not serve; a pivot that is not positive
+// counts as 1 and is reported.  Out of line: nothing of it on the pivots'
+// chain.
+static __device__ __noinline__ double div_rare(double v, double d, int k,
+                                               int *flag) {
+  if (d > 0.0) return v / d;
+  if ((threadIdx.x & 31) == 0 && *flag == 0) *flag = k + 1;
+  return v;
+}
+
+// Column k from its updated values v (a lane per row): V and U = v / d for
+// the updates v_ij -= V_i U_j that need no square root.
+__device__ __forceinline__ void pivot_column(int k, double v, double *V,
+                                             double *U, int *flag) {
   const int lane = threadIdx.x & 31;
   const double d = __shfl_sync(0xffffffffu, v, k);
-  double y = 1.0;
-  if (d > 0.0) y = rsqrt64(d);
-  else if (lane == 0 && *flag == 0) *flag = k + 1;
-  const double l = lane == k ? d * y : v * y;
-  col[lane] = lane >= k ? l : 0.0;
-  if (lane == 0) *piv = y;
-  return l;
+  V[k * kIB + lane] = lane >= k ? v : 0.0;
+  double u = v * rcp64(d);
+  if (!ordinary(d)) u = div_rare(v, d, k, flag);
+  U[k * kIB + lane] = lane > k ? u : 0.0;
 }
 
 // The step of column K in factor_block32 (a template, so that the barrier
 // ids are constants).  Column K + 1's warp brings that column up to date
 // first, writes it and only arrives at the barrier that its readers wait at:
 // its other updates follow while they go on.  Chain of a step: one update,
-// the pivot (5 dependent FP64 instructions), the exchange.
+// the pivot (4 dependent FP64 instructions), the exchange.
 template <int K>
-__device__ __forceinline__ void factor_step(double (&v)[8], double *ex,
-                                            int *flag) {
-  const int t = threadIdx.x, w = (t >> 5) & 3, lane = t & 31;
-  const bool inv = t >= 128;
-  // four exchange columns in turn: a buffer is rewritten four steps on, after
-  // a barrier that every reader has passed
-  double *col = ex + (K & 3) * kIB, *piv = ex + 6 * kIB;
-  constexpr int own = K & 3;
-  if (inv || w != own) bar_sync<1 + (K & 3), kClT>();
-  if (!inv) {
-    const double li = col[lane];
-    constexpr int n1 = K + 1, o1 = n1 & 3, q1 = n1 >> 2;
-    if (n1 < kIB && w == o1) {
-      v[q1 & 7] = fma(-li, col[n1 & 31], v[q1 & 7]);
-      v[q1 & 7] = pivot_column(n1, v[q1 & 7], ex + o1 * kIB, piv + o1, flag);
-      bar_arrive<1 + o1, kClT>();
-    }
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      if (4 * q + w > K && !(w == o1 && q == q1))
-        v[q] = fma(-li, col[4 * q + w], v[q]);
-  } else {
-    double *xr = ex + (4 + (K & 1)) * kIB;
-    constexpr int qk = K >> 2;
-    if (w == own) {
-      const double x = piv[own] * ((lane == K ? 1.0 : 0.0) - v[qk]);
-      v[qk] = x;
-      xr[lane] = x;
-    }
-    bar_sync<5, 128>();
-    const double x = xr[lane];
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      if (4 * q + w > K) v[q] = fma(col[4 * q + w], x, v[q]);
+__device__ __forceinline__ void factor_step(double (&v)[kIB / kFW], double *V,
+                                            double *U, int *flag) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w != K % kFW) bar_sync<1 + (K & 3), kFT>();
+  const double li = V[K * kIB + lane];
+  constexpr int n1 = K + 1, o1 = n1 % kFW, q1 = n1 / kFW;
+  if (n1 < kIB && w == o1) {
+    constexpr int q = q1 % (kIB / kFW);
+    v[q] = fma(-li, U[K * kIB + n1 % kIB], v[q]);
+    pivot_column(n1, v[q], V, U, flag);
+    bar_arrive<1 + (n1 & 3), kFT>();
   }
-  if constexpr (K + 1 < kIB) factor_step<K + 1>(v, ex, flag);
+#pragma unroll
+  for (int q = 0; q < kIB / kFW; q++)
+    if (kFW * q + w > K && !(w == o1 && q == q1))
+      v[q] = fma(-li, U[K * kIB + kFW * q + w], v[q]);
+  if constexpr (K + 1 < kIB) factor_step<K + 1>(v, V, U, flag);
 }
 
-// The jb x jb block D (ld kLd, lower) becomes its factor and X its inverse
-// (both lower, zero above); returns 0 or 1 + the first bad pivot.  Rows and
-// columns past jb are treated as the identity.
-__device__ int factor_block32(int jb, double *D, double *X, double *ex,
-                              int *flag) {
-  const int t = threadIdx.x, w = (t >> 5) & 3, lane = t & 31;
-  const bool inv = t >= 128;
-  // v[q]: factor warps: a[lane][4 q + w]; inverse warps: sum for row 4 q + w,
-  // column lane
-  double v[8];
-#pragma unroll
-  for (int q = 0; q < 8; q++) v[q] = inv ? 0.0 : D[lane * kLd + 4 * q + w];
+// Factors the block whose lower part is in v (v[q]: row lane, column
+// kFW q + w; rows and columns past jb the identity's) into its columns V and
+// U and y = 1/sqrt(pivot): L_ik = V_ik y_k.  Returns 0 or 1 + the first bad
+// pivot.
+__device__ int factor_block32(int jb, double (&v)[kIB / kFW], double *V,
+                              double *U, double *y, int *flag) {
+  const int t = threadIdx.x, w = t >> 5;
   if (t == 0) *flag = 0;
   __syncthreads();
-  if (!inv && w == 0) {
-    v[0] = pivot_column(0, v[0], ex, ex + 6 * kIB, flag);
-    bar_arrive<1, kClT>();
+  if (w == 0) {
+    pivot_column(0, v[0], V, U, flag);
+    bar_arrive<1, kFT>();
   }
-  factor_step<0>(v, ex, flag);
+  if (w < kFW) factor_step<0>(v, V, U, flag);
   __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 8; q++) {
-    const int c = 4 * q + w;
-    if (!inv) D[lane * kLd + c] = c <= lane ? v[q] : 0.0;
-    else X[c * kLd + lane] = lane <= c ? v[q] : 0.0;
+  if (*flag && *flag <= jb) return *flag;
+  if (w == 0) {
+    const double d = V[t * kIB + t];
+    y[t] = d > 0.0 ? rsqrt64(d) : 1.0;
   }
   __syncthreads();
-  return *flag && *flag <= jb ? *flag : 0;
+  return 0;
 }
 
 __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClT)
@@ -174,60 +173,73 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
                 double *__restrict__ X, long long ldx, int base,
                 int *__restrict__ info) {
   extern __shared__ double sh[];
-  double *XD = sh;                                   // diagonal inverses
-  double *D = XD + (kNB / kIB) * kIB * kLd;
-  double *P = D + kIB * kLd;                         // panel rows, then L rows
-  double *C = P + kNB * kLd;                         // own columns of X
-  double *R = C + kNB * (kNB / kCl + 1);             // own rows of A21
-  double *ex = R + (kNB / kCl) * kLd;
+  double *P = sh;                                    // panel rows
+  double *V = P + (kNB - kIB) * kLd;
+  double *U = V + kIB * kIB;
+  double *y = U + kIB * kIB;
   __shared__ int flag;
-  const int t = threadIdx.x, rank = blockIdx.x % kCl;
+  const int t = threadIdx.x, rank = blockIdx.x % kCl, w = t >> 5, lane = t & 31;
   for (int j0 = 0; j0 < kb; j0 += kIB) {
     const int jb = min(kIB, kb - j0);
-    double *Xd = XD + (j0 / kIB) * kIB * kLd;
-    for (int e = t; e < kIB * kIB; e += kClT) {
-      const int i = e / kIB, j = e % kIB;
-      double x = i == j ? 1.0 : 0.0;
-      if (i < jb && j <= i) x = __ldcg(A + (long long)(j0 + i) * lda + j0 + j);
-      D[i * kLd + j] = x;
+    double v[kIB / kFW];
+#pragma unroll
+    for (int q = 0; q < kIB / kFW; q++) {
+      const int c = kFW * q + w;
+      v[q] = lane == c ? 1.0 : 0.0;
+      if (w < kFW && lane < jb && c <= lane)
+        v[q] = __ldcg(A + (long long)(j0 + lane) * lda + j0 + c);
     }
-    __syncthreads();
-    const int bad = factor_block32(jb, D, Xd, ex, &flag);
+    // a warp's row: every kCl-th row below the block, then of the identity
+    const int r0 = j0 + kIB, m = kb - r0;
+    const int nown = m > rank ? (m - rank + kCl - 1) / kCl : 0;
+    static_assert((kNB - kIB) / kCl + kIB / kCl <= kClW, "a row for each warp");
+    const int e = rank + kCl * (w - nown);   // row of the identity, w >= nown
+    double r = 0.0;
+    if (w >= nown)
+      r = lane == e ? 1.0 : 0.0;
+    else if (lane < jb)
+      r = __ldcg(A + (long long)(r0 + rank + kCl * w) * lda + j0 + lane);
+    const int bad = factor_block32(jb, v, V, U, y, &flag);
     if (bad) {   // the same in every CTA: all leave here
       if (rank == 0 && t == 0) atomicCAS(info, 0, base + j0 + bad);
       return;
     }
-    // own rows of the panel: every kCl-th row below the block
-    const int r0 = j0 + kIB, m = kb - r0;
-    const int nown = m > rank ? (m - rank + kCl - 1) / kCl : 0;
-    for (int e = t; e < nown * kIB; e += kClT)
-      R[(e / kIB) * kLd + e % kIB] =
-          __ldcg(A + (long long)(r0 + rank + kCl * (e / kIB)) * lda + j0 + e % kIB);
-    // every CTA has read the diagonal block and this panel's rows are its
-    // own: after this barrier the factor may replace them
-    cluster_barrier();
-    if (rank == 0)
-      for (int e = t; e < kIB * kIB; e += kClT) {
-        const int i = e / kIB, j = e % kIB;
-        if (i < jb && j < jb)
-          A[(long long)(j0 + i) * lda + j0 + j] = D[i * kLd + j];
-      }
-    __syncthreads();
-    for (int e = t; e < nown * kIB; e += kClT) {
-      const int q = e / kIB, c = e % kIB;
-      double s = 0.0;
-      for (int k = 0; k <= c; k++) s = fma(R[q * kLd + k], Xd[c * kLd + k], s);
-      A[(long long)(r0 + rank + kCl * q) * lda + j0 + c] = s;
+    if (w < nown + kIB / kCl) {   // a warp with a row
+#pragma unroll 8
+      for (int k = 0; k < kIB; k++)
+        r = fma(-__shfl_sync(0xffffffffu, r, k), U[k * kIB + lane], r);
     }
-    if (m <= 0) break;
+    r *= y[lane];
+    if (lane < jb) {
+      if (w < nown)
+        A[(long long)(r0 + rank + kCl * w) * lda + j0 + lane] = r;
+      else if (e < jb)
+        X[(long long)(j0 + lane) * ldx + j0 + e] = r;
+    }
+    // every CTA has read the diagonal block before this barrier: the factor
+    // may replace it
     cluster_barrier();
+    if (rank == 0 && lane < jb)
+#pragma unroll
+      for (int q = 0; q < kIB / kClW; q++) {
+        const int c = kClW * q + w;
+        if (c < jb)
+          A[(long long)(j0 + lane) * lda + j0 + c] =
+              lane >= c ? V[c * kIB + lane] * y[c] : 0.0;
+      }
+    if (m <= 0) break;
     for (int e = t; e < m * kIB; e += kClT)
       P[(e / kIB) * kLd + e % kIB] =
           __ldcg(A + (long long)(r0 + e / kIB) * lda + j0 + e % kIB);
     __syncthreads();
-    for (int q = t >> 5; q < nown; q += kClT / 32) {   // a warp per row
+    // own rows' updates, a warp for 32 columns of a row
+    int item = 0;
+    for (int q = 0; q < nown; q++) {
       const int i = rank + kCl * q;
-      for (int c = t & 31; c <= i; c += 32) {
+      for (int c0 = 0; c0 <= i; c0 += 32) {
+        if (item++ % kClW != w) continue;
+        const int c = c0 + lane;
+        if (c > i) continue;
         double s = 0.0;
 #pragma unroll 8
         for (int k = 0; k < kIB; k++) s = fma(P[i * kLd + k], P[c * kLd + k], s);
@@ -237,50 +249,74 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
     }
     cluster_barrier();
   }
-  cluster_barrier();   // all of L is written
-  // columns c = rank mod kCl of X, 32 rows at a time; column slot s holds
-  // column rank + kCl s, four slots to a block of 32 columns
-  constexpr int kOwn = kNB / kCl, kCLd = kOwn + 1, kPerBlk = kIB / kCl;
-  for (int i0 = 0; i0 < kb; i0 += kIB) {
-    const int ib = i0 / kIB, rows = min(kIB, kb - i0);
-    const int act = kPerBlk * (ib + 1);      // columns with entries here
-    // S = E - sum_k L_ik X_k, 32 columns of L at a time
-    constexpr int kOut = kIB * kOwn / kClT;  // outputs a thread
-    double s[kOut] = {};
-    for (int k0 = 0; k0 < i0; k0 += kIB) {
-      __syncthreads();
-      for (int e = t; e < rows * kIB; e += kClT)
-        P[(e / kIB) * kLd + e % kIB] =
-            __ldcg(A + (long long)(i0 + e / kIB) * lda + k0 + e % kIB);
-      __syncthreads();
+}
+
+// The rest of the inverse X of a diagonal block's factor, a CTA for each
+// column c: by 32-row blocks i below the column's own, X_i = -Xd_i (sum over
+// k L_ik X_k) with the inverses Xd of the 32 x 32 diagonal blocks that
+// k_potrf_cluster has left in X; zeros above.  A warp has one FP64 instruction
+// in flight, so four warps take every fourth term of each sum.  By the
+// sixteen CTAs of the cluster, eight columns each, this was 41,000 of its
+// cycles.
+constexpr int kInvT = 128, kInvB = kNB / kIB;
+constexpr int kInvSmem =
+    (kInvB * (kInvB - 1) / 2 + kInvB - 1) * kIB * kLd;   // doubles
+__global__ void __launch_bounds__(kInvT)
+k_potrf_inverse(int kb, const double *__restrict__ A, long long lda,
+                double *X, long long ldx) {
+  extern __shared__ double sh[];
+  constexpr int kBlk = kIB * kLd;
+  double *L = sh;                                  // blocks (i, k), k < i
+  double *D = L + kInvB * (kInvB - 1) / 2 * kBlk;  // Xd_i, i > 0
+  __shared__ double x[kNB], part[4][kIB], sum[kIB];
+  const int c = blockIdx.x, t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const int cb = c / kIB, nb = (kb + kIB - 1) / kIB;
+  for (int i = cb + 1; i < nb; i++)
+    for (int k = cb; k <= i; k++) {
+      double *dst = k < i ? L + (i * (i - 1) / 2 + k) * kBlk : D + (i - 1) * kBlk;
 #pragma unroll
-      for (int o = 0; o < kOut; o++) {
-        const int e = t + o * kClT, r = e % kIB, c = e / kIB;
-        if (c < act && k0 / kIB >= c / kPerBlk && r < rows)
-#pragma unroll 8
-          for (int k = 0; k < kIB; k++)
-            s[o] = fma(P[r * kLd + k], C[(k0 + k) * kCLd + c], s[o]);
+      for (int e = t; e < kIB * kIB; e += kInvT) {
+        const int r = e / kIB, q = e % kIB, row = i * kIB + r;
+        const bool in = row < kb && (k < i || q <= r);
+        const double *src = k < i ? A + (long long)row * lda + k * kIB + q
+                                  : X + (long long)row * ldx + k * kIB + q;
+        // all in flight at once; nothing read (zeros) outside the factor
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;"
+                     ::"r"((unsigned)__cvta_generic_to_shared(dst + r * kLd + q)),
+                       "l"(in ? src : A), "r"(in ? 8 : 0) : "memory");
       }
     }
-    __syncthreads();
+  if (t < kIB) {
+    const int row = cb * kIB + t;
+    x[row] = row < kb ? X[(long long)row * ldx + c] : 0.0;
+  }
+  for (int row = t; row < cb * kIB; row += kInvT) X[(long long)row * ldx + c] = 0.0;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  for (int i = cb + 1; i < nb; i++) {
+    double s = 0.0;
+    for (int k = cb; k < i; k++) {
+      const double *l = L + (i * (i - 1) / 2 + k) * kBlk + lane * kLd;
 #pragma unroll
-    for (int o = 0; o < kOut; o++) {   // S into the panel (rows x columns)
-      const int e = t + o * kClT, r = e % kIB, c = e / kIB;
-      if (c < act)
-        P[r * kLd + c] =
-            (c / kPerBlk == ib && rank + kCl * c == i0 + r ? 1.0 : 0.0) - s[o];
+      for (int q = 0; q < kIB; q += 4) s = fma(l[q + w], x[k * kIB + q + w], s);
     }
+    part[w][lane] = s;
     __syncthreads();
-    const double *Xd = XD + ib * kIB * kLd;
+    if (w == 0)
+      sum[lane] = (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
+    __syncthreads();
+    const double *d = D + (i - 1) * kBlk + lane * kLd;
+    s = 0.0;
 #pragma unroll
-    for (int o = 0; o < kOut; o++) {
-      const int e = t + o * kClT, r = e % kIB, c = e / kIB;
-      if (c >= kOwn || rank + kCl * c >= kb || r >= rows) continue;
-      double x = 0.0;
-      if (c < act)
-        for (int k = 0; k <= r; k++) x = fma(Xd[r * kLd + k], P[k * kLd + c], x);
-      C[(i0 + r) * kCLd + c] = x;
-      X[(long long)(i0 + r) * ldx + rank + kCl * c] = x;
+    for (int q = 0; q < kIB; q += 4) s = fma(-d[q + w], sum[q + w], s);
+    part[w][lane] = s;
+    __syncthreads();
+    if (w == 0) {
+      const double v =
+          (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
+      const int row = i * kIB + lane;
+      x[row] = v;
+      if (row < kb) X[(long long)row * ldx + c] = v;
     }
     __syncthreads();
   }
@@ -554,6 +590,10 @@ int factor(int M, double *A, long long lda, int f, Work &w, cudaStream_t st) {
   FGB_CUDA(cudaFuncSetAttribute(k_potrf_cluster,
                                 cudaFuncAttributeNonPortableClusterSizeAllowed,
                                 1));
+  constexpr int kInvBytes = (int)sizeof(double) * kInvSmem;
+  FGB_CUDA(cudaFuncSetAttribute(k_potrf_inverse,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kInvBytes));
   for (int k0 = 0; k0 < M; k0 += kNB) {
     const int kb = std::min(kNB, M - k0);
     double *A11 = A + (long long)k0 * lda + k0;
@@ -561,6 +601,8 @@ int factor(int M, double *A, long long lda, int f, Work &w, cudaStream_t st) {
     k_potrf_cluster<<<kCl, kClT, kSmem, st>>>(kb, A11, lda, X, kNB, k0,
                                               w.info.as<int>() + f);
     FGB_LAUNCH_CHECK("k_potrf_cluster");
+    k_potrf_inverse<<<kb, kInvT, kInvBytes, st>>>(kb, A11, lda, X, kNB);
+    FGB_LAUNCH_CHECK("k_potrf_inverse");
     const int r = M - k0 - kb;
     if (r == 0) break;
     double *A21 = A + (long long)(k0 + kb) * lda + k0;

@@ -47,3 +47,24 @@ def test_same_rows_in_both_layouts(n):
     u = 2.0 ** -53
     assert np.all(np.abs(L @ L.T - S) <=
                   4 * (n + 1) * u * (np.abs(L) @ np.abs(L).T))
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -990, 2.0 ** 970])
+@pytest.mark.parametrize("n", [5, 33, 128])
+def test_factor_of_extreme_scales(n, scale):
+    """Pivots outside the range of the reciprocal's estimate, in a single
+    diagonal block: the factor of the scaled matrix is the scaled factor."""
+    import torch
+    from flare_gb300 import _lib
+    r = np.random.Generator(np.random.PCG64(n))
+    G = r.normal(size=(n, n))
+    S = G @ G.T + n * np.eye(n)
+    out = []
+    for f in (1.0, scale):
+        A = torch.from_numpy(S * f).cuda()
+        _lib.check(_lib.lib().fgb_cholesky(n, _lib.ptr(A), _lib.stream_ptr()))
+        out.append(A.cpu().numpy() / np.sqrt(f))
+    # each within the backward error of the exact factor, whose condition
+    # here is below 10
+    np.testing.assert_allclose(out[1], out[0], rtol=0,
+                               atol=100 * n * 2.0 ** -53 * np.abs(out[0]).max())
