@@ -193,30 +193,51 @@ __device__ __forceinline__ void visit_lane(int lane, const StrucGeom &g,
   }
 }
 
+// (double)s for |s| < 2^22, exactly, with integer instructions on the FP32
+// value's bits.
+__device__ __forceinline__ double small_int_to_double(int s) {
+  const unsigned f = __float_as_uint(small_int_to_float(s));
+  if (s == 0) return 0.0;
+  const unsigned hi = (f & 0x80000000u) | (((f & 0x7FFFFFFFu) >> 3) + (896u << 20));
+  return __hiloint2double((int)hi, (int)(f << 29));
+}
+
 // The reference's FP64 test for one candidate, in its operation order;
-// returns true (and x, y, z, d) for a pair inside the cutoff.
+// returns true (and x, y, z, d) for a pair inside the cutoff.  An FP64 warp
+// instruction takes the SM 16 cycles, and they bound the fill of a large
+// system.  So the shift terms that are zero are left out (adding zero changes
+// no sum): those of a cell axis along which no active lane's pair is shifted, and
+// those of the cell's zero components; the tests of d >= 0 are made on its
+// bits.  k_fill for 97,556 FCC
+// atoms 357 -> 256 us, for 32 x 1,000 atoms 178 -> 149.
 __device__ __forceinline__ bool exact_pair(const StrucGeom &g,
                                            const double *__restrict__ wrapped,
                                            double wi0, double wi1, double wi2,
                                            int j, int s0, int s1, int s2,
                                            double cutoff, double &x, double &y,
                                            double &z, double &d) {
-  const double e0 = __dsub_rn(wrapped[3 * j], wi0);
-  const double e1 = __dsub_rn(wrapped[3 * j + 1], wi1);
-  const double e2 = __dsub_rn(wrapped[3 * j + 2], wi2);
-  const double f0 = (double)s0, f1 = (double)s1, f2 = (double)s2;
-  x = __dadd_rn(__dadd_rn(__dadd_rn(e0, __dmul_rn(f0, g.cell[0])),
-                          __dmul_rn(f1, g.cell[3])),
-                __dmul_rn(f2, g.cell[6]));
-  y = __dadd_rn(__dadd_rn(__dadd_rn(e1, __dmul_rn(f0, g.cell[1])),
-                          __dmul_rn(f1, g.cell[4])),
-                __dmul_rn(f2, g.cell[7]));
-  z = __dadd_rn(__dadd_rn(__dadd_rn(e2, __dmul_rn(f0, g.cell[2])),
-                          __dmul_rn(f1, g.cell[5])),
-                __dmul_rn(f2, g.cell[8]));
+  x = __dsub_rn(wrapped[3 * j], wi0);
+  y = __dsub_rn(wrapped[3 * j + 1], wi1);
+  z = __dsub_rn(wrapped[3 * j + 2], wi2);
+  const unsigned active = __activemask();
+  const auto shift = [&](int s, const double *cell) {
+    if (!__any_sync(active, s != 0)) return;
+    const double f = small_int_to_double(s);
+    const auto term = [&](double &v, double c) {
+      if (__double_as_longlong(c) << 1)   // c != 0
+        v = __dadd_rn(v, __dmul_rn(f, c));
+    };
+    term(x, cell[0]);
+    term(y, cell[1]);
+    term(z, cell[2]);
+  };
+  shift(s0, g.cell);
+  shift(s1, g.cell + 3);
+  shift(s2, g.cell + 6);
   d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)),
                            __dmul_rn(z, z)));
-  return d < cutoff && d != 0.0;
+  const long long db = __double_as_longlong(d);
+  return db < __double_as_longlong(cutoff) && db != 0;
 }
 
 // Warp per atom: number of pairs.  FP64 only for candidates near the cutoff
