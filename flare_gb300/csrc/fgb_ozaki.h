@@ -1,5 +1,7 @@
 // FP64- and FP32-accurate tensor-core GEMMs by exact BF16 slicing (ozaki.cu).
 #pragma once
+#include <cuda_bf16.h>
+
 #include "fgb_internal.h"
 
 namespace fgb {
@@ -75,13 +77,32 @@ struct SliceSpec {
   const double *rowmax = nullptr;
 };
 
+struct Sliced;
+// An operand's layout and where it lies (no ownership).
+struct Operand {
+  int rows, K, TR, RP, KP, S;
+  __nv_bfloat16 *q;
+  double *scale;
+  size_t values() const { return (size_t)S * RP * KP; }
+  // at value q0 and row scale s0 of a buffer
+  void at(const Sliced &buf, size_t q0, size_t s0);
+};
 struct Sliced {
   int rows = 0, K = 0, TR = 0, RP = 0, KP = 0, S = 0;
   DevBuf q;       // bf16 slices, tiled canonical layout
   DevBuf scale;   // per-row 2^e (kS64 slices: +inf for a non-finite row)
   Sliced() = default;
   explicit Sliced(cudaStream_t st) : q(st), scale(st) {}   // one call's scratch
+  Operand operand() const {
+    return {rows, K, TR, RP, KP, S, q.as<__nv_bfloat16>(), scale.as<double>()};
+  }
 };
+inline void Operand::at(const Sliced &buf, size_t q0, size_t s0) {
+  q = buf.q.as<__nv_bfloat16>() + q0;
+  scale = buf.scale.as<double>() + s0;
+}
+// The layout of rows x K in S slices (not placed yet).
+Operand operand(int rows, int K, int TR, int S);
 
 int pad_to(int x, int m);
 // Size `out` for rows x K in S slices (no conversion).
@@ -89,6 +110,8 @@ int prepare(int rows, int K, int TR, int S, Sliced &out);
 // Slice rows into S = kS64 (FP64 path), kS (FP64-level), 8, 7 or 6 (the mixed path's kernel
 // and variance GEMMs) or kSF32 (FP32-level) digits.
 int slice(const SliceSpec &sp, Sliced &out, cudaStream_t st, int S = kS);
+// kS64 slices of n <= 2 row sets into placed operands, one launch.
+int slice64(const SliceSpec *sp, const Operand *out, int n, cudaStream_t st);
 // Both operands of a kS-slice product (no perm, rownorm or rowmax) in one
 // launch; the same rows are taken apart once.
 int slice_pair(const SliceSpec &a, Sliced &A, const SliceSpec &b, Sliced &B,
@@ -116,6 +139,8 @@ int gemm_axpby(const Sliced &A, const Sliced &B, double *C, long long ldc,
                bool lower = false);
 // B tile height (index into kTN64v) of a kS64- or kS-slice product.
 int tile64(int rows, int cols);
+// ... of n products in one launch.
+int tile64(int n, const int *rows, const int *cols);
 // Products of kS64-slice operands (B tiles of kTN64v rows) for the
 // stored-gradient form and the solved variances:
 //   C[m][n] = (A B^T) inv_a[m] / |s_n|, 1/|s| as hi + lo, zero where either

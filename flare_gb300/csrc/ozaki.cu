@@ -555,14 +555,27 @@ __host__ __device__ constexpr int lower_tiles(int mt, int NTt) {
 // in flight are waited for (bounded) before TMEM is freed and the CTA
 // exits, and `err` reports it.  Energy and variance partials are written
 // per (tile, epilogue warp): NTt * EW slots per row.
-template <class C, class Epi>
+// A launch takes NG products at most (kMaxSpecies: the species of one
+// prediction), their tiles one after the other: products that fill a third
+// of the SMs each then run side by side.
+template <class Epi>
+struct GemmProb {
+  int M, K, KP, MT, NTt, SA;
+  int tile0;   // this product's first tile
+  FastDiv divNT;
+  const __nv_bfloat16 *Asl, *Bsl;
+  const double *Ascale, *Bscale;
+  Epi epi;
+};
+template <class Epi, int NG>
+struct GemmGroup {
+  int n;
+  GemmProb<Epi> p[NG];
+};
+template <class C, class Epi, int NG>
 __global__ void __launch_bounds__(C::THREADS, 1)
-k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
-          int SA, const __nv_bfloat16 *__restrict__ Asl,
-          const double *__restrict__ Ascale,
-          const __nv_bfloat16 *__restrict__ Bsl,
-          const double *__restrict__ Bscale, int tri, int lower, int ntiles,
-          Epi epi, int *__restrict__ err) {
+k_oz_gemm(const __grid_constant__ GemmGroup<Epi, NG> G, int tri, int lower,
+          int ntiles, int *__restrict__ err) {
   constexpr int S = C::S, TN = C::TN, NST = C::STAGES, NCH = C::WCOLS / 16;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t *bar_load = reinterpret_cast<uint64_t *>(smem + NST * C::Stage);
@@ -574,7 +587,6 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
   long long *issued = reinterpret_cast<long long *>(tmem_slot + 2);
   long long *consumed = issued + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int KCH = KP / kKC;
 
   if (warp == 0) {
     tc::tmem_alloc(tmem_slot, kTmemCols);
@@ -605,21 +617,28 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
   // instead of a few (with a triangular B the column tiles differ in cost).
   // lower: only the tiles that reach the diagonal or lie below it (row tile
   // mt has lower_tiles(mt) of them).
-  auto tile_rc = [&](int t, int &mt, int &nt) {
+  auto tile_rc = [&](int t, int &mt, int &nt) -> const GemmProb<Epi> & {
+    int i = 0;
+    if constexpr (NG > 1) {
+      while (i + 1 < G.n && t >= G.p[i + 1].tile0) i++;
+      t -= G.p[i].tile0;
+    }
+    const GemmProb<Epi> &P = G.p[i];
     if (lower) {
       mt = 0;
-      for (int w; t >= (w = lower_tiles<TN>(mt, NTt)); t -= w) mt++;
+      for (int w; t >= (w = lower_tiles<TN>(mt, P.NTt)); t -= w) mt++;
       nt = t;
-      return;
+      return P;
     }
-    mt = fdiv(t, divNT);
-    const int rot = mt - fdiv(mt, divNT) * NTt;
-    nt = t - mt * NTt + rot;
-    if (nt >= NTt) nt -= NTt;
+    mt = fdiv(t, P.divNT);
+    const int rot = mt - fdiv(mt, P.divNT) * P.NTt;
+    nt = t - mt * P.NTt + rot;
+    if (nt >= P.NTt) nt -= P.NTt;
+    return P;
   };
-  auto tile_nch = [&](int nt) {
+  auto tile_nch = [&](const GemmProb<Epi> &P, int nt) {
     const int n0 = nt * TN;
-    const int kmax = tri ? min(K, n0 + TN) : K;
+    const int kmax = tri ? min(P.K, n0 + TN) : P.K;
     return (kmax + kKC - 1) / kKC;
   };
   auto give_up = [&](int why) {   // why: 1 aborted elsewhere, 2 timed out
@@ -635,12 +654,13 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
       bool ok = true;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
         int mt, nt;
-        tile_rc(t, mt, nt);
-        const int nch = tile_nch(nt);
+        const GemmProb<Epi> &P = tile_rc(t, mt, nt);
+        const int nch = tile_nch(P, nt);
         // A blocks hold SA >= S slices per chunk; the first S (the most
         // significant digits) are this product's operand
-        const __nv_bfloat16 *a = Asl + (size_t)mt * KCH * (SA * kTM * kKC);
-        const __nv_bfloat16 *bsrc = Bsl + (size_t)nt * KCH * (S * TN * kKC);
+        const int KCH = P.KP / kKC, SA = P.SA;
+        const __nv_bfloat16 *a = P.Asl + (size_t)mt * KCH * (SA * kTM * kKC);
+        const __nv_bfloat16 *bsrc = P.Bsl + (size_t)nt * KCH * (S * TN * kKC);
         for (int c = 0; c < nch; c++, g++) {
           const int b = (int)(g % NST);
           if (g >= NST) {
@@ -667,8 +687,8 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
       bool ok = true;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
         int mt, nt;
-        tile_rc(t, mt, nt);
-        const int nch = tile_nch(nt);
+        const GemmProb<Epi> &P = tile_rc(t, mt, nt);
+        const int nch = tile_nch(P, nt);
         for (int c = 0; c < nch; c++) {
           const bool seg_first = c % C::SEGC == 0;
           if (seg_first && sg > 0) {
@@ -714,11 +734,11 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
     bool alive = true;
     for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
       int mt, nt;
-      tile_rc(t, mt, nt);
+      const GemmProb<Epi> &P = tile_rc(t, mt, nt);
       const int m0 = mt * kTM, n0 = nt * TN;
       const int m = m0 + q * 32 + lane;
-      const bool row_ok = m < M;
-      const int nseg = (tile_nch(nt) + C::SEGC - 1) / C::SEGC;
+      const bool row_ok = m < P.M;
+      const int nseg = (tile_nch(P, nt) + C::SEGC - 1) / C::SEGC;
       // Phase 1, per K segment.  Group sums are exact integers below 2^24;
       // add them exactly into 64-bit integers, hi = sum_{t <= TSPLIT} g_t
       // 2^(6(TSPLIT-t)) and lo = sum_{t > TSPLIT} g_t 2^(6(S+1-t)), and
@@ -771,14 +791,14 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
       // (FP64 results), or one rounding of hi (FP32 results, no low part).
       // Rows past M (tile padding) still run so that functors can write
       // zero padding.
-      const int er = pow2_exp(Ascale[m]);
+      const int er = pow2_exp(P.Ascale[m]);
       using V = typename Epi::Value;
       V v[NCH][16];
 #pragma unroll
       for (int ch = 0; ch < NCH; ch++) {
 #pragma unroll
         for (int j = 0; j < 16; j++) {
-          const int eb = pow2_exp(Bscale[n0 + c_lo + ch * 16 + j]);
+          const int eb = pow2_exp(P.Bscale[n0 + c_lo + ch * 16 + j]);
           const int e = er + eb;
           if constexpr (Epi::kFloat) {
             static_assert(!C::HAS_LO, "FP32 results take at most 5 slices");
@@ -797,8 +817,8 @@ k_oz_gemm(int M, int N, int K, int KP, int MT, int NTt, FastDiv divNT,
       double acc = 0.0;
 #pragma unroll
       for (int ch = 0; ch < NCH; ch++)
-        acc = epi.chunk(m, row_ok, n0 + c_lo + ch * 16, v[ch], acc);
-      epi.finish(m, row_ok, nt * C::EW + sub, acc);
+        acc = P.epi.chunk(m, row_ok, n0 + c_lo + ch * 16, v[ch], acc);
+      P.epi.finish(m, row_ok, nt * C::EW + sub, acc);
     }
   }
   tc::fence_before_sync();
@@ -889,6 +909,11 @@ struct EpiStoreF32 {
 
 int pad_to(int x, int m) { return (x + m - 1) / m * m; }
 
+Operand operand(int rows, int K, int TR, int S) {
+  return {rows, K, TR, pad_to(std::max(rows, 1), TR),
+          pad_to(std::max(K, 1), kKC), S, nullptr, nullptr};
+}
+
 int prepare(int rows, int K, int TR, int S, Sliced &out) {
   out.rows = rows;
   out.K = K;
@@ -906,10 +931,8 @@ int prepare(int rows, int K, int TR, int S, Sliced &out) {
 // The launch of one operand: its layout, the parts of its rows and where the
 // scales come from.
 template <int S>
-static int slice_op(const SliceSpec &sp, Sliced &out, SliceOp &o,
+static int slice_op(const SliceSpec &sp, const Operand &out, SliceOp &o,
                     cudaStream_t st) {
-  int rc;
-  if ((rc = prepare(sp.rows, sp.K, sp.TR, S, out))) return rc;
   // 16-byte loads need every row start 16-byte aligned
   const int vec = (sp.ld % 2 == 0 &&
                    reinterpret_cast<uintptr_t>(sp.src) % 16 == 0) ? 1 : 0;
@@ -923,8 +946,7 @@ static int slice_op(const SliceSpec &sp, Sliced &out, SliceOp &o,
   while (ceil_div(out.KP, ncols) > 65535) ncols *= 2;   // the grid's y limit
   o = {sp.rows, sp.K, out.RP, out.KP, sp.TR, ncols, ceil_div(out.KP, ncols),
        kScaleRows, vec, sp.src, sp.ld, sp.perm, sp.rownorm, sp.rowmax,
-       out.q.as<__nv_bfloat16>(), nullptr, out.scale.as<double>(), nullptr,
-       0, 0};
+       out.q, nullptr, out.scale, nullptr, 0, 0};
   // a block that finds the scales reads its rows whole: in many parts of
   // long rows that is more than a pass of its own
   if (sp.rowmax) {
@@ -933,10 +955,16 @@ static int slice_op(const SliceSpec &sp, Sliced &out, SliceOp &o,
     o.mode = kScaleGiven;
     k_oz_rowscale<<<ceil_div((long long)out.RP * 32, 256), 256, 0, st>>>(
         sp.rows, sp.K, out.RP, sp.src, sp.ld, sp.perm, sp.rownorm,
-        kEmptyThresh, out.scale.as<double>());
+        kEmptyThresh, out.scale);
     FGB_LAUNCH_CHECK("k_oz_rowscale");
   }
   return FGB_OK;
+}
+template <int S>
+static int slice_op(const SliceSpec &sp, Sliced &out, SliceOp &o,
+                    cudaStream_t st) {
+  const int rc = prepare(sp.rows, sp.K, sp.TR, S, out);
+  return rc ? rc : slice_op<S>(sp, out.operand(), o, st);
 }
 
 template <int S, bool PAIR>
@@ -954,6 +982,15 @@ static int slice_s(const SliceSpec &sp, Sliced &out, cudaStream_t st) {
   SliceOp o;
   const int rc = slice_op<S>(sp, out, o, st);
   return rc ? rc : launch_slice<S, false>(o, nullptr, st);
+}
+
+int slice64(const SliceSpec *sp, const Operand *out, int n, cudaStream_t st) {
+  SliceOp o[2];
+  int rc;
+  for (int i = 0; i < n; i++)
+    if ((rc = slice_op<kS64>(sp[i], out[i], o[i], st))) return rc;
+  return n == 1 ? launch_slice<kS64, false>(o[0], nullptr, st)
+                : launch_slice<kS64, true>(o[0], &o[1], st);
 }
 
 int slice_pair(const SliceSpec &a, Sliced &A, const SliceSpec &b, Sliced &B,
@@ -986,36 +1023,64 @@ int slice(const SliceSpec &sp, Sliced &out, cudaStream_t st, int S) {
 }
 
 
-template <class C, class Epi>
-static int gemm_c(const Sliced &A, const Sliced &B, bool tri, const Epi &epi,
-                  int *err, cudaStream_t st, bool lower = false) {
-  // A may carry more (less significant) slices than the product uses
-  if (A.K != B.K || A.KP != B.KP || A.TR != kTM || B.TR != C::TN ||
-      A.S < C::S || B.S != C::S) {
-    set_error("ozaki gemm: operand layouts disagree");
-    return FGB_EINVAL;
+// n products of operand layouts A[i], B[i] in one launch (NG >= n).
+template <class C, class Epi, int NG>
+static int gemm_group_c(int n, const Operand *A, const Operand *B, bool tri,
+                        const Epi *epi, int *err, cudaStream_t st,
+                        bool lower = false) {
+  GemmGroup<Epi, NG> G{};
+  long long ntiles = 0;
+  for (int i = 0; i < n; i++) {
+    const Operand &a = A[i], &b = B[i];
+    // A may carry more (less significant) slices than the product uses
+    if (a.K != b.K || a.KP != b.KP || a.TR != kTM || b.TR != C::TN ||
+        a.S < C::S || b.S != C::S) {
+      set_error("ozaki gemm: operand layouts disagree");
+      return FGB_EINVAL;
+    }
+    if (a.rows == 0 || b.rows == 0) continue;
+    const int MT = a.RP / kTM, NTt = b.RP / C::TN;
+    G.p[G.n++] = {a.rows, a.K, a.KP, MT, NTt, a.S, (int)ntiles,
+                  make_fastdiv(NTt), a.q, b.q, a.scale, b.scale, epi[i]};
+    if (lower)
+      for (int mt = 0; mt < MT; mt++) ntiles += lower_tiles<C::TN>(mt, NTt);
+    else
+      ntiles += (long long)MT * NTt;
   }
-  if (A.rows == 0 || B.rows == 0) return FGB_OK;
-  FGB_CUDA(cudaFuncSetAttribute(k_oz_gemm<C, Epi>,
+  if (G.n == 0) return FGB_OK;
+  FGB_CUDA(cudaFuncSetAttribute(k_oz_gemm<C, Epi, NG>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)C::Smem));
   int dev = 0, sms = 0;
   FGB_CUDA(cudaGetDevice(&dev));
   FGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int MT = A.RP / kTM, NTt = B.RP / C::TN;
-  int ntiles = MT * NTt;
-  if (lower) {
-    ntiles = 0;
-    for (int mt = 0; mt < MT; mt++) ntiles += lower_tiles<C::TN>(mt, NTt);
-  }
-  const int grid = std::max(1, std::min(ntiles, sms));
-  k_oz_gemm<C, Epi><<<grid, C::THREADS, C::Smem, st>>>(
-      A.rows, B.rows, A.K, A.KP, MT, NTt, make_fastdiv(NTt), A.S,
-      A.q.as<__nv_bfloat16>(),
-      A.scale.as<double>(), B.q.as<__nv_bfloat16>(), B.scale.as<double>(),
-      tri ? 1 : 0, lower ? 1 : 0, ntiles, epi, err);
+  const int grid = (int)std::max(1LL, std::min<long long>(ntiles, sms));
+  k_oz_gemm<C, Epi, NG><<<grid, C::THREADS, C::Smem, st>>>(
+      G, tri ? 1 : 0, lower ? 1 : 0, (int)ntiles, err);
   FGB_LAUNCH_CHECK("k_oz_gemm");
   return FGB_OK;
+}
+
+template <class C, class Epi>
+static int gemm_c(const Sliced &A, const Sliced &B, bool tri, const Epi &epi,
+                  int *err, cudaStream_t st, bool lower = false) {
+  const Operand a = A.operand(), b = B.operand();
+  return gemm_group_c<C, Epi, 1>(1, &a, &b, tri, &epi, err, st, lower);
+}
+
+// Products of kS64-slice operands side by side (all B tiles of one height).
+template <class Epi>
+static int gemm64_group(const std::vector<Operand> &A,
+                        const std::vector<Operand> &B, bool tri,
+                        const std::vector<Epi> &epi, int *err, cudaStream_t st) {
+  const int n = (int)A.size();
+  const auto go = [&](auto c) {
+    return gemm_group_c<decltype(c), Epi, kMaxSpecies>(n, A.data(), B.data(),
+                                                       tri, epi.data(), err, st);
+  };
+  if (B[0].TR == 32) return go(CfgS<kS64, 32>{});
+  if (B[0].TR == 16) return go(CfgS<kS64, 16>{});
+  return go(CfgS<kS64, 48>{});
 }
 
 template <int S, class Epi>
@@ -1545,18 +1610,20 @@ int row_inverse(int M, int nd, const double *rows, double *norms, double2 *inv,
 // and 16 rows cost 20, 16 and 13 (2 x 1,000 sparse, n_d 680, the three
 // products of the FP64 path over both species: 64 atoms 397, 315 and 251 us;
 // 500 atoms 414, 327 and 272; 1,000 atoms 421, 371 and 450; 1,500 atoms 425,
-// 472 and 525; 4,000 atoms 824, 901 and 1,043).
-int tile64(int rows, int cols) {
+// 472 and 525; 4,000 atoms 824, 901 and 1,043; a species at a time).
+int tile64(int n, const int *rows, const int *cols) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
           cudaSuccess)
     return 0;
-  const long long mt = ceil_div(rows, kTM);
   int best = 0, best_cost = 0;
   for (int v = 0; v < kTiles64; v++) {
     constexpr int kCost[kTiles64] = {20, 16, 13};
-    const int c = kCost[v] * ceil_div(mt * ceil_div(cols, kTN64v[v]), sms);
+    long long tiles = 0;
+    for (int i = 0; i < n; i++)
+      tiles += (long long)ceil_div(rows[i], kTM) * ceil_div(cols[i], kTN64v[v]);
+    const int c = kCost[v] * ceil_div(tiles, sms);
     if (v == 0 || c < best_cost) {
       best = v;
       best_cost = c;
@@ -1564,6 +1631,7 @@ int tile64(int rows, int cols) {
   }
   return best;
 }
+int tile64(int rows, int cols) { return tile64(1, &rows, &cols); }
 
 int gemm_cosine(const Sliced &A, const Sliced &B, const int *perm,
                 const double *a_norm, const double2 *s_inv,
@@ -2020,6 +2088,179 @@ bool fp64_stage_sliced(const fgb_model_s *m) {
   return (m->power == 2.0 || m->power == 1.0) && m->finite;
 }
 
+// Species whose products run side by side: those with atoms and sparse
+// environments, where all atoms are one chunk of rows (else 0).
+static int stage64_group(const fgb_model_s *m, const std::vector<int> &counts,
+                         int max_rows) {
+  int n = 0;
+  long long rows = 0;
+  for (int s = 0; s < m->b2.n_species; s++)
+    if (counts[s] > 0 && m->h_counts[s] > 0) {
+      n++;
+      rows += counts[s];
+    }
+  return rows <= max_rows ? n : 0;
+}
+
+// The stage below for several species, each of its products one launch over
+// them all.  At a thousand atoms one species' tiles fill a third of the SMs
+// and a product takes a tile's time (50 to 75 us) whatever their number.
+// 1,000 alloy atoms, 2 x 1,000 sparse, the three products: 366 -> 252 us (64
+// atoms 251 -> 131, 500 atoms 272 -> 175); 2 x 500 sparse, 2,000 atoms, two
+// products: 196 -> 162.
+template <class Ready>
+static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &counts,
+                                   bool want_grad, bool want_var,
+                                   double *d_e_atom, double *d_gB2,
+                                   double *d_var, cudaStream_t st,
+                                   const Ready &ready, bool have_rowmax) {
+  int rc;
+  const B2Params &p = m->b2;
+  const int nd = p.n_d;
+  const double sig2 = m->sigma * m->sigma, xi = m->power;
+  struct Part {
+    int s, N, M, R, off, kslots, vslots;
+    const int *perm;
+    size_t e0, v0;   // first entries in erows and part
+  };
+  std::vector<Part> parts;
+  std::vector<int> rows, mcols, rcols, dcols;
+  int base = 0;
+  for (int s = 0; s < p.n_species; s++) {
+    const int N = counts[s], M = m->h_counts[s];
+    const int *perm = m->ws.perm.as<int>() + base;
+    base += N;
+    if (N > 0 && M == 0 && want_var &&
+        // no sparse environments of this species: k = 0, var = k_self
+        (rc = launch_variance_final(N, 0, nullptr, perm,
+                                    m->ws.norms.as<double>(), sig2, xi, d_var,
+                                    st)))
+      return rc;
+    if (N == 0 || M == 0) continue;
+    parts.push_back({s, N, M, m->h_panel_rows[s], m->h_offsets[s], 0, 0, perm,
+                     0, 0});
+    rows.push_back(N);
+    mcols.push_back(M);
+    rcols.push_back(m->h_panel_rows[s]);
+    dcols.push_back(nd);
+  }
+  const int n = (int)parts.size();
+  const int vk = oz::tile64(n, rows.data(), mcols.data()),
+            vv = oz::tile64(n, rows.data(), rcols.data()),
+            vg = oz::tile64(n, rows.data(), dcols.data());
+  if ((rc = ready(m->oz64S_ready, vk, build_oz64_S)) ||
+      (want_var && (rc = ready(m->oz64L_ready, vv, build_oz64_L))) ||
+      (want_grad && (rc = ready(m->oz64ST_ready, vg, build_oz64_ST))))
+    return rc;
+  // the species' operands one after the other in the workspace's buffers
+  std::vector<oz::Operand> A(n), K(n), W(n), B(n);
+  size_t qa = 0, qk = 0, sa = 0, ne = 0, nv = 0;
+  for (int i = 0; i < n; i++) {
+    Part &P = parts[i];
+    A[i] = oz::operand(P.N, nd, oz::kTM, oz::kS64);
+    K[i] = oz::operand(P.N, P.M, oz::kTM, oz::kS64);
+    P.kslots = m->oz64S[vk][P.s]->RP / 16;
+    P.vslots = want_var ? m->oz64L[vv][P.s]->RP / 16 : 0;
+    P.e0 = ne;
+    P.v0 = nv;
+    ne += (size_t)P.N * P.kslots;
+    nv += (size_t)P.N * P.vslots;
+    qa += A[i].values();
+    qk += K[i].values();
+    sa += A[i].RP;
+  }
+  const size_t h = sizeof(__nv_bfloat16), d = sizeof(double);
+  if ((rc = m->ws.ozA.q.ensure(h * qa)) || (rc = m->ws.ozA.scale.ensure(d * sa)) ||
+      (rc = m->ws.erows.ensure(d * ne)) ||
+      (want_var && ((rc = m->ws.ozK.q.ensure(h * qk)) ||
+                    (rc = m->ws.ozK.scale.ensure(d * sa)) ||
+                    (rc = m->ws.part.ensure(d * nv)))) ||
+      (want_grad && ((rc = m->ws.ozW.q.ensure(h * qk)) ||
+                     (rc = m->ws.ozW.scale.ensure(d * sa)))))
+    return rc;
+  qa = qk = sa = 0;
+  for (int i = 0; i < n; i++) {
+    W[i] = K[i];
+    A[i].at(m->ws.ozA, qa, sa);
+    if (want_var) K[i].at(m->ws.ozK, qk, sa);
+    if (want_grad) W[i].at(m->ws.ozW, qk, sa);
+    qa += A[i].values();
+    qk += K[i].values();
+    sa += A[i].RP;
+  }
+  {
+    StageTimer _pt(kStRowSlice, st, 2);
+    for (int i = 0; i < n; i += 2) {   // two species a launch
+      oz::SliceSpec sp[2];
+      for (int q = i; q < std::min(n, i + 2); q++)
+        sp[q - i] = {parts[q].N, nd, oz::kTM, m->ws.B2.as<double>(), nd,
+                     parts[q].perm, nullptr,
+                     have_rowmax ? m->ws.rowmax.as<double>() : nullptr};
+      if ((rc = oz::slice64(sp, &A[i], std::min(2, n - i), st))) return rc;
+    }
+  }
+  int *err = m->ws.ozerr.as<int>();
+  {
+    StageTimer _pt(kStKernelGemm, st);
+    std::vector<oz::EpiKernel64> epi;
+    for (int i = 0; i < n; i++) {
+      const Part &P = parts[i];
+      const double wmax = m->alpha_max[P.s];
+      B[i] = m->oz64S[vk][P.s]->operand();
+      epi.push_back({want_var ? K[i].q : nullptr, want_grad ? W[i].q : nullptr,
+                     want_var ? K[i].scale : nullptr,
+                     want_grad ? W[i].scale : nullptr, K[i].KP,
+                     wmax > 0.0 ? std::ilogb(wmax) + 1 : 0,
+                     m->ws.erows.as<double>() + P.e0, P.kslots,
+                     m->alpha.as<double>() + P.off,
+                     m->sinv.as<double2>() + P.off,
+                     m->svalid.as<unsigned char>() + P.off, P.perm,
+                     m->ws.norms.as<double>(), xi == 2.0, P.M});
+    }
+    if ((rc = oz::gemm64_group(A, B, false, epi, err, st))) return rc;
+  }
+  {
+    StageTimer _pt(kStRowEnergy, st);
+    for (const Part &P : parts) {
+      oz::k_energy_final<<<ceil_div((long long)P.N * kRowLanes, 128), 128, 0,
+                           st>>>(P.N, P.kslots,
+                                 m->ws.erows.as<double>() + P.e0, P.perm, sig2,
+                                 d_e_atom);
+      FGB_LAUNCH_CHECK("k_energy_final");
+    }
+  }
+  if (want_grad) {
+    StageTimer _pt(kStAdjointGemm, st);
+    std::vector<oz::EpiGrad64> epi;
+    for (int i = 0; i < n; i++) {
+      B[i] = m->oz64ST[vg][parts[i].s]->operand();
+      epi.push_back({parts[i].perm, m->ws.norms.as<double>(),
+                     m->ws.B2.as<double>(), d_e_atom, xi, xi * sig2, d_gB2,
+                     nd});
+    }
+    if ((rc = oz::gemm64_group(W, B, false, epi, err, st))) return rc;
+  }
+  if (want_var) {
+    {
+      StageTimer _pt(kStVarianceGemm, st);
+      std::vector<oz::EpiZsq> epi;
+      for (int i = 0; i < n; i++) {
+        B[i] = m->oz64L[vv][parts[i].s]->operand();
+        epi.push_back({m->ws.part.as<double>() + parts[i].v0, parts[i].vslots,
+                       parts[i].R});
+      }
+      if ((rc = oz::gemm64_group(K, B, true, epi, err, st))) return rc;
+    }
+    for (const Part &P : parts)
+      if ((rc = launch_variance_final(P.N, P.vslots,
+                                      m->ws.part.as<double>() + P.v0, P.perm,
+                                      m->ws.norms.as<double>(), sig2, xi, d_var,
+                                      st, sig2 * sig2)))
+        return rc;
+  }
+  return FGB_OK;
+}
+
 // Kernel, adjoint and variance products of the FP64 path as exact 10-slice
 // products (60 bits of each row's largest entry, integer sums, one
 // rounding): on this GPU an FP64 multiply-add pipe of 2 a clock an SM makes
@@ -2045,6 +2286,9 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
     if (r == FGB_OK) flags[v] = true;
     return r;
   };
+  if (const int g = stage64_group(m, counts, kRows); g > 1)
+    return kernel_stage_fp64_group(m, counts, want_grad, want_var, d_e_atom,
+                                   d_gB2, d_var, st, ready, have_rowmax);
   int base = 0;
   for (int s = 0; s < p.n_species; s++) {
     const int Ns = counts[s], Ms = m->h_counts[s];

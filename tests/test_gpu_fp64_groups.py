@@ -1,0 +1,55 @@
+"""Products of several species in one launch (all atoms within one chunk of
+32,768 rows) against the oracle, and against a species at a time."""
+import numpy as np
+import pytest
+
+from test_gpu_fp64_stage import weighted
+from test_gpu_small_kernels import lattice
+
+import oracle
+from flare_gb300 import synthetic as syn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("atoms,counts", [
+    (64, (5, 130, 49)),        # three species, uneven tiles
+    (200, (16, 0, 33)),        # one without sparse rows between two with
+    (150, (1, 2, 3, 4, 5, 6, 7, 8)),   # the most species
+    (40, (1400, 7)),           # K above one segment beside K of one chunk
+])
+def test_groups_match_oracle(atoms, counts):
+    import flare_gb300 as fg
+    ogp, gp, calc, args = weighted(counts, 3, 2, 2, seed=atoms + 1)
+    S = len(counts)
+    cell, sp, pos = syn.random_alloy(atoms, fractions=[1.0 / S] * S,
+                                     density=0.05, dmin=1.6, seed=70 + atoms)
+    sp[:S] = np.arange(S)
+    st = oracle.Structure(cell, sp, pos, 4.0, [oracle.B2Settings(*args)])
+    ogp.predict_local_uncertainties(st)
+    var = oracle.sort_variances(st, st.local_uncertainties[0])
+    r = gp.predict_batch([fg.Structure(cell, sp, pos, 4.0, [calc])],
+                         precision="fp64")
+    m = st.mean_efs
+    # sums of up to 1,400 terms of FP64 level
+    assert abs(r["energy"][0] - m[0]) <= 1e-10 * max(1.0, abs(m[0]))
+    f = m[1:-6].reshape(-1, 3)
+    np.testing.assert_allclose(r["forces"], f, rtol=0,
+                               atol=1e-10 * max(1.0, np.abs(f).max()))
+    np.testing.assert_allclose(r["local_var"], var, rtol=0,
+                               atol=1e-10 * max(1.0, np.abs(var).max()))
+
+
+def test_a_group_and_a_species_at_a_time_agree():
+    """32,768 atoms in one call (grouped) and the same beside 700 more (a
+    species at a time): the same bits."""
+    import flare_gb300 as fg
+    _, gp, calc, _ = weighted((20, 33), 3, 2, 2, seed=5)
+    big = fg.Structure(*lattice(32768, 1), 4.0, [calc])
+    more = fg.Structure(*lattice(700, 2), 4.0, [calc])
+    a = gp.predict_batch([big], precision="fp64")
+    b = gp.predict_batch([big, more], precision="fp64")
+    assert a["energy"][0] == b["energy"][0]
+    assert np.array_equal(a["forces"], b["forces"][:32768])
+    assert np.array_equal(a["stress"][0], b["stress"][0])
+    assert np.array_equal(a["local_var"], b["local_var"][:32768])
