@@ -206,12 +206,8 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
           if (!ok || !(r.x <= rc)) {
             sj = -1;
           } else if (t < kHalf) {
-            if constexpr (std::is_same<T, double>::value)
-              ylm_eval<T, LC>(p.l_max, r.y, r.z, r.w, sy + lane * NH, nullptr,
-                              r.x);
-            else
-              ylm_eval<T, LC>(p.l_max, T(r.y), T(r.z), T(r.w),
-                              sy + lane * NH, nullptr);
+            ylm_eval<T, LC>(p.l_max, T(r.y), T(r.z), T(r.w), sy + lane * NH,
+                            nullptr);
           } else {
             T g[NC];
             radial_eval<T, NC>(p, T(r.x), T(rc), g, (T *)nullptr);
@@ -266,10 +262,7 @@ k_b2_forward(B2Params p, int n_atoms, const long long *__restrict__ offsets,
         } else {
           radial_eval<T, NC>(p, T(r.x), T(rc), sg + t * nm, (T *)nullptr);
         }
-        if constexpr (std::is_same<T, double>::value)
-          ylm_eval<T, LC>(p.l_max, r.y, r.z, r.w, sy + t * nh, nullptr, r.x);
-        else
-          ylm_eval<T, LC>(p.l_max, T(r.y), T(r.z), T(r.w), sy + t * nh, nullptr);
+        ylm_eval<T, LC>(p.l_max, T(r.y), T(r.z), T(r.w), sy + t * nh, nullptr);
       } else {
         sj = -1;
       }

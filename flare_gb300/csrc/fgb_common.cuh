@@ -5,7 +5,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
-#include <type_traits>
 
 #include "flaregb.h"
 
@@ -347,17 +346,11 @@ __device__ __forceinline__ void radial_eval(const B2Params &p, T r, T rc,
 // m = L..0, l = m..L) with the Cartesian gradient when Grad (zeros
 // otherwise).  LC > 0 fixes l_max at compile time (loops unrolled, the
 // recurrence state kept in registers); LC = 0 takes Lrt.
-// rk > 0: the vector's length, known to the caller.
 template <typename T, int LC, bool Grad, typename Fn>
-__device__ __forceinline__ void ylm_visit(int Lrt, T x, T y, T z, Fn &&fn,
-                                          double rk = 0.0) {
+__device__ __forceinline__ void ylm_visit(int Lrt, T x, T y, T z, Fn &&fn) {
   constexpr int LA = LC > 0 ? LC : kMaxL;
   const int L = LC > 0 ? LC : Lrt;
-  T r;
-  if constexpr (std::is_same<T, double>::value)
-    r = rk > 0.0 ? rk : sqrt(x * x + y * y + z * z);
-  else
-    r = sqrt(x * x + y * y + z * z);
+  T r = sqrt(x * x + y * y + z * z);
   T ir = T(1) / r;
   T ux = x * ir, uy = y * ir, uz = z * ir;
   T C[LA + 1], S[LA + 1];
@@ -427,18 +420,17 @@ __device__ __forceinline__ void ylm_visit(int Lrt, T x, T y, T z, Fn &&fn,
 // The harmonics into Y[] (and, if Yd != nullptr, the Cartesian gradient
 // into Yd[3*idx + k]).
 template <typename T, int LC = 0>
-__device__ __forceinline__ void ylm_eval(int L, T x, T y, T z, T *Y, T *Yd,
-                                         double rk = 0.0) {
+__device__ __forceinline__ void ylm_eval(int L, T x, T y, T z, T *Y, T *Yd) {
   if (Yd) {
     ylm_visit<T, LC, true>(L, x, y, z, [&](int idx, T v, T gx, T gy, T gz) {
       Y[idx] = v;
       Yd[3 * idx] = gx;
       Yd[3 * idx + 1] = gy;
       Yd[3 * idx + 2] = gz;
-    }, rk);
+    });
   } else {
     ylm_visit<T, LC, false>(L, x, y, z,
-                            [&](int idx, T v, T, T, T) { Y[idx] = v; }, rk);
+                            [&](int idx, T v, T, T, T) { Y[idx] = v; });
   }
 }
 

@@ -27,6 +27,10 @@ constexpr int kMaxK = 1472;
 // group then sums to at most 12288 * K.
 constexpr int kS64 = 10;
 constexpr int kMaxK64 = 1360;
+// Triangular operands at kS64 slices count as lower triangular in blocks of
+// this size, whatever the tile: what an inverse has above its diagonal (1e-12
+// of rounding where entries are 1e4) is then taken or left by the matrix alone.
+constexpr int kTriBlock = 64;
 constexpr int kTiles64 = 3;
 constexpr int kTN64v[kTiles64] = {48, 32, 16};   // B tile heights of its products
 // FP32-level configuration (force GEMM of the mixed path): 4 slices, B tiles
@@ -75,6 +79,9 @@ struct SliceSpec {
   // optional: each source row's largest |value| (indexed like src rows);
   // the row scales then come from it instead of a pass over the rows
   const double *rowmax = nullptr;
+  // a lower-triangular matrix in blocks of kTriBlock: row r's entries from
+  // column kTriBlock (r / kTriBlock + 1) on are read as zeros
+  bool lower = false;
 };
 
 struct Sliced;

@@ -310,6 +310,11 @@ __device__ __forceinline__ void store_digits8(long long (&X)[8],
   }
 }
 
+// Columns of row `row` that are read (SliceSpec::lower).
+__device__ __forceinline__ int row_cols(int K, long long row, int lower) {
+  return lower ? (int)min((long long)K, (row / kTriBlock + 1) * kTriBlock) : K;
+}
+
 // The scale of a row of K values (each times `inv`): 2^e with e from its
 // largest magnitude, 2^0 for an empty row; by the lanes of one warp.
 __device__ __forceinline__ double row_scale(int K, const double *sr, double inv) {
@@ -334,7 +339,7 @@ __device__ __forceinline__ double row_scale(int K, const double *sr, double inv)
 __global__ void __launch_bounds__(256)
 k_oz_rowscale(int R, int K, int RP, const double *__restrict__ src,
               long long ld, const int *__restrict__ perm,
-              const double *__restrict__ rownorm, double thresh,
+              const double *__restrict__ rownorm, int lower, double thresh,
               double *__restrict__ scale) {
   const int m = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (m >= RP) return;
@@ -349,7 +354,8 @@ k_oz_rowscale(int R, int K, int RP, const double *__restrict__ src,
       else valid = false;
     }
   }
-  const double x = row_scale(valid ? K : 0, src + row * ld, inv);
+  const double x =
+      row_scale(valid ? row_cols(K, row, lower) : 0, src + row * ld, inv);
   if ((threadIdx.x & 31) == 0) scale[m] = x;
 }
 
@@ -358,7 +364,7 @@ constexpr int kSliceWarps = 4;
 enum { kScaleRows, kScaleMax, kScaleGiven };
 // One operand of k_oz_slice, and optionally a second layout of the same rows.
 struct SliceOp {
-  int R, K, RP, KP, TR, ncols, nparts, mode, vec;
+  int R, K, RP, KP, TR, ncols, nparts, mode, vec, lower;
   const double *src;
   long long ld;
   const int *perm;
@@ -414,7 +420,8 @@ k_oz_slice(const __grid_constant__ SliceOp oa, const __grid_constant__ SliceOp o
       const long long rq = __shfl_sync(0xffffffffu, row, q);
       const bool vq = __shfl_sync(0xffffffffu, (int)valid, q);
       const double iq = __shfl_sync(0xffffffffu, inv, q);
-      const double x = row_scale(vq ? K : 0, o.src + rq * o.ld, iq);
+      const double x =
+          row_scale(vq ? row_cols(K, rq, o.lower) : 0, o.src + rq * o.ld, iq);
       if (lane == 0) s_scale[q] = x;
     }
     __syncthreads();
@@ -430,6 +437,7 @@ k_oz_slice(const __grid_constant__ SliceOp oa, const __grid_constant__ SliceOp o
     if (PAIR && m < o.RP2) o.scale2[m] = sc;
   }
   const double *sr = o.src + row * o.ld;
+  const int Kr = row_cols(K, row, o.lower);
   const int e = pow2_exp(sc), TR = o.TR;
   const bool vec = o.vec, scaled = o.rownorm;
   __nv_bfloat16 *out = o.out;
@@ -439,7 +447,7 @@ k_oz_slice(const __grid_constant__ SliceOp oa, const __grid_constant__ SliceOp o
     // the lane's 8 values: four 16-byte loads when the source rows allow
     // (vec: 16-byte aligned rows) and all 8 lie inside the row
     double v[8];
-    if (vec && valid && k0 + 8 <= K) {
+    if (vec && valid && k0 + 8 <= Kr) {
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const double2 t = reinterpret_cast<const double2 *>(sr + k0)[q];
@@ -448,13 +456,13 @@ k_oz_slice(const __grid_constant__ SliceOp oa, const __grid_constant__ SliceOp o
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; j++) v[j] = (valid && k0 + j < K) ? sr[k0 + j] : 0.0;
+      for (int j = 0; j < 8; j++) v[j] = (valid && k0 + j < Kr) ? sr[k0 + j] : 0.0;
     }
     long long X[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const int k = k0 + j;
-      X[j] = (valid && k < K)
+      X[j] = (valid && k < Kr)
                  ? fixed_rn(scaled ? v[j] * inv : v[j], kBeta * S - e)
                  : 0;
     }
@@ -637,8 +645,9 @@ k_oz_gemm(const __grid_constant__ GemmGroup<Epi, NG> G, int tri, int lower,
     return P;
   };
   auto tile_nch = [&](const GemmProb<Epi> &P, int nt) {
-    const int n0 = nt * TN;
-    const int kmax = tri ? min(P.K, n0 + TN) : P.K;
+    const int n1 = (nt + 1) * TN;
+    const int end = S == kS64 ? (n1 + kTriBlock - 1) / kTriBlock * kTriBlock : n1;
+    const int kmax = tri ? min(P.K, end) : P.K;
     return (kmax + kKC - 1) / kKC;
   };
   auto give_up = [&](int why) {   // why: 1 aborted elsewhere, 2 timed out
@@ -945,7 +954,7 @@ static int slice_op(const SliceSpec &sp, const Operand &out, SliceOp &o,
   int ncols = few ? kStep : 4 * kStep;
   while (ceil_div(out.KP, ncols) > 65535) ncols *= 2;   // the grid's y limit
   o = {sp.rows, sp.K, out.RP, out.KP, sp.TR, ncols, ceil_div(out.KP, ncols),
-       kScaleRows, vec, sp.src, sp.ld, sp.perm, sp.rownorm, sp.rowmax,
+       kScaleRows, vec, sp.lower ? 1 : 0, sp.src, sp.ld, sp.perm, sp.rownorm, sp.rowmax,
        out.q, nullptr, out.scale, nullptr, 0, 0};
   // a block that finds the scales reads its rows whole: in many parts of
   // long rows that is more than a pass of its own
@@ -955,7 +964,7 @@ static int slice_op(const SliceSpec &sp, const Operand &out, SliceOp &o,
     o.mode = kScaleGiven;
     k_oz_rowscale<<<ceil_div((long long)out.RP * 32, 256), 256, 0, st>>>(
         sp.rows, sp.K, out.RP, sp.src, sp.ld, sp.perm, sp.rownorm,
-        kEmptyThresh, out.scale);
+        sp.lower ? 1 : 0, kEmptyThresh, out.scale);
     FGB_LAUNCH_CHECK("k_oz_rowscale");
   }
   return FGB_OK;
@@ -1736,7 +1745,7 @@ static int build_oz64_L(fgb_model_s *m, int v, cudaStream_t st) {
   return build_oz64(m, v, m->oz64L[v], [&](int s, int &) {
     return oz::SliceSpec{m->h_panel_rows[s], m->h_counts[s], 0,
                          m->Lp.as<double>() + m->h_panel_off[s],
-                         m->h_counts[s], nullptr, nullptr};
+                         m->h_counts[s], nullptr, nullptr, nullptr, true};
   }, st);
 }
 

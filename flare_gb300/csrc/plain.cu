@@ -91,8 +91,7 @@ k_pair_basis(B2Params p, long long P, const int *__restrict__ center,
         y[(nh + idx) * P] = gx;
         y[(2 * nh + idx) * P] = gy;
         y[(3 * nh + idx) * P] = gz;
-      },
-      r.x);
+      });
 }
 
 // Radial pairs (n1 <= n2) ordered for a neighbour of species s = blockIdx.x:

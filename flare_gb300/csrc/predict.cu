@@ -1067,7 +1067,7 @@ static int solved_operand(const DevBuf &src, int M, int v, oz::Sliced *out,
                           bool *ready, cudaStream_t st) {
   if (ready[v]) return FGB_OK;
   const int rc = oz::slice({M, M, oz::kTN64v[v], src.as<double>(), M, nullptr,
-                            nullptr},
+                            nullptr, nullptr, true},
                            out[v], st, oz::kS64);
   if (rc == FGB_OK) ready[v] = true;
   return rc;

@@ -53,3 +53,27 @@ def test_a_group_and_a_species_at_a_time_agree():
     assert np.array_equal(a["forces"], b["forces"][:32768])
     assert np.array_equal(a["stress"][0], b["stress"][0])
     assert np.array_equal(a["local_var"], b["local_var"][:32768])
+
+
+@pytest.mark.parametrize("atoms", [8, 1500, 6000])
+def test_triangular_operand_in_blocks(atoms):
+    """What L_inv holds above its diagonal counts inside the 64-row diagonal
+    blocks and nowhere else, whatever the tile height (16, 32 or 48 rows)."""
+    import flare_gb300 as fg
+    M = 130
+    _, gp, calc, _ = weighted((M,), 3, 2, 2, seed=9)
+    r = np.random.Generator(np.random.PCG64(atoms))
+    L = r.normal(size=(M, M)) * 0.1
+    gp.set_weights(gp.sparse_descriptors, gp.alpha, L, [calc])
+    cell, _, pos = lattice(atoms, 3)
+    st = fg.Structure(cell, np.zeros(atoms, int), pos, 4.0, [calc])
+    B, n = (x.cpu().numpy() for x in st.b2_values())
+    d = gp.sparse_descriptors[0].descriptors[0]
+    c = (B / n[:, None]) @ (d / np.linalg.norm(d, axis=1)[:, None]).T
+    block = np.arange(M) // 64
+    z = 1.5 ** 2 * c ** 2 @ (L * (block[None, :] <= block[:, None])).T
+    want = 1.5 ** 2 - (z * z).sum(1)
+    var = gp.predict_batch([st], precision="fp64")["local_var"]
+    # sums of 130 products of FP64 level, squared and summed
+    np.testing.assert_allclose(var, want, rtol=0,
+                               atol=1e-12 * np.abs(want).max())
