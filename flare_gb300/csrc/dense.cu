@@ -9,11 +9,11 @@
 // rounding; about 35x this GPU's FP64 DGEMM rate); the O(M nb^2) work on
 // diagonal blocks of nb = 128 in shared memory:
 //   Cholesky, right-looking by block columns: factor the diagonal block
-//     and invert it (k_potrf_cluster), L21 = A21 L11^-T as a product with
+//     and invert it (k_potrf_cluster, k_potrf_inverse), L21 = A21 L11^-T as a product with
 //     that inverse, then the trailing update A22 -= L21 L21^T;
 //   lower-triangular inverse, recursive: X = [X11 0; X21 X22] with X11,
-//     X22 the inverses of the diagonal halves (leaves of nb inverted by
-//     k_trtri_block, all at once) and X21 = -X22 (L21 X11).
+//     X22 the inverses of the diagonal halves (leaves of nb from the
+//     factorisation, or all at once by k_trtri_block for a given L) and X21 = -X22 (L21 X11).
 // Operation orders differ from Eigen's (the reference's LLT and triangular
 // solves), so results agree with it to FP64 rounding, not bit for bit.
 #include <cmath>

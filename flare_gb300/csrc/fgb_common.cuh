@@ -102,7 +102,8 @@ __device__ __forceinline__ void ylm_norm(int i, float &k) { k = c_ylm_norm_f[i];
 // FP32 head + FP32 tail) and the reciprocals 1/k (k = 1 .. 2 kMaxL + 1,
 // FP32 nearest and its FP32 remainder): the associated-Legendre recurrence
 // multiplies by these instead of dividing (a double-float or FP32 division
-// costs tens of instructions; the FP64 evaluation keeps its divisions).
+// costs tens of instructions, an FP64 one about ten of 16 cycles each; see
+// div_int for how the FP64 quotient stays correctly rounded).
 constexpr int kNumInv = 2 * kMaxL + 2;
 __host__ __device__ constexpr double dfact_value(int m) {
   double v = 1.0;

@@ -13,8 +13,11 @@
 // C = 2^(e_row + e_col) sum_t 2^(-6t) group_t exactly in 64-bit integers,
 // rounding once to FP64 or FP32.  The dropped terms (a + b > S + 1) and the
 // slice residuals are below 2^(-6S) of each row's largest entry.
-//   S = 9, TN = 48:  FP64-level (2^-54); kernel and variance products of the
-//                    sparse GP (energy 4e-12 eV/atom, std 4e-13 against FP64)
+//   S = 10, TN = 48, 32 or 16: the products of the FP64 path and of the
+//                    stored-gradient form (2^-60)
+//   S = 9, TN = 48:  FP64-level (2^-54); the dense solve, and kernel and
+//                    variance products of the mixed path at most (energy
+//                    4e-12 eV/atom, std 4e-13 against FP64)
 //   S = 4, TN = 128: FP32-level (2^-24); the alpha-folded force GEMM
 //
 // Data movement: slices are written by k_oz_slice directly in the tensor

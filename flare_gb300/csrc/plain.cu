@@ -1,6 +1,6 @@
-// Plain FP64 form: the reference's algorithm on the GPU (stored
-// forward-mode descriptor gradients, envs_struc GEMM + scatter), envs_envs,
-// and the FP64 QR solve.
+// The stored-gradient form, the reference's algorithm on the GPU (forward-mode
+// descriptor gradients, envs_struc as exact-slice products and sums over the
+// pairs), envs_envs, and the FP64 QR solve.
 #include <cusolverDn.h>
 
 #include <type_traits>

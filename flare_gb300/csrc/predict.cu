@@ -1,5 +1,7 @@
-// K3/K4: kernel against the sparse set, adjoint GEMM and local variance in
-// FP64, plus the device-resident model and the fgb_predict pipeline.
+// The device-resident model and the fgb_predict pipeline, and K3/K4 (kernel
+// against the sparse set, adjoint GEMM and local variance) as FP64 SIMT
+// kernels: for powers other than 1 and 2 and for non-finite weights.  The
+// others take the exact-slice products of ozaki.cu.
 //
 // For the atoms of species s (rows gathered through a species permutation):
 //   GEMM1 (NT)  C = B2_s S^_s^T;  epilogue c = C/|d|, k = sigma^2 c^xi,
