@@ -568,8 +568,9 @@ def run_ours(args, rank, world, local):
         fp64_fused = {"value": N * k64 / (sum(per64) * 1e-3),
                       "unit": "atoms/s", "steps": k64,
                       "sample": f"the same {B}-structure batch through the "
-                                "fused FP64 path (neighbours, FP64 B2, FP64 "
-                                "SIMT GEMMs, FP64 adjoint), CUDA events"}
+                                "fused FP64 path (neighbours, FP64 B2, "
+                                "10-slice products, FP64 adjoint), CUDA "
+                                "events"}
         e64 = out["e"].cpu().numpy()
         f64 = out["f"].cpu().numpy()
         s64 = out["s"].cpu().numpy()
@@ -651,7 +652,7 @@ def run_ours(args, rank, world, local):
 
     # ---- dominant kernel roofline.  Algorithmic FLOP per launch: the
     # kernel GEMM c = d^ . s^ is 2 M_s n_d per atom of species s (one launch
-    # per species and row chunk), counted once whatever precision scheme
+    # per species and row chunk; FP64: one for all species), counted once whatever precision scheme
     # carries it; the time is the GEMM kernel's own launches (the row
     # slicing is a stage of its own).
     sizes = species_sizes(sp, offsets, gp)
@@ -660,7 +661,7 @@ def run_ours(args, rank, world, local):
                   "adjoint_gemm": sum(2.0 * n_s * m_s * nd_ for n_s, m_s in sizes),
                   "variance_gemm": sum(1.0 * n_s * m_s * (m_s + 1)
                                        for n_s, m_s in sizes)}
-    tensor = args.precision == "mixed" and oz_eligible(gp, b2)
+    tensor = oz_eligible(gp, b2)
     gemm_stage = max(fp64_flops, key=lambda s_: stage.get(s_, (0, 0))[0])
     st_ms, st_n = stage[gemm_stage]
     launches_per_step = st_n / args.steps
@@ -672,7 +673,8 @@ def run_ours(args, rank, world, local):
         # executed on the tensor pipe: S(S+1)/2 BF16 slice products per
         # FP64-level product (S slices of 6 bits, a + b <= S + 1)
         S_ = (guard["variance_slices"] if gemm_stage == "variance_gemm"
-              else guard["kernel_slices"]) if guard else 9
+              else guard["kernel_slices"]) if guard else \
+            10 if args.precision == "fp64" else 9
         products = S_ * (S_ + 1) // 2
         peak, peak_src = bf16_peak()
         roofline = {"kernel": gemm_stage + " (k_oz_gemm, tcgen05, exact BF16 "

@@ -2020,7 +2020,7 @@ int kernel_stage_oz(fgb_model_s *m, int N, const std::vector<int> &counts,
         return rc;
       int vk = 0;
       {
-        StageTimer _pt(kStRowSlice, st, 2);   // row scales, slices
+        StageTimer _pt(kStRowSlice, st);
         if ((rc = oz::slice({Mr, nd, oz::kTM, m->ws.B2.as<double>(), nd, perm,
                              m->ws.norms.as<double>(),
                              m->ws.rowmax.as<double>()},
@@ -2201,7 +2201,7 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
     sa += A[i].RP;
   }
   {
-    StageTimer _pt(kStRowSlice, st, 2);
+    StageTimer _pt(kStRowSlice, st, ceil_div(n, 2));
     for (int i = 0; i < n; i += 2) {   // two species a launch
       oz::SliceSpec sp[2];
       for (int q = i; q < std::min(n, i + 2); q++)
@@ -2335,7 +2335,7 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
            (rc = oz::prepare(Mr, Ms, oz::kTM, oz::kS64, m->ws.ozW))))
         return rc;
       {
-        StageTimer _pt(kStRowSlice, st, 2);
+        StageTimer _pt(kStRowSlice, st);
         if ((rc = oz::slice({Mr, nd, oz::kTM, m->ws.B2.as<double>(), nd, perm,
                              nullptr,
                              have_rowmax ? m->ws.rowmax.as<double>() : nullptr},
