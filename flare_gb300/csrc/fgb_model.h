@@ -36,7 +36,7 @@ struct fgb_workspace {
   fgb::DevBuf redpart;  // chunk sums of structures above one chunk
   fgb::DevBuf rowmax;   // largest |B2| per row (tensor-core row scales)
   fgb::DevBuf gB2, pair_grad, forces, virial;
-  fgb::DevBuf kmat, wmat, erows, part;
+  fgb::DevBuf kmat, wmat, erows, part, vpart;
   fgb::DevBuf b2f, yf;           // mixed path: FP32 normalised rows, D^ B
   // stored-gradient form: pairs grouped by species, basis values, gradients,
   // cosines, force kernel, sparse norms and slices
@@ -204,6 +204,9 @@ namespace fgb {
 int kernel_stage_fp64(fgb_model_s *m, int N, const std::vector<int> &counts,
                       bool want_grad, bool want_var, double *d_e_atom,
                       double *d_gB2, double *d_var, cudaStream_t st);
+// Local variances of Mr rows of species s in the SIMT kernels' order.
+int variance_small(fgb_model_s *m, int s, int Mr, const int *perm,
+                   double *d_var, cudaStream_t st);
 // The FP64 stage of a power-1 or power-2 model with finite weights on the
 // tensor cores (ozaki.cu), else the FP64 SIMT kernels (predict.cu).
 // have_rowmax: ws.rowmax holds each row's largest |B2|; ws.ozerr is cleared

@@ -2100,6 +2100,20 @@ bool fp64_stage_sliced(const fgb_model_s *m) {
   return (m->power == 2.0 || m->power == 1.0) && m->finite;
 }
 
+// Species whose FP64 variances take the SIMT order (variance_small): models
+// of few sparse environments, whose kernel matrix and variance product are at
+// most kSmallVar multiply-adds a row.  Where such a model describes near-equal
+// environments, sigma^2 - |z|^2 cancels to 1e-5 of its terms and the standard
+// deviations of two FP64 summation orders differ by up to 2e-9; these are the
+// SIMT kernels' to the bit.  The model alone decides, so that a structure's
+// results don't depend on its batch.  32 FCC atoms, 64 sparse: 24 us where the
+// sliced product took 9 (and one 64 x 64 SIMT tile 150 for each of the two).
+constexpr long long kSmallVar = 65536;
+static bool small_variance(const fgb_model_s *m, int s) {
+  const long long M = m->h_counts[s];
+  return M * m->b2.n_d + M * M / 2 <= kSmallVar;
+}
+
 // Species whose products run side by side: those with atoms and sparse
 // environments, where all atoms are one chunk of rows (else 0).
 static int stage64_group(const fgb_model_s *m, const std::vector<int> &counts,
@@ -2134,9 +2148,10 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
     int s, N, M, R, off, kslots, vslots;
     const int *perm;
     size_t e0, v0;   // first entries in erows and part
+    bool sv;         // variance by the sliced product
   };
   std::vector<Part> parts;
-  std::vector<int> rows, mcols, rcols, dcols;
+  std::vector<int> rows, mcols, dcols, vrows, vcols;
   int base = 0;
   for (int s = 0; s < p.n_species; s++) {
     const int N = counts[s], M = m->h_counts[s];
@@ -2149,19 +2164,24 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
                                     st)))
       return rc;
     if (N == 0 || M == 0) continue;
+    const bool sv = want_var && !small_variance(m, s);
     parts.push_back({s, N, M, m->h_panel_rows[s], m->h_offsets[s], 0, 0, perm,
-                     0, 0});
+                     0, 0, sv});
     rows.push_back(N);
     mcols.push_back(M);
-    rcols.push_back(m->h_panel_rows[s]);
     dcols.push_back(nd);
+    if (sv) {
+      vrows.push_back(N);
+      vcols.push_back(m->h_panel_rows[s]);
+    }
   }
   const int n = (int)parts.size();
   const int vk = oz::tile64(n, rows.data(), mcols.data()),
-            vv = oz::tile64(n, rows.data(), rcols.data()),
+            vv = oz::tile64((int)vrows.size(), vrows.data(), vcols.data()),
             vg = oz::tile64(n, rows.data(), dcols.data());
+  const bool any_sv = !vrows.empty();
   if ((rc = ready(m->oz64S_ready, vk, build_oz64_S)) ||
-      (want_var && (rc = ready(m->oz64L_ready, vv, build_oz64_L))) ||
+      (any_sv && (rc = ready(m->oz64L_ready, vv, build_oz64_L))) ||
       (want_grad && (rc = ready(m->oz64ST_ready, vg, build_oz64_ST))))
     return rc;
   // the species' operands one after the other in the workspace's buffers
@@ -2172,7 +2192,7 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
     A[i] = oz::operand(P.N, nd, oz::kTM, oz::kS64);
     K[i] = oz::operand(P.N, P.M, oz::kTM, oz::kS64);
     P.kslots = m->oz64S[vk][P.s]->RP / 16;
-    P.vslots = want_var ? m->oz64L[vv][P.s]->RP / 16 : 0;
+    P.vslots = P.sv ? m->oz64L[vv][P.s]->RP / 16 : 0;
     P.e0 = ne;
     P.v0 = nv;
     ne += (size_t)P.N * P.kslots;
@@ -2184,17 +2204,17 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
   const size_t h = sizeof(__nv_bfloat16), d = sizeof(double);
   if ((rc = m->ws.ozA.q.ensure(h * qa)) || (rc = m->ws.ozA.scale.ensure(d * sa)) ||
       (rc = m->ws.erows.ensure(d * ne)) ||
-      (want_var && ((rc = m->ws.ozK.q.ensure(h * qk)) ||
-                    (rc = m->ws.ozK.scale.ensure(d * sa)) ||
-                    (rc = m->ws.part.ensure(d * nv)))) ||
+      (any_sv && ((rc = m->ws.ozK.q.ensure(h * qk)) ||
+                  (rc = m->ws.ozK.scale.ensure(d * sa)) ||
+                  (rc = m->ws.part.ensure(d * nv)))) ||
       (want_grad && ((rc = m->ws.ozW.q.ensure(h * qk)) ||
                      (rc = m->ws.ozW.scale.ensure(d * sa)))))
     return rc;
   qa = qk = sa = 0;
   for (int i = 0; i < n; i++) {
-    W[i] = K[i];
+    W[i] = K[i];   // not placed (null): not wanted
     A[i].at(m->ws.ozA, qa, sa);
-    if (want_var) K[i].at(m->ws.ozK, qk, sa);
+    if (parts[i].sv) K[i].at(m->ws.ozK, qk, sa);
     if (want_grad) W[i].at(m->ws.ozW, qk, sa);
     qa += A[i].values();
     qk += K[i].values();
@@ -2219,9 +2239,7 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
       const Part &P = parts[i];
       const double wmax = m->alpha_max[P.s];
       B[i] = m->oz64S[vk][P.s]->operand();
-      epi.push_back({want_var ? K[i].q : nullptr, want_grad ? W[i].q : nullptr,
-                     want_var ? K[i].scale : nullptr,
-                     want_grad ? W[i].scale : nullptr, K[i].KP,
+      epi.push_back({K[i].q, W[i].q, K[i].scale, W[i].scale, K[i].KP,
                      wmax > 0.0 ? std::ilogb(wmax) + 1 : 0,
                      m->ws.erows.as<double>() + P.e0, P.kslots,
                      m->alpha.as<double>() + P.off,
@@ -2252,24 +2270,27 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
     }
     if ((rc = oz::gemm64_group(W, B, false, epi, err, st))) return rc;
   }
-  if (want_var) {
-    {
-      StageTimer _pt(kStVarianceGemm, st);
-      std::vector<oz::EpiZsq> epi;
-      for (int i = 0; i < n; i++) {
-        B[i] = m->oz64L[vv][parts[i].s]->operand();
-        epi.push_back({m->ws.part.as<double>() + parts[i].v0, parts[i].vslots,
-                       parts[i].R});
-      }
-      if ((rc = oz::gemm64_group(K, B, true, epi, err, st))) return rc;
+  if (any_sv) {
+    StageTimer _pt(kStVarianceGemm, st);
+    std::vector<oz::Operand> Kv, Lv;
+    std::vector<oz::EpiZsq> epi;
+    for (int i = 0; i < n; i++) {
+      if (!parts[i].sv) continue;
+      Kv.push_back(K[i]);
+      Lv.push_back(m->oz64L[vv][parts[i].s]->operand());
+      epi.push_back({m->ws.part.as<double>() + parts[i].v0, parts[i].vslots,
+                     parts[i].R});
     }
-    for (const Part &P : parts)
-      if ((rc = launch_variance_final(P.N, P.vslots,
-                                      m->ws.part.as<double>() + P.v0, P.perm,
-                                      m->ws.norms.as<double>(), sig2, xi, d_var,
-                                      st, sig2 * sig2)))
-        return rc;
+    if ((rc = oz::gemm64_group(Kv, Lv, true, epi, err, st))) return rc;
   }
+  if (want_var)
+    for (const Part &P : parts)
+      if ((rc = P.sv ? launch_variance_final(
+                           P.N, P.vslots, m->ws.part.as<double>() + P.v0,
+                           P.perm, m->ws.norms.as<double>(), sig2, xi, d_var, st,
+                           sig2 * sig2)
+                     : variance_small(m, P.s, P.N, P.perm, d_var, st)))
+        return rc;
   return FGB_OK;
 }
 
@@ -2315,6 +2336,7 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
     }
     if (Ms == 0) continue;
     const int R = m->h_panel_rows[s], off = m->h_offsets[s];
+    const bool sv = want_var && !small_variance(m, s);
     const double wmax = m->alpha_max[s];
     const int eW = wmax > 0.0 ? std::ilogb(wmax) + 1 : 0;
     for (int r0 = 0; r0 < Ns; r0 += kRows) {
@@ -2323,13 +2345,13 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
       const int vk = oz::tile64(Mr, Ms), vv = oz::tile64(Mr, R),
                 vg = oz::tile64(Mr, nd);
       if ((rc = ready(m->oz64S_ready, vk, build_oz64_S)) ||
-          (want_var && (rc = ready(m->oz64L_ready, vv, build_oz64_L))) ||
+          (sv && (rc = ready(m->oz64L_ready, vv, build_oz64_L))) ||
           (want_grad && (rc = ready(m->oz64ST_ready, vg, build_oz64_ST))))
         return rc;
       const oz::Sliced &Sk = *m->oz64S[vk][s];
       const int kslots = Sk.RP / 16;
       if ((rc = m->ws.erows.ensure(sizeof(double) * (size_t)Mr * kslots)) ||
-          (want_var &&
+          (sv &&
            (rc = oz::prepare(Mr, Ms, oz::kTM, oz::kS64, m->ws.ozK))) ||
           (want_grad &&
            (rc = oz::prepare(Mr, Ms, oz::kTM, oz::kS64, m->ws.ozW))))
@@ -2345,9 +2367,9 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
       {
         StageTimer _pt(kStKernelGemm, st);
         const oz::EpiKernel64 epi{
-            want_var ? m->ws.ozK.q.as<__nv_bfloat16>() : nullptr,
+            sv ? m->ws.ozK.q.as<__nv_bfloat16>() : nullptr,
             want_grad ? m->ws.ozW.q.as<__nv_bfloat16>() : nullptr,
-            want_var ? m->ws.ozK.scale.as<double>() : nullptr,
+            sv ? m->ws.ozK.scale.as<double>() : nullptr,
             want_grad ? m->ws.ozW.scale.as<double>() : nullptr,
             oz::pad_to(Ms, oz::kKC), eW, m->ws.erows.as<double>(), kslots,
             m->alpha.as<double>() + off, m->sinv.as<double2>() + off,
@@ -2373,7 +2395,10 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
                            m->ws.ozerr.as<int>(), st)))
           return rc;
       }
-      if (want_var) {
+      if (want_var && !sv &&
+          (rc = variance_small(m, s, Mr, perm, d_var, st)))
+        return rc;
+      if (sv) {
         const oz::Sliced &L = *m->oz64L[vv][s];
         const int vslots = L.RP / 16;
         if ((rc = m->ws.part.ensure(sizeof(double) * (size_t)Mr * vslots)))

@@ -167,6 +167,98 @@ __global__ void k_variance_final(int M, int ntiles, const double *__restrict__ p
   var[atom] = kself - s * scale;
 }
 
+// The kernel matrix and GEMM3 above for models of few sparse environments
+// (small_variance), a thread an element, the same operations in the same
+// order: the same bits.  8 x 16 elements a block, four warps, which the FP64
+// unit of an SM serves in the 64 cycles of one instruction.
+constexpr int kSmT = 128, kSmR = 8, kSmC = 16, kSmK = 48;
+__global__ void __launch_bounds__(kSmT)
+k_kernel_small(int M, int N, int K, const double *__restrict__ B2,
+               const int *__restrict__ perm, const double *__restrict__ norms,
+               const double *__restrict__ S,
+               const unsigned char *__restrict__ svalid, double sig2, double xi,
+               double *__restrict__ Kmat) {
+  __shared__ double As[kSmR][kSmK + 1], Bs[kSmC][kSmK + 1];
+  const int t = threadIdx.x, r = t / kSmC, c = t % kSmC;
+  const int m0 = blockIdx.y * kSmR, n0 = blockIdx.x * kSmC;
+  const int m = m0 + r, n = n0 + c;
+  double acc = 0.0;
+  for (int k0 = 0; k0 < K; k0 += kSmK) {
+    const int kc = min(kSmK, K - k0);
+    for (int e = t; e < (kSmR + kSmC) * kSmK; e += kSmT) {
+      const int row = e / kSmK, k = e % kSmK;
+      double v = 0.0;
+      if (row < kSmR) {
+        if (m0 + row < M && k < kc)
+          v = B2[(long long)perm[m0 + row] * K + k0 + k];
+        As[row][k] = v;
+      } else {
+        if (n0 + row - kSmR < N && k < kc)
+          v = S[(long long)(n0 + row - kSmR) * K + k0 + k];
+        Bs[row - kSmR][k] = v;
+      }
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < kc; k++) acc = fma(As[r][k], Bs[c][k], acc);
+    __syncthreads();
+  }
+  if (m >= M || n >= N) return;
+  const double nd = norms[perm[m]];
+  double kv = 0.0;
+  if (nd >= kEmptyThresh && svalid[n]) {
+    const double x = acc / nd;
+    kv = sig2 * powx(x, xi);
+  }
+  Kmat[(long long)m * N + n] = kv;
+}
+// Two rows and BN columns a block.
+__global__ void __launch_bounds__(kSmT)
+k_variance_small(int M, int R, int Ms, const double *__restrict__ Kmat,
+                 const double *__restrict__ Lp, double *__restrict__ part,
+                 int ntiles) {
+  static_assert(kSmT == 2 * BN, "two rows of a column tile");
+  __shared__ double Ks[2][32], Ls[BN][33], red[2][BN];
+  const int t = threadIdx.x, r = t / BN, c = t % BN;
+  const int m0 = blockIdx.y * 2, n0 = blockIdx.x * BN;
+  const int kmax = min(Ms, n0 + BN);
+  double acc = 0.0;
+  for (int k0 = 0; k0 < kmax; k0 += 32) {
+    const int kc = min(32, kmax - k0);
+    if (t < 64) {
+      const int row = t / 32, k = t % 32;
+      Ks[row][k] = m0 + row < M && k < kc
+                       ? Kmat[(long long)(m0 + row) * Ms + k0 + k] : 0.0;
+    }
+    for (int e = t; e < BN * 32; e += kSmT) {
+      const int row = e / 32, k = e % 32;
+      Ls[row][k] = n0 + row < R && k < kc
+                       ? Lp[(long long)(n0 + row) * Ms + k0 + k] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < kc; k++) acc = fma(Ks[r][k], Ls[c][k], acc);
+    __syncthreads();
+  }
+  red[r][c] = acc;
+  __syncthreads();
+  double s = 0.0;
+  if (c < 16)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const double z = red[r][c + 16 * j];
+      if (n0 + c + 16 * j < R) s += z * z;
+    }
+  __syncthreads();
+  if (c < 16) red[r][c] = s;
+  __syncthreads();
+  if (c == 0 && m0 + r < M) {
+    double v = 0.0;
+    for (int q = 0; q < 16; q++) v += red[r][q];
+    part[(long long)(m0 + r) * ntiles + blockIdx.x] = v;
+  }
+}
+
 // out[m] = sum of the row's partial slots (fixed order, row_slots_sum)
 __global__ void k_sum_parts(int M, int nslots, const double *__restrict__ part,
                             double *__restrict__ out) {
@@ -363,6 +455,36 @@ int launch_kt_alpha(int M, long long ncol, const double *KT,
   k_kt_alpha<<<ceil_div(ncol * 32, 128), 128, 0, st>>>(M, ncol, KT, alpha, out);
   FGB_LAUNCH_CHECK("k_kt_alpha");
   return FGB_OK;
+}
+
+// Local variances of Mr rows of species s by k_kernel_small and
+// k_variance_small, from ws.B2 and ws.norms.
+int variance_small(fgb_model_s *m, int s, int Mr, const int *perm,
+                   double *d_var, cudaStream_t st) {
+  const int Ms = m->h_counts[s], R = m->h_panel_rows[s], nd = m->b2.n_d;
+  const int off = m->h_offsets[s], nt = ceil_div(R, BN);
+  const double sig2 = m->sigma * m->sigma;
+  int rc;
+  if ((rc = m->ws.kmat.ensure(sizeof(double) * (size_t)Mr * Ms)) ||
+      (rc = m->ws.vpart.ensure(sizeof(double) * (size_t)Mr * nt)))
+    return rc;
+  {
+    StageTimer _pt(kStVarianceGemm, st, 2);
+    k_kernel_small<<<dim3(ceil_div(Ms, kSmC), ceil_div(Mr, kSmR)), kSmT, 0,
+                     st>>>(Mr, Ms, nd, m->ws.B2.as<double>(), perm,
+                           m->ws.norms.as<double>(),
+                           m->S.as<double>() + (size_t)off * nd,
+                           m->svalid.as<unsigned char>() + off, sig2, m->power,
+                           m->ws.kmat.as<double>());
+    FGB_LAUNCH_CHECK("k_kernel_small");
+    k_variance_small<<<dim3(nt, ceil_div(Mr, 2)), kSmT, 0, st>>>(
+        Mr, R, Ms, m->ws.kmat.as<double>(),
+        m->Lp.as<double>() + m->h_panel_off[s], m->ws.vpart.as<double>(), nt);
+    FGB_LAUNCH_CHECK("k_variance_small");
+  }
+  return launch_variance_final(Mr, nt, m->ws.vpart.as<double>(), perm,
+                               m->ws.norms.as<double>(), sig2, m->power, d_var,
+                               st);
 }
 
 int launch_variance_final(int Mr, int ntiles, const double *part,

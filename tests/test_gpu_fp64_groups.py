@@ -55,12 +55,16 @@ def test_a_group_and_a_species_at_a_time_agree():
     assert np.array_equal(a["local_var"], b["local_var"][:32768])
 
 
-@pytest.mark.parametrize("atoms", [8, 1500, 6000])
-def test_triangular_operand_in_blocks(atoms):
+@pytest.mark.parametrize("atoms,M", [
+    (8, 400), (1500, 400), (6000, 400),    # slices
+    (1, 1), (9, 63), (8, 130), (33, 65), (1500, 130),   # the SIMT order
+])
+def test_triangular_operand_in_blocks(atoms, M):
     """What L_inv holds above its diagonal counts inside the 64-row diagonal
-    blocks and nowhere else, whatever the tile height (16, 32 or 48 rows)."""
+    blocks and nowhere else, whatever the tile height (16, 32 or 48 rows) and
+    on both sides of the size (about 340 sparse rows here) where the variance
+    product moves to the slices."""
     import flare_gb300 as fg
-    M = 130
     _, gp, calc, _ = weighted((M,), 3, 2, 2, seed=9)
     r = np.random.Generator(np.random.PCG64(atoms))
     L = r.normal(size=(M, M)) * 0.1
