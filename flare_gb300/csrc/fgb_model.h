@@ -10,8 +10,9 @@
 // Host copy of the species counts (and range flag; the stored-gradient form
 // also keeps its pair counts per species here): page-locked with the event
 // recorded after the copy, so that the host can wait for it after queueing
-// more work, or (pageable) plain host memory for a workspace of one call,
-// into which a copy returns complete.
+// more work, or (pageable) plain host memory for a workspace of one call, in
+// which a copy may still be in flight when cudaMemcpyAsync returns: it is
+// waited for where it is queued.
 struct fgb_pinned_counts {
   static constexpr int kInts = 2 * (fgb::kMaxSpecies + 1);
   int *h = nullptr;
@@ -19,6 +20,16 @@ struct fgb_pinned_counts {
   cudaEvent_t ev = nullptr;
   bool pageable = false;
   int host[kInts] = {};
+  // after a copy into h has been queued on st, and before h is read
+  int queued(cudaStream_t st) {
+    if (pageable) FGB_CUDA(cudaStreamSynchronize(st));
+    else FGB_CUDA(cudaEventRecord(ev, st));
+    return FGB_OK;
+  }
+  int wait() const {
+    if (!pageable) FGB_CUDA(cudaEventSynchronize(ev));
+    return FGB_OK;
+  }
   fgb_pinned_counts() = default;
   fgb_pinned_counts(const fgb_pinned_counts &) = delete;
   fgb_pinned_counts &operator=(const fgb_pinned_counts &) = delete;

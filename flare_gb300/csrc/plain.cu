@@ -677,7 +677,7 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
   int *spairs = ws.counts.h + kMaxSpecies + 1;
   FGB_CUDA(cudaMemcpyAsync(spairs, dsp, sizeof(int) * (S + 1),
                            cudaMemcpyDeviceToHost, st));
-  if (ws.counts.ev) FGB_CUDA(cudaEventRecord(ws.counts.ev, st));
+  if ((rc = ws.counts.queued(st))) return rc;
   k_group_rows<<<ceil_div((long long)N * 32, 128), 128, 0, st>>>(
       N, perm, off, start, ws.rows.as<int>());
   FGB_LAUNCH_CHECK("k_group_rows");
@@ -696,7 +696,7 @@ int envs_struc_impl(const B2Params &p, double sigma, double power,
     return rc;
   double *spart = ws.part.as<double>() + (size_t)M * nce;
   FGB_CUDA(cudaMemsetAsync(ws.part.p, 0, sizeof(double) * (size_t)M * nce, st));
-  if (ws.counts.ev) FGB_CUDA(cudaEventSynchronize(ws.counts.ev));
+  if ((rc = ws.counts.wait())) return rc;
   constexpr int kRows = 65536;   // gradient rows sliced at a time
   int base = 0;
   for (int s = 0; s < S; s++) {

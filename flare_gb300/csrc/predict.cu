@@ -592,7 +592,7 @@ int species_permutation_start(int S, fgb_workspace &ws, const int *d_species,
     FGB_CUDA(cudaEventCreateWithFlags(&pc.ev, cudaEventDisableTiming));
   FGB_CUDA(cudaMemcpyAsync(pc.h, tot, sizeof(int) * (S + 1),
                            cudaMemcpyDeviceToHost, st));
-  if (pc.ev) FGB_CUDA(cudaEventRecord(pc.ev, st));
+  if ((rc = pc.queued(st))) return rc;
   pending = true;
   return FGB_OK;
 }
@@ -600,7 +600,8 @@ int species_permutation_start(int S, fgb_workspace &ws, const int *d_species,
 int species_permutation_finish(int S, fgb_workspace &ws,
                                std::vector<int> &counts) {
   const fgb_pinned_counts &pc = ws.counts;
-  if (pc.ev) FGB_CUDA(cudaEventSynchronize(pc.ev));
+  const int rc = pc.wait();
+  if (rc) return rc;
   if (pc.h[S]) {
     set_error("species must lie in [0, %d)", S);
     return FGB_EINVAL;
