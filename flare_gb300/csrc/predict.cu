@@ -729,15 +729,37 @@ extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
                              const double *h_L_inv) {
   if (!m || !h_counts) { set_error("fgb_model_set: invalid arguments"); return FGB_EINVAL; }
   const int S = m->b2.n_species, nd = m->b2.n_d;
-  m->h_counts.assign(h_counts, h_counts + S);
-  m->h_offsets.assign(S + 1, 0);
+  int M = 0;
   for (int s = 0; s < S; s++) {
     if (h_counts[s] < 0) { set_error("fgb_model_set: negative count"); return FGB_EINVAL; }
-    m->h_offsets[s + 1] = m->h_offsets[s] + h_counts[s];
+    M += h_counts[s];
   }
-  const int M = m->h_offsets[S];
-  m->M = M;
   if (M > 0 && !h_desc) { set_error("fgb_model_set: descriptors required"); return FGB_EINVAL; }
+  // nothing of the weights before stays in use, also if this call fails on
+  // the way: neither R_inv (of another Sigma, perhaps of another size) nor
+  // any sliced operand
+  m->solved = false;
+  m->has_rinv = false;
+  m->bmap_ready = false;
+  m->lfull_ready = false;
+  m->slices_chosen = false;
+  m->oz_S = oz::kS;
+  m->oz_Sv = oz::kS;
+  m->oz_err_est = 0.0;
+  m->oz_var_err_est = 0.0;
+  m->force_f64 = false;
+  m->fold_max = 0.0;
+  for (bool &r : m->ozS_ready) r = false;
+  for (bool &r : m->ozL_ready) r = false;
+  for (bool &r : m->ozB_ready) r = false;
+  for (int v = 0; v < oz::kTiles64; v++)
+    m->oz64S_ready[v] = m->oz64ST_ready[v] = m->oz64L_ready[v] =
+        m->oz64R_ready[v] = m->oz64Lfull_ready[v] = false;
+  m->h_counts.assign(h_counts, h_counts + S);
+  m->h_offsets.assign(S + 1, 0);
+  for (int s = 0; s < S; s++)
+    m->h_offsets[s + 1] = m->h_offsets[s] + h_counts[s];
+  m->M = M;
   // normalised sparse descriptors, validity flags (norm >= 1e-8)
   std::vector<double> Sh((size_t)M * nd);
   std::vector<unsigned char> valid(M);
@@ -768,21 +790,6 @@ extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
     FGB_CUDA(cudaMemcpy(m->snorm.p, snorm.data(), sizeof(double) * M,
                         cudaMemcpyHostToDevice));
   }
-  m->solved = false;
-  m->bmap_ready = false;
-  m->lfull_ready = false;
-  m->slices_chosen = false;
-  m->oz_S = oz::kS;
-  m->oz_Sv = oz::kS;
-  m->oz_err_est = 0.0;
-  m->oz_var_err_est = 0.0;
-  m->force_f64 = false;
-  m->fold_max = 0.0;
-  for (bool &r : m->ozS_ready) r = false;
-  for (bool &r : m->ozL_ready) r = false;
-  for (bool &r : m->ozB_ready) r = false;
-  for (int v = 0; v < oz::kTiles64; v++)
-    m->oz64S_ready[v] = m->oz64ST_ready[v] = m->oz64L_ready[v] = false;
   m->finite = true;
   for (int t = 0; t < M; t++) m->finite &= std::isfinite(snorm[t]);
   if (!h_alpha || !h_L_inv) return FGB_OK;

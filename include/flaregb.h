@@ -187,7 +187,9 @@ int fgb_model_destroy(fgb_model_t m);
 /* h_counts[n_species]: sparse environments per species; h_desc[M * n_d]
  * species-grouped rows (species 0 first); h_alpha[M]; h_L_inv[M * M]
  * row-major (the kernel's block of L_inv).  h_alpha/h_L_inv may be NULL to
- * load only the sparse set (model is then stale for prediction). */
+ * load only the sparse set (model is then stale for prediction).  R_inv of
+ * earlier weights is dropped: fgb_predict_sor and fgb_predict_dtc return
+ * FGB_ESTALE until fgb_model_set_R_inv follows. */
 int fgb_model_set(fgb_model_t m, const int *h_counts, const double *h_desc,
                   const double *h_alpha, const double *h_L_inv);
 
