@@ -318,8 +318,16 @@ __device__ __forceinline__ int row_cols(int K, long long row, int lower) {
   return lower ? (int)min((long long)K, (row / kTriBlock + 1) * kTriBlock) : K;
 }
 
-// The scale of a row of K values (each times `inv`): 2^e with e from its
-// largest magnitude, 2^0 for an empty row; by the lanes of one warp.
+// The scale of a row from its largest magnitude (as bits, times `inv`): 2^e
+// above it, 2^0 for an empty row.  An infinity or NaN in the row: +inf, which
+// makes every product of the row NaN at kS64 slices.
+__device__ __forceinline__ double max_scale(unsigned long long mb, double inv) {
+  if (mb >= 0x7FF0000000000000ULL) return __longlong_as_double(0x7FF0000000000000LL);
+  const double mx = __longlong_as_double((long long)mb) * inv;
+  return ldexp(1.0, mx > 0.0 ? ilogb(mx) + 1 : 0);
+}
+
+// The scale of a row of K values (each times `inv`), by the lanes of one warp.
 __device__ __forceinline__ double row_scale(int K, const double *sr, double inv) {
   unsigned long long mb = 0;
   for (int k = threadIdx.x & 31; k < K; k += 32)
@@ -328,12 +336,7 @@ __device__ __forceinline__ double row_scale(int K, const double *sr, double inv)
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1)
     mb = max(mb, (unsigned long long)__shfl_xor_sync(0xffffffffu, (long long)mb, off));
-  const double mx = __longlong_as_double((long long)mb) * inv;
-  const int e = mx > 0.0 ? ilogb(mx) + 1 : 0;
-  // an infinity or NaN in the row: scale +inf, which makes every product of
-  // the row NaN at kS64 slices
-  const bool bad = mb >= 0x7FF0000000000000ULL;
-  return bad ? __longlong_as_double(0x7FF0000000000000LL) : ldexp(1.0, e);
+  return max_scale(mb, inv);
 }
 
 // Row scales (after the optional division by the row norm), one warp per
@@ -430,8 +433,8 @@ k_oz_slice(const __grid_constant__ SliceOp oa, const __grid_constant__ SliceOp o
     __syncthreads();
     sc = s_scale[r];
   } else if (o.mode == kScaleMax) {
-    const double mx = valid ? o.rowmax[row] * inv : 0.0;
-    sc = ldexp(1.0, mx > 0.0 ? ilogb(mx) + 1 : 0);
+    sc = max_scale(valid ? (unsigned long long)__double_as_longlong(o.rowmax[row])
+                         : 0, inv);
   } else {
     sc = !PAIR || m < o.RP ? o.scale[m] : 1.0;
   }
