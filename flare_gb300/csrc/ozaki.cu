@@ -1513,14 +1513,15 @@ struct EpiCosine {
                           double acc) const {
     if (!row_ok) return acc;
     const double nd = a_norm[perm[m]];
-    const double inv = nd >= kEmptyThresh ? 1.0 / nd : 0.0;
+    const bool dok = nd >= kEmptyThresh;   // also an infinite norm: 1/|d| = 0
+    const double inv = dok ? 1.0 / nd : 0.0;
     double *c = C + (long long)m * N + n0;
 #pragma unroll
     for (int j = 0; j < 16; j++)
       if (n0 + j < N) {
         const double t = v[j] * inv;
         const double2 si = s_inv[n0 + j];
-        c[j] = inv != 0.0 && s_norm[n0 + j] >= kEmptyThresh
+        c[j] = dok && s_norm[n0 + j] >= kEmptyThresh
                    ? fma(t, si.y, t * si.x) : 0.0;
       }
     return acc;

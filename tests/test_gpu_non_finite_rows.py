@@ -50,3 +50,16 @@ def test_predictions(M, power):
     for at in (0, 4):
         assert np.array_equal(b["local_var"][at:at + 2], a["local_var"])
         assert np.array_equal(b["forces"][at:at + 2], a["forces"])
+
+
+@pytest.mark.parametrize("power", [1, 2, 3])
+def test_stored_gradients(power):
+    import flare_gb300 as fg
+    _, calc, cd = model(40, power)
+    k = fg.NormalizedDotProduct(1.5, power)
+    K = k.envs_struc(cd, structure(calc, GOOD + BAD))
+    G = k.envs_struc(cd, structure(calc, GOOD))
+    assert np.isfinite(G).all()
+    assert np.isnan(K[:, 0]).all()
+    assert np.array_equal(K[:, 1:7], G[:, 1:7])
+    assert np.isnan(K[:, [7, 10]]).all()   # x forces of the overflowed pair
