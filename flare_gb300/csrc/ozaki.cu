@@ -1366,6 +1366,18 @@ __global__ void k_oz_row_inv(int M, int nd, const double *__restrict__ S,
   for (int off = 16; off > 0; off >>= 1)
     dd_add(hi, lo, __shfl_xor_sync(0xffffffffu, hi, off),
            __shfl_xor_sync(0xffffffffu, lo, off));
+  if (__any_sync(0xffffffffu, !isfinite(hi))) {
+    // the TwoSums turn an infinity into NaN, which would count as an empty
+    // row: the plain sum
+    hi = lo = 0.0;
+    for (int k = 0; k < nd; k++)
+      hi = fma(S[(long long)m * nd + k], S[(long long)m * nd + k], hi);
+    if (lane == 0) {
+      out[m] = make_double2(1.0 / sqrt(hi), 0.0);
+      if (norms) norms[m] = sqrt(hi);
+    }
+    return;
+  }
   if (lane) return;
   double y = 0.0, y_lo = 0.0;
   if (hi > 0.0) {

@@ -63,3 +63,19 @@ def test_stored_gradients(power):
     assert np.isnan(K[:, 0]).all()
     assert np.array_equal(K[:, 1:7], G[:, 1:7])
     assert np.isnan(K[:, [7, 10]]).all()   # x forces of the overflowed pair
+
+
+def test_sparse_rows():
+    """An infinite entry makes its row of the kernel matrix NaN, a norm that
+    overflows makes it zero (finite over infinite); the others stay."""
+    import flare_gb300 as fg
+    _, calc, cd = model(40, 2)
+    k, st = fg.NormalizedDotProduct(1.5, 2), structure(calc, GOOD)
+    K = k.envs_struc(cd, st)
+    cd.descriptors[0][7, 3] = np.inf
+    cd.descriptors[0][9, 3] = 1e200
+    G = k.envs_struc(cd, st)
+    assert np.isnan(G[7, 0]) and np.isnan(G[7, 1]) and np.isnan(G[7, 4])
+    assert (G[9] == 0.0).all()
+    keep = np.delete(np.arange(40), [7, 9])
+    assert np.array_equal(G[keep], K[keep])
