@@ -80,21 +80,14 @@ __device__ __forceinline__ void bar_arrive() {
 __device__ __forceinline__ bool ordinary(double d) {
   return (unsigned)(__double2hiint(d) >> 20) - 60u < 1920u;
 }
-// From the hardware's estimates y (about 20 bits) by one third-order step of
-// the Householder iteration: 1/d, y (1 + e + e^2) with e = 1 - d y;
-// 1/sqrt(d), y (1 + e/2 + 3 e^2/8) with e = 1 - d y^2.
+// 1/d of an ordinary d from the hardware's estimate y (20 bits of mantissa)
+// by one third-order step of Householder's iteration, y (1 + e + e^2) with e =
+// 1 - d y: e^3 leaves 2^-60, so within one ulp of the rounded quotient.
 __device__ __forceinline__ double rcp64(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double e = fma(-d, y, 1.0);
   return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double rsqrt64(double d) {
-  if (!ordinary(d)) return rsqrt(d);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double t = d * y, e = fma(-t, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // v / d where the estimate does not serve; a pivot that is not positive
@@ -162,7 +155,7 @@ __device__ int factor_block32(int jb, double (&v)[kIB / kFW], double *V,
   if (*flag && *flag <= jb) return *flag;
   if (w == 0) {
     const double d = V[t * kIB + t];
-    y[t] = d > 0.0 ? rsqrt64(d) : 1.0;
+    y[t] = d > 0.0 ? rsqrt(d) : 1.0;
   }
   __syncthreads();
   return 0;
@@ -249,6 +242,17 @@ k_potrf_cluster(int kb, double *__restrict__ A, long long lda,
     }
     cluster_barrier();
   }
+}
+
+// fgb_fp64_check: 1/x as a pivot's column is scaled (k = 0), or x / k.
+__global__ void k_fp64_check(int k, long long n, const double *__restrict__ x,
+                             double *__restrict__ y) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double d = x[i];
+  int flag = 0;
+  if (k > 0) y[i] = div_int(d, k);
+  else y[i] = ordinary(d) ? rcp64(d) : div_rare(1.0, d, 0, &flag);
 }
 
 // The rest of the inverse X of a diagonal block's factor, a CTA for each
@@ -797,6 +801,20 @@ int build_At(int M, int nl, const double *Kuf, const double *noise,
 }  // namespace fgb
 
 using namespace fgb;
+
+extern "C" int fgb_fp64_check(int k, long long n, const double *d_x,
+                              double *d_y, void *stream) {
+  if (k < 0 || k >= kNumInv || n < 0 || n > (1LL << 30) ||
+      (n > 0 && (!d_x || !d_y))) {
+    set_error("fgb_fp64_check: invalid arguments (k in [0, %d])", kNumInv - 1);
+    return FGB_EINVAL;
+  }
+  if (n == 0) return FGB_OK;
+  dense::k_fp64_check<<<ceil_div(n, 256), 256, 0, (cudaStream_t)stream>>>(
+      k, n, d_x, d_y);
+  FGB_LAUNCH_CHECK("k_fp64_check");
+  return FGB_OK;
+}
 
 extern "C" int fgb_cholesky(int M, double *d_A, void *stream) {
   if (M < 0 || (M > 0 && !d_A)) {

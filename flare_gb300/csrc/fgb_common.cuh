@@ -129,8 +129,9 @@ __device__ __forceinline__ void dfact_const(int m, double &v) { v = c_dfact[m]; 
 __device__ __forceinline__ void dfact_const(int m, float &v) { v = c_dfact_f[m]; }
 // x / k for a small positive integer k.  FP64: the product with 1/k rounded
 // to nearest and Markstein's correction step (P. W. Markstein, IBM J. Res.
-// Dev. 34, 1990), which rounds the quotient correctly: 3 FP64 instructions
-// where a division takes about ten.
+// Dev. 34, 1990), which rounds the quotient correctly (all k of the table,
+// 2^-900 <= |x| <= 2^1000): 3 FP64 instructions where a division takes about
+// ten.
 __device__ __forceinline__ double div_int(double x, int k) {
   const double inv = c_inv[k], q = x * inv;
   if ((k & (k - 1)) == 0) return q;     // powers of two are exact

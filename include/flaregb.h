@@ -336,6 +336,14 @@ int fgb_model_set_slices(fgb_model_t m, int kernel_slices,
  * abort) with the context still usable, or another status on failure. */
 int fgb_wait_expiry_check(long long polls, int *h_how, void *stream);
 
+/* Self-check of the FP64 quotients that the kernels form themselves, y[i]
+ * from x[i] (n device values, queued on `stream`): k = 0, 1/x as the
+ * Cholesky pivots take it (within one ulp of the rounded quotient); k = 1 ..
+ * 21, x / k as the Legendre recurrence takes it (the rounded quotient for
+ * 2^-900 <= |x| <= 2^1000).  No reference counterpart. */
+int fgb_fp64_check(int k, long long n, const double *d_x, double *d_y,
+                   void *stream);
+
 /* Thin Q (rows x cols, column-major) of the Householder QR of A (rows x
  * cols, column-major, rows >= cols), device buffers; the varmap
  * coefficients (normalized_dot_product.cpp:769-830) are its leading rows. */
