@@ -870,18 +870,35 @@ __global__ void k_forces(int n_atoms, const long long *__restrict__ offsets,
 }
 
 // Per-structure energy and stress: fixed-order tree sums over chunks of
-// kRedChunk atoms, a block per (structure, chunk); the chunks of a larger
-// structure are then added in order (k_struct_final).  The chunking follows
-// the structure's own atoms alone, so its sums do not depend on the batch.
+// kRedChunk atoms, a block per chunk; the chunks of a larger structure are
+// then added in order (k_struct_final).  The chunking follows the structure's
+// own atoms alone, so its sums do not depend on the batch.
 // One block for 97,556 atoms took 355 us, 48 blocks and the final sum 18.
+// Where all structures are one chunk (`many` false) block b takes structure
+// b; else structure s has the blocks from red_block(s) to red_block(s + 1),
+// at least one and enough for its chunks, so that their number is bounded by
+// the atoms and structures, not by their product.
 constexpr int kRedChunk = 2048;
+__host__ __device__ inline int red_block(int s, int atom0) {
+  return s + atom0 / kRedChunk;
+}
 __global__ void __launch_bounds__(256)
-k_struct_reduce(const StrucGeom *__restrict__ geom,
+k_struct_reduce(int n_struc, bool many, const StrucGeom *__restrict__ geom,
                 const double *__restrict__ e_atom,
                 const double *__restrict__ virial, double *__restrict__ part,
                 double *__restrict__ energy, double *__restrict__ stress) {
   __shared__ double red[7][256];
-  const int s = blockIdx.y, ch = blockIdx.x, t = threadIdx.x;
+  const int b = blockIdx.x, t = threadIdx.x;
+  int s = b, ch = 0;
+  if (many) {
+    s = 0;
+    for (int hi = n_struc; hi - s > 1;) {
+      const int mid = (s + hi) >> 1;
+      if (red_block(mid, geom[mid].atom0) <= b) s = mid;
+      else hi = mid;
+    }
+    ch = b - red_block(s, geom[s].atom0);
+  }
   const int a0 = geom[s].atom0, na = geom[s].natoms;
   if (ch > 0 && ch * kRedChunk >= na) return;
   const int a1 = a0 + min(na, (ch + 1) * kRedChunk);
@@ -899,20 +916,21 @@ k_struct_reduce(const StrucGeom *__restrict__ geom,
     __syncthreads();
   }
   if (t >= 7) return;
-  if (na > kRedChunk) part[((long long)s * gridDim.x + ch) * 7 + t] = red[t][0];
+  if (na > kRedChunk) part[7LL * b + t] = red[t][0];
   else if (t == 0) { if (energy) energy[s] = red[0][0]; }
   else if (stress) stress[6 * s + t - 1] = -red[t][0] / geom[s].volume;
 }
 
-__global__ void k_struct_final(const StrucGeom *__restrict__ geom, int maxch,
+__global__ void k_struct_final(const StrucGeom *__restrict__ geom,
                                const double *__restrict__ part,
                                double *__restrict__ energy,
                                double *__restrict__ stress) {
   const int s = blockIdx.x, t = threadIdx.x, na = geom[s].natoms;
   if (t >= 7 || na <= kRedChunk) return;
   const int nch = (na + kRedChunk - 1) / kRedChunk;
+  const double *p = part + 7LL * red_block(s, geom[s].atom0);
   double x = 0.0;
-  for (int c = 0; c < nch; c++) x += part[((long long)s * maxch + c) * 7 + t];
+  for (int c = 0; c < nch; c++) x += p[7LL * c + t];
   if (t == 0) { if (energy) energy[s] = x; }
   else if (stress) stress[6 * s + t - 1] = -x / geom[s].volume;
 }
@@ -1083,28 +1101,21 @@ int launch_forces(const fgb_nlist_s *nl, const void *d_pair_grad, bool fp32,
 int launch_struct_reduce(const fgb_nlist_s *nl, const double *d_e_atom,
                          const double *d_virial, double *d_energy,
                          double *d_stress, DevBuf &part, cudaStream_t st) {
-  int most = 0;
-  for (int s = 0; s < nl->n_struc; s++)
-    most = std::max(most, nl->h_atom_offsets[s + 1] - nl->h_atom_offsets[s]);
-  const int maxch = std::max(1, ceil_div(most, kRedChunk));
+  const int S = nl->n_struc;
+  bool many = false;
+  for (int s = 0; s < S; s++)
+    many |= nl->h_atom_offsets[s + 1] - nl->h_atom_offsets[s] > kRedChunk;
+  const int blocks = many ? red_block(S, nl->n_atoms) : S;
   int rc;
-  if (maxch > 1 &&
-      (rc = part.ensure(sizeof(double) * 7 * (size_t)maxch * nl->n_struc)))
-    return rc;
-  // the grid's second dimension holds up to 65,535 structures
-  for (int s0 = 0; s0 < nl->n_struc; s0 += 65535) {
-    const int ns = std::min(65535, nl->n_struc - s0);
-    const StrucGeom *g = nl->geom.as<StrucGeom>() + s0;
-    double *p = maxch > 1 ? part.as<double>() + 7LL * maxch * s0 : nullptr;
-    double *e = d_energy ? d_energy + s0 : nullptr;
-    double *t = d_stress ? d_stress + 6LL * s0 : nullptr;
-    k_struct_reduce<<<dim3(maxch, ns), 256, 0, st>>>(g, d_e_atom, d_virial, p,
-                                                     e, t);
-    FGB_LAUNCH_CHECK("k_struct_reduce");
-    if (maxch > 1) {
-      k_struct_final<<<ns, 32, 0, st>>>(g, maxch, p, e, t);
-      FGB_LAUNCH_CHECK("k_struct_final");
-    }
+  if (many && (rc = part.ensure(sizeof(double) * 7 * (size_t)blocks))) return rc;
+  if (S == 0) return FGB_OK;
+  const StrucGeom *g = nl->geom.as<StrucGeom>();
+  k_struct_reduce<<<blocks, 256, 0, st>>>(S, many, g, d_e_atom, d_virial,
+                                          part.as<double>(), d_energy, d_stress);
+  FGB_LAUNCH_CHECK("k_struct_reduce");
+  if (many) {
+    k_struct_final<<<S, 32, 0, st>>>(g, part.as<double>(), d_energy, d_stress);
+    FGB_LAUNCH_CHECK("k_struct_final");
   }
   return FGB_OK;
 }
