@@ -465,6 +465,38 @@ __global__ void k_transpose32(long long R, int C, const double *__restrict__ in,
       out[(c0 + k) * R + r0 + threadIdx.x] = t[threadIdx.x][k];
 }
 
+// The products' bounded waits: a kernel matrix of which a tile is missing
+// becomes NaN as a whole, in the order of the stream (the host does not wait).
+__global__ void k_nan_on_flag(long long n, const int *__restrict__ flag,
+                              double *__restrict__ out) {
+  if (*flag == 0) return;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x)
+    out[i] = __longlong_as_double(0x7FF8000000000000LL);
+}
+
+int envs_envs_sliced(const double *d1, const double *norm1, int n1,
+                     const double *d2, const double *norm2, int n2, int nd,
+                     double sig2, double power, double *d_kern,
+                     cudaStream_t st) {
+  oz::Sliced A(st), B(st);
+  DevBuf err(st);
+  const int v = oz::tile64(n1, n2);
+  int rc;
+  if ((rc = err.ensure(sizeof(int)))) return rc;
+  FGB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+  if ((rc = oz::slice({n1, nd, oz::kTM, d1, nd, nullptr, nullptr}, A, st,
+                      oz::kS64)) ||
+      (rc = oz::slice({n2, nd, oz::kTN64v[v], d2, nd, nullptr, nullptr}, B, st,
+                      oz::kS64)) ||
+      (rc = oz::gemm_envs(A, B, norm1, norm2, sig2, power, d_kern,
+                          err.as<int>(), st)))
+    return rc;
+  k_nan_on_flag<<<32, 256, 0, st>>>((long long)n1 * n2, err.as<int>(), d_kern);
+  FGB_LAUNCH_CHECK("k_nan_on_flag");
+  return FGB_OK;
+}
+
 }  // namespace
 
 int launch_b2_dervs(const B2Params &p, const fgb_nlist_s *nl,
@@ -557,32 +589,15 @@ extern "C" int fgb_envs_envs(const double *d_desc1, const double *d_norm1,
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
     cudaGetLastError();
-    cs = cudaStreamCaptureStatusActive;   // unknown: do not synchronise
+    cs = cudaStreamCaptureStatusActive;   // unknown: allocate nothing
   }
   if (cs == cudaStreamCaptureStatusNone) {
-    oz::Sliced A(st), B(st);
-    DevBuf err(st);
-    const int v = oz::tile64(n1, n2);
-    int rc, h = 0;
-    if ((rc = err.ensure(sizeof(int)))) return rc;
-    FGB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    if ((rc = oz::slice({n1, n_desc, oz::kTM, d_desc1, n_desc, nullptr,
-                         nullptr}, A, st, oz::kS64)) ||
-        (rc = oz::slice({n2, n_desc, oz::kTN64v[v], d_desc2, n_desc, nullptr,
-                         nullptr}, B, st, oz::kS64)) ||
-        (rc = oz::gemm_envs(A, B, d_norm1, d_norm2, sig2, power, d_kern,
-                            err.as<int>(), st)))
-      return rc;
-    FGB_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost,
-                             st));
-    FGB_CUDA(cudaStreamSynchronize(st));
-    if (h) {
-      set_error("fgb_envs_envs: a bounded device wait ran out");
-      return FGB_ETIMEOUT;
-    }
-    return FGB_OK;
+    const int rc = envs_envs_sliced(d_desc1, d_norm1, n1, d_desc2, d_norm2, n2,
+                                    n_desc, sig2, power, d_kern, st);
+    if (rc != FGB_ENOMEM) return rc;
   }
-  // a call being captured cannot read the products' time-out flag back
+  // a call being captured, whose graph then holds no allocation, or without
+  // room for the slices
   dim3 g(ceil_div(n2, BN), ceil_div(n1, BM));
   k_envs_envs<<<g, GT, 0, st>>>(n1, n2, n_desc, d_desc1, d_norm1, d_desc2,
                                 d_norm2, sig2, power, d_kern);

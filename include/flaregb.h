@@ -435,7 +435,12 @@ int fgb_serve_stop(fgb_server_t s);
 /* NormalizedDotProduct::envs_envs (normalized_dot_product.cpp:28-89) for
  * one species block in FP64: d_kern[n1 * n2] (row-major) =
  * sig2 * (d1.d2 / (norm1 norm2))^power, zero where either norm < 1e-8.
- * d_desc1[n1 * n_desc], d_norm1[n1], d_desc2[n2 * n_desc], d_norm2[n2]. */
+ * d_desc1[n1 * n_desc], d_norm1[n1], d_desc2[n2 * n_desc], d_norm2[n2].
+ * Queued on `stream` without waiting, with scratch from the stream-ordered
+ * pool; d_kern is NaN throughout if a bounded device wait ran out.  While
+ * `stream` is being captured, and where the scratch cannot be had, the
+ * product runs as one FP64 kernel without scratch instead of exact slices:
+ * the same values to the FP64 rounding of n_desc-term sums, not bit for bit. */
 int fgb_envs_envs(const double *d_desc1, const double *d_norm1, int n1,
                   const double *d_desc2, const double *d_norm2, int n2,
                   int n_desc, double sig2, double power, double *d_kern,
