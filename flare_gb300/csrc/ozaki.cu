@@ -2116,16 +2116,23 @@ bool fp64_stage_sliced(const fgb_model_s *m) {
   return (m->power == 2.0 || m->power == 1.0) && m->finite;
 }
 
-// Species whose FP64 variances take the SIMT order (variance_small): models
-// of few sparse environments, whose kernel matrix and variance product are at
-// most kSmallVar multiply-adds a row.  Where such a model describes near-equal
-// environments, sigma^2 - |z|^2 cancels to 1e-5 of its terms and the standard
-// deviations of two FP64 summation orders differ by up to 2e-9; these are the
-// SIMT kernels' to the bit.  The model alone decides, so that a structure's
-// results don't depend on its batch.  32 FCC atoms, 64 sparse: 24 us where the
-// sliced product took 9 (and one 64 x 64 SIMT tile 150 for each of the two).
-// 64 x 256 atoms, 200 sparse: the call 2.0 -> 3.9 ms, the FP64 unit's time for
-// 0.8 G multiply-adds and more (6.2 ms with SIMT tiles throughout).
+// Species whose FP64 variances take the SIMT products' order of summation
+// (variance_small), to the bit.  The standard deviation of an environment
+// that the sparse set nearly contains is the root of a difference sigma^2 -
+// |z|^2 that cancels to 1e-5 of its terms and beyond, so that two FP64 orders
+// give standard deviations 1e-9 to 1e-6 apart; small models, for whose calls
+// the order costs little, keep the one they had.  That is the reason, not
+// accuracy: against 128-bit sums the variances of 32 FCC atoms (n_d 144, 64 to
+// 500 sparse rows) are off by 3.2e-16 to 4.6e-16 sigma^2 by the slices and
+// 1.0e-15 to 2.6e-15 in the SIMT order.  And the line, on the multiply-adds
+// of the kernel and variance products a row, is one of cost: one structure of
+// 32 atoms, or 64 of 256, take by the slices and in the SIMT order
+//      64 sparse (11,264)     265 and 281 us     1.86 and 2.25 ms
+//     200 sparse (48,800)     276 and 299        2.02 and 3.92
+//     280 sparse (79,520)     280 and 311        2.06 and 4.89
+//     500 sparse (197,000)    299 and 341        2.36 and 8.43
+// The model alone decides, so that a structure's results don't depend on its
+// batch.
 constexpr long long kSmallVar = 65536;
 static bool small_variance(const fgb_model_s *m, int s) {
   const long long M = m->h_counts[s];
