@@ -2110,7 +2110,8 @@ int kernel_stage_oz(fgb_model_s *m, int N, const std::vector<int> &counts,
 }
 
 // Power 1 or 2 and finite weights: k and the adjoint weights then stay below
-// fixed scales, and no infinity or NaN has to come through.  Other powers
+// fixed scales, and an infinity or NaN can only come from a descriptor row,
+// whose scale carries it through.  Other powers
 // (pow of a small or negative c) and non-finite weights keep the SIMT form.
 bool fp64_stage_sliced(const fgb_model_s *m) {
   return (m->power == 2.0 || m->power == 1.0) && m->finite;

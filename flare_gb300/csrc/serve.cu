@@ -33,9 +33,16 @@ struct Request {
   std::vector<double> forces, var;
 };
 
-// Device bytes per atom of the prediction pipeline for this model (the
+// Device bytes per atom of the prediction pipeline for this model: the
 // workspace buffers of predict.cu, neighbour arrays at up to 128 neighbours
-// per atom, and the widest per-species GEMM rows).
+// per atom, and the widest per-species GEMM rows.  The sum covers either
+// precision (mixed: nine slices of rows and kernel values, FP32 rows of the
+// force product; FP64: 36 n_d + 40 M_s of descriptors, their gradients and ten
+// slices of rows, kernel values and adjoint weights, for the 42 n_d + 42 M_s
+// here).  Measured from 16,000 to 32,000 atoms in FP64, and this estimate:
+//   n_d 680, 2 x 1,000 sparse 83.5 of 88.2 kB; 2 x 100 sparse 47.6 of 50.4
+//   n_d 385, 1,000 sparse     70.3 of 76.6;      100 sparse   32.2 of 38.8
+// The model's own operands are not in it.
 long long footprint_per_atom(const fgb_model_s *m) {
   const B2Params &p = m->b2;
   long long mmax = 1;
