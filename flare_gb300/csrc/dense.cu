@@ -494,16 +494,15 @@ int transpose(int rows, int cols, const double *in, long long ldi, double *out,
 constexpr int kMaxFactors = 4;
 struct Work {
   oz::Sliced A, B;
-  DevBuf err, t1, t2, dinv, info;
+  DevBuf flags, t1, t2, dinv;   // flags: time-out, then info[kMaxFactors]
   explicit Work(cudaStream_t st)
-      : A(st), B(st), err(st), t1(st), t2(st), dinv(st), info(st) {}
+      : A(st), B(st), flags(st), t1(st), t2(st), dinv(st) {}
+  int *err() const { return flags.as<int>(); }
+  int *info(int f) const { return flags.as<int>() + 1 + f; }
   int start(cudaStream_t st) {
-    int rc;
-    if ((rc = err.ensure(sizeof(int))) ||
-        (rc = info.ensure(sizeof(int) * kMaxFactors)))
-      return rc;
-    FGB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    FGB_CUDA(cudaMemsetAsync(info.p, 0, sizeof(int) * kMaxFactors, st));
+    const int rc = flags.ensure(sizeof(int) * (1 + kMaxFactors));
+    if (rc) return rc;
+    FGB_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * (1 + kMaxFactors), st));
     return FGB_OK;
   }
 };
@@ -520,25 +519,23 @@ int gemm_nt(int m, int n, int k, const double *A, long long lda,
            {n, k, oz::kTN64v[oz::tile64(m, n)], B, ldb, nullptr, nullptr}, w.B,
            st)))
     return rc;
-  return oz::gemm_axpby(w.A, w.B, C, ldc, a, b, w.err.as<int>(), st, lower);
+  return oz::gemm_axpby(w.A, w.B, C, ldc, a, b, w.err(), st, lower);
 }
 
-// Waits for the stream and reports the first factorisation that met a bad
-// pivot, then a product whose bounded wait ran out.
+// Waits for the stream and reports a product whose bounded wait ran out, then
+// the first factorisation that met a bad pivot (one copy of all flags).
 int finish(Work &w, cudaStream_t st, const char *what) {
-  int h = 0, info[kMaxFactors] = {};
-  FGB_CUDA(cudaMemcpyAsync(&h, w.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  FGB_CUDA(cudaMemcpyAsync(info, w.info.p, sizeof(info), cudaMemcpyDeviceToHost,
-                           st));
+  int h[1 + kMaxFactors] = {};
+  FGB_CUDA(cudaMemcpyAsync(h, w.flags.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   FGB_CUDA(cudaStreamSynchronize(st));
-  if (h) {
+  if (h[0]) {
     set_error("%s: a bounded device wait ran out", what);
     return FGB_ETIMEOUT;
   }
-  for (int f : info)
-    if (f) {
+  for (int f = 1; f <= kMaxFactors; f++)
+    if (h[f]) {
       set_error("Cholesky of Kuu + jitter failed (leading minor %d not "
-                "positive definite)", f);
+                "positive definite)", h[f]);
       return FGB_EINVAL;
     }
   return FGB_OK;
@@ -603,7 +600,7 @@ int factor(int M, double *A, long long lda, int f, Work &w, cudaStream_t st) {
     double *A11 = A + (long long)k0 * lda + k0;
     double *X = w.dinv.as<double>() + (size_t)(k0 / kNB) * kNB * kNB;
     k_potrf_cluster<<<kCl, kClT, kSmem, st>>>(kb, A11, lda, X, kNB, k0,
-                                              w.info.as<int>() + f);
+                                              w.info(f));
     FGB_LAUNCH_CHECK("k_potrf_cluster");
     k_potrf_inverse<<<kb, kInvT, kInvBytes, st>>>(kb, A11, lda, X, kNB);
     FGB_LAUNCH_CHECK("k_potrf_inverse");
