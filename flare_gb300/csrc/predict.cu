@@ -724,6 +724,18 @@ extern "C" int fgb_model_destroy(fgb_model_t m) {
   return FGB_OK;
 }
 
+// On the bits, without a branch: 4 M entries of L_inv one by one with
+// std::isfinite took 2 of the 10 ms of a call.
+static bool all_finite(const double *x, int n) {
+  unsigned bad = 0;
+  for (int i = 0; i < n; i++) {
+    unsigned long long b;
+    std::memcpy(&b, x + i, sizeof(b));
+    bad |= (b << 1) >= 0xFFE0000000000000ULL;
+  }
+  return !bad;
+}
+
 extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
                              const double *h_desc, const double *h_alpha,
                              const double *h_L_inv) {
@@ -809,6 +821,7 @@ extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
   // [c_s, c_s + M_s); R_s = M_s when everything below the diagonal block is
   // exactly zero (the single-kernel case), else M - c_s.
   std::vector<double> panels;
+  bool finite = true;
   m->h_panel_rows.assign(S, 0);
   m->h_panel_off.assign(S, 0);
   for (int s = 0; s < S; s++) {
@@ -820,11 +833,13 @@ extern "C" int fgb_model_set(fgb_model_t m, const int *h_counts,
     const int R = below_zero ? Ms : M - cs;
     m->h_panel_rows[s] = R;
     m->h_panel_off[s] = (long long)panels.size();
-    for (int r = 0; r < R; r++)
-      for (int c = 0; c < Ms; c++)
-        panels.push_back(h_L_inv[(size_t)(cs + r) * M + cs + c]);
+    for (int r = 0; r < R; r++) {
+      const double *row = h_L_inv + (size_t)(cs + r) * M + cs;
+      panels.insert(panels.end(), row, row + Ms);
+      finite &= all_finite(row, Ms);   // while it is in the cache
+    }
   }
-  for (double x : panels) m->finite &= std::isfinite(x);
+  m->finite &= finite;
   if ((rc = m->Lp.ensure(sizeof(double) * (panels.size() + 1)))) return rc;
   if (!panels.empty())
     FGB_CUDA(cudaMemcpy(m->Lp.p, panels.data(), sizeof(double) * panels.size(),
