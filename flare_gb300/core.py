@@ -261,15 +261,17 @@ class ClusterDescriptor:
 
 
 # ---------------------------------------------------------- structure
-def _species_int32(species):
-    """A species list as an int32 array; small non-negative codes go through
-    bytes (5 us per 1,000 against 35 for a list)."""
-    if type(species) in (list, tuple):
+def _species_int32(*species):
+    """Species lists, joined, as an int32 array; small non-negative codes go
+    through bytes (5 us per 1,000 against 35 for a list; 3,000 lists of 4
+    joined as bytes 0.6 ms, as arrays 2.3)."""
+    if all(type(s) in (list, tuple) for s in species):
         try:
-            return np.frombuffer(bytes(species), np.uint8).astype(np.int32)
+            return np.frombuffer(b"".join([bytes(s) for s in species]),
+                                 np.uint8).astype(np.int32)
         except (TypeError, ValueError):
             pass
-    return np.asarray(species, np.int32)
+    return np.concatenate([np.asarray(s, np.int32) for s in species])
 
 
 class _NList:
@@ -980,8 +982,7 @@ def pack_structures(structures):
     cells = np.ascontiguousarray(np.stack([s.cell.reshape(-1)
                                            for s in structures]))
     pos = np.ascontiguousarray(np.concatenate([s.positions for s in structures]))
-    sp = np.ascontiguousarray(np.concatenate(
-        [_species_int32(s.species) for s in structures]))
+    sp = _species_int32(*[s.species for s in structures])
     return offsets, cells, pos, sp
 
 
