@@ -97,7 +97,8 @@ struct Operand {
 struct Sliced {
   int rows = 0, K = 0, TR = 0, RP = 0, KP = 0, S = 0;
   DevBuf q;       // bf16 slices, tiled canonical layout
-  DevBuf scale;   // per-row 2^e (kS64 slices: +inf for a non-finite row)
+  DevBuf scale;   // per-row 2^e by its exponent bits (pow2_scale; a non-finite
+                  // row: +inf, whose products are NaN at kS64 slices)
   Sliced() = default;
   explicit Sliced(cudaStream_t st) : q(st), scale(st) {}   // one call's scratch
   Operand operand() const {

@@ -183,9 +183,14 @@ __device__ __forceinline__ size_t tiled_index(int m, int k, int KP, int TR) {
 // doubles with integer instructions; the results are the same doubles the
 // FP64 expressions give.
 
-// e for a power-of-two scale 2^e.
+// A power-of-two scale 2^e is kept as the double of that value, read by its
+// exponent bits alone: e + 1023 in the upper twelve (with sign: below -1022,
+// the scales of rows of subnormal numbers, the bits are not the value's).
+__device__ __forceinline__ double pow2_scale(int e) {
+  return __hiloint2double((e + 1023) * (1 << 20), 0);
+}
 __device__ __forceinline__ int pow2_exp(double s) {
-  return (int)((__double_as_longlong(s) >> 52) & 0x7FF) - 1023;
+  return (__double2hiint(s) >> 20) - 1023;
 }
 
 // Out of line so that its FP64 instructions stay off the common path.
@@ -318,13 +323,20 @@ __device__ __forceinline__ int row_cols(int K, long long row, int lower) {
   return lower ? (int)min((long long)K, (row / kTriBlock + 1) * kTriBlock) : K;
 }
 
+static __device__ __noinline__ double max_scale_rare(double mx) {
+  return pow2_scale(mx > 0.0 ? ilogb(mx) + 1 : 0);
+}
+
 // The scale of a row from its largest magnitude (as bits, times `inv`): 2^e
 // above it, 2^0 for an empty row.  An infinity or NaN in the row: +inf, which
-// makes every product of the row NaN at kS64 slices.
+// makes every product of the row NaN at kS64 slices.  At most 2^1023, so that
+// a finite row in the last binade is not taken for one (its top digits reach
+// 128, which BF16 and short sums hold exactly).
 __device__ __forceinline__ double max_scale(unsigned long long mb, double inv) {
-  if (mb >= 0x7FF0000000000000ULL) return __longlong_as_double(0x7FF0000000000000LL);
   const double mx = __longlong_as_double((long long)mb) * inv;
-  return ldexp(1.0, mx > 0.0 ? ilogb(mx) + 1 : 0);
+  const int field = (__double2hiint(mx) >> 20) & 0x7FF;
+  if (field == 0) return max_scale_rare(mx);
+  return pow2_scale(field == 2047 ? 1024 : min(field - 1022, 1023));
 }
 
 // The scale of a row of K values (each times `inv`), by the lanes of one warp.
@@ -1335,7 +1347,7 @@ struct EpiKernel {
   }
   __device__ void finish(int m, bool row_ok, int slot, double acc) const {
     if (row_ok) epart[(long long)m * nslots + slot] = acc;
-    if (Ksl && slot == 0) Kscale[m] = ldexp(1.0, eK);
+    if (Ksl && slot == 0) Kscale[m] = pow2_scale(eK);
   }
 };
 
@@ -1445,8 +1457,8 @@ struct EpiKernel64 {
   __device__ void finish(int m, bool row_ok, int slot, double acc) const {
     if (row_ok) epart[(long long)m * nslots + slot] = acc;
     if (slot == 0) {
-      if (Ksl) Kscale[m] = ldexp(1.0, eK);
-      if (Wsl) Wscale[m] = ldexp(1.0, eW);
+      if (Ksl) Kscale[m] = pow2_scale(eK);
+      if (Wsl) Wscale[m] = pow2_scale(eW);
     }
   }
 };
@@ -2266,7 +2278,7 @@ static int kernel_stage_fp64_group(fgb_model_s *m, const std::vector<int> &count
       const double wmax = m->alpha_max[P.s];
       B[i] = m->oz64S[vk][P.s]->operand();
       epi.push_back({K[i].q, W[i].q, K[i].scale, W[i].scale, K[i].KP,
-                     wmax > 0.0 ? std::ilogb(wmax) + 1 : 0,
+                     wmax > 0.0 ? std::min(std::ilogb(wmax) + 1, 1023) : 0,
                      m->ws.erows.as<double>() + P.e0, P.kslots,
                      m->alpha.as<double>() + P.off,
                      m->sinv.as<double2>() + P.off,
@@ -2364,7 +2376,7 @@ int kernel_stage_fp64_oz(fgb_model_s *m, const std::vector<int> &counts,
     const int R = m->h_panel_rows[s], off = m->h_offsets[s];
     const bool sv = want_var && !small_variance(m, s);
     const double wmax = m->alpha_max[s];
-    const int eW = wmax > 0.0 ? std::ilogb(wmax) + 1 : 0;
+    const int eW = wmax > 0.0 ? std::min(std::ilogb(wmax) + 1, 1023) : 0;
     for (int r0 = 0; r0 < Ns; r0 += kRows) {
       const int Mr = std::min(kRows, Ns - r0);
       const int *perm = perm_s + r0;

@@ -56,3 +56,22 @@ def test_entries_with_all_their_bits():
     B = r.integers(-15, 16, size=(7, 40)) * 2.0 ** -24
     A[:, 0], B[:, 0], B[:, 1], A[:, 1] = 1.0, 0.0, 1.0, 0.0
     assert np.array_equal(product(A, B), A @ B.T)
+
+
+@pytest.mark.parametrize("up,down", [(1023, -1018), (1022, -1040), (-1040, 1000)])
+def test_rows_at_the_ends_of_the_range(up, down):
+    """Finite rows up to the largest double, and subnormal ones."""
+    K = 40
+    r = np.random.Generator(np.random.PCG64(up + 2000))
+    A = np.ldexp(r.uniform(-2.0, 2.0, size=(5, K)), up)
+    A[:, 3] = np.ldexp(1.875, up)
+    B = np.ldexp(r.uniform(-2.0, 2.0, size=(7, K)), down)
+    assert np.isfinite(A).all()
+    # scaled exactly to where the sums can neither overflow nor underflow
+    exact = np.array([[float(sum(Fraction(a) * Fraction(b)
+                                 for a, b in zip(x, y))) for y in B]
+                      for x in A])
+    top = np.ldexp(np.abs(np.ldexp(A, -up)).max(1)[:, None] *
+                   np.abs(np.ldexp(B, -down)).max(1)[None, :], up + down)
+    assert np.all(np.abs(product(A, B) - exact) <= 2.0 ** -56 * K * top +
+                  2.0 ** -52 * np.abs(exact))
